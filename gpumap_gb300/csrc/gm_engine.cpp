@@ -119,7 +119,7 @@ Session::Session(const gm_params &p) : p_(p) {
     d_rows_ = (int *)dalloc(Nm * sizeof(int));
     d_rows2_ = (int *)dalloc(Nm * sizeof(int));
     d_batch_ = (int *)dalloc(Nm * sizeof(int));
-    d_cnt_ = (int *)dalloc(16 * sizeof(int));
+    d_cnt_ = (int *)dalloc((16 + kInsertIters) * sizeof(int));
     d_tmp_ = (int *)dalloc(std::max(scan_tmp_ints((int)Nm), compact_tmp_ints((int)Nm)) *
                            sizeof(int) + 64);
 
@@ -705,15 +705,8 @@ uint32_t Session::insert(uint32_t n_ops) {
   } else {
     ensure_cand(B);
     wait_init();
-    launch_random_init(st_, row0, nb, n, window_start, seed, s);
-    for (int it = 0; it < kInsertIters; ++it) {
-      launch_sample_candidates(st_, row0, nb, n, cand_, cand_cnt_, s);
-      timed_begin(1);
-      launch_candidate_dists(st_, row0, nb, cand_, cand_cnt_, cand_dist_, s);
-      timed_end(1);
-      launch_forward_merge(st_, row0, nb, cand_, cand_cnt_, cand_dist_, s);
-      if (row0 > 0) launch_reverse_insert(st_, row0, nb, cand_, cand_cnt_, cand_dist_, s);
-    }
+    launch_nnd_insert(st_, row0, nb, n, window_start, seed, cand_, cand_cnt_, cand_dist_, d_cnt_ + 16,
+                      sms_, [this](bool begin) { begin ? timed_begin(1) : timed_end(1); }, s);
   }
   // existing rows whose list changed, ascending
   compact_flags(st_.dirty, row0, -1, d_rows_, d_cnt_, d_tmp_, s);
