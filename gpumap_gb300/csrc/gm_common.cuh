@@ -241,16 +241,37 @@ GM_HD int key_id(Key k) { return (int)(uint32_t)(k & 0xffffffffu); }
 GM_D float key_dist(Key k) { return __uint_as_float((uint32_t)(k >> 32)); }
 GM_HD bool key_is_placeholder(Key k) { return (uint32_t)(k >> 32) == kFltMaxBits; }
 
-// Offers m candidate keys to node t's 32-wide sorted list under t's lock.
-// Per candidate: if its id is listed with a finite distance, nothing
-// happens; if its id is listed as a placeholder, the placeholder is removed
-// and the candidate inserted; otherwise the candidate is inserted before the
-// first entry it is smaller than, dropping the last entry.  (The reference,
-// update_kernel.cuh:310-375, skips any listed id; whether a placeholder was
-// evicted before its id is offered then depends on lock order.  Replacing
-// the placeholder makes the final list independent of the order of offers.)
-// Returns the smallest insert position (kListW if nothing changed, -1 if the
-// lock wait ran out).
+// Offers key ck to a 32-wide sorted list held by a warp (lane l: entry l).
+// If its id is listed with a finite distance, nothing happens; if its id is
+// listed as a placeholder, the placeholder is removed and the key inserted;
+// otherwise the key is inserted before the first entry it is smaller than,
+// dropping the last entry.  (The reference, update_kernel.cuh:310-375, skips
+// any listed id; whether a placeholder was evicted before its id is offered
+// then depends on lock order.  Replacing the placeholder makes the final list
+// independent of the order of offers.)  Returns the insert position, kListW
+// if nothing changed.
+GM_D int warp_insert(Key &mine, Key ck) {
+  const int lane = threadIdx.x & 31;
+  const unsigned match = __ballot_sync(0xffffffffu, key_id(mine) == key_id(ck));
+  if (match) {
+    const int at = __ffs(match) - 1;
+    const Key there = __shfl_sync(0xffffffffu, mine, at);
+    if (!key_is_placeholder(there)) return kListW;
+    const Key nxt = __shfl_down_sync(0xffffffffu, mine, 1);
+    if (lane >= at) mine = (lane == kListW - 1) ? kEmptyKey : nxt;
+  }
+  const unsigned msk = __ballot_sync(0xffffffffu, ck < mine);
+  if (msk == 0u) return kListW;
+  const int pos = __ffs(msk) - 1;
+  const Key prev = __shfl_up_sync(0xffffffffu, mine, 1);
+  if (lane > pos) mine = prev;
+  else if (lane == pos) mine = ck;
+  return pos;
+}
+
+// Offers m candidate keys to node t's list under t's lock.  Returns the
+// smallest insert position (kListW if nothing changed, -1 if the lock wait
+// ran out).
 GM_D int warp_locked_merge(int t, const Key *cands, int m, Key *g_key, int *locks,
                            unsigned *err) {
   const int lane = threadIdx.x & 31;
@@ -258,25 +279,7 @@ GM_D int warp_locked_merge(int t, const Key *cands, int m, Key *g_key, int *lock
   Key *row = g_key + (size_t)t * kListW;
   Key mine = __ldcg(&row[lane]);
   int minpos = kListW;
-  for (int q = 0; q < m; ++q) {
-    const Key ck = cands[q];
-    const int cid = key_id(ck);
-    const unsigned match = __ballot_sync(0xffffffffu, key_id(mine) == cid);
-    if (match) {
-      const int at = __ffs(match) - 1;
-      const Key there = __shfl_sync(0xffffffffu, mine, at);
-      if (!key_is_placeholder(there)) continue;
-      const Key nxt = __shfl_down_sync(0xffffffffu, mine, 1);
-      if (lane >= at) mine = (lane == kListW - 1) ? kEmptyKey : nxt;
-    }
-    const unsigned msk = __ballot_sync(0xffffffffu, ck < mine);
-    if (msk == 0u) continue;
-    const int pos = __ffs(msk) - 1;
-    const Key prev = __shfl_up_sync(0xffffffffu, mine, 1);
-    if (lane > pos) mine = prev;
-    else if (lane == pos) mine = ck;
-    minpos = min(minpos, pos);
-  }
+  for (int q = 0; q < m; ++q) minpos = min(minpos, warp_insert(mine, cands[q]));
   if (minpos < kListW) __stcg(&row[lane], mine);
   warp_unlock(&locks[t]);
   return minpos;

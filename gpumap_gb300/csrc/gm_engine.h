@@ -146,7 +146,7 @@ class Session {
   size_t fixed_bytes_ = 0;
 
   // insertion candidates (grow on demand)
-  int *cand_ = nullptr, *cand_cnt_ = nullptr;
+  int *cand_ = nullptr, *cand_cnt_ = nullptr, *cand_next_ = nullptr;
   float *cand_dist_ = nullptr;
   size_t cand_rows_ = 0;
 

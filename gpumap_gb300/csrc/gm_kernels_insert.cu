@@ -220,66 +220,101 @@ __global__ void __launch_bounds__(kSampWarps * 32)
   if (lane == 0) cand_cnt[rl] = min(base, kMaxCand);
 }
 
+// Offers of an iteration by target: row j has 32 chains, heads[j * 32 + l]
+// the newest offer of the batch rows with id mod 32 = l (-1: none), next[]
+// the one before it.  Offer e is candidate slot e of the launch: from its
+// row e / 256, at distance cand_dist[e].
+struct OfferChains {
+  int *heads;  // -1 before the first iteration, left so by k_merge_offers
+  int *next;
+};
+
 // Candidate distances and, for existing candidates (id < row0), the reverse
 // offers (reference: compute_candidate_distances_kernel,
 // insertion_kernel.cuh:337-405, and :548-640, which scatters up to 32
-// arrivals per row and merges them; merging every offer gives the same list
-// as merging the best 32, one of the reference's outcomes).  A warp takes
-// (row, chunk of 32 candidates) tasks in a grid stride: 32 canonical chains
-// (gm_rowdot.cuh), then each offer that can change its target's list (below
-// its last entry, not listed) is merged under the target's lock.
-// The distances are bound by L2 (a row's candidates are 100-200 feature rows),
-// the offers by the locks.  An insertion of 500 rows x 784 features at k = 15
-// took 1.35 ms over its ten iterations with a CTA per row and two barriers per
-// chunk, then a warp per row for the offers; this form takes 0.36 ms, nearly
-// all of it merges under locks.
+// arrivals per row; here every one is kept, one of the reference's outcomes).
+// A warp takes (row, chunk of 32 candidates) tasks in a grid stride: 32
+// canonical chains (gm_rowdot.cuh), then each offer that can change its
+// target's list (below its last entry; not listed already, which an earlier
+// iteration may have done: scan_listed) is put on one of the target's chains.
+// Bound by L2: a row's candidates are 100-200 feature rows.  An insertion of
+// 500 rows x 784 features at k = 15 took 1.35 ms over its ten iterations with
+// a CTA per row, two barriers per chunk and every offer merged under its
+// target's lock; 0.36 ms with one iteration of this form but the locks (the
+// recent window's rows get most of the offers); 0.05 ms with the chains, their merge
+// included.
 constexpr int kCandWarps = 2;
 __global__ void __launch_bounds__(kCandWarps * 32)
-    k_candidate_offers(const float *X, const float *norms, int ld, int row0, int nrows, int chunks,
-                       const int *cand, const int *cand_cnt, float *cand_dist, Key *g_key,
-                       int *locks, int *dirty, unsigned *err, int *changed_out, const int *changed,
+    k_candidate_offers(const float *X, const float *norms, int ld, int row0, int first, int nrows, int chunks,
+                       const int *cand, const int *cand_cnt, float *cand_dist, const Key *g_key,
+                       OfferChains chains, int scan_listed, const int *changed,
                        unsigned long long *stat) {
   if (changed && *changed == 0) return;
   __shared__ __align__(16) RowDotTiles tiles[kCandWarps];
-  __shared__ Key s_key[kCandWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tasks = nrows * chunks;
   for (int task = blockIdx.x * kCandWarps + warp; task < tasks; task += gridDim.x * kCandWarps) {
     const int rl = task / chunks, s = (task - rl * chunks) * 32 + lane;
     const int cnt = cand_cnt[rl];
     if (s - lane >= cnt) continue;
-    const int gid = row0 + rl;
+    const int gid = first + rl;
     const int j = s < cnt ? cand[(size_t)rl * kMaxCand + s] : gid;
     if (stat && lane == 0) atomicAdd(&stat[4], (unsigned long long)(min(32, cnt - s) + (s == 0)));
     const float dot = warp_row_dot(X, ld, X + (size_t)gid * ld, j, tiles[warp]);
     const float dv = canon_dist(norms[gid], norms[j], dot);
-    if (s < cnt && cand_dist) cand_dist[(size_t)rl * kMaxCand + s] = dv;
+    const size_t e = (size_t)rl * kMaxCand + s;
+    if (s < cnt) cand_dist[e] = dv;
     bool want = false;
-    Key ck = 0;
     if (s < cnt && j < row0 && dv >= 0.0f) {
-      ck = make_key(dv, gid);
+      const Key ck = make_key(dv, gid);
       const Key *row = g_key + (size_t)j * kListW;
       if (ck < __ldcg(&row[kListW - 1])) {
         want = true;
-        for (int w = 0; w < kListW; ++w)
-          if (__ldcg(&row[w]) == ck) want = false;
+        if (scan_listed)
+          for (int w = 0; w < kListW; ++w)
+            if (__ldcg(&row[w]) == ck) want = false;
       }
     }
-    unsigned bal = __ballot_sync(0xffffffffu, want);
-    while (bal) {
-      const int src = __ffs(bal) - 1;
-      bal &= bal - 1u;
-      const int tj = __shfl_sync(0xffffffffu, j, src);
-      const Key tk = __shfl_sync(0xffffffffu, ck, src);
-      if (lane == 0) s_key[warp] = tk;
-      __syncwarp();
-      const int pos = warp_locked_merge(tj, &s_key[warp], 1, g_key, locks, err);
-      if (lane == 0 && pos >= 0 && pos < kListW) {
-        dirty[tj] = 1;
-        if (changed_out) *changed_out = 1;
-      }
-      __syncwarp();
+    if (want) chains.next[e] = atomicExch(&chains.heads[(size_t)j * 32 + (gid & 31)], (int)e);
+  }
+}
+
+// Merges the offers on each existing row's chains into its list, a warp per
+// row, a chain per lane, without a lock: no other warp of this launch touches
+// the row.  The order of offers does not matter (warp_insert).
+constexpr int kOfferWarps = 8;
+__global__ void __launch_bounds__(kOfferWarps * 32)
+    k_merge_offers(Key *g_key, int row0, int first, OfferChains chains, const float *cand_dist, int *dirty,
+                   int *changed_out, const int *changed) {
+  if (changed && *changed == 0) return;
+  const int lane = threadIdx.x & 31;
+  const int j = blockIdx.x * kOfferWarps + (threadIdx.x >> 5);
+  if (j >= row0) return;
+  const unsigned full = 0xffffffffu;
+  int e = chains.heads[(size_t)j * 32 + lane];
+  if (!__any_sync(full, e >= 0)) return;
+  chains.heads[(size_t)j * 32 + lane] = -1;
+  Key *row = g_key + (size_t)j * kListW;
+  Key mine = row[lane];
+  bool moved = false;
+  while (__any_sync(full, e >= 0)) {
+    Key ck = ~(Key)0;
+    if (e >= 0) {
+      ck = make_key(cand_dist[e], first + e / kMaxCand);
+      e = chains.next[e];
     }
+    unsigned todo = __ballot_sync(full, ck < __shfl_sync(full, mine, kListW - 1));
+    while (todo) {
+      const int src = __ffs(todo) - 1;
+      todo &= todo - 1u;
+      moved |= warp_insert(mine, __shfl_sync(full, ck, src)) < kListW;
+    }
+  }
+  if (!moved) return;
+  row[lane] = mine;
+  if (lane == 0) {
+    dirty[j] = 1;
+    if (changed_out) *changed_out = 1;
   }
 }
 
@@ -431,9 +466,9 @@ void launch_row_norms(const DevState &st, int row0, int nrows, cudaStream_t s) {
   note_launch();
 }
 
-void launch_nnd_insert(const DevState &st, int row0, int nrows, int n, int window_start,
-                       uint64_t seed, int *cand, int *cand_cnt, float *cand_dist, int *changed,
-                       int sms, const std::function<void(bool)> &timed, cudaStream_t s) {
+void launch_nnd_insert(const DevState &st, const UpdScratch &u, int row0, int nrows, int n, int window_start,
+                       uint64_t seed, int *cand, int *cand_cnt, float *cand_dist, int *next,
+                       int *changed, int sms, const std::function<void(bool)> &timed, cudaStream_t s) {
   if (nrows <= 0) return;
   k_random_init<<<cdiv(nrows, kInitWarps), kInitWarps * 32, 0, s>>>(st.g_key, row0, nrows, n,
                                                                     window_start, seed);
@@ -466,7 +501,10 @@ void launch_nnd_insert(const DevState &st, int row0, int nrows, int n, int windo
     }
   }
   const int chunks = cdiv(std::min(P, kMaxCand), 32);
-  const int grid = (int)std::min<long>(cdiv((long)nrows * chunks, kCandWarps), 6L * std::max(sms, 1) * 4);
+  // the chains' heads lie over one of the update's sample lists (n_cap x 32,
+  // not in use during an insertion)
+  const OfferChains chains{u.fwd_new, next};
+  if (row0 > 0) cudaMemsetAsync(chains.heads, 0xff, (size_t)row0 * 32 * sizeof(int), s);
   if (merges) cudaMemsetAsync(changed, 0, kInsertIters * sizeof(int), s);
   for (int it = 0; it < iters; ++it) {
     // an iteration that follows one without any change repeats it: its
@@ -476,12 +514,22 @@ void launch_nnd_insert(const DevState &st, int row0, int nrows, int n, int windo
     k_sample_candidates<<<cdiv(nrows, kSampWarps), kSampWarps * 32, smem, s>>>(
         st.g_key, row0, nrows, n, k, slots, merges ? 0 : 1, cand, cand_cnt, go);
     note_launch();
-    timed(true);
-    k_candidate_offers<<<grid, kCandWarps * 32, 0, s>>>(
-        st.X, st.norms, st.ld, row0, nrows, chunks, cand, cand_cnt, merges ? cand_dist : nullptr,
-        st.g_key, st.locks, st.dirty, st.err, mark, go, st.stat);
-    note_launch();
-    timed(false);
+    for (int r = 0; r < nrows; r += kOfferRows) {
+      const int m = std::min(kOfferRows, nrows - r);
+      const size_t at = (size_t)r * kMaxCand;
+      const int grid = (int)std::min<long>(cdiv((long)m * chunks, kCandWarps), 24L * std::max(sms, 1));
+      timed(true);
+      k_candidate_offers<<<grid, kCandWarps * 32, 0, s>>>(
+          st.X, st.norms, st.ld, row0, row0 + r, m, chunks, cand + at, cand_cnt + r, cand_dist + at,
+          st.g_key, chains, merges ? 1 : 0, go, st.stat);
+      note_launch();
+      timed(false);
+      if (row0 > 0) {
+        k_merge_offers<<<cdiv(row0, kOfferWarps), kOfferWarps * 32, 0, s>>>(
+            st.g_key, row0, row0 + r, chains, cand_dist + at, st.dirty, mark, go);
+        note_launch();
+      }
+    }
     if (merges) {
       k_forward_merge<<<cdiv(nrows, kFwdWarps), kFwdWarps * 32, 0, s>>>(
           st.g_key, row0, nrows, cand, cand_cnt, cand_dist, mark, go);
