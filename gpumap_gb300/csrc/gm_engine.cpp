@@ -32,9 +32,12 @@ void ck(cudaError_t e, const char *what) {
 
 size_t round_up(size_t v, size_t m) { return (v + m - 1) / m * m; }
 
-// Insertion scratch for r batch rows: candidates, distances, counts, chains.
-size_t cand_bytes(size_t r) {
-  return r * (size_t)kMaxCand * (sizeof(int) + sizeof(float)) + r * sizeof(int) +
+// From 256 two-hop positions on, insertion iterates and keeps distances.
+bool reuses_dists(int k) { return k * k >= kMaxCand; }
+// Insertion scratch for r batch rows (CandScratch).
+size_t cand_bytes(size_t r, int k) {
+  return r * ((size_t)kMaxCand * (sizeof(int) + sizeof(float)) + sizeof(int)) +
+         (reuses_dists(k) ? r * (kMaxCand + sizeof(int)) : 0) +
          std::min<size_t>(r, kOfferRows) * kMaxCand * sizeof(int);
 }
 
@@ -297,10 +300,7 @@ Session::~Session() {
     cudaEventDestroy(pr.b);
   }
   for (void *q : allocs_) cudaFree(q);
-  if (cand_) cudaFree(cand_);
-  if (cand_cnt_) cudaFree(cand_cnt_);
-  if (cand_dist_) cudaFree(cand_dist_);
-  if (cand_next_) cudaFree(cand_next_);
+  free_cand();
   free_embed(es_);
   free_embed(es_alt_);
   if (h_pin_) cudaFreeHost(h_pin_);
@@ -360,23 +360,28 @@ void Session::check_device_error(const char *phase) {
   }
 }
 
+void Session::free_cand() {
+  for (void *q : {(void *)cs_.cand, (void *)cs_.cnt, (void *)cs_.dist, (void *)cs_.todo,
+                  (void *)cs_.todo_cnt, (void *)cs_.next})
+    if (q) cudaFree(q);
+  cs_ = CandScratch{};
+  cand_rows_ = 0;
+}
+
 void Session::ensure_cand(size_t rows) {
   if (rows <= cand_rows_) return;
   sync();
-  if (cand_) cudaFree(cand_);
-  if (cand_cnt_) cudaFree(cand_cnt_);
-  if (cand_dist_) cudaFree(cand_dist_);
-  if (cand_next_) cudaFree(cand_next_);
-  cand_ = nullptr;
-  cand_cnt_ = nullptr;
-  cand_dist_ = nullptr;
-  cand_next_ = nullptr;
-  cand_rows_ = 0;
-  const size_t r = std::max<size_t>(rows, 1024);
-  ck(cudaMalloc(&cand_, r * kMaxCand * sizeof(int)), "cudaMalloc cand");
-  ck(cudaMalloc(&cand_cnt_, r * sizeof(int)), "cudaMalloc cand");
-  ck(cudaMalloc(&cand_dist_, r * kMaxCand * sizeof(float)), "cudaMalloc cand");
-  ck(cudaMalloc(&cand_next_, std::min<size_t>(r, kOfferRows) * kMaxCand * sizeof(int)), "cudaMalloc cand");
+  free_cand();
+  const size_t r = std::max<size_t>(rows, 1024), slots = r * kMaxCand;
+  auto get = [&](auto *&p, size_t n) { ck(cudaMalloc(&p, n * sizeof(*p)), "cudaMalloc cand"); };
+  get(cs_.cand, slots);
+  get(cs_.cnt, r);
+  get(cs_.dist, slots);
+  if (reuses_dists(st_.k)) {
+    get(cs_.todo, slots);
+    get(cs_.todo_cnt, r);
+  }
+  get(cs_.next, std::min<size_t>(r, kOfferRows) * kMaxCand);
   cand_rows_ = r;
 }
 
@@ -402,7 +407,7 @@ void Session::set_keep_tile(bool on) {
 
 size_t Session::device_bytes() const {
   size_t b = fixed_bytes_;
-  b += cand_bytes(cand_rows_);
+  b += cand_bytes(cand_rows_, st_.k);
   for (const EmbedScratch *e : {&es_, &es_alt_})
     if (e->coo_row) b += e->cap_coo * 9 * 4 + (compact_tmp_ints((int)e->cap_coo) + 64) * sizeof(int);
   return b;
@@ -412,7 +417,7 @@ size_t Session::growth_bytes(uint32_t n_ins, uint32_t n_emb) const {
   size_t g = 0;
   if (p_.precision == 0 && n_ins > cand_rows_) {
     const size_t r = std::max<size_t>(n_ins, 1024);
-    g += cand_bytes(r);
+    g += cand_bytes(r, st_.k);
   }
   // an embedding batch takes the queued new rows plus the cursor's rows
   const size_t nb = std::max<size_t>(n_emb, n_inserted_ + n_ins - emb_new_head_);
@@ -715,8 +720,8 @@ uint32_t Session::insert(uint32_t n_ops) {
   } else {
     ensure_cand(B);
     wait_init();
-    launch_nnd_insert(st_, us_, row0, nb, n, window_start, seed, cand_, cand_cnt_, cand_dist_, cand_next_,
-                      d_cnt_ + 16, sms_, [this](bool begin) { begin ? timed_begin(1) : timed_end(1); }, s);
+    launch_nnd_insert(st_, us_, row0, nb, n, window_start, seed, cs_, d_cnt_ + 16, sms_,
+                      [this](bool begin) { begin ? timed_begin(1) : timed_end(1); }, s);
   }
   // existing rows whose list changed, ascending
   compact_flags(st_.dirty, row0, -1, d_rows_, d_cnt_, d_tmp_, s);

@@ -98,6 +98,7 @@ class Session {
   void check_launch_error(const char *phase);
   void check_device_error(const char *phase);
   void ensure_cand(size_t rows);
+  void free_cand();
   void ensure_embed(EmbedScratch &e, size_t nb);
   void free_embed(EmbedScratch &e);
   void sync_embed_streams();
@@ -146,8 +147,7 @@ class Session {
   size_t fixed_bytes_ = 0;
 
   // insertion candidates (grow on demand)
-  int *cand_ = nullptr, *cand_cnt_ = nullptr, *cand_next_ = nullptr;
-  float *cand_dist_ = nullptr;
+  CandScratch cs_;
   size_t cand_rows_ = 0;
 
   // device row lists / counters

@@ -77,15 +77,24 @@ void compact_list(const int *list, const int *n_dev, int n_max, const int *pred,
 void launch_row_norms(const DevState &st, int row0, int nrows, cudaStream_t s);
 // Batch rows whose offers are chained and merged together.
 constexpr int kOfferRows = 1 << 16;
+// Insertion scratch per batch row: 256 candidates, their distances and
+// counts; the slots without a known distance (for k^2 >= 256 only); the
+// offers' chains (kOfferRows rows at most).
+struct CandScratch {
+  int *cand = nullptr, *cnt = nullptr;
+  float *dist = nullptr;
+  uint8_t *todo = nullptr;
+  int *todo_cnt = nullptr;
+  int *next = nullptr;
+};
 // NN-Descent insertion of rows [row0, row0 + nrows): random initial lists,
 // then the iterations of two-hop candidates, distances, offers and forward
-// merge.  One of u's sample lists holds the offers' chain heads.  cand,
-// cand_dist: nrows x 256; next: as many for up to kOfferRows rows; changed:
-// kInsertIters ints; timed
-// brackets each distance launch (true before, false after).
-void launch_nnd_insert(const DevState &st, const UpdScratch &u, int row0, int nrows, int n, int window_start,
-                       uint64_t seed, int *cand, int *cand_cnt, float *cand_dist, int *next,
-                       int *changed, int sms, const std::function<void(bool)> &timed, cudaStream_t s);
+// merge.  One of u's sample lists holds the offers' chain heads; changed:
+// kInsertIters ints; timed brackets each distance launch (true before, false
+// after).
+void launch_nnd_insert(const DevState &st, const UpdScratch &u, int row0, int nrows, int n,
+                       int window_start, uint64_t seed, const CandScratch &c, int *changed, int sms,
+                       const std::function<void(bool)> &timed, cudaStream_t s);
 // Copies the first k working entries of rows [row0,row0+nrows) and of the
 // listed rows into the authoritative list and publishes them.
 void launch_adopt_and_publish(const DevState &st, int row0, int nrows,

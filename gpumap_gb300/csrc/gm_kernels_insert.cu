@@ -2,7 +2,6 @@
 // Restates the reference's insertion_kernel.cuh (run_insertion, :926-1095)
 // with a deterministic reverse step and a canonical FP32 distance.
 #include <algorithm>
-#include <atomic>
 #include <climits>
 
 #include "gm_common.cuh"
@@ -138,43 +137,77 @@ __global__ void __launch_bounds__(kInitWarps * 32)
 // first 256 kept positions in order are the candidates
 // (reference: sample_forward_candidates_kernel, insertion_kernel.cuh:250-321).
 // First occurrences come from a shared-memory hash table of the ids (linear
-// probing, at most two thirds full) that keeps each id's smallest position;
-// the row's own neighbours are entered at position -1.  Comparing every
-// position with every earlier one was O(k^4): 36 us for 500 rows at k = 15
-// and 606 us for 10,000 at k = 30, this form 10 us and 142 us.  The
-// neighbours' lists are read row by row, k adjacent keys at a time.
+// probing) that keeps each id's smallest position; the row's own neighbours are
+// entered at position -1.  Positions are taken kHopBlock slots of every
+// neighbour at a time, in order, and the rest is left unread once 256 are
+// kept, so the table holds at most k + 256 + kHopBlock k ids, whatever k is.
+// Candidates of the previous iteration keep the distance they have (and were
+// offered then); only the others are listed in todo, by slot.
+// Comparing every position with every earlier one was O(k^4): 36 us for 500
+// rows at k = 15 and 606 us for 10,000 at k = 30; this form 10 us and 70 us (142 us
+// with every position read).
 // exist_only: only candidates below row0 are written (see launch_nnd_insert).
 constexpr int kSampWarps = 4;
-GM_HD int hop_slots(int k) {  // hash slots: a power of two, at least 1.5 (k^2 + k)
+constexpr int kHopBlock = 8;
+GM_HD int hop_slots(int k) {  // hash slots: a power of two, at most two thirds full
   int h = 32;
-  while (h < k * k + k + (k * k + k) / 2) h *= 2;
+  while (h < 1024 && h < k * k + k + (k * k + k) / 2) h *= 2;
   return h;
 }
-GM_HD size_t hop_ints(int k) { return (size_t)2 * hop_slots(k) + kListW + (k * k + 3) / 4 * 4; }
+static_assert(kListW + kMaxCand + kHopBlock * kListW <= 2 * 1024 / 3, "hash table too full");
+static_assert(kSampWarps * (2 * 1024 + kListW + kHopBlock * kListW + kMaxCand / 32) * 4 <= 48 * 1024, "shared memory");
+// table ids, table positions, neighbours, the block's slots, known candidates
+GM_HD size_t hop_ints(int k) {
+  return (size_t)2 * hop_slots(k) + kListW + kHopBlock * kListW + kMaxCand / 32;
+}
+struct HopOut {
+  int *cand;        // 256 per row
+  int *cnt;         // per row
+  float *dist;      // 256 per row: known distances are written
+  uint8_t *todo;    // 256 per row: slots without a known distance (null: all)
+  int *todo_cnt;    // per row
+};
 __global__ void __launch_bounds__(kSampWarps * 32)
     k_sample_candidates(const Key *g_key, int row0, int nrows, int n, int k, int slots,
-                        int exist_only, int *cand, int *cand_cnt, const int *changed) {
+                        int exist_only, HopOut o, int iter, const int *changed) {
   if (changed && *changed == 0) return;
   extern __shared__ __align__(16) int smem_sc[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rl = blockIdx.x * kSampWarps + warp;
   if (rl >= nrows) return;
-  const int P = k * k;
   int *hid = smem_sc + (size_t)warp * hop_ints(k);
   int *hpos = hid + slots;
   int *nb = hpos + slots;
-  int *at = nb + kListW;  // position -> slot (-1: none)
+  int *at = nb + kListW;  // the block's positions -> table slot (-1: none)
+  unsigned *known = reinterpret_cast<unsigned *>(at + kHopBlock * kListW);
   const int gid = row0 + rl;
+  int *out = o.cand + (size_t)rl * kMaxCand;
+  float *dist = o.dist + (size_t)rl * kMaxCand;
+  // the previous iteration's candidates
+  int pid[kMaxCand / 32];
+  float pd[kMaxCand / 32];
+  const bool reuse = o.todo && iter > 0;
+  if (reuse) {
+    const int pc = o.cnt[rl];
+#pragma unroll
+    for (int c = 0; c < kMaxCand / 32; ++c) {
+      const int i = c * 32 + lane;
+      pid[c] = i < pc ? out[i] : -1;
+      pd[c] = i < pc ? dist[i] : 0.0f;
+    }
+  }
   const int mine = key_id(g_key[(size_t)gid * kListW + lane]);
   nb[lane] = (lane < k && mine >= 0 && mine < n) ? mine : kIdSentinel;
+  if (lane < kMaxCand / 32) known[lane] = 0u;
   for (int i = lane * 4; i < slots; i += 128) {
     *reinterpret_cast<int4 *>(hid + i) = make_int4(-1, -1, -1, -1);
     *reinterpret_cast<int4 *>(hpos + i) = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
   }
   __syncwarp();
   const unsigned mask = (unsigned)slots - 1u;
+  auto first_slot = [&](int id) { return ((unsigned)id * 2654435761u >> 10) & mask; };
   auto enter = [&](int id, int pos) {
-    unsigned h = ((unsigned)id * 2654435761u >> 10) & mask;
+    unsigned h = first_slot(id);
     for (;;) {
       const int old = atomicCAS(&hid[h], -1, id);
       if (old == -1 || old == id) break;
@@ -185,39 +218,68 @@ __global__ void __launch_bounds__(kSampWarps * 32)
   };
   if (nb[lane] != kIdSentinel) enter(nb[lane], -1);
   __syncwarp();
-  // 32 / w neighbours at a time, w lanes (a power of two >= k) on each list
-  const int w = k <= 8 ? 8 : k <= 16 ? 16 : 32;
-  const int kk = lane & (w - 1), step = 32 / w;
-  constexpr int kAhead = 8;
-  for (int j0 = lane / w; j0 < k; j0 += step * kAhead) {
+  // lane: slot kb + lane % 8 of neighbours lane / 8, lane / 8 + 4, ...
+  constexpr int kSpan = 32 / kHopBlock, kAhead = kListW / kSpan;
+  const int sub = lane % kHopBlock;
+  int base = 0;
+  for (int kb = 0; kb < k && base < kMaxCand; kb += kHopBlock) {
+    const int kk = kb + sub;
     int e[kAhead];
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
-      const int j = j0 + u * step;
-      const int nbr = j < k ? nb[j] : kIdSentinel;
-      e[u] = (nbr != kIdSentinel && kk < k) ? key_id(g_key[(size_t)nbr * kListW + kk]) : -1;
+      const int j = lane / kHopBlock + u * kSpan;
+      const int nbr = (j < k && kk < k) ? nb[j] : kIdSentinel;
+      e[u] = nbr != kIdSentinel ? key_id(g_key[(size_t)nbr * kListW + kk]) : -1;
     }
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
-      const int j = j0 + u * step;
+      const int j = lane / kHopBlock + u * kSpan;
       if (j < k && kk < k)
-        at[kk * k + j] = ((uint32_t)e[u] < (uint32_t)n && e[u] != gid) ? enter(e[u], kk * k + j) : -1;
+        at[sub * k + j] = ((uint32_t)e[u] < (uint32_t)n && e[u] != gid) ? enter(e[u], kk * k + j) : -1;
     }
+    __syncwarp();
+    const int p_end = min(kHopBlock, k - kb) * k;
+    for (int p0 = 0; p0 < p_end && base < kMaxCand; p0 += 32) {
+      const int p = p0 + lane;
+      const int sl = p < p_end ? at[p] : -1;
+      const int id = sl >= 0 ? hid[sl] : -1;
+      const bool keep = sl >= 0 && hpos[sl] == kb * k + p && !(exist_only && id >= row0);
+      const unsigned bal = __ballot_sync(0xffffffffu, keep);
+      const int idx = base + __popc(bal & ((1u << lane) - 1u));
+      if (keep && idx < kMaxCand) {
+        out[idx] = id;
+        hpos[sl] = -2 - idx;  // below every position: later entries change nothing
+      }
+      base += __popc(bal);
+    }
+    __syncwarp();
   }
-  __syncwarp();
-  int *out = cand + (size_t)rl * kMaxCand;
-  int base = 0;
-  for (int p0 = 0; p0 < P && base < kMaxCand; p0 += 32) {
-    const int p = p0 + lane;
-    const int sl = p < P ? at[p] : -1;
-    const int id = sl >= 0 ? hid[sl] : -1;
-    const bool keep = sl >= 0 && hpos[sl] == p && !(exist_only && id >= row0);
-    const unsigned bal = __ballot_sync(0xffffffffu, keep);
-    const int idx = base + __popc(bal & ((1u << lane) - 1u));
-    if (keep && idx < kMaxCand) out[idx] = id;
-    base += __popc(bal);
+  const int cnt = min(base, kMaxCand);
+  if (lane == 0) o.cnt[rl] = cnt;
+  if (!o.todo) return;
+  if (reuse) {
+#pragma unroll
+    for (int c = 0; c < kMaxCand / 32; ++c) {
+      if (pid[c] < 0) continue;
+      unsigned h = first_slot(pid[c]);
+      while (hid[h] != -1 && hid[h] != pid[c]) h = (h + 1u) & mask;
+      const int idx = hid[h] == pid[c] ? -2 - hpos[h] : -1;
+      if (idx >= 0) {
+        dist[idx] = pd[c];
+        atomicOr(&known[idx >> 5], 1u << (idx & 31));
+      }
+    }
+    __syncwarp();
   }
-  if (lane == 0) cand_cnt[rl] = min(base, kMaxCand);
+  int left = 0;
+  for (int c = 0; c * 32 < cnt; ++c) {
+    const bool open = c * 32 + lane < cnt && !((known[c] >> lane) & 1u);
+    const unsigned bal = __ballot_sync(0xffffffffu, open);
+    if (open)
+      o.todo[(size_t)rl * kMaxCand + left + __popc(bal & ((1u << lane) - 1u))] = (uint8_t)(c * 32 + lane);
+    left += __popc(bal);
+  }
+  if (lane == 0) o.todo_cnt[rl] = left;
 }
 
 // Offers of an iteration by target: row j has 32 chains, heads[j * 32 + l]
@@ -234,9 +296,9 @@ struct OfferChains {
 // insertion_kernel.cuh:337-405, and :548-640, which scatters up to 32
 // arrivals per row; here every one is kept, one of the reference's outcomes).
 // A warp takes (row, chunk of 32 candidates) tasks in a grid stride: 32
-// canonical chains (gm_rowdot.cuh), then each offer that can change its
-// target's list (below its last entry; not listed already, which an earlier
-// iteration may have done: scan_listed) is put on one of the target's chains.
+// canonical chains (gm_rowdot.cuh), then each offer below its target's last
+// entry is put on one of the target's chains.  todo (null: every candidate)
+// lists the slots to do.
 // Bound by L2: a row's candidates are 100-200 feature rows.  An insertion of
 // 500 rows x 784 features at k = 15 took 1.35 ms over its ten iterations with
 // a CTA per row, two barriers per chunk and every offer merged under its
@@ -246,36 +308,28 @@ struct OfferChains {
 constexpr int kCandWarps = 2;
 __global__ void __launch_bounds__(kCandWarps * 32)
     k_candidate_offers(const float *X, const float *norms, int ld, int row0, int first, int nrows, int chunks,
-                       const int *cand, const int *cand_cnt, float *cand_dist, const Key *g_key,
-                       OfferChains chains, int scan_listed, const int *changed,
+                       const int *cand, const uint8_t *todo, const int *todo_cnt,
+                       float *cand_dist, const Key *g_key, OfferChains chains, const int *changed,
                        unsigned long long *stat) {
   if (changed && *changed == 0) return;
   __shared__ __align__(16) RowDotTiles tiles[kCandWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tasks = nrows * chunks;
   for (int task = blockIdx.x * kCandWarps + warp; task < tasks; task += gridDim.x * kCandWarps) {
-    const int rl = task / chunks, s = (task - rl * chunks) * 32 + lane;
-    const int cnt = cand_cnt[rl];
-    if (s - lane >= cnt) continue;
+    const int rl = task / chunks, i = (task - rl * chunks) * 32 + lane;
+    const int cnt = todo_cnt[rl];
+    if (i - lane >= cnt) continue;
     const int gid = first + rl;
-    const int j = s < cnt ? cand[(size_t)rl * kMaxCand + s] : gid;
-    if (stat && lane == 0) atomicAdd(&stat[4], (unsigned long long)(min(32, cnt - s) + (s == 0)));
+    const size_t e = (size_t)rl * kMaxCand + (i < cnt && todo ? todo[(size_t)rl * kMaxCand + i] : i);
+    const int j = i < cnt ? cand[e] : gid;
+    if (stat && lane == 0) atomicAdd(&stat[4], (unsigned long long)(min(32, cnt - i) + (i == 0)));
     const float dot = warp_row_dot(X, ld, X + (size_t)gid * ld, j, tiles[warp]);
     const float dv = canon_dist(norms[gid], norms[j], dot);
-    const size_t e = (size_t)rl * kMaxCand + s;
-    if (s < cnt) cand_dist[e] = dv;
-    bool want = false;
-    if (s < cnt && j < row0 && dv >= 0.0f) {
-      const Key ck = make_key(dv, gid);
-      const Key *row = g_key + (size_t)j * kListW;
-      if (ck < __ldcg(&row[kListW - 1])) {
-        want = true;
-        if (scan_listed)
-          for (int w = 0; w < kListW; ++w)
-            if (__ldcg(&row[w]) == ck) want = false;
-      }
+    if (i < cnt) {
+      cand_dist[e] = dv;
+      if (j < row0 && dv >= 0.0f && make_key(dv, gid) < g_key[(size_t)j * kListW + kListW - 1])
+        chains.next[e] = atomicExch(&chains.heads[(size_t)j * 32 + (gid & 31)], (int)e);
     }
-    if (want) chains.next[e] = atomicExch(&chains.heads[(size_t)j * 32 + (gid & 31)], (int)e);
   }
 }
 
@@ -467,8 +521,8 @@ void launch_row_norms(const DevState &st, int row0, int nrows, cudaStream_t s) {
 }
 
 void launch_nnd_insert(const DevState &st, const UpdScratch &u, int row0, int nrows, int n, int window_start,
-                       uint64_t seed, int *cand, int *cand_cnt, float *cand_dist, int *next,
-                       int *changed, int sms, const std::function<void(bool)> &timed, cudaStream_t s) {
+                       uint64_t seed, const CandScratch &c, int *changed, int sms,
+                       const std::function<void(bool)> &timed, cudaStream_t s) {
   if (nrows <= 0) return;
   k_random_init<<<cdiv(nrows, kInitWarps), kInitWarps * 32, 0, s>>>(st.g_key, row0, nrows, n,
                                                                     window_start, seed);
@@ -489,21 +543,10 @@ void launch_nnd_insert(const DevState &st, const UpdScratch &u, int row0, int nr
   const int iters = merges ? kInsertIters : (row0 > 0 ? 1 : 0);
   const int slots = hop_slots(k);
   const size_t smem = (size_t)kSampWarps * hop_ints(k) * sizeof(int);
-  {
-    // the largest table (k = 32) needs more than 48 KB per CTA
-    static std::atomic<unsigned> configured{0u};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 32 && !(configured.load() & (1u << dev))) {
-      cudaFuncSetAttribute(k_sample_candidates, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)(kSampWarps * hop_ints(kListW) * sizeof(int)));
-      configured.fetch_or(1u << dev);
-    }
-  }
   const int chunks = cdiv(std::min(P, kMaxCand), 32);
   // the chains' heads lie over one of the update's sample lists (n_cap x 32,
   // not in use during an insertion)
-  const OfferChains chains{u.fwd_new, next};
+  const OfferChains chains{u.fwd_new, c.next};
   if (row0 > 0) cudaMemsetAsync(chains.heads, 0xff, (size_t)row0 * 32 * sizeof(int), s);
   if (merges) cudaMemsetAsync(changed, 0, kInsertIters * sizeof(int), s);
   for (int it = 0; it < iters; ++it) {
@@ -512,7 +555,8 @@ void launch_nnd_insert(const DevState &st, const UpdScratch &u, int row0, int nr
     const int *go = it > 0 ? changed + it - 1 : nullptr;
     int *mark = merges ? changed + it : nullptr;
     k_sample_candidates<<<cdiv(nrows, kSampWarps), kSampWarps * 32, smem, s>>>(
-        st.g_key, row0, nrows, n, k, slots, merges ? 0 : 1, cand, cand_cnt, go);
+        st.g_key, row0, nrows, n, k, slots, merges ? 0 : 1,
+        HopOut{c.cand, c.cnt, c.dist, merges ? c.todo : nullptr, c.todo_cnt}, it, go);
     note_launch();
     for (int r = 0; r < nrows; r += kOfferRows) {
       const int m = std::min(kOfferRows, nrows - r);
@@ -520,19 +564,19 @@ void launch_nnd_insert(const DevState &st, const UpdScratch &u, int row0, int nr
       const int grid = (int)std::min<long>(cdiv((long)m * chunks, kCandWarps), 24L * std::max(sms, 1));
       timed(true);
       k_candidate_offers<<<grid, kCandWarps * 32, 0, s>>>(
-          st.X, st.norms, st.ld, row0, row0 + r, m, chunks, cand + at, cand_cnt + r, cand_dist + at,
-          st.g_key, chains, merges ? 1 : 0, go, st.stat);
+          st.X, st.norms, st.ld, row0, row0 + r, m, chunks, c.cand + at, merges ? c.todo + at : nullptr,
+          (merges ? c.todo_cnt : c.cnt) + r, c.dist + at, st.g_key, chains, go, st.stat);
       note_launch();
       timed(false);
       if (row0 > 0) {
         k_merge_offers<<<cdiv(row0, kOfferWarps), kOfferWarps * 32, 0, s>>>(
-            st.g_key, row0, row0 + r, chains, cand_dist + at, st.dirty, mark, go);
+            st.g_key, row0, row0 + r, chains, c.dist + at, st.dirty, mark, go);
         note_launch();
       }
     }
     if (merges) {
       k_forward_merge<<<cdiv(nrows, kFwdWarps), kFwdWarps * 32, 0, s>>>(
-          st.g_key, row0, nrows, cand, cand_cnt, cand_dist, mark, go);
+          st.g_key, row0, nrows, c.cand, c.cnt, c.dist, mark, go);
       note_launch();
     }
   }
