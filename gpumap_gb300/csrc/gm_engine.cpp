@@ -817,24 +817,18 @@ size_t Session::update_round(std::vector<uint32_t> &batch, std::vector<uint32_t>
   std::memcpy(h_pin_, batch.data(), (size_t)nb * sizeof(uint32_t));
   ck(cudaMemcpyAsync(d_batch_, h_pin_, (size_t)nb * sizeof(int), cudaMemcpyHostToDevice, s),
      "batch");
-  ck(cudaMemsetAsync(us_.sizes, 0, (size_t)n * sizeof(int4), s), "sizes");
-  ck(cudaMemsetAsync(st_.dirty, 0, (size_t)n * sizeof(int), s), "dirty");
-  launch_sample_graph(st_, us_, d_batch_, nb, n, s);
+  int *counters = d_cnt_ + 1;  // after the report count
   bloom_clean_ = false;
-  build_reverse(st_, us_, d_batch_, nb, n, 0, d_tmp_, s);
-  build_reverse(st_, us_, d_batch_, nb, n, 1, d_tmp_, s);
-  launch_join_flags(us_, n, us_.hflag, s);
-  compact_flags(us_.hflag, n, -1, d_rows_, d_cnt_ + 3, d_tmp_, s);
+  launch_join_nodes(st_, us_, d_batch_, nb, n, d_rows_, d_rows2_, counters, s);
   timed_begin(0);
-  launch_local_join(st_, us_, d_rows_, d_cnt_ + 3, n, n, s);
+  launch_local_join(st_, us_, d_rows_, d_rows2_, counters, n, s);
   timed_end(0);
-  ck(cudaMemsetAsync(d_cnt_ + 1, 0, sizeof(int), s), "edges");
-  launch_merge_publish(st_, us_, nullptr, nullptr, n, n, d_cnt_ + 1, us_.hflag, s);
-  compact_flags(us_.hflag, n, -1, d_rows_, d_cnt_ + 2, d_tmp_, s);
-  ck(cudaMemcpyAsync(h_pin_, d_cnt_, 4 * sizeof(int), cudaMemcpyDeviceToHost, s), "counts");
+  launch_merge_publish(st_, n, counters + kUpdEdges, us_.hflag, s);
+  compact_flags(us_.hflag, n, -1, d_rows_, d_cnt_, d_tmp_, s);
+  ck(cudaMemcpyAsync(h_pin_, d_cnt_, 2 * sizeof(int), cudaMemcpyDeviceToHost, s), "counts");
   sync();
-  const int edges = (int)h_pin_[1];
-  const int na = (int)h_pin_[2];
+  const int na = (int)h_pin_[0];
+  const int edges = (int)h_pin_[1 + kUpdEdges];
   if (na > 0) {
     ck(cudaMemcpyAsync(h_pin_, d_rows_, (size_t)na * sizeof(int), cudaMemcpyDeviceToHost, s),
        "affected");

@@ -39,14 +39,11 @@ struct UpdScratch {
   int *rev_new = nullptr;  // n_cap x 32
   int *rev_old = nullptr;  // n_cap x 32
   int4 *sizes = nullptr;   // n_cap: (fwd new, rev new, fwd old, rev old)
-  int *cnt = nullptr;      // n_cap reverse in-degree
-  int *off = nullptr;      // n_cap + 1 exclusive offsets
-  int *fill = nullptr;     // n_cap
+  int *cnt = nullptr;      // n_cap new sources per row
+  int *off = nullptr;      // n_cap + 1 offsets of the new sources
+  int *fill = nullptr;     // n_cap old sources per row
   int *csr = nullptr;      // n_cap x 32 reverse sources
-  int *hflag = nullptr;    // n_cap per-row host-side dirty state
-  int *rowtmp = nullptr;   // n_cap row list scratch
-  int *rowtmp2 = nullptr;  // n_cap row list scratch
-  int *counters = nullptr; // small device counters
+  int *hflag = nullptr;    // n_cap offsets of the old sources, then report flags
 };
 
 // ---- utilities (gm_kernels_util.cu) ----
@@ -158,21 +155,19 @@ void launch_exact_screen(const DevState &st, int row0, int blk0, int nrows, int 
                          const ExactScreen &x, long ldD, int sms, cudaStream_t s);
 
 // ---- update (gm_kernels_update.cu) ----
-void launch_sample_graph(const DevState &st, const UpdScratch &u,
-                         const int *batch, int nb, int n, cudaStream_t s);
-// Builds rev[j] from fwd lists of the batch rows, keeping the 32 smallest
-// source ids per target.  which = 0 new, 1 old.
-void build_reverse(const DevState &st, const UpdScratch &u, const int *batch,
-                   int nb, int n, int which, int *tmp, cudaStream_t s);
-void launch_local_join(const DevState &st, const UpdScratch &u,
-                       const int *join_nodes, const int *n_join_dev, int n_join_max,
-                       int n, cudaStream_t s);
-// Merges working lists into the authoritative lists for dirty rows,
-// re-sorts them, publishes changed rows and flags rows to report.
-void launch_join_flags(const UpdScratch &u, int n, int *flag, cudaStream_t s);
-void launch_merge_publish(const DevState &st, const UpdScratch &u,
-                          const int *rows, const int *n_rows_dev, int n_rows_max,
-                          int n, int *edge_counter, int *report_flag,
+// Counters of an update round (device ints): edges changed, sources, then
+// small and large join nodes and their tickets.
+constexpr int kUpdEdges = 0, kUpdSources = 1, kUpdNodes = 2, kUpdCounters = 6;
+// Samples the batch rows' lists and builds every row's join lists; clears
+// the round's per-row state and counters first.  Nodes with a pair to form
+// land in small_nodes (at most 32 members) and large_nodes (n ids each).
+void launch_join_nodes(const DevState &st, const UpdScratch &u, const int *batch, int nb, int n,
+                       int *small_nodes, int *large_nodes, int *counters, cudaStream_t s);
+void launch_local_join(const DevState &st, const UpdScratch &u, const int *small_nodes,
+                       const int *large_nodes, int *counters, int n, cudaStream_t s);
+// Merges working lists into the authoritative lists, re-sorts them, publishes
+// changed rows and flags rows to report.
+void launch_merge_publish(const DevState &st, int n, int *edge_counter, int *report_flag,
                           cudaStream_t s);
 
 // ---- embedding (gm_kernels_embed.cu) ----

@@ -1,12 +1,13 @@
 // Update phase: one NN-Descent local-join round over a batch of rows.
 // Restates the reference's UpdateAlgo (update_kernel.cuh:689-1054) with the
 // sampling, reverse lists, merge and publish all on the device.
+#include <algorithm>
+#include <climits>
 #include <mutex>
 
 #include "gm_common.cuh"
 #include "gm_kernels.h"
-
-#include <algorithm>
+#include "gm_rowdot.cuh"
 
 namespace gm {
 
@@ -30,359 +31,435 @@ GM_D uint32_t bloom_h1(uint32_t v) {
   v ^= v << 5;
   return v;
 }
-GM_D bool bloom_check(const uint32_t *bits, uint32_t key) {
-  const uint32_t base = (key % 4u) * 512u;
-  uint32_t h = bloom_h0(key);
-  const uint32_t h1 = bloom_h1(key);
-  for (int i = 0; i < 4; ++i) {
-    if (i > 0) h += h1;
-    const uint32_t b = base + h % 512u;
-    if (!((bits[b >> 5] >> (b & 31u)) & 1u)) return false;
-  }
-  return true;
+// The four bits of a key: set key % 4, bits (h0 + i h1) % 512 of it.
+GM_D int bloom_bit(uint32_t key, int i) {
+  return (int)((key % 4u) * 512u + (bloom_h0(key) + (uint32_t)i * bloom_h1(key)) % 512u);
 }
-GM_D void bloom_add(uint32_t *bits, uint32_t key) {
-  const uint32_t base = (key % 4u) * 512u;
-  uint32_t h = bloom_h0(key);
-  const uint32_t h1 = bloom_h1(key);
-  for (int i = 0; i < 4; ++i) {
-    if (i > 0) h += h1;
-    const uint32_t b = base + h % 512u;
-    bits[b >> 5] |= (1u << (b & 31u));
-  }
+
+// Zeroes the per-row state of an update round and its counters.
+__global__ void k_update_reset(int n, int4 *sizes, int *dirty, int *cnt_new, int *cnt_old,
+                               int *counters, int n_counters) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n_counters) counters[i] = 0;
+  if (i >= n) return;
+  sizes[i] = make_int4(0, 0, 0, 0);
+  dirty[i] = 0;
+  cnt_new[i] = 0;
+  cnt_old[i] = 0;
 }
 
 // New/old samples of each batch row from its authoritative k-list: new
 // entries (up to 32) are sampled, marked old and recorded in the Bloom
 // filter; old entries the filter has not seen are sampled (up to 32)
 // (reference: UpdateAlgo::sample_graph, update_kernel.cuh:750-807).
-__global__ void k_sample_graph(int *knn_ids, uint32_t *bloom, const int *batch,
-                               int nb, int n, int k, int *fwd_new, int *fwd_old,
-                               int4 *sizes) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// A warp per row, entry j on lane j.  In list order an old entry sees the bits
+// that the new entries before it have set: each new entry's bits are handed
+// round and the lanes behind it note the ones they ask for.  The position of
+// each sample among its target's sources (pos_*, any order) is taken here, so
+// that the reverse lists need no second count.  One thread per row took 26 us
+// for 2,000 rows at k = 15, this form 5 us.
+constexpr int kSgWarps = 8;
+__global__ void __launch_bounds__(kSgWarps * 32)
+    k_sample_graph(int *knn_ids, uint32_t *bloom, const int *batch, int nb, int n, int k,
+                   int *fwd_new, int *fwd_old, int *pos_new, int *pos_old, int *cnt_new,
+                   int *cnt_old, int4 *sizes) {
+  __shared__ uint32_t s_bits[kSgWarps][64];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * kSgWarps + warp;
   if (i >= nb) return;
+  const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
   const int row = batch[i];
   int *list = knn_ids + (size_t)row * k;
   uint32_t *bits = bloom + (size_t)row * 64;
-  int xn = 0, xo = 0;
-  for (int j = 0; j < k; ++j) {
-    const int e = list[j];
-    const bool isnew = e >= 0;
-    const int id = isnew ? e : -e - 1;
-    if ((uint32_t)id >= (uint32_t)n) continue;
-    if (!isnew) {
-      if (bloom_check(bits, (uint32_t)id)) continue;
-      if (xo < kSamples) fwd_old[(size_t)row * kSamples + xo++] = id;
-    } else if (xn < kSamples) {
-      list[j] = -id - 1;
-      fwd_new[(size_t)row * kSamples + xn++] = id;
-      bloom_add(bits, (uint32_t)id);
-    }
-    if (xo == kSamples && xn == kSamples) break;
+  uint32_t *sb = s_bits[warp];
+  const int e = lane < k ? list[lane] : kIdSentinel;
+  sb[lane] = bits[lane];
+  sb[lane + 32] = bits[lane + 32];
+  __syncwarp();
+  const int id = e >= 0 ? e : -e - 1;
+  const bool valid = lane < k && (uint32_t)id < (uint32_t)n;
+  const bool isnew = valid && e >= 0;
+  int b[4];
+  unsigned seen = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    b[q] = bloom_bit((uint32_t)id, q);
+    if (valid && ((sb[b[q] >> 5] >> (b[q] & 31)) & 1u)) seen |= 1u << q;
   }
-  int4 sz = sizes[row];
-  sz.x = xn;
-  sz.z = xo;
-  sizes[row] = sz;
+  __syncwarp();
+  const unsigned news = __ballot_sync(full, isnew);
+  for (unsigned m = news; m; m &= m - 1u) {
+    const int src = __ffs(m) - 1;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const int x = __shfl_sync(full, b[p], src);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (src < lane && b[q] == x) seen |= 1u << q;
+    }
+  }
+  const bool isold = valid && e < 0 && seen != 15u;
+  const unsigned olds = __ballot_sync(full, isold);
+  const size_t at = (size_t)row * kSamples;
+  if (isnew) {
+    list[lane] = -id - 1;
+    const int s = __popc(news & lt);
+    fwd_new[at + s] = id;
+    pos_new[at + s] = atomicAdd(&cnt_new[id], 1);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) atomicOr(&sb[b[q] >> 5], 1u << (b[q] & 31));
+  }
+  if (isold) {
+    const int s = __popc(olds & lt);
+    fwd_old[at + s] = id;
+    pos_old[at + s] = atomicAdd(&cnt_old[id], 1);
+  }
+  __syncwarp();
+  if (news) {
+    bits[lane] = sb[lane];
+    bits[lane + 32] = sb[lane + 32];
+  }
+  if (lane == 0) sizes[row] = make_int4(__popc(news), 0, __popc(olds), 0);
 }
 
-GM_D int fwd_count(int4 s, int which) { return which ? s.z : s.x; }
+// A segment of the source array for every target's new, then old sources
+// (segments in any order; both together hold at most one entry per list slot
+// of the batch, so n_cap x 32 entries are enough).
+__global__ void k_rev_segments(int n, const int *cnt_new, const int *cnt_old, int *off_new,
+                               int *off_old, int *total) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  const int a = j < n ? cnt_new[j] : 0, c = j < n ? cnt_old[j] : 0;
+  int v = a + c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += y;
+  }
+  int base = 0;
+  if (lane == 31 && v) base = atomicAdd(total, v);
+  base = __shfl_sync(0xffffffffu, base, 31) + v - a - c;
+  if (j < n) {
+    off_new[j] = base;
+    off_old[j] = base + a;
+  }
+}
 
-__global__ void k_rev_count(const int *batch, int nb, int n, const int *fwd,
-                            const int4 *sizes, int which, int *cnt) {
+__global__ void k_rev_place(const int *batch, int nb, const int *fwd_new, const int *fwd_old,
+                            const int *pos_new, const int *pos_old, const int4 *sizes,
+                            const int *off_new, const int *off_old, int *src) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= nb * kSamples) return;
-  const int i = tid / kSamples, s = tid - i * kSamples;
-  const int row = batch[i];
-  if (s >= fwd_count(sizes[row], which)) return;
-  const int j = fwd[(size_t)row * kSamples + s];
-  if (j < 0 || j >= n) return;
-  atomicAdd(&cnt[j], 1);
+  const int row = batch[tid / kSamples], s = tid % kSamples;
+  const size_t at = (size_t)row * kSamples + s;
+  const int4 sz = sizes[row];
+  if (s < sz.x) src[off_new[fwd_new[at]] + pos_new[at]] = row;
+  if (s < sz.z) src[off_old[fwd_old[at]] + pos_old[at]] = row;
 }
 
-__global__ void k_rev_fill(const int *batch, int nb, int n, const int *fwd,
-                           const int4 *sizes, int which, const int *off, int *fill,
-                           int *csr) {
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= nb * kSamples) return;
-  const int i = tid / kSamples, s = tid - i * kSamples;
-  const int row = batch[i];
-  if (s >= fwd_count(sizes[row], which)) return;
-  const int j = fwd[(size_t)row * kSamples + s];
-  if (j < 0 || j >= n) return;
-  const int pos = off[j] + atomicAdd(&fill[j], 1);
-  csr[pos] = row;
-}
-
-// Reverse list of j: its sources in ascending id order, capped at the 32
-// smallest.  The reference keeps the first 32 atomic arrivals
-// (add_rev_edges_kernel, update_kernel.cuh:122-146); ascending-id is one of
-// its possible outcomes and makes the round deterministic.
-__global__ void k_rev_finalize(int n, const int *cnt, const int *off, const int *csr,
-                               int *rev, int4 *sizes, int which) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const int c = cnt[j];
-  if (c == 0) return;
-  int v[kSamples];
-  int m = 0;
-  const int *src = csr + off[j];
-  for (int q = 0; q < c; ++q) {
-    const int x = src[q];
-    if (m == kSamples && x >= v[kSamples - 1]) continue;
-    int pos = (m < kSamples) ? m : kSamples - 1;
-    while (pos > 0 && v[pos - 1] > x) {
-      v[pos] = v[pos - 1];
-      --pos;
+// Join lists of every row with new samples or sources: N = forward-new, then
+// reverse-new not in forward-new; O = forward-old, then reverse-old not in
+// forward-old.  A reverse list is its target's 32 smallest source ids in
+// ascending order.  (The reference keeps the first 32 atomic arrivals,
+// add_rev_edges_kernel, update_kernel.cuh:122-146; ascending ids are one of
+// its outcomes and make the round deterministic.)  A warp per row; the kept
+// reverse samples replace the positions in rev_*, sizes becomes (forward new,
+// kept reverse new, forward old, kept reverse old), and rows with a pair to
+// form are appended to the small (at most 32 members) or the large node list
+// (any order).
+constexpr int kListWarps = 8;
+GM_D int warp_smallest(const int *src, int c) {
+  // lane l: the l-th smallest of c distinct ids (INT_MAX past the end)
+  const int lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu;
+  int mine = INT_MAX;
+  for (int c0 = 0; c0 < c; c0 += 32) {
+    const int v = c0 + lane < c ? src[c0 + lane] : INT_MAX;
+    unsigned todo = __ballot_sync(full, v < __shfl_sync(full, mine, 31));
+    while (todo) {
+      const int x = __shfl_sync(full, v, __ffs(todo) - 1);
+      todo &= todo - 1u;
+      const unsigned after = __ballot_sync(full, x < mine);
+      if (!after) continue;
+      const int pos = __ffs(after) - 1;
+      const int prev = __shfl_up_sync(full, mine, 1);
+      if (lane > pos) mine = prev;
+      else if (lane == pos) mine = x;
     }
-    v[pos] = x;
-    if (m < kSamples) ++m;
   }
-  int *out = rev + (size_t)j * kSamples;
-  for (int q = 0; q < m; ++q) out[q] = v[q];
-  int4 sz = sizes[j];
-  if (which) sz.w = m; else sz.y = m;
-  sizes[j] = sz;
+  return mine;
+}
+__global__ void __launch_bounds__(kListWarps * 32)
+    k_join_lists(int n, const int *fwd_new, const int *fwd_old, int *rev_new, int *rev_old,
+                 const int *cnt_new, const int *cnt_old, const int *off_new, const int *off_old,
+                 const int *src, int4 *sizes, int *small_nodes, int *large_nodes, int *counts) {
+  __shared__ int s_cls[kListWarps];
+  __shared__ int s_base[2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int j = blockIdx.x * kListWarps + warp;
+  const unsigned full = 0xffffffffu;
+  int cls = 0;
+  if (j < n) {
+    const int4 sz = sizes[j];
+    const int cn = cnt_new[j];
+    if (sz.x + cn > 0) {
+      const int co = cnt_old[j];
+      const size_t at = (size_t)j * kSamples;
+      auto side = [&](const int *fwd, int *rev, int nf, int c, int off) {
+        const int f = lane < nf ? fwd[at + lane] : -1;
+        const int r = warp_smallest(src + off, c);
+        bool keep = lane < c && r != INT_MAX;
+        for (int q = 0; q < nf; ++q) keep &= __shfl_sync(full, f, q) != r;
+        const unsigned bal = __ballot_sync(full, keep);
+        if (keep) rev[at + __popc(bal & ((1u << lane) - 1u))] = r;
+        return __popc(bal);
+      };
+      const int rn = side(fwd_new, rev_new, sz.x, cn, off_new[j]);
+      const int ro = side(fwd_old, rev_old, sz.z, co, off_old[j]);
+      if (lane == 0) sizes[j] = make_int4(sz.x, rn, sz.z, ro);
+      const int m = sz.x + rn + sz.z + ro;
+      cls = m < 2 ? 0 : m <= 32 ? 1 : 2;
+    }
+  }
+  if (lane == 0) s_cls[warp] = cls;
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    int c = 0;
+    for (int w = 0; w < kListWarps; ++w) c += s_cls[w] == (int)threadIdx.x + 1;
+    s_base[threadIdx.x] = c ? atomicAdd(&counts[threadIdx.x], c) : 0;
+  }
+  __syncthreads();
+  if (lane == 0 && cls) {
+    int at = s_base[cls - 1];
+    for (int w = 0; w < warp; ++w) at += s_cls[w] == cls;
+    (cls == 1 ? small_nodes : large_nodes)[at] = j;
+  }
 }
 
-__global__ void k_join_flags(const int4 *sizes, int n, int *flag) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const int4 s = sizes[j];
-  flag[j] = (s.x + s.y) > 0 ? 1 : 0;
+// Local join of a node's lists N and O.  Distances of N x (N ++ O) are FP32,
+// a sequential fma chain per pair; every pair is then offered to both
+// endpoints' lists: N members get all other N and O members, O members get
+// the N members (reference: local_join_kernel, update_kernel.cuh:377-687).
+//
+// W warps work on a node: the CTA's four on a large one, a single warp on a
+// small one (at most 32 members), the four warps of a CTA on different nodes.
+// The members' rows come 32 features at a time by 16-byte cp.async into a ring
+// of kJoinRing slots (36 words a row: conflict-free 16-byte reads), each row
+// once; member row r of N is on warp r % W, member column c on lane c % 32, so
+// a thread's products take its own columns and broadcast rows, and its sums
+// stay in registers.  The distance tile then goes over the ring, and each
+// warp takes every W-th member as a target: its list (read one target ahead)
+// decides which offers can act, and only then its lock is taken.
+//
+// Bound by latency: rows from L2, list snapshots and the lock's round trips
+// (about 2.5 us a merge), so what counts is the number of nodes in flight:
+// 16 warps an SM on as many small nodes, where a CTA of eight warps per node
+// had three.  45 rounds of 2,000 rows over 20k x 784 (k = 15): 28.4 -> 12.0 ms;
+// 10 rounds of 10,000 rows over 100k x 128 (k = 30): 12.8 -> 6.1 ms.
+constexpr int kJoinWarps = 4;
+constexpr int kJoinRing = 3;
+constexpr int kJoinLd = 36;
+constexpr int kJoinCols = 2 * kJoinMax;  // members of a large node
+
+struct JoinArgs {
+  const int *fwd_new, *fwd_old, *rev_new, *rev_old;
+  const int4 *sizes;
+  const float *X, *norms;
+  int ld, k;
+  Key *g_key;
+  int *locks, *dirty;
+  unsigned *err;
+  unsigned long long *stat;
+};
+
+template <int W>
+GM_D void join_sync() {
+  if (W == 1) __syncwarp();
+  else __syncthreads();
 }
 
-// Local join of one node per CTA.  New list N = forward-new + unseen
-// reverse-new, old list O = forward-old + unseen reverse-old.  Distances of
-// N x (N ++ O) are formed as an FP32 tile with a sequential fma chain per
-// pair; every pair is then offered to both endpoints' lists: N members get
-// all other N and O members, O members get the N members
-// (reference: local_join_kernel, update_kernel.cuh:377-687).
-constexpr int kLJThreads = 256;
-constexpr int kLJWarps = kLJThreads / 32;
-constexpr int kLJKC = 32;
-constexpr int kLJR = kJoinMax;      // 64 tile rows (N)
-constexpr int kLJC = 2 * kJoinMax;  // 128 tile cols (N ++ O)
-
-// One feature chunk of the node's rows: N (A) and N ++ O (B), feature-major.
-struct LJStage {
-  float As[kLJKC][kLJR + 4];
-  float Bs[kLJKC][kLJC + 4];
-};
-struct LJSmem {
-  int cid[kLJC];
-  float nrm[kLJC];
-  // two chunk stages (chunk i in stage i & 1: one barrier per chunk), and
-  // over them, once the products are done, the node's distance tile
-  union {
-    LJStage st[2];
-    float D[kLJR][kLJC + 1];
-  } u;
-  Key lst[kLJWarps][kListW];
-  Key cb[kLJWarps][kLJC];
-  int nN, nC;
-};
-
-__global__ void __launch_bounds__(kLJThreads, 3) k_local_join(
-    const int *join_nodes, const int *n_join_dev, const int *fwd_new,
-    const int *fwd_old, const int *rev_new, const int *rev_old, const int4 *sizes,
-    const float *X, const float *norms, int ld, int d, int n, int k, Key *g_key,
-    int *locks, int *dirty, unsigned *err, unsigned long long *stat) {
-  extern __shared__ __align__(16) unsigned char lj_raw[];
-  LJSmem &S = *reinterpret_cast<LJSmem *>(lj_raw);
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int n_join = *n_join_dev;
-  // Persistent CTAs: each walks the join list with a grid stride.
-  for (int bi = blockIdx.x; bi < n_join; bi += gridDim.x) {
-    __syncthreads();  // previous node's shared data is no longer read
-    const int u = join_nodes[bi];
-    if (warp == 0) {
-      // join lists built by warp 0, entries in sample order (ballot
-      // compaction): N = forward-new ++ reverse-new not already in
-      // forward-new, then forward-old ++ reverse-old not in forward-old
-      const int4 sz = sizes[u];
-      const unsigned lt = (1u << lane) - 1u;
-      const int *fn = fwd_new + (size_t)u * kSamples;
-      const int *rn = rev_new + (size_t)u * kSamples;
-      const int *fo = fwd_old + (size_t)u * kSamples;
-      const int *ro = rev_old + (size_t)u * kSamples;
-      int v = lane < sz.x ? fn[lane] : -1;
-      bool ok = v >= 0 && v < n;
-      unsigned bal = __ballot_sync(0xffffffffu, ok);
-      if (ok) S.cid[__popc(bal & lt)] = v;
-      const int nfn = __popc(bal);
-      __syncwarp();
-      v = lane < sz.y ? rn[lane] : -1;
-      ok = v >= 0 && v < n;
-      for (int q = 0; q < nfn && ok; ++q) ok = S.cid[q] != v;
-      bal = __ballot_sync(0xffffffffu, ok);
-      if (ok) S.cid[nfn + __popc(bal & lt)] = v;
-      const int nN = nfn + __popc(bal);
-      __syncwarp();
-      v = lane < sz.z ? fo[lane] : -1;
-      ok = v >= 0 && v < n;
-      bal = __ballot_sync(0xffffffffu, ok);
-      if (ok) S.cid[nN + __popc(bal & lt)] = v;
-      const int nfo = nN + __popc(bal);
-      __syncwarp();
-      v = lane < sz.w ? ro[lane] : -1;
-      ok = v >= 0 && v < n;
-      for (int q = nN; q < nfo && ok; ++q) ok = S.cid[q] != v;
-      bal = __ballot_sync(0xffffffffu, ok);
-      if (ok) S.cid[nfo + __popc(bal & lt)] = v;
-      const int nC = nfo + __popc(bal);
-      if (lane == 0) {
-        S.nN = nN;
-        S.nC = nC;
-        if (stat && nN > 0) {
-          atomicAdd(&stat[0], 1ull);
-          atomicAdd(&stat[1], (unsigned long long)nC);
-          atomicAdd(&stat[2], (unsigned long long)nN * (unsigned long long)nC);
+// Products of one feature chunk: the thread's CG column groups against its
+// warp's rows, four features at a time.
+template <int W, int CG, int R, int C>
+GM_D void join_products(const float *slot, int nq, int nr, int w, int lane, float (&acc)[R][C]) {
+  for (int f = 0; f < nq; ++f) {
+    float4 b[CG];
+#pragma unroll
+    for (int g = 0; g < CG; ++g)
+      b[g] = *reinterpret_cast<const float4 *>(slot + (g * 32 + lane) * kJoinLd + 4 * f);
+#pragma unroll
+    for (int r0 = 0; r0 < R; r0 += 4) {
+      if (r0 >= nr) break;
+#pragma unroll
+      for (int r = r0; r < r0 + 4; ++r) {
+        const float4 a = *reinterpret_cast<const float4 *>(slot + (r * W + w) * kJoinLd + 4 * f);
+#pragma unroll
+        for (int g = 0; g < CG; ++g) {
+          acc[r][g] = __fmaf_rn(a.x, b[g].x, acc[r][g]);
+          acc[r][g] = __fmaf_rn(a.y, b[g].y, acc[r][g]);
+          acc[r][g] = __fmaf_rn(a.z, b[g].z, acc[r][g]);
+          acc[r][g] = __fmaf_rn(a.w, b[g].w, acc[r][g]);
         }
       }
     }
-    __syncthreads();
-    const int nN = S.nN, nC = S.nC;
-    if (nN == 0) continue;
-    for (int c = t; c < nC; c += kLJThreads) S.nrm[c] = norms[S.cid[c]];
+  }
+}
 
-    // ---- FP32 distance tile over the node's real extent (rows N, columns
-    // N ++ O): one 4 x 4 micro-tile per thread when the tile has at most
-    // kLJThreads of them (every node at k <= 16: about 30 x 90), else 4 x 8
-    // (at most 16 x 16); the threads past the last micro-tile only stage
-    const bool narrow = ((nN + 3) >> 2) * ((nC + 3) >> 2) <= kLJThreads;
-    const int mw = narrow ? 4 : 8;
-    const int mtc = (nC + mw - 1) / mw;
-    const bool active = t < ((nN + 3) >> 2) * mtc;
-    const int r0 = active ? (t / mtc) * 4 : 0, c0 = active ? (t % mtc) * mw : 0;
-    float acc[4][8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+template <int W>
+GM_D void join_node(int u, const JoinArgs &g, float *ring, int *cid, float *nrm) {
+  constexpr int kRows = 32 * W;             // ring rows
+  constexpr int kGroups = W == 1 ? 1 : kJoinCols / 32;
+  constexpr int kMine = W == 1 ? 32 : kJoinMax / W;  // rows of N per warp
+  constexpr int kLdD = kRows + 1;
+  const int lane = threadIdx.x & 31, w = W == 1 ? 0 : (int)(threadIdx.x >> 5);
+  const int t = W == 1 ? lane : (int)threadIdx.x;
+  const int4 sz = g.sizes[u];
+  const int nN = sz.x + sz.y, nC = nN + sz.z + sz.w;
+  const size_t at = (size_t)u * kSamples;
+  if (t < kSamples) {
+    if (lane < sz.x) cid[lane] = g.fwd_new[at + lane];
+    if (lane < sz.y) cid[sz.x + lane] = g.rev_new[at + lane];
+    if (lane < sz.z) cid[nN + lane] = g.fwd_old[at + lane];
+    if (lane < sz.w) cid[nN + sz.z + lane] = g.rev_old[at + lane];
+  }
+  join_sync<W>();
+  for (int c = t; c < nC; c += 32 * W) nrm[c] = g.norms[cid[c]];
 
-    // feature chunks: the next chunk's loads are issued before this chunk's
-    // products, so their latency overlaps the arithmetic
-    float4 pa[2], pb[4];
-    auto fetch = [&](int k0) {
+  const int q = t & 7, r0 = t >> 3;
+  const float *src[8];
 #pragma unroll
-      for (int p = 0; p < 2; ++p) {
-        const int f = t + p * kLJThreads;
-        const int r = f >> 3, q = f & 7;
-        const int col = k0 + 4 * q;
-        pa[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < nN && col < ld)
-          pa[p] = __ldg(reinterpret_cast<const float4 *>(X + (size_t)S.cid[r] * ld + col));
-      }
+  for (int i = 0; i < 8; ++i) {
+    const int r = r0 + 4 * W * i;
+    src[i] = g.X + (size_t)(r < nC ? cid[r] : 0) * g.ld + 4 * q;
+  }
+  const int nch = (g.ld + 31) / 32;
+  auto issue = [&](int c) {
+    if (c * 32 + 4 * q < g.ld) {
+      float *slot = ring + (size_t)(c % kJoinRing) * kRows * kJoinLd + 4 * q;
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        const int f = t + p * kLJThreads;
-        const int r = f >> 3, q = f & 7;
-        const int col = k0 + 4 * q;
-        pb[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < nC && col < ld)
-          pb[p] = __ldg(reinterpret_cast<const float4 *>(X + (size_t)S.cid[r] * ld + col));
+      for (int i = 0; i < 8; ++i) {
+        const int r = r0 + 4 * W * i;
+        if (r < nC) dot_cp16(slot + r * kJoinLd, src[i] + c * 32);
       }
+    }
+    dot_commit();
+  };
+  float acc[kMine][kGroups];
+#pragma unroll
+  for (int r = 0; r < kMine; ++r)
+#pragma unroll
+    for (int c = 0; c < kGroups; ++c) acc[r][c] = 0.0f;
+  const int nr = (nN - w + W - 1) / W;  // rows of this warp
+  for (int c = 0; c < kJoinRing - 1; ++c) issue(c);
+  for (int c = 0; c < nch; ++c) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kJoinRing - 2) : "memory");
+    join_sync<W>();  // chunk c has landed, and every thread is done with chunk c - 1
+    issue(c + kJoinRing - 1);
+    const float *slot = ring + (size_t)(c % kJoinRing) * kRows * kJoinLd;
+    const int nq = min(32, g.ld - c * 32) >> 2;
+    if (W == 1 || nC <= 32) join_products<W, 1>(slot, nq, nr, w, lane, acc);
+    else if (nC <= 64) join_products<W, (W == 1 ? 1 : 2)>(slot, nq, nr, w, lane, acc);
+    else if (nC <= 96) join_products<W, (W == 1 ? 1 : 3)>(slot, nq, nr, w, lane, acc);
+    else join_products<W, kGroups>(slot, nq, nr, w, lane, acc);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  join_sync<W>();  // every product is done before the tile overwrites the ring
+  float *D = ring;
+#pragma unroll
+  for (int r = 0; r < kMine; ++r)
+#pragma unroll
+    for (int c = 0; c < kGroups; ++c) {
+      const int row = r * W + w, col = c * 32 + lane;
+      if (row < nN && col < nC) D[row * kLdD + col] = canon_dist(nrm[row], nrm[col], acc[r][c]);
+    }
+  join_sync<W>();
+
+  // ---- offers, one target per warp at a time
+  const unsigned full = 0xffffffffu;
+  Key snap = w < nC ? __ldcg(&g.g_key[(size_t)cid[w] * kListW + lane]) : 0;
+  for (int tt = w; tt < nC; tt += W) {
+    const Key list = snap;
+    if (tt + W < nC) snap = __ldcg(&g.g_key[(size_t)cid[tt + W] * kListW + lane]);
+    const int idt = cid[tt];
+    const bool in_n = tt < nN;
+    const int ncand = in_n ? nC : nN;
+    auto key_of = [&](int c) {
+      if (c >= ncand || c == tt || cid[c] == idt) return ~(Key)0;
+      return make_key(in_n ? D[tt * kLdD + c] : D[c * kLdD + tt], cid[c]);
     };
-    // chunk i is stored in stage i & 1, whose last readers (the products of
-    // chunk i - 2) every thread has finished before the barrier of chunk
-    // i - 1, so one barrier per chunk orders both uses
-    fetch(0);
-    int sb = 0;
-    for (int k0 = 0; k0 < d; k0 += kLJKC, sb ^= 1) {
-      LJStage &G = S.u.st[sb];
-#pragma unroll
-      for (int p = 0; p < 2; ++p) {
-        const int f = t + p * kLJThreads;
-        const int r = f >> 3, q = f & 7;
-        G.As[4 * q][r] = pa[p].x; G.As[4 * q + 1][r] = pa[p].y;
-        G.As[4 * q + 2][r] = pa[p].z; G.As[4 * q + 3][r] = pa[p].w;
-      }
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        const int f = t + p * kLJThreads;
-        const int r = f >> 3, q = f & 7;
-        G.Bs[4 * q][r] = pb[p].x; G.Bs[4 * q + 1][r] = pb[p].y;
-        G.Bs[4 * q + 2][r] = pb[p].z; G.Bs[4 * q + 3][r] = pb[p].w;
-      }
-      __syncthreads();
-      if (k0 + kLJKC < d) fetch(k0 + kLJKC);
-      if (active) {
-        const int kend = min(kLJKC, d - k0);
-        for (int kk = 0; kk < kend; ++kk) {
-          const float4 a = *reinterpret_cast<const float4 *>(&G.As[kk][r0]);
-          const float4 b0 = *reinterpret_cast<const float4 *>(&G.Bs[kk][c0]);
-          const float av[4] = {a.x, a.y, a.z, a.w};
-          const float bv[4] = {b0.x, b0.y, b0.z, b0.w};
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = __fmaf_rn(av[i], bv[j], acc[i][j]);
-          if (!narrow) {
-            const float4 b1 = *reinterpret_cast<const float4 *>(&G.Bs[kk][c0 + 4]);
-            const float bw[4] = {b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-              for (int j = 0; j < 4; ++j) acc[i][4 + j] = __fmaf_rn(av[i], bw[j], acc[i][4 + j]);
-          }
-        }
+    // an offer acts if it is below the last entry and not listed already
+    const Key worst = __shfl_sync(full, list, kListW - 1);
+    bool act = false;
+    for (int c0 = 0; c0 < ncand && !act; c0 += 32) {
+      const Key ck = key_of(c0 + lane);
+      unsigned todo = __ballot_sync(full, ck < worst);
+      while (todo && !act) {
+        const Key x = __shfl_sync(full, ck, __ffs(todo) - 1);
+        todo &= todo - 1u;
+        act = !__any_sync(full, list == x);
       }
     }
-    __syncthreads();  // every product is done before the tile overwrites the stages
-    if (active) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int r = r0 + i, c = c0 + j;
-          if (j < mw && r < nN && c < nC) S.u.D[r][c] = canon_dist(S.nrm[r], S.nrm[c], acc[i][j]);
-        }
+    if (!act) continue;
+    if (!warp_lock(&g.locks[idt], g.err)) continue;
+    Key *row = g.g_key + (size_t)idt * kListW;
+    Key mine = __ldcg(&row[lane]);
+    int minpos = kListW;
+    for (int c0 = 0; c0 < ncand; c0 += 32) {
+      const Key ck = key_of(c0 + lane);
+      unsigned todo = __ballot_sync(full, ck < __shfl_sync(full, mine, kListW - 1));
+      while (todo) {
+        const int s = __ffs(todo) - 1;
+        todo &= todo - 1u;
+        minpos = min(minpos, warp_insert(mine, __shfl_sync(full, ck, s)));
+      }
     }
-    __syncthreads();
+    if (minpos < kListW) __stcg(&row[lane], mine);
+    warp_unlock(&g.locks[idt]);
+    if (lane == 0) {
+      if (minpos < kListW) atomicMax(&g.dirty[idt], minpos < g.k ? 2 : 1);
+      if (g.stat) atomicAdd(&g.stat[3], 1ull);
+    }
+  }
+  if (g.stat && t == 0) {
+    atomicAdd(&g.stat[0], 1ull);
+    atomicAdd(&g.stat[1], (unsigned long long)nC);
+    atomicAdd(&g.stat[2], (unsigned long long)nN * (unsigned long long)nC);
+  }
+}
 
-    // ---- offer pairs to both endpoints, one target per warp at a time.
-    // An offer can only act if it is below the target's last entry and not
-    // already listed with this distance; the snapshot (8-byte slots, never
-    // torn) filters the rest without taking the lock.
-    for (int tt = warp; tt < nC; tt += kLJWarps) {
-      const int idt = S.cid[tt];
-      S.lst[warp][lane] = __ldcg(&g_key[(size_t)idt * kListW + lane]);
-      __syncwarp();
-      const Key worst = S.lst[warp][kListW - 1];
-      const int ncand = (tt < nN) ? nC : nN;
-      int m = 0;
-      for (int c0b = 0; c0b < ncand; c0b += 32) {
-        const int c = c0b + lane;
-        bool pass = false;
-        Key ck = 0;
-        if (c < ncand && c != tt) {
-          const int cidv = S.cid[c];
-          const float dv = (tt < nN) ? S.u.D[tt][c] : S.u.D[c][tt];
-          ck = make_key(dv, cidv);
-          if (cidv != idt && ck < worst) {
-            pass = true;
-            for (int q = 0; q < kListW; ++q)
-              if (S.lst[warp][q] == ck) {
-                pass = false;
-                break;
-              }
-          }
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, pass);
-        if (pass) S.cb[warp][m + __popc(bal & ((1u << lane) - 1u))] = ck;
-        m += __popc(bal);
-      }
-      __syncwarp();
-      if (m > 0) {
-        const int pos = warp_locked_merge(idt, S.cb[warp], m, g_key, locks, err);
-        if (lane == 0) {
-          if (pos >= 0 && pos < kListW) atomicMax(&dirty[idt], pos < k ? 2 : 1);
-          if (stat) atomicAdd(&stat[3], 1ull);
-        }
-      }
-      __syncwarp();
-    }
+// Persistent CTAs take the large nodes together, then their warps the small
+// ones, by tickets (counts[0] / counts[1] small / large nodes, counts[2] /
+// counts[3] their tickets).
+struct JoinSmem {
+  float ring[kJoinRing * kJoinCols * kJoinLd];
+  int cid[kJoinCols];
+  float nrm[kJoinCols];
+  int ticket;
+};
+static_assert(sizeof(float) * kJoinRing * kJoinCols * kJoinLd >= sizeof(float) * kJoinMax * (kJoinCols + 1),
+              "the tile of a large node does not fit its ring");
+__global__ void __launch_bounds__(kJoinWarps * 32, 4)
+    k_local_join(const int *small_nodes, const int *large_nodes, int *counts, JoinArgs g) {
+  extern __shared__ __align__(16) unsigned char join_raw[];
+  JoinSmem &S = *reinterpret_cast<JoinSmem *>(join_raw);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n_small = counts[0], n_large = counts[1];
+  for (;;) {
+    __syncthreads();  // the previous node's shared data is no longer read
+    if (threadIdx.x == 0) S.ticket = n_large ? atomicAdd(&counts[3], 1) : 0;
+    __syncthreads();
+    if (S.ticket >= n_large) break;
+    join_node<kJoinWarps>(large_nodes[S.ticket], g, S.ring, S.cid, S.nrm);
+  }
+  int next = 0;
+  if (lane == 0 && n_small) next = atomicAdd(&counts[2], 1);
+  for (;;) {
+    const int i = __shfl_sync(0xffffffffu, next, 0);
+    if (i >= n_small) break;
+    if (lane == 0) next = atomicAdd(&counts[2], 1);
+    __syncwarp();
+    join_node<1>(small_nodes[i], g, S.ring + (size_t)warp * kJoinRing * 32 * kJoinLd, S.cid + warp * 32,
+                 S.nrm + warp * 32);
+    __syncwarp();
   }
 }
 
@@ -390,91 +467,96 @@ __global__ void __launch_bounds__(kLJThreads, 3) k_local_join(
 // 986-1050) for every row, as the reference does: a row whose working list
 // did not change this round can still gain an entry, when an id that was a
 // placeholder in its k-list (and so skipped as a duplicate) has since been
-// pushed out of the k-list.  rows == nullptr means rows 0..n-1.
-__global__ void k_merge_publish(const int *rows, const int *n_rows_dev,
-                                const Key *g_key, int *knn_ids,
-                                float *knn_dists, const int *dirty,
-                                uint32_t *pub_idx, float *pub_dist, int k, int n,
-                                int *edge_counter, int *report_flag) {
-  const int nr = rows ? *n_rows_dev : n;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nr; i += gridDim.x * blockDim.x) {
-  const int row = rows ? rows[i] : i;
-  int lid[kListW];
-  float ldv[kListW];
+// pushed out of the k-list.
+// A warp per row, entry j of both lists on lane j.  Most rows change nothing:
+// every working entry that could enter is listed already, and none does.
+// Otherwise the working entries are taken in order, as insert_to_ordered_list
+// does (update_kernel.cuh:87-120).  One thread per row took 206 us for 100,000
+// rows at k = 30, this form 56 us.
+constexpr int kMpWarps = 8;
+__global__ void __launch_bounds__(kMpWarps * 32)
+    k_merge_publish(const Key *g_key, int *knn_ids, float *knn_dists, const int *dirty,
+                    uint32_t *pub_idx, float *pub_dist, int k, int n, int *edge_counter,
+                    int *report_flag) {
+  const int lane = threadIdx.x & 31;
+  const int row = blockIdx.x * kMpWarps + (threadIdx.x >> 5);
+  if (row >= n) return;
+  const unsigned full = 0xffffffffu, ks = k >= 32 ? full : (1u << k) - 1u;
   int *kl = knn_ids + (size_t)row * k;
   float *kd = knn_dists + (size_t)row * k;
-  for (int j = 0; j < k; ++j) {
-    lid[j] = kl[j];
-    ldv[j] = kd[j];
-  }
+  int le = lane < k ? kl[lane] : 0;
+  float lv = lane < k ? kd[lane] : 0.0f;
+  const Key key = g_key[(size_t)row * kListW + lane];
+  const float nd = key_dist(key);
+  const int nid = key_id(key);
+  auto listed_id = [](int e) { return e >= 0 ? e : -e - 1; };
+  const float tail0 = __shfl_sync(full, lv, k - 1);
+  // entries up to the first empty or placeholder one
+  const unsigned end = __ballot_sync(full, nd == FLT_MAX);
+  const bool cand = (end ? lane < __ffs(end) - 1 : true) && nid >= 0 && nid < n && nid != row &&
+                    !(nd > tail0);
+  bool dup = false;
+  for (int q = 0; q < k; ++q) dup |= __shfl_sync(full, listed_id(le), q) == nid;
   int h = 0, edges = 0;
-  for (int j = 0; j < kListW; ++j) {
-    const Key key = g_key[(size_t)row * kListW + j];
-    const float nd = key_dist(key);
-    if (nd == FLT_MAX) break;
-    const int nid = key_id(key);
-    if (nid < 0 || nid >= n || nid == row) continue;
-    // insert_to_ordered_list (update_kernel.cuh:87-120)
-    if (nd > ldv[k - 1]) continue;
-    int idx = k;
-    bool dup = false;
-    for (int q = 0; q < k; ++q) {
-      const int e = lid[q];
-      if ((e >= 0 ? e : -e - 1) == nid) {
-        dup = true;
-        break;
-      }
-      if (idx == k && ldv[q] > nd) idx = q;
+  unsigned todo = __ballot_sync(full, cand);
+  if (!__any_sync(full, cand && !dup)) todo = 0;
+  while (todo) {
+    const int j = __ffs(todo) - 1;
+    todo &= todo - 1u;
+    const float d = __shfl_sync(full, nd, j);
+    const int id = __shfl_sync(full, nid, j);
+    if (d > __shfl_sync(full, lv, k - 1)) continue;
+    if (__ballot_sync(full, listed_id(le) == id) & ks) continue;
+    const unsigned above = __ballot_sync(full, lv > d) & ks;
+    if (!above) continue;
+    const int idx = __ffs(above) - 1;
+    const int pe = __shfl_up_sync(full, le, 1);
+    const float pv = __shfl_up_sync(full, lv, 1);
+    if (lane > idx) {
+      le = pe;
+      lv = pv;
+    } else if (lane == idx) {
+      le = id;
+      lv = d;
     }
-    if (dup || idx == k) continue;
-    for (int q = k - 1; q > idx; --q) {
-      lid[q] = lid[q - 1];
-      ldv[q] = ldv[q - 1];
-    }
-    lid[idx] = nid;
-    ldv[idx] = nd;
     h = 2;
     ++edges;
   }
-  const int dd = dirty[row];
-  if (dd > h) h = dd;
+  h = max(h, dirty[row]);
   int report = 0;
   if (h >= 1) {
     // sort_lists: ascending (dist, id_with_flag)
-    for (int a = 1; a < k; ++a) {
-      const int e = lid[a];
-      const float dv = ldv[a];
-      int b = a;
-      while (b > 0 && (ldv[b - 1] > dv || (ldv[b - 1] == dv && lid[b - 1] > e))) {
-        lid[b] = lid[b - 1];
-        ldv[b] = ldv[b - 1];
-        --b;
-      }
-      lid[b] = e;
-      ldv[b] = dv;
+    int rank = 0;
+    for (int q = 0; q < k; ++q) {
+      const float v = __shfl_sync(full, lv, q);
+      const int e = __shfl_sync(full, le, q);
+      rank += v < lv || (v == lv && (e < le || (e == le && q < lane)));
     }
-    for (int j = 0; j < k; ++j) {
-      kl[j] = lid[j];
-      kd[j] = ldv[j];
+    int from = 0;
+    for (int q = 0; q < k; ++q)
+      if (__shfl_sync(full, rank, q) == lane) from = q;
+    le = __shfl_sync(full, le, from);
+    lv = __shfl_sync(full, lv, from);
+    if (lane < k) {
+      kl[lane] = le;
+      kd[lane] = lv;
     }
     if (h == 2) {
-      bool valid_row = false;
-      for (int j = 0; j < k; ++j) {
-        const int e = lid[j];
-        const int id = e >= 0 ? e : -e - 1;
-        const bool valid = id >= 0 && id < n && id != row;
-        valid_row |= valid;
-        pub_idx[(size_t)row * (k + 1) + j] = valid ? (uint32_t)id : kPubIdxSentinel;
-        pub_dist[(size_t)row * (k + 1) + j] = valid ? ldv[j] : FLT_MAX;
+      const int id = listed_id(le);
+      const bool valid = lane < k && id >= 0 && id < n && id != row;
+      if (lane < k) {
+        pub_idx[(size_t)row * (k + 1) + lane] = valid ? (uint32_t)id : kPubIdxSentinel;
+        pub_dist[(size_t)row * (k + 1) + lane] = valid ? lv : FLT_MAX;
       }
-      if (valid_row) {
-        pub_idx[(size_t)row * (k + 1) + k] = 1u;
+      if (__any_sync(full, valid)) {
+        if (lane == 0) pub_idx[(size_t)row * (k + 1) + k] = 1u;
         report = 1;
       }
     }
   }
-  report_flag[row] = report;
-  if (edges) atomicAdd(edge_counter, edges);
+  if (lane == 0) {
+    report_flag[row] = report;
+    if (edges) atomicAdd(edge_counter, edges);
   }
 }
 
@@ -482,38 +564,30 @@ inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace
 
-void launch_sample_graph(const DevState &st, const UpdScratch &u, const int *batch,
-                         int nb, int n, cudaStream_t s) {
-  if (nb <= 0) return;
-  k_sample_graph<<<cdiv(nb, 128), 128, 0, s>>>(st.knn_ids, st.bloom, batch, nb, n,
-                                                st.k, u.fwd_new, u.fwd_old, u.sizes);
-  note_launch();
-}
-
-void build_reverse(const DevState &st, const UpdScratch &u, const int *batch, int nb,
-                   int n, int which, int *tmp, cudaStream_t s) {
+void launch_join_nodes(const DevState &st, const UpdScratch &u, const int *batch, int nb, int n,
+                       int *small_nodes, int *large_nodes, int *counters, cudaStream_t s) {
   if (nb <= 0 || n <= 0) return;
-  const int *fwd = which ? u.fwd_old : u.fwd_new;
-  int *rev = which ? u.rev_old : u.rev_new;
-  cudaMemsetAsync(u.cnt, 0, sizeof(int) * (size_t)n, s);
-  cudaMemsetAsync(u.fill, 0, sizeof(int) * (size_t)n, s);
-  const int work = nb * kSamples;
-  k_rev_count<<<cdiv(work, 256), 256, 0, s>>>(batch, nb, n, fwd, u.sizes, which, u.cnt);
-  note_launch();
-  exclusive_scan(u.cnt, u.off, n, tmp, s);
-  k_rev_fill<<<cdiv(work, 256), 256, 0, s>>>(batch, nb, n, fwd, u.sizes, which, u.off,
-                                            u.fill, u.csr);
-  note_launch();
-  k_rev_finalize<<<cdiv(n, 128), 128, 0, s>>>(n, u.cnt, u.off, u.csr, rev, u.sizes,
-                                              which);
-  note_launch();
-  (void)st;
+  // new sources are counted in u.cnt, old ones in u.fill; the positions of the
+  // samples wait in the batch rows' reverse lists until k_join_lists writes them
+  int *off_new = u.off, *off_old = u.hflag;
+  k_update_reset<<<cdiv(std::max(n, kUpdCounters), 256), 256, 0, s>>>(n, u.sizes, st.dirty, u.cnt, u.fill,
+                                                                      counters, kUpdCounters);
+  k_sample_graph<<<cdiv(nb, kSgWarps), kSgWarps * 32, 0, s>>>(
+      st.knn_ids, st.bloom, batch, nb, n, st.k, u.fwd_new, u.fwd_old, u.rev_new, u.rev_old, u.cnt, u.fill,
+      u.sizes);
+  k_rev_segments<<<cdiv(n, 256), 256, 0, s>>>(n, u.cnt, u.fill, off_new, off_old, counters + kUpdSources);
+  k_rev_place<<<cdiv((long)nb * kSamples, 256), 256, 0, s>>>(batch, nb, u.fwd_new, u.fwd_old, u.rev_new,
+                                                            u.rev_old, u.sizes, off_new, off_old, u.csr);
+  k_join_lists<<<cdiv(n, kListWarps), kListWarps * 32, 0, s>>>(
+      n, u.fwd_new, u.fwd_old, u.rev_new, u.rev_old, u.cnt, u.fill, off_new, off_old, u.csr, u.sizes,
+      small_nodes, large_nodes, counters + kUpdNodes);
+  note_launch(5);
 }
 
-void launch_local_join(const DevState &st, const UpdScratch &u, const int *join_nodes,
-                       const int *n_join_dev, int n_join_max, int n, cudaStream_t s) {
-  if (n_join_max <= 0) return;
-  const size_t smem = sizeof(LJSmem);
+void launch_local_join(const DevState &st, const UpdScratch &u, const int *small_nodes,
+                       const int *large_nodes, int *counters, int n, cudaStream_t s) {
+  if (n <= 0) return;
+  const size_t smem = sizeof(JoinSmem);
   // per device, once (sessions on several host threads may launch at once)
   static std::mutex mu;
   static int ctas[32] = {0};
@@ -526,34 +600,24 @@ void launch_local_join(const DevState &st, const UpdScratch &u, const int *join_
       cudaFuncSetAttribute(k_local_join, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       int sms = 0, per_sm = 0;
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_local_join, kLJThreads, smem);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_local_join, kJoinWarps * 32, smem);
       ctas[dev] = std::max(1, sms * std::max(per_sm, 1));
     }
     grid_ctas = ctas[dev];
   }
-
-  const int grid = std::min(n_join_max, grid_ctas > 0 ? grid_ctas : 1024);
-  k_local_join<<<grid, kLJThreads, smem, s>>>(
-      join_nodes, n_join_dev, u.fwd_new, u.fwd_old, u.rev_new, u.rev_old, u.sizes, st.X,
-      st.norms, st.ld, st.d, n, st.k, st.g_key, st.locks, st.dirty, st.err, st.stat);
+  const int grid = std::min(n, grid_ctas > 0 ? grid_ctas : 1024);
+  const JoinArgs g{u.fwd_new, u.fwd_old, u.rev_new, u.rev_old, u.sizes, st.X, st.norms, st.ld, st.k,
+                   st.g_key, st.locks, st.dirty, st.err, st.stat};
+  k_local_join<<<grid, kJoinWarps * 32, smem, s>>>(small_nodes, large_nodes, counters + kUpdNodes, g);
   note_launch();
 }
 
-void launch_join_flags(const UpdScratch &u, int n, int *flag, cudaStream_t s) {
+void launch_merge_publish(const DevState &st, int n, int *edge_counter, int *report_flag, cudaStream_t s) {
   if (n <= 0) return;
-  k_join_flags<<<cdiv(n, 256), 256, 0, s>>>(u.sizes, n, flag);
+  k_merge_publish<<<cdiv(n, kMpWarps), kMpWarps * 32, 0, s>>>(st.g_key, st.knn_ids, st.knn_dists, st.dirty,
+                                                             st.pub_idx, st.pub_dist, st.k, n, edge_counter,
+                                                             report_flag);
   note_launch();
-}
-
-void launch_merge_publish(const DevState &st, const UpdScratch &u, const int *rows,
-                          const int *n_rows_dev, int n_rows_max, int n,
-                          int *edge_counter, int *report_flag, cudaStream_t s) {
-  if (n_rows_max <= 0) return;
-  k_merge_publish<<<std::min(cdiv(n_rows_max, 128), 2048), 128, 0, s>>>(
-      rows, n_rows_dev, st.g_key, st.knn_ids, st.knn_dists, st.dirty,
-      st.pub_idx, st.pub_dist, st.k, n, edge_counter, report_flag);
-  note_launch();
-  (void)u;
 }
 
 }  // namespace gm
