@@ -91,6 +91,7 @@ _SIGS = [
     ("gm_debug_copy", C.c_int, [_P, C.c_int, _P, C.c_uint64]),
     ("gm_debug_keep_tiles", C.c_int, [_P, C.c_int]),
     ("gm_debug_pre_capacity", C.c_int, [_P, C.c_int]),
+    ("gm_debug_join_words", C.c_int, [_P, C.c_uint64]),
     ("gm_debug_scalars", C.c_int, [_P, C.POINTER(C.c_int64), C.c_int]),
     ("gm_debug_update_queue", C.c_int, [_P, _P, C.c_uint64, C.POINTER(C.c_uint64)]),
     ("gm_op_fuzzy_schedule", C.c_int,
@@ -206,6 +207,9 @@ class Session:
 
     def pre_capacity(self, cap: int) -> None:
         check(self._lib.gm_debug_pre_capacity(self._h, int(cap)))
+
+    def join_words(self, words: int) -> None:
+        check(self._lib.gm_debug_join_words(self._h, int(words)))
 
     def set_stats(self, on: bool) -> None:
         check(self._lib.gm_set_stats(self._h, 1 if on else 0))

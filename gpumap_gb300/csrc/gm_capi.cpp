@@ -284,6 +284,11 @@ int gm_debug_pre_capacity(gm_session *s, int cap) {
   return guarded([&] { s->impl->set_pre_cap(cap); });
 }
 
+int gm_debug_join_words(gm_session *s, uint64_t words) {
+  if (!s) return fail(GM_ERR_INVALID, "null session");
+  return guarded([&] { s->impl->set_join_part((size_t)words); });
+}
+
 int gm_debug_scalars(const gm_session *s, int64_t *out, int n) {
   if (!s || !out) return fail(GM_ERR_INVALID, "null argument");
   s->impl->debug_scalars(out, n);

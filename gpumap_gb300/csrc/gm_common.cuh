@@ -1,6 +1,6 @@
 // Shared device-side definitions for the GB300 progressive-UMAP engine:
 // list widths, status bits, the counter-based RNG, bit-reproducible float
-// math, the bounded per-node lock and the warp-cooperative 32-list merge.
+// math and the warp-cooperative 32-list insertion.
 //
 // Every floating-point expression whose result feeds a comparison on the
 // k-NN path is written with explicit round-to-nearest intrinsics and the
@@ -26,12 +26,8 @@ constexpr int kIdSentinel = 0x7fffffff;       // INT_MAX: empty list slot
 constexpr uint32_t kPubIdxSentinel = 0xffffffffu;
 
 // Device error bits, OR-ed into the session's error word.
-constexpr unsigned kDevErrLock = 1u;  // a per-node lock wait ran out
-constexpr unsigned kDevErrSpin = 2u;  // another bounded wait ran out
+constexpr unsigned kDevErrSpin = 2u;  // a bounded wait ran out
 constexpr unsigned kDevErrOverflow = 4u;  // a scratch pool would have overflowed (work skipped)
-
-// Lock wait bound: about a second at the longest back-off.
-constexpr uint32_t kLockSpinLimit = 1u << 20;
 
 #define GM_HD __host__ __device__ __forceinline__
 #define GM_D __device__ __forceinline__
@@ -184,40 +180,6 @@ GM_HD bool item_less(float da, int ia, float db, int ib) {
 }
 
 // ---------------------------------------------------------------------------
-// Bounded per-node lock.  Lane 0 spins with back-off; after kLockSpinLimit
-// failed attempts it records kDevErrLock and reports failure.
-// ---------------------------------------------------------------------------
-GM_D bool warp_lock(int *lock, unsigned *err) {
-  const int lane = threadIdx.x & 31;
-  int ok = 0;
-  if (lane == 0) {
-    for (uint32_t it = 0; it < kLockSpinLimit; ++it) {
-      if (atomicCAS(lock, 0, 1) == 0) {
-        ok = 1;
-        break;
-      }
-      __nanosleep(it < 64u ? 32u : 256u);
-    }
-    if (!ok) atomicOr(err, kDevErrLock);
-  }
-  // acquire: every lane is ordered after lane 0's successful CAS
-  __syncwarp();
-  ok = __shfl_sync(0xffffffffu, ok, 0);
-  __threadfence();
-  return ok != 0;
-}
-
-GM_D void warp_unlock(int *lock) {
-  // release: all lanes' list stores precede lane 0's fence and unlock
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0) {
-    __threadfence();
-    atomicExch(lock, 0);
-  }
-  __syncwarp();
-}
-
-// ---------------------------------------------------------------------------
 // Working-list entries are 64-bit keys: high word = bits of the non-negative
 // float distance, low word = id.  Unsigned key order is the lexicographic
 // (dist, id) order, and an 8-byte load of one slot is never torn.
@@ -267,22 +229,6 @@ GM_D int warp_insert(Key &mine, Key ck) {
   if (lane > pos) mine = prev;
   else if (lane == pos) mine = ck;
   return pos;
-}
-
-// Offers m candidate keys to node t's list under t's lock.  Returns the
-// smallest insert position (kListW if nothing changed, -1 if the lock wait
-// ran out).
-GM_D int warp_locked_merge(int t, const Key *cands, int m, Key *g_key, int *locks,
-                           unsigned *err) {
-  const int lane = threadIdx.x & 31;
-  if (!warp_lock(&locks[t], err)) return -1;
-  Key *row = g_key + (size_t)t * kListW;
-  Key mine = __ldcg(&row[lane]);
-  int minpos = kListW;
-  for (int q = 0; q < m; ++q) minpos = min(minpos, warp_insert(mine, cands[q]));
-  if (minpos < kListW) __stcg(&row[lane], mine);
-  warp_unlock(&locks[t]);
-  return minpos;
 }
 
 }  // namespace gm

@@ -102,7 +102,6 @@ Session::Session(const gm_params &p) : p_(p) {
     st_.norms = (float *)dalloc(Nm * sizeof(float));
     st_.snorms = (float *)dalloc(Nm * sizeof(float));
     st_.g_key = (unsigned long long *)dalloc(Nm * kListW * sizeof(unsigned long long));
-    st_.locks = (int *)dalloc(Nm * sizeof(int));
     st_.dirty = (int *)dalloc(Nm * sizeof(int));
     st_.knn_ids = (int *)dalloc(Nm * k * sizeof(int));
     st_.knn_dists = (float *)dalloc(Nm * k * sizeof(float));
@@ -224,7 +223,6 @@ Session::Session(const gm_params &p) : p_(p) {
   ck(cudaMemsetAsync(st_.norms, 0, Nm * sizeof(float), s), "memset");
   ck(cudaMemsetAsync(st_.snorms, 0, Nm * sizeof(float), s), "memset");
   fill_u64(st_.g_key, kEmptyKey, Nm * kListW, s);
-  ck(cudaMemsetAsync(st_.locks, 0, Nm * sizeof(int), s), "memset");
   ck(cudaMemsetAsync(st_.dirty, 0, Nm * sizeof(int), s), "memset");
   fill_u32(st_.knn_ids, (uint32_t)kIdSentinel, Nm * k, s);
   fill_u32(st_.knn_dists, kFltMaxBits, Nm * k, s);
@@ -301,6 +299,7 @@ Session::~Session() {
   }
   for (void *q : allocs_) cudaFree(q);
   free_cand();
+  if (join_pool_) cudaFree(join_pool_);
   free_embed(es_);
   free_embed(es_alt_);
   if (h_pin_) cudaFreeHost(h_pin_);
@@ -385,6 +384,26 @@ void Session::ensure_cand(size_t rows) {
   cand_rows_ = r;
 }
 
+// The join pool: words for every block of a round, up to kJoinPartWords.
+void Session::ensure_join(size_t words) {
+  const size_t w = join_part(words);
+  if (w <= join_words_) return;
+  sync();
+  if (join_pool_) cudaFree(join_pool_);
+  join_pool_ = nullptr;
+  join_words_ = 0;
+  ck(cudaMalloc(&join_pool_, (w + kJoinSlackWords) * sizeof(int)), "cudaMalloc join");
+  join_words_ = w;
+}
+
+void Session::set_join_part(size_t words) {
+  drain();
+  if (join_pool_) cudaFree(join_pool_);
+  join_pool_ = nullptr;
+  join_words_ = 0;
+  join_part_max_ = std::max<size_t>(2, std::min(words, kJoinPartWords) & ~(size_t)1);
+}
+
 void Session::set_pre_cap(int cap) {
   drain();
   xs_.pre_cap = std::max(0, std::min(cap, pre_cap_alloc_));
@@ -408,13 +427,19 @@ void Session::set_keep_tile(bool on) {
 size_t Session::device_bytes() const {
   size_t b = fixed_bytes_;
   b += cand_bytes(cand_rows_, st_.k);
+  if (join_pool_) b += (join_words_ + kJoinSlackWords) * sizeof(int);
   for (const EmbedScratch *e : {&es_, &es_alt_})
     if (e->coo_row) b += e->cap_coo * 9 * 4 + (compact_tmp_ints((int)e->cap_coo) + 64) * sizeof(int);
   return b;
 }
 
-size_t Session::growth_bytes(uint32_t n_ins, uint32_t n_emb) const {
+size_t Session::growth_bytes(uint32_t n_ins, uint32_t n_upd, uint32_t n_emb) const {
   size_t g = 0;
+  if (n_upd > 0 && !upd_done_) {
+    const size_t rows = std::min<size_t>(n_upd, n_inserted_ + n_ins);
+    const size_t w = join_part(join_pool_words((int)rows, st_.k));
+    if (w > join_words_) g += (w + kJoinSlackWords) * sizeof(int);
+  }
   if (p_.precision == 0 && n_ins > cand_rows_) {
     const size_t r = std::max<size_t>(n_ins, 1024);
     g += cand_bytes(r, st_.k);
@@ -817,18 +842,29 @@ size_t Session::update_round(std::vector<uint32_t> &batch, std::vector<uint32_t>
   std::memcpy(h_pin_, batch.data(), (size_t)nb * sizeof(uint32_t));
   ck(cudaMemcpyAsync(d_batch_, h_pin_, (size_t)nb * sizeof(int), cudaMemcpyHostToDevice, s),
      "batch");
-  int *counters = d_cnt_ + 1;  // after the report count
+  int *counters = d_cnt_ + 2;  // after the report count (8-byte aligned)
+  const size_t bound = join_pool_words(nb, st_.k);
+  ensure_join(bound);
   bloom_clean_ = false;
   launch_join_nodes(st_, us_, d_batch_, nb, n, d_rows_, d_rows2_, counters, s);
   timed_begin(0);
-  launch_local_join(st_, us_, d_rows_, d_rows2_, counters, n, s);
+  launch_local_join(st_, us_, d_rows_, d_rows2_, counters, join_pool_, join_words_, 0, n, s);
+  if (bound > join_words_) {
+    // the pool may not hold every block: as many passes as their words take
+    ck(cudaMemcpyAsync(h_pin_, counters + kUpdPool, sizeof(uint64_t), cudaMemcpyDeviceToHost, s), "words");
+    sync();
+    uint64_t words = 0;
+    std::memcpy(&words, h_pin_, sizeof(words));
+    for (int pass = 1; (uint64_t)pass * join_words_ < words; ++pass)
+      launch_local_join(st_, us_, d_rows_, d_rows2_, counters, join_pool_, join_words_, pass, n, s);
+  }
   timed_end(0);
   launch_merge_publish(st_, n, counters + kUpdEdges, us_.hflag, s);
   compact_flags(us_.hflag, n, -1, d_rows_, d_cnt_, d_tmp_, s);
-  ck(cudaMemcpyAsync(h_pin_, d_cnt_, 2 * sizeof(int), cudaMemcpyDeviceToHost, s), "counts");
+  ck(cudaMemcpyAsync(h_pin_, d_cnt_, 3 * sizeof(int), cudaMemcpyDeviceToHost, s), "counts");
   sync();
   const int na = (int)h_pin_[0];
-  const int edges = (int)h_pin_[1 + kUpdEdges];
+  const int edges = (int)h_pin_[2 + kUpdEdges];
   if (na > 0) {
     ck(cudaMemcpyAsync(h_pin_, d_rows_, (size_t)na * sizeof(int), cudaMemcpyDeviceToHost, s),
        "affected");

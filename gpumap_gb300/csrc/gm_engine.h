@@ -74,10 +74,12 @@ class Session {
   // device memory the session holds now, and what a run with these op
   // counts could add (its scratch grows on demand)
   size_t device_bytes() const;
-  size_t growth_bytes(uint32_t n_ins, uint32_t n_emb) const;
+  size_t growth_bytes(uint32_t n_ins, uint32_t n_upd, uint32_t n_emb) const;
   // keep each insertion block's approximate distance tile (tests)
   void set_keep_tile(bool on);
   void set_pre_cap(int cap);
+  // words of the join pool a pass covers, at most (tests)
+  void set_join_part(size_t words);
   void drain();
   // consumer waits (on the device) for everything queued on this session
   void order_after(cudaStream_t consumer) const;
@@ -99,6 +101,10 @@ class Session {
   void check_device_error(const char *phase);
   void ensure_cand(size_t rows);
   void free_cand();
+  void ensure_join(size_t words);
+  size_t join_part(size_t words) const {
+    return std::min(std::max<size_t>((words + 1) & ~(size_t)1, 4096), join_part_max_);
+  }
   void ensure_embed(EmbedScratch &e, size_t nb);
   void free_embed(EmbedScratch &e);
   void sync_embed_streams();
@@ -148,6 +154,8 @@ class Session {
 
   // insertion candidates (grow on demand)
   CandScratch cs_;
+  int *join_pool_ = nullptr;  // join blocks of an update round (grows on demand)
+  size_t join_words_ = 0, join_part_max_ = kJoinPartWords;
   size_t cand_rows_ = 0;
 
   // device row lists / counters

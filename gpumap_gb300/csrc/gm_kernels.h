@@ -7,6 +7,8 @@
 #include <functional>
 #include <cuda_runtime.h>
 
+#include "gm_common.cuh"
+
 namespace gm {
 
 // Resident session state in HBM (all device pointers, capacity n_cap rows).
@@ -20,7 +22,6 @@ struct DevState {
   float *norms = nullptr;     // n_cap squared L2 norms
   float *snorms = nullptr;    // n_cap sqrt of norms rounded up (exact-mode bounds)
   unsigned long long *g_key = nullptr;  // n_cap x 32 working lists, (dist bits << 32 | id)
-  int *locks = nullptr;       // n_cap per-node locks (0 = free)
   int *dirty = nullptr;       // n_cap device dirty flags (0/1/2)
   int *knn_ids = nullptr;     // n_cap x k authoritative list, old flag = sign
   float *knn_dists = nullptr; // n_cap x k
@@ -155,16 +156,27 @@ void launch_exact_screen(const DevState &st, int row0, int blk0, int nrows, int 
                          const ExactScreen &x, long ldD, int sms, cudaStream_t s);
 
 // ---- update (gm_kernels_update.cu) ----
-// Counters of an update round (device ints): edges changed, sources, then
-// small and large join nodes and their tickets.
-constexpr int kUpdEdges = 0, kUpdSources = 1, kUpdNodes = 2, kUpdCounters = 6;
+// Counters of an update round (device ints): edges changed, sources, small
+// and large join nodes and their tickets, words of all join blocks (64 bits,
+// 8-byte aligned).
+constexpr int kUpdEdges = 0, kUpdSources = 1, kUpdNodes = 2, kUpdPool = 6, kUpdCounters = 8;
+// Words of the join pool's part that one pass covers, at most, and the slack
+// past it (a block may start anywhere in the part).
+constexpr size_t kJoinPartWords = (size_t)32 << 20;
+constexpr size_t kJoinSlackWords = 2 * kJoinMax * (kJoinMax + 3);
+// Upper bound on the words of all join blocks of a round over nb batch rows.
+size_t join_pool_words(int nb, int k);
 // Samples the batch rows' lists and builds every row's join lists; clears
 // the round's per-row state and counters first.  Nodes with a pair to form
 // land in small_nodes (at most 32 members) and large_nodes (n ids each).
 void launch_join_nodes(const DevState &st, const UpdScratch &u, const int *batch, int nb, int n,
                        int *small_nodes, int *large_nodes, int *counters, cudaStream_t s);
+// Distances of the nodes whose block starts in words [pass * part_words,
+// +part_words), and the merge of their offers; pool: part_words +
+// kJoinSlackWords words.
 void launch_local_join(const DevState &st, const UpdScratch &u, const int *small_nodes,
-                       const int *large_nodes, int *counters, int n, cudaStream_t s);
+                       const int *large_nodes, int *counters, int *pool, size_t part_words, int pass,
+                       int n, cudaStream_t s);
 // Merges working lists into the authoritative lists, re-sorts them, publishes
 // changed rows and flags rows to report.
 void launch_merge_publish(const DevState &st, int n, int *edge_counter, int *report_flag,

@@ -165,8 +165,12 @@ __global__ void k_rev_place(const int *batch, int nb, const int *fwd_new, const 
 // reverse samples replace the positions in rev_*, sizes becomes (forward new,
 // kept reverse new, forward old, kept reverse old), and rows with a pair to
 // form are appended to the small (at most 32 members) or the large node list
-// (any order).
+// and get a place in the pool for their block (any order; its words in
+// off_new / off_old, low and high half).
 constexpr int kListWarps = 8;
+// Words of a node's block: per member its chain entry (next, node) and id,
+// then the N x (N ++ O) tile; a whole number of chain entries.
+GM_D int join_block_words(int nN, int nC) { return (nC * (nN + 3) + 1) & ~1; }
 GM_D int warp_smallest(const int *src, int c) {
   // lane l: the l-th smallest of c distinct ids (INT_MAX past the end)
   const int lane = threadIdx.x & 31;
@@ -190,14 +194,16 @@ GM_D int warp_smallest(const int *src, int c) {
 }
 __global__ void __launch_bounds__(kListWarps * 32)
     k_join_lists(int n, const int *fwd_new, const int *fwd_old, int *rev_new, int *rev_old,
-                 const int *cnt_new, const int *cnt_old, const int *off_new, const int *off_old,
-                 const int *src, int4 *sizes, int *small_nodes, int *large_nodes, int *counts) {
-  __shared__ int s_cls[kListWarps];
+                 const int *cnt_new, const int *cnt_old, int *off_new, int *off_old,
+                 const int *src, int4 *sizes, int *small_nodes, int *large_nodes, int *counts,
+                 unsigned long long *pool_words) {
+  __shared__ int s_cls[kListWarps], s_words[kListWarps];
   __shared__ int s_base[2];
+  __shared__ unsigned long long s_pool;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int j = blockIdx.x * kListWarps + warp;
   const unsigned full = 0xffffffffu;
-  int cls = 0;
+  int cls = 0, words = 0;
   if (j < n) {
     const int4 sz = sizes[j];
     const int cn = cnt_new[j];
@@ -218,43 +224,67 @@ __global__ void __launch_bounds__(kListWarps * 32)
       if (lane == 0) sizes[j] = make_int4(sz.x, rn, sz.z, ro);
       const int m = sz.x + rn + sz.z + ro;
       cls = m < 2 ? 0 : m <= 32 ? 1 : 2;
+      words = cls ? join_block_words(sz.x + rn, m) : 0;
     }
   }
-  if (lane == 0) s_cls[warp] = cls;
+  if (lane == 0) {
+    s_cls[warp] = cls;
+    s_words[warp] = words;
+  }
   __syncthreads();
   if (threadIdx.x < 2) {
     int c = 0;
     for (int w = 0; w < kListWarps; ++w) c += s_cls[w] == (int)threadIdx.x + 1;
     s_base[threadIdx.x] = c ? atomicAdd(&counts[threadIdx.x], c) : 0;
+  } else if (threadIdx.x == 2) {
+    int c = 0;
+    for (int w = 0; w < kListWarps; ++w) c += s_words[w];
+    s_pool = c ? atomicAdd(pool_words, (unsigned long long)c) : 0ull;
   }
   __syncthreads();
   if (lane == 0 && cls) {
     int at = s_base[cls - 1];
-    for (int w = 0; w < warp; ++w) at += s_cls[w] == cls;
+    unsigned long long pos = s_pool;
+    for (int w = 0; w < warp; ++w) {
+      at += s_cls[w] == cls;
+      pos += (unsigned long long)s_words[w];
+    }
     (cls == 1 ? small_nodes : large_nodes)[at] = j;
+    off_new[j] = (int)(uint32_t)pos;
+    off_old[j] = (int)(pos >> 32);
   }
 }
 
-// Local join of a node's lists N and O.  Distances of N x (N ++ O) are FP32,
-// a sequential fma chain per pair; every pair is then offered to both
-// endpoints' lists: N members get all other N and O members, O members get
-// the N members (reference: local_join_kernel, update_kernel.cuh:377-687).
+// Local join of a node's lists N and O, in two kernels (reference:
+// local_join_kernel, update_kernel.cuh:377-687).
 //
-// W warps work on a node: the CTA's four on a large one, a single warp on a
-// small one (at most 32 members), the four warps of a CTA on different nodes.
-// The members' rows come 32 features at a time by 16-byte cp.async into a ring
-// of kJoinRing slots (36 words a row: conflict-free 16-byte reads), each row
-// once; member row r of N is on warp r % W, member column c on lane c % 32, so
-// a thread's products take its own columns and broadcast rows, and its sums
-// stay in registers.  The distance tile then goes over the ring, and each
-// warp takes every W-th member as a target: its list (read one target ahead)
-// decides which offers can act, and only then its lock is taken.
+// k_join_tiles forms the distances of N x (N ++ O), FP32, a sequential fma
+// chain per pair, and stores the tile in the node's block of the pool.  W
+// warps work on a node: the CTA's four on a large one, a single warp on a small
+// one (at most 32 members), the four warps of a CTA on different nodes.  The
+// members' rows come 32 features at a time by 16-byte cp.async into a ring of
+// kJoinRing slots (36 words a row: conflict-free 16-byte reads), each row once;
+// member row r of N is on warp r % W, member column c on lane c % 32, so a
+// thread's products take its own columns and broadcast rows, and its sums stay
+// in registers until the tile goes over the ring.  A member whose list some
+// offer can change then goes on one of its row's 32 chains (heads[row * 32 +
+// node % 32]); a node without one leaves its block unwritten.
 //
-// Bound by latency: rows from L2, list snapshots and the lock's round trips
-// (about 2.5 us a merge), so what counts is the number of nodes in flight:
-// 16 warps an SM on as many small nodes, where a CTA of eight warps per node
-// had three.  45 rounds of 2,000 rows over 20k x 784 (k = 15): 28.4 -> 12.0 ms;
-// 10 rounds of 10,000 rows over 100k x 128 (k = 30): 12.8 -> 6.1 ms.
+// k_join_merge, a warp per row, walks the row's chains, 32 memberships at a
+// time, and offers it the other side of each tile: as a member of N all other
+// members, as a member of O the members of N.
+//
+// A round whose blocks do not fit the pool takes several passes, each over the
+// nodes whose block starts in its part of the (virtual) pool.
+//
+// Bound by latency (rows from L2, then list and tile reads), so what counts is
+// the number of nodes in flight: 16 an SM here, three with a CTA of eight warps
+// per node.  Merging every (node, member) under the member's lock instead, as
+// the kernel before did, cost most of its time (about 2.5 us a merge, in turn
+// for a row in many nodes: 250 of 272 us at 600 rows).  45 rounds of 2,000 rows
+// over 20k x 784 (k = 15): 28.4 ms with a CTA per node, 12.0 with a warp per
+// small node and locks, 9.5 now; 10 rounds of 10,000 rows over 100k x 128
+// (k = 30): 12.8, 6.1, 5.6 ms.
 constexpr int kJoinWarps = 4;
 constexpr int kJoinRing = 3;
 constexpr int kJoinLd = 36;
@@ -263,13 +293,23 @@ constexpr int kJoinCols = 2 * kJoinMax;  // members of a large node
 struct JoinArgs {
   const int *fwd_new, *fwd_old, *rev_new, *rev_old;
   const int4 *sizes;
+  const int *pos_lo, *pos_hi;   // a node's block: its first word, low and high half
+  int *pool;                    // this pass's part, from word pass * part_words on
+  unsigned long long part_words;
+  int pass;
+  int *heads;                   // n_cap x 32 chain heads (-1: none)
+  const Key *g_key;
   const float *X, *norms;
-  int ld, k;
-  Key *g_key;
-  int *locks, *dirty;
-  unsigned *err;
+  int ld;
   unsigned long long *stat;
 };
+// The node's first word in this pass's pool; false if it belongs to another.
+GM_D bool join_block(const JoinArgs &g, int u, int &at) {
+  const unsigned long long pos = ((unsigned long long)(uint32_t)g.pos_hi[u] << 32) | (uint32_t)g.pos_lo[u];
+  const unsigned long long from = (unsigned long long)g.pass * g.part_words;
+  at = (int)(pos - from);
+  return pos >= from && pos - from < g.part_words;
+}
 
 template <int W>
 GM_D void join_sync() {
@@ -310,6 +350,8 @@ GM_D void join_node(int u, const JoinArgs &g, float *ring, int *cid, float *nrm)
   constexpr int kGroups = W == 1 ? 1 : kJoinCols / 32;
   constexpr int kMine = W == 1 ? 32 : kJoinMax / W;  // rows of N per warp
   constexpr int kLdD = kRows + 1;
+  int block;
+  if (!join_block(g, u, block)) return;
   const int lane = threadIdx.x & 31, w = W == 1 ? 0 : (int)(threadIdx.x >> 5);
   const int t = W == 1 ? lane : (int)threadIdx.x;
   const int4 sz = g.sizes[u];
@@ -361,7 +403,6 @@ GM_D void join_node(int u, const JoinArgs &g, float *ring, int *cid, float *nrm)
     else if (nC <= 96) join_products<W, (W == 1 ? 1 : 3)>(slot, nq, nr, w, lane, acc);
     else join_products<W, kGroups>(slot, nq, nr, w, lane, acc);
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
   join_sync<W>();  // every product is done before the tile overwrites the ring
   float *D = ring;
 #pragma unroll
@@ -373,24 +414,26 @@ GM_D void join_node(int u, const JoinArgs &g, float *ring, int *cid, float *nrm)
     }
   join_sync<W>();
 
-  // ---- offers, one target per warp at a time
+  // members that an offer acts on (below the last entry of the member's list
+  // and not listed already), one member per warp at a time, the next one's
+  // list on its way
   const unsigned full = 0xffffffffu;
-  Key snap = w < nC ? __ldcg(&g.g_key[(size_t)cid[w] * kListW + lane]) : 0;
+  int2 *ent = reinterpret_cast<int2 *>(g.pool + block);
+  bool any = false;
+  Key next = w < nC ? g.g_key[(size_t)cid[w] * kListW + lane] : 0;
   for (int tt = w; tt < nC; tt += W) {
-    const Key list = snap;
-    if (tt + W < nC) snap = __ldcg(&g.g_key[(size_t)cid[tt + W] * kListW + lane]);
+    const Key list = next;
+    if (tt + W < nC) next = g.g_key[(size_t)cid[tt + W] * kListW + lane];
     const int idt = cid[tt];
     const bool in_n = tt < nN;
     const int ncand = in_n ? nC : nN;
-    auto key_of = [&](int c) {
-      if (c >= ncand || c == tt || cid[c] == idt) return ~(Key)0;
-      return make_key(in_n ? D[tt * kLdD + c] : D[c * kLdD + tt], cid[c]);
-    };
-    // an offer acts if it is below the last entry and not listed already
     const Key worst = __shfl_sync(full, list, kListW - 1);
     bool act = false;
     for (int c0 = 0; c0 < ncand && !act; c0 += 32) {
-      const Key ck = key_of(c0 + lane);
+      const int c = c0 + lane;
+      Key ck = ~(Key)0;
+      if (c < ncand && c != tt && cid[c] != idt)
+        ck = make_key(in_n ? D[tt * kLdD + c] : D[c * kLdD + tt], cid[c]);
       unsigned todo = __ballot_sync(full, ck < worst);
       while (todo && !act) {
         const Key x = __shfl_sync(full, ck, __ffs(todo) - 1);
@@ -398,26 +441,16 @@ GM_D void join_node(int u, const JoinArgs &g, float *ring, int *cid, float *nrm)
         act = !__any_sync(full, list == x);
       }
     }
-    if (!act) continue;
-    if (!warp_lock(&g.locks[idt], g.err)) continue;
-    Key *row = g.g_key + (size_t)idt * kListW;
-    Key mine = __ldcg(&row[lane]);
-    int minpos = kListW;
-    for (int c0 = 0; c0 < ncand; c0 += 32) {
-      const Key ck = key_of(c0 + lane);
-      unsigned todo = __ballot_sync(full, ck < __shfl_sync(full, mine, kListW - 1));
-      while (todo) {
-        const int s = __ffs(todo) - 1;
-        todo &= todo - 1u;
-        minpos = min(minpos, warp_insert(mine, __shfl_sync(full, ck, s)));
-      }
-    }
-    if (minpos < kListW) __stcg(&row[lane], mine);
-    warp_unlock(&g.locks[idt]);
-    if (lane == 0) {
-      if (minpos < kListW) atomicMax(&g.dirty[idt], minpos < g.k ? 2 : 1);
-      if (g.stat) atomicAdd(&g.stat[3], 1ull);
-    }
+    if (act && lane == 0)
+      ent[tt] = make_int2(atomicExch(&g.heads[(size_t)idt * 32 + (u & 31)], block / 2 + tt), u);
+    any |= act;
+  }
+  if (W == 1 ? any : __syncthreads_or(any)) {
+    int *ids = g.pool + block + 2 * nC;
+    float *out = reinterpret_cast<float *>(ids + nC);
+    for (int c = t; c < nC; c += 32 * W) ids[c] = cid[c];
+    for (int r = w; r < nN; r += W)
+      for (int c = lane; c < nC; c += 32) out[r * nC + c] = D[r * kLdD + c];
   }
   if (g.stat && t == 0) {
     atomicAdd(&g.stat[0], 1ull);
@@ -435,10 +468,10 @@ struct JoinSmem {
   float nrm[kJoinCols];
   int ticket;
 };
-static_assert(sizeof(float) * kJoinRing * kJoinCols * kJoinLd >= sizeof(float) * kJoinMax * (kJoinCols + 1),
-              "the tile of a large node does not fit its ring");
+static_assert(kJoinRing * kJoinCols * kJoinLd >= kJoinMax * (kJoinCols + 1) && kJoinRing * 32 * kJoinLd >= 32 * 33,
+              "a node's tile does not fit its ring");
 __global__ void __launch_bounds__(kJoinWarps * 32, 4)
-    k_local_join(const int *small_nodes, const int *large_nodes, int *counts, JoinArgs g) {
+    k_join_tiles(const int *small_nodes, const int *large_nodes, int *counts, JoinArgs g) {
   extern __shared__ __align__(16) unsigned char join_raw[];
   JoinSmem &S = *reinterpret_cast<JoinSmem *>(join_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -460,6 +493,74 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 4)
     join_node<1>(small_nodes[i], g, S.ring + (size_t)warp * kJoinRing * 32 * kJoinLd, S.cid + warp * 32,
                  S.nrm + warp * 32);
     __syncwarp();
+  }
+}
+
+constexpr int kJmWarps = 8;
+__global__ void __launch_bounds__(kJmWarps * 32)
+    k_join_merge(int n, JoinArgs g, Key *g_key, int *dirty, int k) {
+  const int lane = threadIdx.x & 31;
+  const int t = blockIdx.x * kJmWarps + (threadIdx.x >> 5);
+  if (t >= n) return;
+  const unsigned full = 0xffffffffu;
+  int e = g.heads[(size_t)t * 32 + lane];
+  if (!__any_sync(full, e >= 0)) return;
+  g.heads[(size_t)t * 32 + lane] = -1;
+  Key *row = g_key + (size_t)t * kListW;
+  Key mine = row[lane];
+  int minpos = kListW;
+  const int2 *entries = reinterpret_cast<const int2 *>(g.pool);
+  for (unsigned live; (live = __ballot_sync(full, e >= 0)) != 0u;) {
+    // lane: its membership's ids, tile, member number and list sizes
+    int ids = 0, c = 0, nN = 0, nC = 0;
+    if (e >= 0) {
+      const int2 ent = entries[e];
+      int block;
+      join_block(g, ent.y, block);
+      const int4 sz = g.sizes[ent.y];
+      nN = sz.x + sz.y;
+      nC = nN + sz.z + sz.w;
+      c = e - block / 2;
+      ids = block + 2 * nC;
+      e = ent.x;
+    }
+    // candidate c0 + lane of membership m (all ones: none)
+    auto key_of = [&](int m, int c0) {
+      const int mi = __shfl_sync(full, ids, m), mc = __shfl_sync(full, c, m);
+      const int mN = __shfl_sync(full, nN, m), mC = __shfl_sync(full, nC, m);
+      const bool in_n = mc < mN;
+      const int i = c0 + lane;
+      if (i >= (in_n ? mC : mN) || i == mc) return ~(Key)0;
+      const int id = g.pool[mi + i];
+      const float d = __int_as_float(g.pool[mi + mC + (in_n ? mc * mC + i : i * mC + mc)]);
+      return id == t ? ~(Key)0 : make_key(d, id);
+    };
+    Key ahead = key_of(__ffs(live) - 1, 0);
+    while (live) {
+      const int m = __ffs(live) - 1;
+      live &= live - 1u;
+      const int mc = __shfl_sync(full, c, m), mN = __shfl_sync(full, nN, m);
+      const int ncand = mc < mN ? __shfl_sync(full, nC, m) : mN;
+      Key ck = ahead;
+      if (live) ahead = key_of(__ffs(live) - 1, 0);
+      for (int c0 = 0;;) {
+        unsigned todo = __ballot_sync(full, ck < __shfl_sync(full, mine, kListW - 1));
+        while (todo) {
+          const int s = __ffs(todo) - 1;
+          todo &= todo - 1u;
+          minpos = min(minpos, warp_insert(mine, __shfl_sync(full, ck, s)));
+        }
+        c0 += 32;
+        if (c0 >= ncand) break;
+        ck = key_of(m, c0);
+      }
+    }
+  }
+  if (minpos == kListW) return;
+  row[lane] = mine;
+  if (lane == 0) {
+    dirty[t] = max(dirty[t], minpos < k ? 2 : 1);
+    if (g.stat) atomicAdd(&g.stat[3], 1ull);
   }
 }
 
@@ -580,12 +681,20 @@ void launch_join_nodes(const DevState &st, const UpdScratch &u, const int *batch
                                                             u.rev_old, u.sizes, off_new, off_old, u.csr);
   k_join_lists<<<cdiv(n, kListWarps), kListWarps * 32, 0, s>>>(
       n, u.fwd_new, u.fwd_old, u.rev_new, u.rev_old, u.cnt, u.fill, off_new, off_old, u.csr, u.sizes,
-      small_nodes, large_nodes, counters + kUpdNodes);
+      small_nodes, large_nodes, counters + kUpdNodes, (unsigned long long *)(counters + kUpdPool));
   note_launch(5);
 }
 
+size_t join_pool_words(int nb, int k) {
+  // a node's members are its forward samples and its sources, at most nb k of
+  // each over all nodes, and its block takes nN + 3 <= k + 32 + 3 words for
+  // each, rounded up to a whole entry
+  return 2 * (size_t)nb * (size_t)k * (size_t)(k + kSamples + 4);
+}
+
 void launch_local_join(const DevState &st, const UpdScratch &u, const int *small_nodes,
-                       const int *large_nodes, int *counters, int n, cudaStream_t s) {
+                       const int *large_nodes, int *counters, int *pool, size_t part_words, int pass,
+                       int n, cudaStream_t s) {
   if (n <= 0) return;
   const size_t smem = sizeof(JoinSmem);
   // per device, once (sessions on several host threads may launch at once)
@@ -597,19 +706,24 @@ void launch_local_join(const DevState &st, const UpdScratch &u, const int *small
   if (dev < 32) {
     std::lock_guard<std::mutex> g(mu);
     if (!ctas[dev]) {
-      cudaFuncSetAttribute(k_local_join, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_join_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       int sms = 0, per_sm = 0;
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_local_join, kJoinWarps * 32, smem);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_join_tiles, kJoinWarps * 32, smem);
       ctas[dev] = std::max(1, sms * std::max(per_sm, 1));
     }
     grid_ctas = ctas[dev];
   }
   const int grid = std::min(n, grid_ctas > 0 ? grid_ctas : 1024);
-  const JoinArgs g{u.fwd_new, u.fwd_old, u.rev_new, u.rev_old, u.sizes, st.X, st.norms, st.ld, st.k,
-                   st.g_key, st.locks, st.dirty, st.err, st.stat};
-  k_local_join<<<grid, kJoinWarps * 32, smem, s>>>(small_nodes, large_nodes, counters + kUpdNodes, g);
-  note_launch();
+  // the sources' array is free once the join lists stand: chain heads
+  const JoinArgs g{u.fwd_new, u.fwd_old, u.rev_new, u.rev_old, u.sizes, u.off, u.hflag, pool,
+                   (unsigned long long)part_words, pass, u.csr, st.g_key, st.X, st.norms, st.ld,
+                   st.stat};
+  if (pass == 0) cudaMemsetAsync(u.csr, 0xff, (size_t)n * 32 * sizeof(int), s);
+  else cudaMemsetAsync(counters + kUpdNodes + 2, 0, 2 * sizeof(int), s);  // the tickets
+  k_join_tiles<<<grid, kJoinWarps * 32, smem, s>>>(small_nodes, large_nodes, counters + kUpdNodes, g);
+  k_join_merge<<<cdiv(n, kJmWarps), kJmWarps * 32, 0, s>>>(n, g, st.g_key, st.dirty, st.k);
+  note_launch(2);
 }
 
 void launch_merge_publish(const DevState &st, int n, int *edge_counter, int *report_flag, cudaStream_t s) {

@@ -96,7 +96,7 @@ Request *gm_server::take(std::unique_lock<std::mutex> &) {
     Request *r = *it;
     Slot &sl = sessions.at(r->session);
     if (sl.busy) continue;
-    const size_t grow = sl.h->impl->growth_bytes((uint32_t)r->n_rows, r->n_emb);
+    const size_t grow = sl.h->impl->growth_bytes((uint32_t)r->n_rows, r->n_upd, r->n_emb);
     if (bytes_in_use + grow > p.hbm_budget) {
       if (running > 0) continue;
       pending.erase(it);

@@ -91,7 +91,7 @@ typedef struct gm_stats {
   uint64_t join_nodes;        /* nodes joined */
   uint64_t join_rows;         /* feature rows loaded by the join (sum over nodes) */
   uint64_t join_pairs;        /* distance pairs formed by the join */
-  uint64_t join_merges;       /* locked list merges */
+  uint64_t join_merges;       /* lists changed by the join's offers */
   uint64_t cand_launches;     /* insertion candidate-distance launches */
   double cand_ms;
   uint64_t cand_rows;         /* candidate feature rows loaded */

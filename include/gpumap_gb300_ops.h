@@ -53,6 +53,10 @@ int gm_debug_keep_tiles(struct gm_session *s, int on);
  * exceed it makes the heap and candidate passes run for its block
  * (gm_stats.exact_overflow_blocks). */
 int gm_debug_pre_capacity(struct gm_session *s, int cap);
+/* Words of the join pool that one pass of an update round covers, at most
+ * (clamped to [2, 2^25], the default; frees the pool).  A round whose node
+ * blocks take more words runs in several passes; its lists are the same. */
+int gm_debug_join_words(struct gm_session *s, uint64_t words);
 /* Host and device scalars, out[0..n):
  *  0 n_inserted, 1 insertion-queue head, 2 new-row embedding-queue head,
  *  3 embedding cursor (-1 = none), 4 embedding sweeps, 5 last nnz,
