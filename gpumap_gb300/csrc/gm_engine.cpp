@@ -185,8 +185,8 @@ Session::Session(const gm_params &p) : p_(p) {
       xs_.pool_j = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
       xs_.pool_m = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
       xs_.pool_d = (float *)dalloc((size_t)xs_.pool_cap * sizeof(float));
-      xs_.pool_j2 = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
-      xs_.pool_m2 = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
+      xs_.pair_j = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
+      xs_.pair_m = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
       xs_.row_t = (float *)dalloc((size_t)ex_block_ * sizeof(float));
       xs_.seed = (float *)dalloc((size_t)ex_block_ * sizeof(float));
       // pre-candidate segments: one per (block row, CTA of a row tile), for
@@ -201,9 +201,10 @@ Session::Session(const gm_params &p) : p_(p) {
       xs_.pre_cnt = (int *)dalloc((size_t)ex_block_ * xs_.pre_gx * sizeof(int));
       xs_.pre_over = (int *)dalloc(sizeof(int));
       xs_.heaps = (float *)dalloc((size_t)ex_block_ * std::max(sms_, 1) * 32 * sizeof(float));
-      xs_.pcnt = (int *)dalloc((Nm + 1) * sizeof(int));
-      xs_.poff = (int *)dalloc((Nm + 1) * sizeof(int));
-      xs_.tmp = (int *)dalloc(scan_tmp_ints((int)Nm) * sizeof(int));
+      xs_.pcnt = (int *)dalloc((size_t)ex_block_ * sizeof(int));
+      xs_.poff = (int *)dalloc(((size_t)ex_block_ + 1) * sizeof(int));
+      xs_.pfill = (int *)dalloc((size_t)ex_block_ * sizeof(int));
+      xs_.heads = us_.fwd_new;  // not in use during an insertion
       xs_.counter = (int *)dalloc(16 * sizeof(int));
     }
   } catch (...) {
@@ -727,6 +728,7 @@ uint32_t Session::insert(uint32_t n_ops) {
     // columns: the rows inserted so far (rows appended but still queued have
     // no norms or shadow rows yet)
     const int ncol = row0 + nb;
+    ck(cudaMemsetAsync(xs_.heads, 0xff, (size_t)row0 * 32 * sizeof(int), s), "heads");
     for (int b0 = 0; b0 < nb; b0 += ex_block_) {
       const int rows = std::min(ex_block_, nb - b0);
       timed_begin(3);

@@ -18,8 +18,8 @@
 //                32 nearest; per existing row, the batch rows that may enter
 //                its list
 //  k_row_threshold  per batch row: its exact threshold from the CTAs' heaps
-//  k_row_dists / k_pair_dists   canonical FP32 re-score of the survivors
-//  k_row_select / k_col_merge   exact top-32 merges
+//  k_rescore     canonical FP32 re-score of the survivors
+//  k_row_select / k_merge_offers   exact top-32 merges
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -31,6 +31,7 @@
 
 #include "gm_common.cuh"
 #include "gm_kernels.h"
+#include "gm_rowdot.cuh"
 
 namespace gm {
 
@@ -680,23 +681,18 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
 //  k_row_threshold  warp per batch row: T = 32nd smallest upper bound over all
 //                columns, from the union of the CTAs' heaps (pass 1), for the
 //                candidate test of pass 2
-//  k_pool_count / k_pool_scatter   groups the column pairs by existing row
+//  k_pool_count / k_pool_place   groups the column pairs by batch row
 //                (counting sort; order inside a group is free)
-//  k_row_dists   canonical distances of the row candidates
-//  k_pair_dists  canonical distances of the column pairs
+//  k_rescore     canonical distances of the row candidates and of the column
+//                pairs, whose offers go on the existing rows' chains
 //  k_row_select  warp per batch row: exact top-32 keys of its candidates
-//  k_col_merge   warp per existing row: merges its pairs into its list
+//  k_merge_offers (gm_kernels_insert.cu)  warp per existing row: merges its
+//                chains into its list
 // Both merges are order independent: a list ends as the 32 smallest keys of
 // its old entries and every candidate, and keys are unique (distinct ids).
 //
-// Canonical distances are sequential FP32 fused multiply-add chains over the
-// features; a warp forms 32 chains at once, one per lane, from feature rows
-// staged 32 columns at a time in shared memory by coalesced loads (lane l
-// reads tile row l at column i: bank (l * 33 + i) mod 32, conflict free).
 // fmaf(a, b, c) = fmaf(b, a, c) exactly, so d(x, y) = d(y, x) bit for bit.
 
-constexpr int kTile = 32;
-constexpr int kTileLd = 33;
 constexpr int kFinalWarps = 4;
 
 // Merges each lane's value u into the warp's ascending top 32 (lane l holds
@@ -831,148 +827,89 @@ __global__ void __launch_bounds__(kFinalWarps * 32)
   }
 }
 
-__global__ void k_pool_count(const int *pool_j, const int *counter, long pool_cap, int *pcnt,
-                             unsigned long long *stat) {
+// Pairs per batch row (at most 1,024 rows a block, counted in shared memory
+// first), then, in one CTA, the groups' offsets and fill cursors.
+constexpr int kMaxBlockRows = 1024;
+__global__ void __launch_bounds__(256)
+    k_pool_count(const int *pool_m, const int *counter, long pool_cap, int nrows, int *cnt,
+                 unsigned long long *stat) {
+  __shared__ int s_cnt[kMaxBlockRows];
   const long total = min((long)*counter, pool_cap);
+  for (int i = threadIdx.x; i < nrows; i += blockDim.x) s_cnt[i] = 0;
+  __syncthreads();
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x)
-    atomicAdd(&pcnt[pool_j[e]], 1);
+    atomicAdd(&s_cnt[pool_m[e]], 1);
+  __syncthreads();
+  for (int i = threadIdx.x; i < nrows; i += blockDim.x)
+    if (s_cnt[i]) atomicAdd(&cnt[i], s_cnt[i]);
   if (stat && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&stat[6], (unsigned long long)total);
 }
-// pcnt: zeroed again before this launch (it serves as the fill cursor)
-__global__ void k_pool_scatter(const int *pool_j, const int *pool_m, const int *counter,
-                               long pool_cap, const int *poff, int *pcnt, int *pool_j2,
-                               int *pool_m2) {
+__global__ void __launch_bounds__(kMaxBlockRows)
+    k_pool_offsets(int nrows, const int *cnt, int *off, int *fill) {
+  __shared__ int s_tot[32];
+  const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
+  const int c = i < nrows ? cnt[i] : 0;
+  int v = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += y;
+  }
+  if (lane == 31) s_tot[warp] = v;
+  __syncthreads();
+  int base = 0;
+  for (int w = 0; w < warp; ++w) base += s_tot[w];
+  if (i < nrows) {
+    off[i] = fill[i] = base + v - c;
+    if (i == nrows - 1) off[nrows] = base + v;
+  }
+}
+__global__ void k_pool_place(const int *pool_j, const int *pool_m, const int *counter, long pool_cap,
+                             int *fill, int *pair_j, int *pair_m) {
   const long total = min((long)*counter, pool_cap);
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
-    const int j = pool_j[e];
-    const int q = poff[j] + atomicAdd(&pcnt[j], 1);
-    pool_j2[q] = j;
-    pool_m2[q] = pool_m[e];
+    const int m = pool_m[e], q = atomicAdd(&fill[m], 1);
+    pair_j[q] = pool_j[e];
+    pair_m[q] = m;
   }
 }
 
-// 32 canonical chains per warp, one per lane (pair ra, rb; dummies for idle
-// lanes).  Feature chunks of 32 columns of the 64 rows are copied into a ring
-// of kRing shared-memory slots by 4-byte cp.async (each lane copies column
-// `lane` of every row: coalesced), kRing - 1 chunks ahead of the chain.
-constexpr int kRing = 4;
-constexpr int kPairWarps = 2;
-struct PairTiles {
-  float a[kRing][kTile][kTileLd];
-  float b[kRing][kTile][kTileLd];
-  int ra[kTile], rb[kTile];
-};
-constexpr size_t kPairSmem = sizeof(PairTiles) * kPairWarps;
-
-GM_D void cp_async4(float *dst, const float *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src)
-               : "memory");
-}
-GM_D void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-GM_D void cp_async_wait_ring() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 1) : "memory");
-}
-
-GM_D float warp_pair_dot(const float *X, int ld, int d, int ra, int rb, PairTiles &t) {
-  const int lane = threadIdx.x & 31;
-  t.ra[lane] = ra;
-  t.rb[lane] = rb;
-  __syncwarp();
-  const int nch = (d + kTile - 1) / kTile;
-  // one commit group per chunk index (empty past the last chunk), so that
-  // "at most kRing - 1 groups pending" means chunk c has landed
-  auto issue = [&](int c) {
-    const int col = c * kTile + lane;
-    if (c < nch && col < d) {
-      const int slot = c % kRing;
-#pragma unroll 8
-      for (int r = 0; r < kTile; ++r) {
-        cp_async4(&t.a[slot][r][lane], X + (size_t)t.ra[r] * ld + col);
-        cp_async4(&t.b[slot][r][lane], X + (size_t)t.rb[r] * ld + col);
-      }
-    }
-    cp_async_commit();
-  };
-  for (int c = 0; c < kRing - 1; ++c) issue(c);
-  float dot = 0.0f;
-  for (int c = 0; c < nch; ++c) {
-    issue(c + kRing - 1);  // refills the slot the previous iteration consumed
-    cp_async_wait_ring();
-    __syncwarp();
-    const int slot = c % kRing, lim = min(kTile, d - c * kTile);
-    for (int i = 0; i < lim; ++i) dot = __fmaf_rn(t.a[slot][lane][i], t.b[slot][lane][i], dot);
-    __syncwarp();
-  }
-  return dot;
-}
-
-__global__ void __launch_bounds__(kPairWarps * 32)
-    k_pair_dists(const float *X, int ld, int d, const float *norms, int brow0, const int *pool_j,
-                 const int *pool_m, float *pool_d, const int *counter, long pool_cap) {
-  extern __shared__ __align__(16) unsigned char pair_smem[];
-  PairTiles &t = reinterpret_cast<PairTiles *>(pair_smem)[threadIdx.x >> 5];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long total = min((long)*counter, pool_cap);
-  const long nw = (long)gridDim.x * kPairWarps;
-  for (long g = ((long)blockIdx.x * kPairWarps + w) * 32; g < total; g += nw * 32) {
-    const long e = g + lane;
-    const bool ok = e < total;
-    const int a = ok ? pool_j[e] : 0;
-    const int b = ok ? brow0 + pool_m[e] : 0;
-    const float dot = warp_pair_dot(X, ld, d, a, b, t);
-    if (ok) pool_d[e] = canon_dist(norms[a], norms[b], dot);
-  }
-}
-
-// Row candidates: the batch row is common to the warp, so only the candidate
-// rows go through the ring; lane l holds feature c0 + l of the batch row and
-// hands it to every chain by a shuffle.
-constexpr int kRowDistWarps = 4;
-struct RowTiles {
-  float b[kRing][kTile][kTileLd];
-  float a[kRing][kTile];
-  int rb[kTile];
-};
-constexpr size_t kRowSmem = sizeof(RowTiles) * kRowDistWarps;
-
-__global__ void __launch_bounds__(kRowDistWarps * 32)
-    k_row_dists(const float *X, int ld, int d, const float *norms, int brow0, const int *cand,
-                long cand_ld, const int *row_cnt, float *cand_d) {
-  extern __shared__ __align__(16) unsigned char row_smem[];
-  RowTiles &t = reinterpret_cast<RowTiles *>(row_smem)[threadIdx.x >> 5];
-  const int ml = blockIdx.x, row = brow0 + ml;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int cnt = row_cnt[ml];
-  const int *cl = cand + (long)ml * cand_ld;
+// Canonical distances, 32 chains per warp against one batch row
+// (gm_rowdot.cuh): kRescoreSplit warps walk each row's candidates, as many its
+// column pairs.  A pair's offer goes on one of its existing row's chains, as
+// in the NN-Descent insertion (its entry is its place in pair_j).
+// Bound by memory (a feature row per chain).  500 rows x 784 features
+// against 70,000: candidates by a CTA of four warps per row (4-byte copies, 1.1
+// waves) 73 us and pairs with both rows gathered 57 us; together 79 us now, of which
+// reading most of the 220 MB of rows once is half.
+constexpr int kRescoreWarps = 2;
+constexpr int kRescoreSplit = 4;
+__global__ void __launch_bounds__(kRescoreWarps * 32)
+    k_rescore(const float *X, int ld, const float *norms, int brow0, int nrows, const int *cand,
+              long cand_ld, const int *row_cnt, float *cand_d, const int *pair_j, const int *pair_off,
+              float *pair_d, const Key *g_key, OfferChains chains) {
+  __shared__ __align__(16) RowDotTiles tiles[kRescoreWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int task = blockIdx.x * kRescoreWarps + warp;
+  const int ml = task / (2 * kRescoreSplit), part = task % (2 * kRescoreSplit);
+  if (ml >= nrows) return;
+  const int row = brow0 + ml;
   const float *xa = X + (size_t)row * ld;
-  const int nch = (d + kTile - 1) / kTile;
-  for (int g = w * 32; g < cnt; g += kRowDistWarps * 32) {
-    const int c = g + lane;
-    t.rb[lane] = c < cnt ? cl[c] : row;
-    __syncwarp();
-    auto issue = [&](int ch) {
-      const int col = ch * kTile + lane;
-      if (ch < nch && col < d) {
-        const int slot = ch % kRing;
-        cp_async4(&t.a[slot][lane], xa + col);
-#pragma unroll 8
-        for (int r = 0; r < kTile; ++r)
-          cp_async4(&t.b[slot][r][lane], X + (size_t)t.rb[r] * ld + col);
-      }
-      cp_async_commit();
-    };
-    for (int ch = 0; ch < kRing - 1; ++ch) issue(ch);
-    float dot = 0.0f;
-    for (int ch = 0; ch < nch; ++ch) {
-      issue(ch + kRing - 1);
-      cp_async_wait_ring();
-      __syncwarp();
-      const int slot = ch % kRing, lim = min(kTile, d - ch * kTile);
-      for (int i = 0; i < lim; ++i) dot = __fmaf_rn(t.a[slot][i], t.b[slot][lane][i], dot);
-      __syncwarp();
+  const bool pairs = part >= kRescoreSplit;
+  if (pairs && !pair_off) return;
+  const int begin = pairs ? pair_off[ml] : 0;
+  const int cnt = pairs ? pair_off[ml + 1] - begin : row_cnt[ml];
+  const int *ids = pairs ? pair_j + begin : cand + (long)ml * cand_ld;
+  float *out = pairs ? pair_d + begin : cand_d + (long)ml * cand_ld;
+  for (int i0 = (part % kRescoreSplit) * 32; i0 < cnt; i0 += kRescoreSplit * 32) {
+    const int i = i0 + lane;
+    const int j = i < cnt ? ids[i] : row;
+    const float dv = canon_dist(norms[row], norms[j], warp_row_dot(X, ld, xa, j, tiles[warp]));
+    if (i < cnt) {
+      out[i] = dv;
+      if (pairs && make_key(dv, row) < g_key[(size_t)j * kListW + kListW - 1])
+        chains.next[begin + i] = atomicExch(&chains.heads[(size_t)j * 32 + (row & 31)], begin + i);
     }
-    if (c < cnt) cand_d[(long)ml * cand_ld + c] = canon_dist(norms[row], norms[t.rb[lane]], dot);
-    __syncwarp();
   }
 }
 
@@ -1003,39 +940,6 @@ __global__ void k_row_select(const float *cand_d, int brow0, int nrows, const in
   }
   g_key[(size_t)(brow0 + ml) * kListW + lane] = mine;
   if (stat && lane == 0) atomicAdd(&stat[6], (unsigned long long)cnt);
-}
-
-// Warp per existing row j with pairs: lane l holds entry l of j's sorted list;
-// each new key is inserted by a ballot on the lanes whose entry it precedes.
-constexpr int kMergeWarps = 8;
-__global__ void k_col_merge(int n_exist, int brow0, const int *poff, const int *pool_m,
-                            const float *pool_d, Key *g_key, int *dirty) {
-  const int lane = threadIdx.x & 31;
-  const int j = blockIdx.x * kMergeWarps + (threadIdx.x >> 5);
-  if (j >= n_exist) return;
-  const int base = poff[j], cnt = poff[j + 1] - poff[j];
-  if (!cnt) return;
-  Key *lst = g_key + (size_t)j * kListW;
-  Key mine = lst[lane];
-  bool changed = false;
-  for (int c0 = 0; c0 < cnt; c0 += 32) {
-    const int c = c0 + lane;
-    const Key ck = c < cnt ? make_key(pool_d[base + c], brow0 + pool_m[base + c]) : ~(Key)0;
-    for (int src = 0; src < 32 && c0 + src < cnt; ++src) {
-      const Key k = __shfl_sync(0xffffffffu, ck, src);
-      const unsigned msk = __ballot_sync(0xffffffffu, k < mine);
-      if (!msk) continue;
-      changed = true;
-      const int pos = __ffs(msk) - 1;
-      const Key prev = __shfl_up_sync(0xffffffffu, mine, 1);
-      if (lane > pos) mine = prev;
-      else if (lane == pos) mine = k;
-    }
-  }
-  if (changed) {
-    lst[lane] = mine;
-    if (lane == 0) dirty[j] = 1;
-  }
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
@@ -1227,40 +1131,22 @@ void launch_exact_screen(const DevState &st, int row0, int blk0, int nrows, int 
   if (nrows <= 0 || n <= 0) return;
   const int brow0 = row0 + blk0;  // global first row of the block
   const int grid = 4 * std::max(sms, 1);
+  // the pairs as found are done with once placed: pool_m holds the chains
+  const OfferChains chains{x.heads, x.pool_m};
   if (row0 > 0) {
-    cudaMemsetAsync(x.pcnt, 0, (size_t)row0 * sizeof(int), s);
-    k_pool_count<<<grid, 256, 0, s>>>(x.pool_j, x.counter, x.pool_cap, x.pcnt, st.stat);
-    note_launch();
-    exclusive_scan(x.pcnt, x.poff, row0, x.tmp, s);
-    cudaMemsetAsync(x.pcnt, 0, (size_t)row0 * sizeof(int), s);
-    k_pool_scatter<<<grid, 256, 0, s>>>(x.pool_j, x.pool_m, x.counter, x.pool_cap, x.poff, x.pcnt,
-                                        x.pool_j2, x.pool_m2);
-    note_launch();
+    cudaMemsetAsync(x.pcnt, 0, (size_t)nrows * sizeof(int), s);
+    k_pool_count<<<grid, 256, 0, s>>>(x.pool_m, x.counter, x.pool_cap, nrows, x.pcnt, st.stat);
+    k_pool_offsets<<<1, kMaxBlockRows, 0, s>>>(nrows, x.pcnt, x.poff, x.pfill);
+    k_pool_place<<<grid, 256, 0, s>>>(x.pool_j, x.pool_m, x.counter, x.pool_cap, x.pfill, x.pair_j, x.pair_m);
+    note_launch(3);
   }
-  static std::atomic<unsigned> pair_configured{0u};
-  {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 32 && !(pair_configured.load() & (1u << dev))) {
-      cudaFuncSetAttribute(k_row_dists, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmem);
-      cudaFuncSetAttribute(k_pair_dists, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem);
-      pair_configured.fetch_or(1u << dev);
-    }
-  }
-  k_row_dists<<<nrows, kRowDistWarps * 32, kRowSmem, s>>>(st.X, st.ld, st.d, st.norms, brow0,
-                                                         x.cand, ldD, x.row_cnt, x.cand_d);
-  note_launch();
+  k_rescore<<<cdiv((long)nrows * 2 * kRescoreSplit, kRescoreWarps), kRescoreWarps * 32, 0, s>>>(
+      st.X, st.ld, st.norms, brow0, nrows, x.cand, ldD, x.row_cnt, x.cand_d, x.pair_j,
+      row0 > 0 ? x.poff : nullptr, x.pool_d, st.g_key, chains);
   k_row_select<<<cdiv(nrows, kRowWarps), kRowWarps * 32, 0, s>>>(x.cand_d, brow0, nrows, x.cand,
                                                                  ldD, x.row_cnt, st.g_key, st.stat);
-  note_launch();
-  if (row0 > 0) {
-    k_pair_dists<<<grid, kPairWarps * 32, kPairSmem, s>>>(
-        st.X, st.ld, st.d, st.norms, brow0, x.pool_j2, x.pool_m2, x.pool_d, x.counter, x.pool_cap);
-    note_launch();
-    k_col_merge<<<cdiv(row0, kMergeWarps), kMergeWarps * 32, 0, s>>>(
-        row0, brow0, x.poff, x.pool_m2, x.pool_d, st.g_key, st.dirty);
-    note_launch();
-  }
+  note_launch(2);
+  if (row0 > 0) launch_merge_offers(st, row0, brow0, chains, x.pool_d, x.pair_m, nullptr, nullptr, s);
 }
 
 }  // namespace gm

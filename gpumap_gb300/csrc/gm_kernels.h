@@ -93,6 +93,19 @@ struct CandScratch {
 void launch_nnd_insert(const DevState &st, const UpdScratch &u, int row0, int nrows, int n,
                        int window_start, uint64_t seed, const CandScratch &c, int *changed, int sms,
                        const std::function<void(bool)> &timed, cudaStream_t s);
+// Offers by target: row j has 32 chains, heads[j * 32 + l] the newest offer of
+// the batch rows with id mod 32 = l (-1: none), next[] the one before it.
+struct OfferChains {
+  int *heads;  // -1 before the first offer, left so by launch_merge_offers
+  int *next;
+};
+// Merges the offers on the chains of rows [0, row0) into their lists.  Offer
+// e comes from row first + e_row[e] (e_row null: first + e / 256) at distance
+// dist[e].  changed_out (or null) is set when a list changes; changed (or
+// null): nothing is done unless it is set.
+void launch_merge_offers(const DevState &st, int row0, int first, const OfferChains &chains,
+                         const float *dist, const int *e_row, int *changed_out, const int *changed,
+                         cudaStream_t s);
 // Copies the first k working entries of rows [row0,row0+nrows) and of the
 // listed rows into the authoritative list and publishes them.
 void launch_adopt_and_publish(const DevState &st, int row0, int nrows,
@@ -131,12 +144,13 @@ struct ExactScreen {
   int pre_cap = 0, pre_gx = 0;
   bool pre_fixed = false;
   int *pre_over = nullptr;
-  int *pool_j = nullptr, *pool_m = nullptr;    // column pairs as found
-  int *pool_j2 = nullptr, *pool_m2 = nullptr;  // grouped by existing row
+  int *pool_j = nullptr, *pool_m = nullptr;  // column pairs as found
+  int *pair_j = nullptr, *pair_m = nullptr;  // grouped by batch row
   float *pool_d = nullptr;    // their canonical distances
-  int *pcnt = nullptr;        // n_cap + 1 pairs per existing row, then fill cursors
-  int *poff = nullptr;        // n_cap + 1 group offsets
-  int *tmp = nullptr;         // scan scratch, scan_tmp_ints(n_cap)
+  int *pcnt = nullptr;        // pairs per batch row
+  int *poff = nullptr;        // the groups' offsets (rows + 1) and fill cursors
+  int *pfill = nullptr;
+  int *heads = nullptr;       // chain heads of the existing rows (n_cap x 32, all -1)
   int *counter = nullptr;     // pairs in the pool
   long pool_cap = 0;
 };

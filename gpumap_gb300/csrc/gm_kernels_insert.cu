@@ -282,15 +282,6 @@ __global__ void __launch_bounds__(kSampWarps * 32)
   if (lane == 0) o.todo_cnt[rl] = left;
 }
 
-// Offers of an iteration by target: row j has 32 chains, heads[j * 32 + l]
-// the newest offer of the batch rows with id mod 32 = l (-1: none), next[]
-// the one before it.  Offer e is candidate slot e of the launch: from its
-// row e / 256, at distance cand_dist[e].
-struct OfferChains {
-  int *heads;  // -1 before the first iteration, left so by k_merge_offers
-  int *next;
-};
-
 // Candidate distances and, for existing candidates (id < row0), the reverse
 // offers (reference: compute_candidate_distances_kernel,
 // insertion_kernel.cuh:337-405, and :548-640, which scatters up to 32
@@ -338,8 +329,8 @@ __global__ void __launch_bounds__(kCandWarps * 32)
 // the row.  The order of offers does not matter (warp_insert).
 constexpr int kOfferWarps = 8;
 __global__ void __launch_bounds__(kOfferWarps * 32)
-    k_merge_offers(Key *g_key, int row0, int first, OfferChains chains, const float *cand_dist, int *dirty,
-                   int *changed_out, const int *changed) {
+    k_merge_offers(Key *g_key, int row0, int first, OfferChains chains, const float *dist,
+                   const int *e_row, int *dirty, int *changed_out, const int *changed) {
   if (changed && *changed == 0) return;
   const int lane = threadIdx.x & 31;
   const int j = blockIdx.x * kOfferWarps + (threadIdx.x >> 5);
@@ -354,7 +345,7 @@ __global__ void __launch_bounds__(kOfferWarps * 32)
   while (__any_sync(full, e >= 0)) {
     Key ck = ~(Key)0;
     if (e >= 0) {
-      ck = make_key(cand_dist[e], first + e / kMaxCand);
+      ck = make_key(dist[e], first + (e_row ? e_row[e] : e / kMaxCand));
       e = chains.next[e];
     }
     unsigned todo = __ballot_sync(full, ck < __shfl_sync(full, mine, kListW - 1));
@@ -520,6 +511,14 @@ void launch_row_norms(const DevState &st, int row0, int nrows, cudaStream_t s) {
   note_launch();
 }
 
+void launch_merge_offers(const DevState &st, int row0, int first, const OfferChains &chains,
+                         const float *dist, const int *e_row, int *changed_out, const int *changed,
+                         cudaStream_t s) {
+  k_merge_offers<<<cdiv(row0, kOfferWarps), kOfferWarps * 32, 0, s>>>(
+      st.g_key, row0, first, chains, dist, e_row, st.dirty, changed_out, changed);
+  note_launch();
+}
+
 void launch_nnd_insert(const DevState &st, const UpdScratch &u, int row0, int nrows, int n, int window_start,
                        uint64_t seed, const CandScratch &c, int *changed, int sms,
                        const std::function<void(bool)> &timed, cudaStream_t s) {
@@ -568,11 +567,7 @@ void launch_nnd_insert(const DevState &st, const UpdScratch &u, int row0, int nr
           (merges ? c.todo_cnt : c.cnt) + r, c.dist + at, st.g_key, chains, go, st.stat);
       note_launch();
       timed(false);
-      if (row0 > 0) {
-        k_merge_offers<<<cdiv(row0, kOfferWarps), kOfferWarps * 32, 0, s>>>(
-            st.g_key, row0, row0 + r, chains, c.dist + at, st.dirty, mark, go);
-        note_launch();
-      }
+      if (row0 > 0) launch_merge_offers(st, row0, row0 + r, chains, c.dist + at, nullptr, mark, go, s);
     }
     if (merges) {
       k_forward_merge<<<cdiv(nrows, kFwdWarps), kFwdWarps * 32, 0, s>>>(
