@@ -407,7 +407,7 @@ int gm_op_sgd(float *emb, int64_t n, const int32_t *head, const int32_t *tail,
     int *isc = (int *)sc;
     const cudaError_t le = gm::launch_sgd_call(
         emb, head, tail, eps, (float *)ns, (float *)nn, isc, (const float *)((char *)sc + 64),
-        alpha0, gamma, a, b, n_epochs, neg_rate, seed, (unsigned *)(isc + gm::kIscalBarrier),
+        (int)nnz, alpha0, gamma, a, b, n_epochs, neg_rate, seed, (unsigned *)(isc + gm::kIscalBarrier),
         (unsigned *)(isc + 10), dev, s);
     unsigned dev_err = 0;
     if (le == cudaSuccess) cudaMemcpyAsync(&dev_err, isc + 10, sizeof(unsigned), cudaMemcpyDeviceToHost, s);

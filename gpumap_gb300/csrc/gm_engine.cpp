@@ -986,7 +986,7 @@ uint32_t Session::embed(uint32_t n_ops) {
     launch_add_noise(st_.emb, ni, es_.batch, nb, 0.001f, noise_seed, es_, s);
   }
   timed_begin(2, s);
-  run_sgd(s);
+  run_sgd((int)std::min<size_t>(2 * (size_t)nb * (size_t)k, INT32_MAX), s);
   timed_end(2, s);
   if (nu > 0) launch_heuristic(heur_idx, heur_dist, ni, k, euclid, es_.unsel, nu, st_.emb, es_, s);
   if (p_.overlap) {
@@ -1007,15 +1007,13 @@ void Session::flush_init() {
 
 // The max_epoch SGD epochs of one embedding call: one cooperative launch
 // with a grid barrier between epochs (sizes are read from device scalars).
-// t_col (free once the schedule is built) holds the edge grouping and
-// ipartial its bins.
-void Session::run_sgd(cudaStream_t s) {
+void Session::run_sgd(int max_edges, cudaStream_t s) {
   if (p_.max_epoch == 0) return;
   // overlapped: half the SMs, the other half stays free for the next cycle's
   // distance work (the per-epoch time does not depend on it)
   const int max_ctas = p_.overlap ? std::max(1, sms_ / 2) : 0;
   ck(launch_sgd_call(st_.emb, es_.t_row, es_.flag_tail, es_.t_val, es_.next_s, es_.next_n,
-                     es_.iscal, es_.fscal, p_.alpha, 1.0f, p_.a, p_.b, (int)p_.max_epoch,
+                     es_.iscal, es_.fscal, max_edges, p_.alpha, 1.0f, p_.a, p_.b, (int)p_.max_epoch,
                      (int)p_.negative_sample_rate, 42ull, (unsigned *)(es_.iscal + kIscalBarrier),
                      st_.err, device_, s, st_.stat, max_ctas),
      "SGD launch");

@@ -115,7 +115,7 @@ class Session {
   void timed_begin(int slot, cudaStream_t s = nullptr);
   void timed_end(int slot, cudaStream_t s = nullptr);
   void collect_timings(bool block = true);
-  void run_sgd(cudaStream_t s);
+  void run_sgd(int max_edges, cudaStream_t s);
 
   gm_params p_;
   int device_ = 0;
