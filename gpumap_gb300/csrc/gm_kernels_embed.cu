@@ -14,9 +14,10 @@ namespace gm {
 // Scalar slots in EmbedScratch.
 //   fscal: 0 mean_dist, 1 max_w, 2 rounding, 3 x_min, 4 x_max
 //   iscal: 0 nnz (directed + extras), 1 extras, 2 nnz after trim, 3 max degree,
-//          4 rows n (read by the SGD epochs so a captured graph stays valid)
+//          4 rows n (read by the SGD epochs so a captured graph stays valid),
+//          5 rows left for k_fix_sigma
 enum { FS_MEAN = 0, FS_MAXW = 1, FS_ROUND = 2, FS_XMIN = 3, FS_XMAX = 4 };
-enum { IS_NNZ = 0, IS_EXTRA = 1, IS_NNZ2 = 2, IS_MAXDEG = 3, IS_N = 4 };
+enum { IS_NNZ = 0, IS_EXTRA = 1, IS_NNZ2 = 2, IS_MAXDEG = 3, IS_N = 4, IS_MARKED = 5 };
 
 namespace {
 
@@ -75,124 +76,100 @@ __global__ void k_mean_partial(const float *pub_dist, int n, int k, int euclid,
   }
 }
 
-// Ordered sum of the partials: a block stages them in shared memory by
-// coalesced loads, then thread 0 adds them in index order.
-constexpr int kMeanStage = 4096;
-__global__ void k_mean_final(const float *part, const int *ipart, int nb, float *fscal) {
-  __shared__ float sp[kMeanStage];
-  __shared__ int si[kMeanStage];
+// The mean of the partials, added in index order by one thread (each addition
+// waits for the one before it; the partials come through shared memory, four
+// per read).  The whole block calls it.
+constexpr int kMeanStage = 2048;
+GM_D void mean_final(const float *part, const int *ipart, int nb, float *fscal, float *stage) {
   float s = 0.0f;
-  long c = 0;
+  int c = 0;
   for (int i0 = 0; i0 < nb; i0 += kMeanStage) {
     const int m = min(kMeanStage, nb - i0);
     __syncthreads();
-    for (int i = threadIdx.x; i < m; i += blockDim.x) {
-      sp[i] = part[i0 + i];
-      si[i] = ipart[i0 + i];
+    for (int i = threadIdx.x; i < (m + 3) / 4 * 4; i += blockDim.x) {
+      stage[i] = i < m ? part[i0 + i] : 0.0f;
+      c += i < m ? ipart[i0 + i] : 0;
     }
     __syncthreads();
-    if (threadIdx.x == 0)
-      for (int i = 0; i < m; ++i) {
-        s = __fadd_rn(s, sp[i]);
-        c += si[i];
+    if (threadIdx.x == 0) {
+      // (the partials are not negative: adding a +0 of the padding is exact)
+#pragma unroll 8
+      for (int i = 0; i < m; i += 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(stage + i);
+        s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v.x), v.y), v.z), v.w);
       }
+    }
   }
+  __shared__ unsigned long long s_c;
+  if (threadIdx.x == 0) s_c = 0ull;
+  __syncthreads();
+  if (c) atomicAdd(&s_c, (unsigned long long)c);
+  __syncthreads();
   if (threadIdx.x == 0)
-    fscal[FS_MEAN] = (c > 0 && isfinite(s) && s > 0.0f) ? __fdiv_rn(s, (float)c) : 1.0f;
+    fscal[FS_MEAN] = (s_c > 0ull && isfinite(s) && s > 0.0f) ? __fdiv_rn(s, (float)(long)s_c) : 1.0f;
 }
 
-// sigma / rho per row, one warp per row; the bisection's target sum is
-// accumulated in FP64 by a fixed butterfly (reference smooth_knn_dist_kernel,
-// embedding_kernel.cuh:135-207).
-// sigma / rho by bisection (reference smooth_knn_dist, one warp per row for
-// k > 16).  The bisection's target sum is accumulated in FP64 by the fixed
-// xor-butterfly order of 32 lanes, term c on lane c (the terms of lanes >= k
-// are +0, adding them is exact).
-__global__ void k_smooth_knn(const float *pub_dist, int n, int k, int euclid,
-                             const float *fscal, double target, float *sigma,
-                             float *rho) {
-  const int lane = threadIdx.x & 31;
-  const long gid = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (gid >= n) return;
-  const int row = (int)gid;
-  const float raw = lane < k ? edist(pub_dist, k, row, lane, euclid) : 0.0f;
-  const float san = (lane < k && valid_d(raw)) ? raw : 0.0f;
-  float sum = 0.0f;
-  for (int c = 0; c < k; ++c) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, san, c));
-  const unsigned nz = __ballot_sync(0xffffffffu, lane < k && san > 0.0f);
-  const float mean_dist = fscal[FS_MEAN];
-  if (nz == 0u) {
-    if (lane == 0) {
-      rho[row] = 0.0f;
-      sigma[row] = __fmul_rn(kMinKDistScale, mean_dist);
-    }
+// Exact sum of two floats: s + e (Knuth, The Art of Computer Programming,
+// vol. 2, 4.2.2, theorem B).
+GM_D void two_sum(float a, float b, float &s, float &e) {
+  s = __fadd_rn(a, b);
+  const float bb = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+}
+
+// sigma / rho by bisection (reference smooth_knn_dist_kernel,
+// embedding_kernel.cuh:135-207), L lanes per row (4 for k <= 16, 8 for k <=
+// 32), terms q, q + L, q + 2L, q + 3L on lane q.  The bisection's target sum is
+// defined in FP64, by the xor butterfly of 32 lanes with term c on lane c (the
+// terms of lanes >= k are +0, adding them is exact).  Its only use is two
+// comparisons (within the tolerance of the target; above it), so it is formed
+// in FP32 with exact error terms, to within 1e-12, and FP64 additions run only
+// where that cannot decide (within kUnsure of the tolerance's edge): FP64 has
+// 1/64 of the FP32 rate here and bound the kernel.  The other terms of the
+// FP64 tree: (t0 + t2) + (t1 + t3) on each lane, then xor L/2 .. 1.
+// 70,000 rows at k = 15: 151 -> 56 us; 100,000 at k = 30 (a warp per row): 1508
+// -> 187 us.
+// The first CTA takes the global mean meanwhile, which only rows without a
+// positive distance need: those are left marked (sigma < 0, *marked set) for
+// k_fix_sigma.
+constexpr float kUnsure = 1e-10f;
+constexpr int kSmoothThreads = 256;
+template <int L>
+__global__ void __launch_bounds__(kSmoothThreads)
+    k_smooth_knn(const float *pub_dist, int n, int k, int euclid, double target, float t_hi,
+                 float t_lo, float *sigma, float *rho, const float *part, const int *ipart, int nb,
+                 float *fscal, int *marked) {
+  __shared__ __align__(16) float stage[kMeanStage];
+  if (blockIdx.x == 0) {
+    mean_final(part, ipart, nb, fscal, stage);
     return;
   }
-  const float r = __shfl_sync(0xffffffffu, raw, __ffs(nz) - 1);
-  const float row_mean = __fdiv_rn(sum, (float)k);
-  float lo = 0.0f, hi = FLT_MAX, mid = 1.0f;
-  const bool contrib = lane >= 2 && lane < k;
-  const float dj = __fsub_rn(san, r);
-  for (int it = 0; it < 64; ++it) {
-    double term = 0.0;
-    if (contrib) term = (dj > 0.0f) ? (double)gm_expf(__fdiv_rn(-dj, mid)) : 1.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) term += __shfl_xor_sync(0xffffffffu, term, o);
-    if (fabs(term - target) < (double)kSmoothTol) break;
-    if (term > target) {
-      hi = mid;
-      mid = __fmul_rn(__fadd_rn(lo, hi), 0.5f);
-    } else {
-      lo = mid;
-      mid = (hi == FLT_MAX) ? __fmul_rn(mid, 2.0f) : __fmul_rn(__fadd_rn(lo, hi), 0.5f);
-    }
-  }
-  if (lane != 0) return;
-  if (!isfinite(mid) || mid <= 0.0f) mid = 1.0f;
-  const float min_scale = __fmul_rn(kMinKDistScale, (r > 0.0f) ? row_mean : mean_dist);
-  rho[row] = r;
-  sigma[row] = mid < min_scale ? min_scale : mid;
-}
-
-// The same for k <= 16 with four lanes per row (eight rows per warp).  Lane
-// q of a row holds terms c = q, q+4, q+8, q+12 and forms
-// (t[q] + t[q+8]) + (t[q+4] + t[q+12]); two more xor steps over the four
-// lanes finish the sum.  For k <= 16 this is exactly the 32-lane butterfly's
-// tree (its first step only adds the exact zeros of lanes 16-31, the next two
-// are these per-lane additions), so every bit agrees with the warp-per-row
-// form, with a quarter of the FP64 additions (FP64 is slow on this part).
-__global__ void k_smooth_knn4(const float *pub_dist, int n, int k, int euclid,
-                              const float *fscal, double target, float *sigma,
-                              float *rho) {
+  const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const int q = lane & 3, base = lane - q;
-  const long gid = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+  const int q = lane & (L - 1), base = lane - q;
+  const long gid = ((long)(blockIdx.x - 1) * kSmoothThreads + threadIdx.x) / L;
   const bool live = gid < n;
   const int row = live ? (int)gid : 0;
   float raw[4], san[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const int c = q + 4 * j;
+    const int c = q + L * j;
     raw[j] = (live && c < k) ? edist(pub_dist, k, row, c, euclid) : 0.0f;
     san[j] = (live && c < k && valid_d(raw[j])) ? raw[j] : 0.0f;
   }
   // row sum in column order, first nonzero column
-  float sum = 0.0f;
-  int first = 64;
+  float sum = 0.0f, r = 0.0f;
+  bool found = false;
 #pragma unroll
-  for (int c = 0; c < 16; ++c) {
-    const float v = __shfl_sync(0xffffffffu, san[c >> 2], base + (c & 3));
+  for (int c = 0; c < 4 * L; ++c) {
+    const float v = __shfl_sync(full, san[c / L], base + (c & (L - 1)));
     if (c < k) {
       sum = __fadd_rn(sum, v);
-      if (first == 64 && v > 0.0f) first = c;
+      if (!found && v > 0.0f) {
+        found = true;
+        r = v;
+      }
     }
-  }
-  const float mean_dist = fscal[FS_MEAN];
-  float r = 0.0f;
-#pragma unroll
-  for (int c = 0; c < 16; ++c) {
-    const float v = __shfl_sync(0xffffffffu, raw[c >> 2], base + (c & 3));
-    if (c == first) r = v;
   }
   const float row_mean = __fdiv_rn(sum, (float)k);
   float lo = 0.0f, hi = FLT_MAX, mid = 1.0f;
@@ -200,28 +177,48 @@ __global__ void k_smooth_knn4(const float *pub_dist, int n, int k, int euclid,
   bool contrib[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const int c = q + 4 * j;
+    const int c = q + L * j;
     contrib[j] = c >= 2 && c < k;
     dj[j] = __fsub_rn(san[j], r);
   }
-  bool done = !live || first == 64;
+  bool done = !live || !found;
   for (int it = 0; it < 64; ++it) {
-    if (__all_sync(0xffffffffu, done)) break;
-    double t[4];
+    if (__all_sync(full, done)) break;
+    float t[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      t[j] = 0.0;
-      if (contrib[j] && !done) t[j] = (dj[j] > 0.0f) ? (double)gm_expf(__fdiv_rn(-dj[j], mid)) : 1.0;
+      t[j] = 0.0f;
+      if (contrib[j] && !done) t[j] = (dj[j] > 0.0f) ? gm_expf(__fdiv_rn(-dj[j], mid)) : 1.0f;
     }
-    double term = (t[0] + t[2]) + (t[1] + t[3]);
-    term += __shfl_xor_sync(0xffffffffu, term, 2);
-    term += __shfl_xor_sync(0xffffffffu, term, 1);
+    float s0, e0, s1, e1, s, e;
+    two_sum(t[0], t[2], s0, e0);
+    two_sum(t[1], t[3], s1, e1);
+    two_sum(s0, s1, s, e);
+    e = __fadd_rn(e, __fadd_rn(e0, e1));
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) {
+      const float so = __shfl_xor_sync(full, s, o), eo = __shfl_xor_sync(full, e, o);
+      float sn, en;
+      two_sum(s, so, sn, en);
+      s = sn;
+      e = __fadd_rn(en, __fadd_rn(e, eo));
+    }
+    const float off = __fadd_rn(__fsub_rn(s, t_hi), __fsub_rn(e, t_lo));
+    bool within = fabsf(off) < kSmoothTol, above = off > 0.0f;
+    const bool unsure = !done && fabsf(__fsub_rn(fabsf(off), kSmoothTol)) <= kUnsure;
+    if (__any_sync(full, unsure)) {
+      double term = ((double)t[0] + (double)t[2]) + ((double)t[1] + (double)t[3]);
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) term += __shfl_xor_sync(full, term, o);
+      if (unsure) {
+        within = fabs(term - target) < (double)kSmoothTol;
+        above = term > target;
+      }
+    }
     if (done) continue;
-    if (fabs(term - target) < (double)kSmoothTol) {
+    if (within) {
       done = true;
-      continue;
-    }
-    if (term > target) {
+    } else if (above) {
       hi = mid;
       mid = __fmul_rn(__fadd_rn(lo, hi), 0.5f);
     } else {
@@ -230,15 +227,24 @@ __global__ void k_smooth_knn4(const float *pub_dist, int n, int k, int euclid,
     }
   }
   if (!live || q != 0) return;
-  if (first == 64) {
+  if (!found) {
     rho[row] = 0.0f;
-    sigma[row] = __fmul_rn(kMinKDistScale, mean_dist);
+    sigma[row] = -1.0f;
+    *marked = 1;
     return;
   }
   if (!isfinite(mid) || mid <= 0.0f) mid = 1.0f;
-  const float min_scale = __fmul_rn(kMinKDistScale, (r > 0.0f) ? row_mean : mean_dist);
+  // (r > 0: the row's own mean is the scale, never the global one)
+  const float min_scale = __fmul_rn(kMinKDistScale, row_mean);
   rho[row] = r;
   sigma[row] = mid < min_scale ? min_scale : mid;
+}
+
+// Rows without a positive distance: a share of the global mean.
+__global__ void k_fix_sigma(int n, const float *fscal, float *sigma, const int *marked) {
+  if (!*marked) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n && sigma[i] < 0.0f) sigma[i] = __fmul_rn(kMinKDistScale, fscal[FS_MEAN]);
 }
 
 // Directed membership p_ij for batch rows and the fuzzy union
@@ -778,15 +784,17 @@ void launch_fuzzy_graph(const uint32_t *pub_idx, const float *pub_dist, int n, i
   const int nbl = cdiv(total, 256);
   k_mean_partial<<<nbl, 256, 0, s>>>(pub_dist, n, k, euclidean, e.partial, e.ipartial);
   note_launch();
-  k_mean_final<<<1, 256, 0, s>>>(e.partial, e.ipartial, nbl, e.fscal);
-  note_launch();
-  if (k <= 16)
-    k_smooth_knn4<<<cdiv((long)n * 4, 256), 256, 0, s>>>(pub_dist, n, k, euclidean, e.fscal,
-                                                         log2_target, e.sigma, e.rho);
-  else
-    k_smooth_knn<<<cdiv((long)n * 32, 256), 256, 0, s>>>(pub_dist, n, k, euclidean, e.fscal,
-                                                         log2_target, e.sigma, e.rho);
-  note_launch();
+  cudaMemsetAsync(e.iscal + IS_MARKED, 0, sizeof(int), s);
+  const float t_hi = (float)log2_target, t_lo = (float)(log2_target - (double)t_hi);
+  auto smooth = [&](auto kernel, int lanes) {
+    kernel<<<1 + cdiv((long)n * lanes, kSmoothThreads), kSmoothThreads, 0, s>>>(
+        pub_dist, n, k, euclidean, log2_target, t_hi, isfinite(log2_target) ? t_lo : 0.0f, e.sigma, e.rho,
+        e.partial, e.ipartial, nbl, e.fscal, e.iscal + IS_MARKED);
+  };
+  if (k <= 16) smooth(k_smooth_knn<4>, 4);
+  else smooth(k_smooth_knn<8>, 8);
+  k_fix_sigma<<<cdiv(n, 256), 256, 0, s>>>(n, e.fscal, e.sigma, e.iscal + IS_MARKED);
+  note_launch(2);
   const int ndir = nb * k;
   if (ndir > 0)
     k_memb_sym<<<cdiv(ndir, 256), 256, 0, s>>>(pub_idx, pub_dist, n, k, euclidean, e.sigma,
