@@ -71,6 +71,10 @@ Session::Session(const gm_params &p) : p_(p) {
   ck(cudaFree(nullptr), "CUDA context");
   ck(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
   ck(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_), "attr");
+  int host_tables = 0;
+  ck(cudaDeviceGetAttribute(&host_tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device_),
+     "attr");
+  reads_host_ = host_tables != 0;
   if (p.overlap) {
     // the embedding stream gets the higher priority: its cooperative SGD
     // launch is placed as soon as SMs free up
@@ -569,12 +573,14 @@ void Session::get_stats(gm_stats *out) {
 // ---------------------------------------------------------------------------
 // Appends rows at [n_inserted, +n_rows) of X (row stride ld; reference
 // append_host, matrix_utils.cuh:50-63, a cudaMemcpy2DAsync into stride d+1).
-// Host rows go through the ingest ring: a copy stream and two pinned staging
-// slots.  Rows already in page-locked memory are copied from where they are;
-// pageable rows are first copied into the next slot (waiting only for that
-// slot's previous transfer).  The main stream waits for the transfer on the
-// device, so the host returns as soon as it is queued and the transfer of
-// the next chunk overlaps the work still running (an overlapped embedding).
+// Host rows are copied on a stream of their own, so that the next chunk's
+// transfer runs beside work still going (an overlapped embedding); the main
+// stream waits for it on the device.  Rows in page-locked memory are copied
+// from where they are.  Pageable rows are read in place by a kernel where the
+// GPU shares the CPU's page tables (launch_copy_rows); elsewhere they go
+// through two pinned staging slots (waiting only for the slot's previous
+// transfer).  Where the caller's buffer is read, the call returns after the
+// copy, so that the buffer can be reused.
 void Session::append(const float *rows, size_t n_rows, size_t n_cols, bool on_device) {
   if (closed_) throw Error(GM_ERR_CLOSED, "session is closed");
   if (n_rows == 0) return;
@@ -600,7 +606,8 @@ void Session::append(const float *rows, size_t n_rows, size_t n_cols, bool on_de
     RingSlot &slot = ring_[ring_next_];
     ring_next_ = (ring_next_ + 1) % kRingSlots;
     const float *src = rows;
-    if (!pinned) {
+    const bool direct = !pinned && reads_host_;
+    if (!pinned && !direct) {
       const size_t bytes = n_rows * width;
       ck(cudaEventSynchronize(slot.done), "ingest slot");  // its previous transfer
       if (slot.cap < bytes) {
@@ -613,11 +620,16 @@ void Session::append(const float *rows, size_t n_rows, size_t n_cols, bool on_de
       std::memcpy(slot.buf, rows, bytes);
       src = (const float *)slot.buf;
     }
-    ck(cudaMemcpy2DAsync(dst, pitch, src, width, width, n_rows, cudaMemcpyHostToDevice, cstream_),
-       "append copy");
+    if (direct) {
+      launch_copy_rows(src, dst, n_rows, st_.d, st_.ld, sms_, cstream_);
+      ck(cudaGetLastError(), "append copy");
+    } else {
+      ck(cudaMemcpy2DAsync(dst, pitch, src, width, width, n_rows, cudaMemcpyHostToDevice, cstream_),
+         "append copy");
+    }
     ck(cudaEventRecord(slot.done, cstream_), "ingest event");
     ck(cudaStreamWaitEvent(stream_, slot.done, 0), "ingest wait");
-    if (pinned) {
+    if (pinned || direct) {
       // the caller's buffer is in use until the transfer ends: block here
       // rather than let the caller overwrite it (the slot event covers it)
       ck(cudaEventSynchronize(slot.done), "append copy");

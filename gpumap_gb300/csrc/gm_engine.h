@@ -135,8 +135,9 @@ class Session {
   bool emb_pending_ = false, snap_pending_ = false, init_wait_ = false;
   bool defer_init_ = false, init_pending_ = false;
   int init_row0_ = 0, init_nb_ = 0, init_n_ = 0;
-  // ingest ring: host-to-device row transfers on their own stream, pageable
-  // rows staged through two pinned slots
+  // ingest ring: host-to-device row transfers on their own stream; pageable
+  // rows are read in place (reads_host_) or staged through two pinned slots
+  bool reads_host_ = false;
   static constexpr int kRingSlots = 2;
   struct RingSlot {
     void *buf = nullptr;

@@ -55,6 +55,9 @@ uint64_t launch_counter();
 void fill_u32(void *p, uint32_t v, size_t n, cudaStream_t s);
 void fill_u64(void *p, unsigned long long v, size_t n, cudaStream_t s);
 void launch_counter_reset();
+// Rows x d floats at src, memory the device can read (host memory included),
+// into dst with row stride ld.
+void launch_copy_rows(const float *src, float *dst, size_t rows, int d, int ld, int sms, cudaStream_t s);
 // Exclusive scan of in[0..n) into out[0..n]; out[n] = total.  tmp needs
 // scan_tmp_ints(n) ints.
 size_t scan_tmp_ints(int n);
