@@ -712,10 +712,38 @@ GM_D void top32_merge(float &top, float u, int lane) {
   }
 }
 
-// The 32nd smallest of cnt values at v (inf when fewer than 32 are finite),
-// one warp; eight 32-value chunks are loaded together, then merged.
+// The 32nd smallest of values >= 0 (inf included), by a search over its bits:
+// the smallest x that `count` (the warp's number of values <= x) puts at 32 or
+// more; inf when there are fewer.
+template <typename F>
+GM_D float bits_32nd(F &&count) {
+  unsigned x = 0;
+#pragma unroll 1
+  for (int b = 30; b >= 0; --b)
+    if (count(__uint_as_float(x | ((1u << b) - 1u))) < kListTop) x |= 1u << b;
+  return __uint_as_float(min(x, 0x7f800000u));
+}
+
+// The 32nd smallest of cnt values >= 0 at v (inf when there are fewer), one
+// warp.  Up to 512 are held in registers and searched by bits (31 counts);
+// inserting them one at a time took 10 us a launch for 128 values, this 3 us.
+// Past that, eight 32-value chunks are loaded together, then inserted.
 GM_D float warp_32nd(const float *v, int cnt, int lane) {
   const float inf = __int_as_float(0x7f800000);
+  constexpr int kHeld = 16;
+  if (cnt <= kHeld * 32) {
+    float u[kHeld];
+#pragma unroll
+    for (int q = 0; q < kHeld; ++q) u[q] = q * 32 + lane < cnt ? v[q * 32 + lane] : inf;
+    const int used = (cnt + 31) / 32;
+    return bits_32nd([&](float x) {
+      int c = 0;
+#pragma unroll
+      for (int q = 0; q < kHeld; ++q)
+        if (q < used) c += u[q] <= x;
+      return (int)__reduce_add_sync(0xffffffffu, (unsigned)c);
+    });
+  }
   float top = inf;
   for (int c0 = 0; c0 < cnt; c0 += 8 * 32) {
     float u[8];
@@ -751,78 +779,129 @@ __global__ void __launch_bounds__(kFinalWarps * 32)
 }
 
 // Warp per batch row: the seed, the 32nd smallest of the row's chunk minima
-// from pass 0 (the largest upper bound of 32 distinct columns).
+// from pass 0 (the largest upper bound of 32 distinct columns).  Clears the
+// counters of the passes after it.
 __global__ void __launch_bounds__(kFinalWarps * 32)
-    k_seed_select(const float *mins, int mins_ld, int nrows, float *seed) {
+    k_seed_select(const float *mins, int mins_ld, int nrows, float *seed, int *row_cnt, int *pcnt,
+                  int *counter, int *pre_over) {
   const int lane = threadIdx.x & 31;
   const int ml = blockIdx.x * kFinalWarps + (threadIdx.x >> 5);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *counter = *pre_over = 0;
   if (ml >= nrows) return;
   const float T = warp_32nd(mins + (size_t)ml * mins_ld, mins_ld, lane);
-  if (lane == 0) seed[ml] = T;
+  if (lane == 0) {
+    seed[ml] = T;
+    row_cnt[ml] = pcnt[ml] = 0;
+  }
 }
 
-// Warp per batch row, after pass 3: T = the 32nd smallest stored upper
+// CTA per batch row, after pass 3: T = the 32nd smallest stored upper
 // bound (exact: every column whose upper bound is at most T was stored),
-// then the row's candidates, the stored columns with lower bound <= T.  Lane
-// l walks segments l, l + 32, ... (a row tile has at least 19 CTAs on 152
-// SMs with blocks of up to 1,024 rows); entry i of every lane's segment is
-// handled together, four entries loaded ahead.  Does nothing when a segment
-// overflowed (the heap passes then run instead).
-__global__ void __launch_bounds__(kFinalWarps * 32)
+// then the row's candidates, the stored columns with lower bound <= T.  Does
+// nothing when a segment overflowed (the heap passes then run instead).
+// The entries (about 0.8 % of the columns: the seed is a 32 / 4096 quantile)
+// are gathered from the row's segments, a warp per segment, into shared memory,
+// and the bounds, held in registers, searched by bits with one barrier a bit.
+// A warp per row that inserted the bounds one at a time was bound by latency: 33
+// us for 500 rows of ~600 entries, this form @P us.  A row with more than
+// kPreStage entries is worked through where they lie, by its first warp.
+constexpr int kPreThreads = 128, kPreWarps = kPreThreads / 32;
+constexpr int kPreStage = 2048, kPreSegs = 512;
+__global__ void __launch_bounds__(kPreThreads)
     k_pre_select(const unsigned long long *pre, const float *pre_ub, const int *pre_cnt, int gx,
-                 int cap, const int *pre_over, int nrows, int n, float *row_t, int *cand,
-                 long cand_ld, int *row_cnt, unsigned long long *stat) {
+                 int cap, const int *pre_over, int n, float *row_t, int *cand, long cand_ld,
+                 int *row_cnt, unsigned long long *stat) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, m = blockIdx.x;
   if (*pre_over) {
-    if (stat && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&stat[9], 1ull);
+    if (stat && m == 0 && threadIdx.x == 0) atomicAdd(&stat[9], 1ull);
     return;
   }
-  const int lane = threadIdx.x & 31;
-  const int m = blockIdx.x * kFinalWarps + (threadIdx.x >> 5);
-  if (m >= nrows) return;
+  __shared__ float s_ub[kPreStage];
+  __shared__ unsigned long long s_ent[kPreStage];
+  __shared__ int s_off[kPreSegs + 1], s_count[32], s_kept;
+  const unsigned full = 0xffffffffu;
   const float inf = __int_as_float(0x7f800000);
-  float top = inf;
-  for (int c0 = 0; c0 < gx; c0 += 32) {
-    const int c = c0 + lane;
-    const size_t seg = (size_t)m * gx + c;
-    const int len = c < gx ? pre_cnt[seg] : 0;
-    const float *u = pre_ub + seg * (size_t)cap;
-    int maxlen = len;
-    for (int o = 16; o > 0; o >>= 1) maxlen = max(maxlen, __shfl_xor_sync(0xffffffffu, maxlen, o));
-    for (int i0 = 0; i0 < maxlen; i0 += 4) {
-      float v[4];
+  const int *cnts = pre_cnt + (size_t)m * gx;
+  const size_t seg0 = (size_t)m * gx * (size_t)cap;
+  if (warp == 0) {
+    s_count[lane] = 0;
+    int run = 0;
+    for (int c0 = 0; c0 < gx; c0 += 32) {
+      const int v = c0 + lane < gx ? cnts[c0 + lane] : 0;
+      int incl = v;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = i0 + q < len ? u[i0 + q] : inf;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) top32_merge(top, v[q], lane);
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(full, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (c0 + lane < min(gx, kPreSegs)) s_off[c0 + lane] = run + incl - v;
+      run += __shfl_sync(full, incl, 31);
+    }
+    if (lane == 0) {
+      s_off[kPreSegs] = run;
+      s_kept = 0;
     }
   }
-  // fewer than 32 other rows: every column is a candidate
-  const float T = n - 1 < kListTop ? inf : __shfl_sync(0xffffffffu, top, 31);
+  __syncthreads();
+  const int total = s_off[kPreSegs];
   int *out = cand + (long)m * cand_ld;
-  int cnt = 0;
-  for (int c0 = 0; c0 < gx; c0 += 32) {
-    const int c = c0 + lane;
-    const size_t seg = (size_t)m * gx + c;
-    const int len = c < gx ? pre_cnt[seg] : 0;
-    const unsigned long long *e = pre + seg * (size_t)cap;
-    int maxlen = len;
-    for (int o = 16; o > 0; o >>= 1) maxlen = max(maxlen, __shfl_xor_sync(0xffffffffu, maxlen, o));
-    for (int i0 = 0; i0 < maxlen; i0 += 4) {
-      unsigned long long v[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = i0 + q < len ? e[i0 + q] : 0ull;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const bool keep = i0 + q < len && __uint_as_float((unsigned)(v[q] >> 32)) <= T;
-        const unsigned bal = __ballot_sync(0xffffffffu, keep);
-        if (keep) out[cnt + __popc(bal & ((1u << lane) - 1u))] = (int)(unsigned)v[q];
-        cnt += __popc(bal);
+  auto keep = [&](bool in, unsigned long long e, float T) {
+    const bool ok = in && __uint_as_float((unsigned)(e >> 32)) <= T;
+    const unsigned bal = __ballot_sync(full, ok);
+    int base = 0;
+    if (lane == 0 && bal) base = atomicAdd(&s_kept, __popc(bal));
+    base = __shfl_sync(full, base, 0);
+    if (ok) out[base + __popc(bal & ((1u << lane) - 1u))] = (int)(unsigned)e;
+  };
+  float T = inf;
+  if (total <= kPreStage && gx <= kPreSegs) {
+    for (int c = warp; c < gx; c += kPreWarps) {
+      const int off = s_off[c], len = (c + 1 < gx ? s_off[c + 1] : total) - off;
+      const size_t from = seg0 + (size_t)c * cap;
+      for (int i = lane; i < len; i += 32) {
+        s_ub[off + i] = pre_ub[from + i];
+        s_ent[off + i] = pre[from + i];
       }
     }
+    __syncthreads();
+    float u[kPreStage / kPreThreads];
+#pragma unroll
+    for (int q = 0; q < kPreStage / kPreThreads; ++q) {
+      const int i = q * kPreThreads + threadIdx.x;
+      u[q] = i < total ? s_ub[i] : inf;
+    }
+    const int used = (total + kPreThreads - 1) / kPreThreads;
+    int bit = 30;
+    T = bits_32nd([&](float x) {
+      int c = 0;
+#pragma unroll
+      for (int q = 0; q < kPreStage / kPreThreads; ++q)
+        if (q < used) c += u[q] <= x;
+      c = (int)__reduce_add_sync(full, (unsigned)c);
+      if (lane == 0 && c) atomicAdd(&s_count[bit], c);
+      __syncthreads();
+      return s_count[bit--];
+    });
+    // fewer than 32 other rows: every column is a candidate
+    if (n - 1 < kListTop) T = inf;
+    for (int i = warp * 32; i < total; i += kPreThreads)
+      keep(i + lane < total, i + lane < total ? s_ent[i + lane] : 0ull, T);
+  } else if (warp == 0) {
+    T = bits_32nd([&](float x) {
+      int c = 0;
+      for (int g = 0; g < gx; ++g)
+        for (int i = lane; i < cnts[g]; i += 32) c += pre_ub[seg0 + (size_t)g * cap + i] <= x;
+      return (int)__reduce_add_sync(full, (unsigned)c);
+    });
+    if (n - 1 < kListTop) T = inf;
+    for (int g = 0; g < gx; ++g)
+      for (int i = 0; i < cnts[g]; i += 32)
+        keep(i + lane < cnts[g], i + lane < cnts[g] ? pre[seg0 + (size_t)g * cap + i + lane] : 0ull, T);
   }
-  if (lane == 0) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
     row_t[m] = T;
-    row_cnt[m] = cnt;
+    row_cnt[m] = s_kept;
     if (stat) atomicAdd(&stat[5], (unsigned long long)n);
   }
 }
@@ -913,6 +992,23 @@ __global__ void __launch_bounds__(kRescoreWarps * 32)
   }
 }
 
+// Exact top 32 of a row's candidates, a warp per row: chunks of 32 keys are
+// sorted by a bitonic network and merged with the 32 smallest so far (the
+// elementwise minimum of one list and the other reversed is bitonic and holds
+// the 32 smallest of both).  Inserting one key at a time took 10.3 us for 500
+// rows of ~100 candidates, this @R us.
+GM_D Key bitonic_step(Key k, int partner, bool up) {
+  const Key o = __shfl_xor_sync(0xffffffffu, k, partner);
+  return ((threadIdx.x & partner) == 0) == up ? (k < o ? k : o) : (k < o ? o : k);
+}
+GM_D Key warp_sort32(Key k) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int size = 2; size <= 32; size *= 2)
+#pragma unroll
+    for (int j = size / 2; j > 0; j /= 2) k = bitonic_step(k, j, (lane & size) == 0);
+  return k;
+}
 constexpr int kRowWarps = 4;
 __global__ void k_row_select(const float *cand_d, int brow0, int nrows, const int *cand,
                              long cand_ld, const int *row_cnt, Key *g_key,
@@ -926,17 +1022,13 @@ __global__ void k_row_select(const float *cand_d, int brow0, int nrows, const in
   Key mine = kEmptyKey;
   for (int c0 = 0; c0 < cnt; c0 += 32) {
     const int c = c0 + lane;
-    const Key ck = c < cnt ? make_key(dr[c], cl[c]) : ~(Key)0;
-    // insert the (up to) 32 new keys one at a time into the sorted warp list
-    for (int src = 0; src < 32 && c0 + src < cnt; ++src) {
-      const Key k = __shfl_sync(0xffffffffu, ck, src);
-      const unsigned msk = __ballot_sync(0xffffffffu, k < mine);
-      if (!msk) continue;
-      const int pos = __ffs(msk) - 1;
-      const Key prev = __shfl_up_sync(0xffffffffu, mine, 1);
-      if (lane > pos) mine = prev;
-      else if (lane == pos) mine = k;
-    }
+    Key ck = c < cnt ? make_key(dr[c], cl[c]) : ~(Key)0;
+    if (!__any_sync(0xffffffffu, ck < __shfl_sync(0xffffffffu, mine, 31))) continue;
+    ck = warp_sort32(ck);
+    ck = __shfl_sync(0xffffffffu, ck, 31 - lane);
+    mine = ck < mine ? ck : mine;
+#pragma unroll
+    for (int j = 16; j > 0; j /= 2) mine = bitonic_step(mine, j, true);
   }
   g_key[(size_t)(brow0 + ml) * kListW + lane] = mine;
   if (stat && lane == 0) atomicAdd(&stat[6], (unsigned long long)cnt);
@@ -1076,8 +1168,6 @@ void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int ro
   // CTAs per row tile so that the grid covers the SMs once
   const int gx = std::max(1, std::min(n_tiles, std::max(1, sms / m_tiles)));
   const bool kd = keep_d && x.D;
-  cudaMemsetAsync(x.row_cnt, 0, (size_t)nrows * sizeof(int), s);
-  cudaMemsetAsync(x.counter, 0, sizeof(int), s);
   const int tiles = exact_seed_tiles(n_tiles);
   // entries per stored segment: the row's whole allocation shared by its
   // tile's CTAs (fewer CTAs per row tile, longer segments)
@@ -1090,16 +1180,16 @@ void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int ro
     const int mins_ld = tiles * (kTN / 32);
     launch_tile<0, false>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx0, m_tiles, tiles, stride,
                           nullptr, 0, mins_ld, 0, nullptr, s);
-    k_seed_select<<<cdiv(nrows, kFinalWarps), kFinalWarps * 32, 0, s>>>(x.mins, mins_ld, nrows, x.seed);
-    cudaMemsetAsync(x.pre_over, 0, sizeof(int), s);
+    k_seed_select<<<cdiv(nrows, kFinalWarps), kFinalWarps * 32, 0, s>>>(
+        x.mins, mins_ld, nrows, x.seed, x.row_cnt, x.pcnt, x.counter, x.pre_over);
     if (kd)
       launch_tile<3, true>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx, m_tiles, n_tiles, 1, x.seed,
                            cap, 0, 0, nullptr, s);
     else
       launch_tile<3, false>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx, m_tiles, n_tiles, 1, x.seed,
                             cap, 0, 0, nullptr, s);
-    k_pre_select<<<cdiv(nrows, kFinalWarps), kFinalWarps * 32, 0, s>>>(
-        x.pre, x.pre_ub, x.pre_cnt, gx, cap, x.pre_over, nrows, n, x.row_t, x.cand, ldD, x.row_cnt,
+    k_pre_select<<<nrows, kPreThreads, 0, s>>>(
+        x.pre, x.pre_ub, x.pre_cnt, gx, cap, x.pre_over, n, x.row_t, x.cand, ldD, x.row_cnt,
         st.stat);
     note_launch(2);
     // after an overflow only: the heap pass (seed-capped; its pairs were
@@ -1113,6 +1203,9 @@ void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int ro
                           0, 0, x.pre_over, s);
     return;
   }
+  cudaMemsetAsync(x.row_cnt, 0, (size_t)nrows * sizeof(int), s);
+  cudaMemsetAsync(x.pcnt, 0, (size_t)nrows * sizeof(int), s);
+  cudaMemsetAsync(x.counter, 0, sizeof(int), s);
   if (kd)
     launch_tile<1, true>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx, m_tiles, n_tiles, 1, nullptr, 0,
                          0, 1, nullptr, s);
@@ -1134,7 +1227,6 @@ void launch_exact_screen(const DevState &st, int row0, int blk0, int nrows, int 
   // the pairs as found are done with once placed: pool_m holds the chains
   const OfferChains chains{x.heads, x.pool_m};
   if (row0 > 0) {
-    cudaMemsetAsync(x.pcnt, 0, (size_t)nrows * sizeof(int), s);
     k_pool_count<<<grid, 256, 0, s>>>(x.pool_m, x.counter, x.pool_cap, nrows, x.pcnt, st.stat);
     k_pool_offsets<<<1, kMaxBlockRows, 0, s>>>(nrows, x.pcnt, x.poff, x.pfill);
     k_pool_place<<<grid, 256, 0, s>>>(x.pool_j, x.pool_m, x.counter, x.pool_cap, x.pfill, x.pair_j, x.pair_m);
