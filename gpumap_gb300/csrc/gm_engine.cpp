@@ -74,7 +74,10 @@ Session::Session(const gm_params &p) : p_(p) {
   int host_tables = 0;
   ck(cudaDeviceGetAttribute(&host_tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device_),
      "attr");
-  reads_host_ = host_tables != 0;
+  // (not in overlap mode: beside the SGD the reads take 154 us for 500 rows x
+  // 784 instead of 18, and the staging copy is hidden behind it: 163.7 ms for a
+  // 70k x 784 build against 159.7 staged)
+  reads_host_ = host_tables != 0 && !p.overlap;
   if (p.overlap) {
     // the embedding stream gets the higher priority: its cooperative SGD
     // launch is placed as soon as SMs free up
@@ -989,13 +992,18 @@ uint32_t Session::embed(uint32_t n_ops) {
     ck(cudaEventRecord(ev_snap_, s), "record snapshot");
     snap_pending_ = true;
     if (emb_pending_) ck(cudaStreamWaitEvent(s, ev_emb_, 0), "wait embedding");
-    if (init_pending_) {
-      launch_embed_init(st_, init_row0_, init_nb_, init_n_, s);
+    const bool init = init_pending_;
+    if (init) launch_embed_init(st_, init_row0_, init_nb_, init_n_, s);
+    launch_add_noise(st_.emb, ni, es_.batch, nb, 0.001f, noise_seed, es_, s);
+    if (init) {
+      // recorded last before the SGD: what waits for it (the next insertion's
+      // screen) fills every SM, and a cooperative launch that comes after it
+      // waits for half of them to drain (35 us a cycle when recorded before
+      // the noise)
       ck(cudaEventRecord(ev_init_, s), "record row embedding");
       init_pending_ = false;
       init_wait_ = true;
     }
-    launch_add_noise(st_.emb, ni, es_.batch, nb, 0.001f, noise_seed, es_, s);
   }
   timed_begin(2, s);
   run_sgd((int)std::min<size_t>(2 * (size_t)nb * (size_t)k, INT32_MAX), s);
