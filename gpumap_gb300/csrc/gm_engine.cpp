@@ -16,6 +16,8 @@
 #include <numeric>
 #include <unordered_set>
 
+#include <unistd.h>
+
 namespace gm {
 
 namespace {
@@ -624,6 +626,13 @@ void Session::append(const float *rows, size_t n_rows, size_t n_cols, bool on_de
       src = (const float *)slot.buf;
     }
     if (direct) {
+      // one read per page on the CPU: a page whose entry the kernel has
+      // withdrawn for a moment (NUMA balancing does, also of a VM on its host) costs the
+      // GPU a fault of 0.7 ms, the CPU one of a microsecond
+      static const size_t page = (size_t)std::max<long>(sysconf(_SC_PAGESIZE), 4096);
+      const volatile char *b = (const volatile char *)rows;
+      for (size_t at = 0; at < n_rows * width; at += page) (void)b[at];
+      (void)b[n_rows * width - 1];
       launch_copy_rows(src, dst, n_rows, st_.d, st_.ld, sms_, cstream_);
       ck(cudaGetLastError(), "append copy");
     } else {
