@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "gm_engine.h"
+#include "gm_pool.h"
 #include "../../include/gpumap_gb300.h"
 #include "../../include/gpumap_gb300_ops.h"
 
@@ -316,11 +317,12 @@ int gm_op_fuzzy_schedule(const uint32_t *pub_idx, const float *pub_dist, int64_t
   return guarded([&] {
     gm::EmbedScratch e;
     std::vector<void *> al;
+    int dev = 0;
+    cudaGetDevice(&dev);
     auto dalloc = [&](size_t bytes) {
       void *p = nullptr;
-      if (cudaMalloc(&p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
-        cudaGetLastError();
-        for (void *q : al) cudaFree(q);
+      if (gm::device_alloc(&p, std::max<size_t>(bytes, 16), dev, s) != cudaSuccess) {
+        for (void *q : al) gm::device_free(q, s);
         throw gm::Error(GM_ERR_OOM, "cudaMalloc");
       }
       al.push_back(p);
@@ -358,7 +360,7 @@ int gm_op_fuzzy_schedule(const uint32_t *pub_idx, const float *pub_dist, int64_t
     cudaMemcpyAsync(iscal, e.iscal, sizeof(iscal), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(fscal, e.fscal, sizeof(fscal), cudaMemcpyDeviceToHost, s);
     const cudaError_t err = cudaStreamSynchronize(s);
-    for (void *q : al) cudaFree(q);
+    for (void *q : al) gm::device_free(q, s);
     if (err != cudaSuccess) throw gm::Error(GM_ERR_CUDA, cudaGetErrorString(err));
     if (counts_out) {
       counts_out[0] = iscal[0];
@@ -384,12 +386,15 @@ int gm_op_sgd(float *emb, int64_t n, const int32_t *head, const int32_t *tail,
   return guarded([&] {
     if (nnz == 0 || n_epochs == 0) return;
     void *ns = nullptr, *nn = nullptr, *sc = nullptr;
-    if (cudaMalloc(&ns, (size_t)nnz * 4) != cudaSuccess || cudaMalloc(&nn, (size_t)nnz * 4) != cudaSuccess ||
-        cudaMalloc(&sc, 128) != cudaSuccess) {
-      cudaGetLastError();
-      cudaFree(ns);
-      cudaFree(nn);
-      cudaFree(sc);
+    int dev = 0;
+    cudaGetDevice(&dev);
+    auto release = [&] {
+      for (void *q : {ns, nn, sc}) gm::device_free(q, s);
+    };
+    if (gm::device_alloc(&ns, (size_t)nnz * 4, dev, s) != cudaSuccess ||
+        gm::device_alloc(&nn, (size_t)nnz * 4, dev, s) != cudaSuccess ||
+        gm::device_alloc(&sc, 128, dev, s) != cudaSuccess) {
+      release();
       throw gm::Error(GM_ERR_OOM, "cudaMalloc");
     }
     int iscal[16] = {0};
@@ -400,8 +405,6 @@ int gm_op_sgd(float *emb, int64_t n, const int32_t *head, const int32_t *tail,
     cudaMemcpyAsync(sc, iscal, 64, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync((char *)sc + 64, fscal, 64, cudaMemcpyHostToDevice, s);
     gm::launch_epoch_init(eps, (int)nnz, neg_rate, (float *)ns, (float *)nn, s);
-    int dev = 0;
-    cudaGetDevice(&dev);
     // scalars: iscal[0..16) at sc, fscal at sc + 64; grid-barrier words in
     // iscal[8..9], device error word in iscal[10]
     int *isc = (int *)sc;
@@ -413,9 +416,7 @@ int gm_op_sgd(float *emb, int64_t n, const int32_t *head, const int32_t *tail,
     if (le == cudaSuccess) cudaMemcpyAsync(&dev_err, isc + 10, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
     const cudaError_t err = le != cudaSuccess ? le : cudaStreamSynchronize(s);
     if (le != cudaSuccess) cudaGetLastError();
-    cudaFree(ns);
-    cudaFree(nn);
-    cudaFree(sc);
+    release();
     if (err != cudaSuccess) throw gm::Error(GM_ERR_CUDA, cudaGetErrorString(err));
     if (dev_err) throw gm::Error(GM_ERR_DEVICE, "SGD grid barrier wait ran out");
   });

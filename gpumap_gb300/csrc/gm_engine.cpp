@@ -6,6 +6,7 @@
 #include "gm_engine.h"
 
 #include "gm_common.cuh"
+#include "gm_pool.h"
 
 #include <algorithm>
 #include <cfloat>
@@ -101,7 +102,7 @@ Session::Session(const gm_params &p) : p_(p) {
 
   auto dalloc = [&](size_t bytes) -> void * {
     void *ptr = nullptr;
-    ck(cudaMalloc(&ptr, std::max<size_t>(bytes, 16)), "cudaMalloc");
+    ck(device_alloc(&ptr, std::max<size_t>(bytes, 16), device_, stream_), "cudaMalloc");
     allocs_.push_back(ptr);
     fixed_bytes_ += std::max<size_t>(bytes, 16);
     return ptr;
@@ -167,10 +168,10 @@ Session::Session(const gm_params &p) : p_(p) {
     alloc_side(es_, es_cnt_);
     if (p.overlap) alloc_side(es_alt_, es_cnt_alt_);
 
-    ck(cudaMallocHost((void **)&h_pin_, (Nm + 64) * sizeof(uint32_t)), "cudaMallocHost");
-    ck(cudaMallocHost((void **)&h_emb_pin_, (Nm + 64) * sizeof(uint32_t)), "cudaMallocHost");
-    if (p.overlap)
-      ck(cudaMallocHost((void **)&h_emb_pin_alt_, (Nm + 64) * sizeof(uint32_t)), "cudaMallocHost");
+    pin_bytes_ = (Nm + 64) * sizeof(uint32_t);
+    ck(host_alloc((void **)&h_pin_, pin_bytes_), "cudaMallocHost");
+    ck(host_alloc((void **)&h_emb_pin_, pin_bytes_), "cudaMallocHost");
+    if (p.overlap) ck(host_alloc((void **)&h_emb_pin_alt_, pin_bytes_), "cudaMallocHost");
     if (p.precision == 1) {
       // split-BF16 shadow rows (hi | lo, 2 x dh bf16 each) plus a block of
       // candidate / pair scratch for the worst case (every column a
@@ -217,11 +218,7 @@ Session::Session(const gm_params &p) : p_(p) {
       xs_.counter = (int *)dalloc(16 * sizeof(int));
     }
   } catch (...) {
-    for (void *q : allocs_) cudaFree(q);
-    allocs_.clear();
-    if (h_pin_) cudaFreeHost(h_pin_);
-    if (h_emb_pin_) cudaFreeHost(h_emb_pin_);
-    if (h_emb_pin_alt_) cudaFreeHost(h_emb_pin_alt_);
+    release_memory();
     release_streams();
     throw;
   }
@@ -255,14 +252,7 @@ Session::Session(const gm_params &p) : p_(p) {
   ck(cudaStreamSynchronize(s), "init sync");
   if (xh_) {
     if (!make_row_maps(xh_, (int)Nm, dh_, &maps_)) {
-      for (void *q : allocs_) cudaFree(q);
-      allocs_.clear();
-      cudaFreeHost(h_pin_);
-      h_pin_ = nullptr;
-      cudaFreeHost(h_emb_pin_);
-      h_emb_pin_ = nullptr;
-      if (h_emb_pin_alt_) cudaFreeHost(h_emb_pin_alt_);
-      h_emb_pin_alt_ = nullptr;
+      release_memory();
       release_streams();
       throw Error(GM_ERR_CUDA, "cuTensorMapEncodeTiled unavailable or failed");
     }
@@ -270,6 +260,17 @@ Session::Session(const gm_params &p) : p_(p) {
   upd_q_.reset(N);
   ensure_embed(es_, 1);
   if (p.overlap) ensure_embed(es_alt_, 1);
+}
+
+// The fixed buffers, after every stream has been waited for.
+void Session::release_memory() {
+  if (stream_) cudaStreamSynchronize(stream_);
+  for (void *q : allocs_) device_free(q, stream_);
+  allocs_.clear();
+  for (uint32_t **h : {&h_pin_, &h_emb_pin_, &h_emb_pin_alt_}) {
+    host_free(*h, pin_bytes_);
+    *h = nullptr;
+  }
 }
 
 void Session::release_streams() {
@@ -294,31 +295,33 @@ void Session::free_embed(EmbedScratch &e) {
   for (void *q : {(void *)e.coo_row, (void *)e.coo_col, (void *)e.coo_val, (void *)e.t_row,
                   (void *)e.t_col, (void *)e.flag_tail, (void *)e.t_val, (void *)e.next_s,
                   (void *)e.next_n, (void *)e.tmp2})
-    cudaFree(q);
+    device_free(q, stream_);
   e.coo_row = nullptr;
   e.cap_coo = 0;
 }
 
 Session::~Session() {
-  for (cudaStream_t q : {stream_, estream_, estream_alt_})
-    if (q) cudaStreamSynchronize(q);
+  // everything on the device: a consumer's stream may still be reading a view,
+  // and the pool hands the memory on (cudaFree would have waited as well)
+  int current = 0;
+  cudaGetDevice(&current);
+  if (current != device_) cudaSetDevice(device_);
+  cudaDeviceSynchronize();
+  if (current != device_) cudaSetDevice(current);
   for (auto &e : ev_pool_) cudaEventDestroy(e);
   for (auto &pr : ev_pending_) {
     cudaEventDestroy(pr.a);
     cudaEventDestroy(pr.b);
   }
-  for (void *q : allocs_) cudaFree(q);
+  if (cstream_) cudaStreamSynchronize(cstream_);
   free_cand();
-  if (join_pool_) cudaFree(join_pool_);
+  device_free(join_pool_, stream_);
   free_embed(es_);
   free_embed(es_alt_);
-  if (h_pin_) cudaFreeHost(h_pin_);
-  if (h_emb_pin_) cudaFreeHost(h_emb_pin_);
-  if (h_emb_pin_alt_) cudaFreeHost(h_emb_pin_alt_);
-  if (cstream_) cudaStreamSynchronize(cstream_);
+  release_memory();
   for (auto &slot : ring_) {
     if (slot.done) cudaEventDestroy(slot.done);
-    if (slot.buf) cudaFreeHost(slot.buf);
+    host_free(slot.buf, slot.cap);
   }
   if (cstream_) cudaStreamDestroy(cstream_);
   release_streams();
@@ -372,7 +375,7 @@ void Session::check_device_error(const char *phase) {
 void Session::free_cand() {
   for (void *q : {(void *)cs_.cand, (void *)cs_.cnt, (void *)cs_.dist, (void *)cs_.todo,
                   (void *)cs_.todo_cnt, (void *)cs_.next})
-    if (q) cudaFree(q);
+    device_free(q, stream_);
   cs_ = CandScratch{};
   cand_rows_ = 0;
 }
@@ -382,7 +385,9 @@ void Session::ensure_cand(size_t rows) {
   sync();
   free_cand();
   const size_t r = std::max<size_t>(rows, 1024), slots = r * kMaxCand;
-  auto get = [&](auto *&p, size_t n) { ck(cudaMalloc(&p, n * sizeof(*p)), "cudaMalloc cand"); };
+  auto get = [&](auto *&p, size_t n) {
+    ck(device_alloc((void **)&p, n * sizeof(*p), device_, stream_), "cudaMalloc cand");
+  };
   get(cs_.cand, slots);
   get(cs_.cnt, r);
   get(cs_.dist, slots);
@@ -399,16 +404,17 @@ void Session::ensure_join(size_t words) {
   const size_t w = join_part(words);
   if (w <= join_words_) return;
   sync();
-  if (join_pool_) cudaFree(join_pool_);
+  device_free(join_pool_, stream_);
   join_pool_ = nullptr;
   join_words_ = 0;
-  ck(cudaMalloc(&join_pool_, (w + kJoinSlackWords) * sizeof(int)), "cudaMalloc join");
+  ck(device_alloc((void **)&join_pool_, (w + kJoinSlackWords) * sizeof(int), device_, stream_),
+     "cudaMalloc join");
   join_words_ = w;
 }
 
 void Session::set_join_part(size_t words) {
   drain();
-  if (join_pool_) cudaFree(join_pool_);
+  device_free(join_pool_, stream_);
   join_pool_ = nullptr;
   join_words_ = 0;
   join_part_max_ = std::max<size_t>(2, std::min(words, kJoinPartWords) & ~(size_t)1);
@@ -425,7 +431,7 @@ void Session::set_keep_tile(bool on) {
     drain();
     const size_t bytes = (size_t)ex_block_ * std::max<size_t>(p_.n_instances, 1) * sizeof(float);
     void *ptr = nullptr;
-    ck(cudaMalloc(&ptr, bytes), "cudaMalloc tile");
+    ck(device_alloc(&ptr, bytes, device_, stream_), "cudaMalloc tile");
     allocs_.push_back(ptr);
     fixed_bytes_ += bytes;
     ex_D_ = (float *)ptr;
@@ -470,16 +476,20 @@ void Session::ensure_embed(EmbedScratch &e, size_t nb) {
   sync_embed_streams();
   free_embed(e);
   const size_t c = std::max(need, (size_t)4096);
-  ck(cudaMalloc(&e.coo_row, c * sizeof(int)), "cudaMalloc coo");
-  ck(cudaMalloc(&e.coo_col, c * sizeof(int)), "cudaMalloc coo");
-  ck(cudaMalloc(&e.coo_val, c * sizeof(float)), "cudaMalloc coo");
-  ck(cudaMalloc(&e.t_row, c * sizeof(int)), "cudaMalloc coo");
-  ck(cudaMalloc(&e.t_col, c * sizeof(int)), "cudaMalloc coo");
-  ck(cudaMalloc(&e.flag_tail, c * sizeof(int)), "cudaMalloc coo");
-  ck(cudaMalloc(&e.t_val, c * sizeof(float)), "cudaMalloc coo");
-  ck(cudaMalloc(&e.next_s, c * sizeof(float)), "cudaMalloc coo");
-  ck(cudaMalloc(&e.next_n, c * sizeof(float)), "cudaMalloc coo");
-  ck(cudaMalloc(&e.tmp2, (compact_tmp_ints((int)c) + 64) * sizeof(int)), "cudaMalloc coo");
+  auto get = [&](auto *&p, size_t n) {
+    ck(device_alloc((void **)&p, n * sizeof(*p), device_, stream_), "cudaMalloc coo");
+  };
+  get(e.coo_row, c);
+  get(e.coo_col, c);
+  get(e.coo_val, c);
+  get(e.t_row, c);
+  get(e.t_col, c);
+  get(e.flag_tail, c);
+  get(e.t_val, c);
+  get(e.next_s, c);
+  get(e.next_n, c);
+  get(e.tmp2, compact_tmp_ints((int)c) + 64);
+  sync();  // (the embedding may run on another stream)
   e.cap_coo = c;
 }
 
@@ -616,10 +626,10 @@ void Session::append(const float *rows, size_t n_rows, size_t n_cols, bool on_de
       const size_t bytes = n_rows * width;
       ck(cudaEventSynchronize(slot.done), "ingest slot");  // its previous transfer
       if (slot.cap < bytes) {
-        if (slot.buf) cudaFreeHost(slot.buf);
+        host_free(slot.buf, slot.cap);
         slot.buf = nullptr;
         slot.cap = 0;
-        ck(cudaMallocHost(&slot.buf, std::max<size_t>(bytes, (size_t)8 << 20)), "cudaMallocHost ingest");
+        ck(host_alloc(&slot.buf, std::max<size_t>(bytes, (size_t)8 << 20)), "cudaMallocHost ingest");
         slot.cap = std::max<size_t>(bytes, (size_t)8 << 20);
       }
       std::memcpy(slot.buf, rows, bytes);

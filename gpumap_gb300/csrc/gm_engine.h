@@ -112,6 +112,7 @@ class Session {
   template <typename... A> void log(const char *fmt, A... a) const;
   void sync();
   void release_streams();
+  void release_memory();
   void timed_begin(int slot, cudaStream_t s = nullptr);
   void timed_end(int slot, cudaStream_t s = nullptr);
   void collect_timings(bool block = true);
@@ -163,6 +164,7 @@ class Session {
   int *d_rows_ = nullptr, *d_rows2_ = nullptr, *d_batch_ = nullptr;
   int *d_cnt_ = nullptr;  // [0] list count, [1] edges, [2] report count, [3] join count
   int *d_tmp_ = nullptr;
+  size_t pin_bytes_ = 0;           // of each pinned staging buffer
   uint32_t *h_pin_ = nullptr;      // pinned staging (n_cap + 16 words)
   uint32_t *h_emb_pin_ = nullptr;  // the embedding phase's pinned staging
   int *es_cnt_ = nullptr;          // the embedding phase's compaction counter

@@ -10,6 +10,8 @@ queued work on torch's current stream), else the engine's view object.
 """
 from __future__ import annotations
 
+import functools
+
 import numpy as np
 from scipy.optimize import curve_fit
 
@@ -33,17 +35,24 @@ def find_ab_params(spread, min_dist):
     return params[0], params[1]
 
 
+@functools.cache
+def _cupy():
+    """CuPy, or None (a failing import searches the whole path every time)."""
+    try:
+        import cupy
+    except ImportError:
+        return None
+    return cupy
+
+
 def _device_array(view):
     """A device array over an engine view: CuPy through the CUDA Array
     Interface when CuPy is installed, else a torch tensor through DLPack (the
     view makes torch's current stream wait for the session's queued work),
     else the view itself.  The memory stays the engine's."""
-    try:
-        import cupy as cp  # noqa: F401
-
+    cp = _cupy()
+    if cp is not None:
         return cp.asarray(view)
-    except ImportError:
-        pass
     try:
         import torch
     except ImportError:
