@@ -119,7 +119,6 @@ Session::Session(const gm_params &p) : p_(p) {
     st_.pub_dist = (float *)dalloc(Nm * (k + 1) * sizeof(float));
     st_.emb = (float *)dalloc(Nm * 2 * sizeof(float));
     st_.bloom = (uint32_t *)dalloc(Nm * 64 * sizeof(uint32_t));
-    st_.err = (unsigned *)dalloc(16);
     d_stat_ = (unsigned long long *)dalloc(16 * sizeof(unsigned long long));
     st_.stat = d_stat_;
 
@@ -137,7 +136,8 @@ Session::Session(const gm_params &p) : p_(p) {
     d_rows_ = (int *)dalloc(Nm * sizeof(int));
     d_rows2_ = (int *)dalloc(Nm * sizeof(int));
     d_batch_ = (int *)dalloc(Nm * sizeof(int));
-    d_cnt_ = (int *)dalloc((16 + kInsertIters) * sizeof(int));
+    d_cnt_ = (int *)dalloc(kCounters * sizeof(int));
+    st_.err = (unsigned *)(d_cnt_ + kErrAt);
     d_tmp_ = (int *)dalloc(std::max(scan_tmp_ints((int)Nm), compact_tmp_ints((int)Nm)) *
                            sizeof(int) + 64);
 
@@ -168,7 +168,7 @@ Session::Session(const gm_params &p) : p_(p) {
     alloc_side(es_, es_cnt_);
     if (p.overlap) alloc_side(es_alt_, es_cnt_alt_);
 
-    pin_bytes_ = (Nm + 64) * sizeof(uint32_t);
+    pin_bytes_ = (Nm + kCounters) * sizeof(uint32_t);
     ck(host_alloc((void **)&h_pin_, pin_bytes_), "cudaMallocHost");
     ck(host_alloc((void **)&h_emb_pin_, pin_bytes_), "cudaMallocHost");
     if (p.overlap) ck(host_alloc((void **)&h_emb_pin_alt_, pin_bytes_), "cudaMallocHost");
@@ -237,7 +237,7 @@ Session::Session(const gm_params &p) : p_(p) {
   fill_u32(st_.pub_dist, kFltMaxBits, Nm * (k + 1), s);
   ck(cudaMemsetAsync(st_.emb, 0, Nm * 2 * sizeof(float), s), "memset");
   ck(cudaMemsetAsync(st_.bloom, 0, Nm * 64 * sizeof(uint32_t), s), "memset");
-  ck(cudaMemsetAsync(st_.err, 0, 16, s), "memset");
+  ck(cudaMemsetAsync(d_cnt_, 0, kCounters * sizeof(int), s), "memset");
   ck(cudaMemsetAsync(d_stat_, 0, 16 * sizeof(unsigned long long), s), "memset");
   ck(cudaMemsetAsync(us_.sizes, 0, Nm * sizeof(int4), s), "memset");
   for (EmbedScratch *e : {&es_, &es_alt_}) {
@@ -362,14 +362,39 @@ void Session::check_launch_error(const char *phase) {
 
 void Session::check_device_error(const char *phase) {
   check_launch_error(phase);
-  unsigned e = 0;
-  ck(cudaMemcpyAsync(&e, st_.err, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_), "err");
+  ck(cudaMemcpyAsync(h_pin_ + kErrAt, st_.err, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_), "err");
   sync();
-  if (e != 0u) {
-    cudaMemsetAsync(st_.err, 0, sizeof(unsigned), stream_);
-    throw Error(GM_ERR_DEVICE, std::string(phase) + ": a bounded device wait ran out (bits " +
-                                   std::to_string(e) + ")");
+  report_device_error(phase, h_pin_[kErrAt]);
+}
+
+void Session::report_device_error(const char *phase, unsigned e) {
+  if (e == 0u) return;
+  cudaMemsetAsync(st_.err, 0, sizeof(unsigned), stream_);
+  throw Error(GM_ERR_DEVICE, std::string(phase) + ": a bounded device wait ran out (bits " +
+                                 std::to_string(e) + ")");
+}
+
+// Ends a phase that compacted a row list into d_rows_ (count in d_cnt_[0], at
+// most `bound` rows): its counters, error word and first rows come in one wait
+// (three waits, for the count, the rows and the error word, were 30 us a
+// phase).  Counters are then at h_pin_, the rows after them; returns their
+// number.
+size_t Session::finish_phase(const char *phase, size_t bound) {
+  check_launch_error(phase);
+  const size_t ahead = std::min(bound, kRowsAhead);
+  uint32_t *rows = h_pin_ + kCounters;
+  ck(cudaMemcpyAsync(h_pin_, d_cnt_, kCounters * sizeof(int), cudaMemcpyDeviceToHost, stream_), "counts");
+  if (ahead)
+    ck(cudaMemcpyAsync(rows, d_rows_, ahead * sizeof(int), cudaMemcpyDeviceToHost, stream_), "rows");
+  sync();
+  report_device_error(phase, h_pin_[kErrAt]);
+  const size_t n = h_pin_[0];
+  if (n > ahead) {
+    ck(cudaMemcpyAsync(rows + ahead, d_rows_ + ahead, (n - ahead) * sizeof(int), cudaMemcpyDeviceToHost,
+                       stream_), "rows");
+    sync();
   }
+  return n;
 }
 
 void Session::free_cand() {
@@ -675,8 +700,6 @@ gm_result Session::run(uint32_t n_ins, uint32_t n_upd, uint32_t n_emb) {
   if (!ins_done_) {
     const auto t0 = Clock::now();
     r.n_insertion_ops = insert(n_ins);
-    sync();
-    check_device_error("insertion");
     const auto t1 = Clock::now();
     r.insertion_time = std::chrono::duration<float>(t1 - t0).count();
     ins_done_ = (ins_head_ == n_inserted_) && n_inserted_ == p_.n_instances;
@@ -686,8 +709,6 @@ gm_result Session::run(uint32_t n_ins, uint32_t n_upd, uint32_t n_emb) {
     size_t changed = 0;
     const auto t0 = Clock::now();
     r.n_update_ops = update(n_upd, changed);
-    sync();
-    check_device_error("update");
     const auto t1 = Clock::now();
     r.n_update_changed_edges = changed;
     r.update_time = std::chrono::duration<float>(t1 - t0).count();
@@ -699,7 +720,6 @@ gm_result Session::run(uint32_t n_ins, uint32_t n_upd, uint32_t n_emb) {
     const auto t0 = Clock::now();
     r.n_embedding_ops = embed(n_emb);
     if (!p_.overlap) {
-      sync();
       check_device_error("embedding");
     } else {
       check_launch_error("embedding");
@@ -781,7 +801,7 @@ uint32_t Session::insert(uint32_t n_ops) {
   } else {
     ensure_cand(B);
     wait_init();
-    launch_nnd_insert(st_, us_, row0, nb, n, window_start, seed, cs_, d_cnt_ + 16, sms_,
+    launch_nnd_insert(st_, us_, row0, nb, n, window_start, seed, cs_, d_cnt_ + kFlagsAt, sms_,
                       [this](bool begin) { begin ? timed_begin(1) : timed_end(1); }, s);
   }
   // existing rows whose list changed, ascending
@@ -802,18 +822,11 @@ uint32_t Session::insert(uint32_t n_ops) {
     if (emb_pending_) ck(cudaStreamWaitEvent(s, ev_emb_, 0), "wait embedding");
     launch_embed_init(st_, row0, nb, n, s);
   }
-  ck(cudaMemcpyAsync(h_pin_, d_cnt_, sizeof(int), cudaMemcpyDeviceToHost, s), "count");
-  sync();
+  const size_t nd = finish_phase("insertion", (size_t)row0);
   if (!defer_init_) emb_pending_ = snap_pending_ = false;  // the stream waited for it above
-  const int nd = (int)h_pin_[0];
-  if (nd > 0) {
-    ck(cudaMemcpyAsync(h_pin_, d_rows_, (size_t)nd * sizeof(int), cudaMemcpyDeviceToHost, s),
-       "rows");
-    sync();
-  }
   // affected = batch rows then changed existing rows (insertion_kernel.cuh:1039-1089)
   for (int i = 0; i < nb; ++i) upd_q_.push((uint32_t)(row0 + i));
-  for (int i = 0; i < nd; ++i) upd_q_.push(h_pin_[i]);
+  for (size_t i = 0; i < nd; ++i) upd_q_.push(h_pin_[kCounters + i]);
   return (uint32_t)B;
 }
 
@@ -897,16 +910,9 @@ size_t Session::update_round(std::vector<uint32_t> &batch, std::vector<uint32_t>
   timed_end(0);
   launch_merge_publish(st_, n, counters + kUpdEdges, us_.hflag, s);
   compact_flags(us_.hflag, n, -1, d_rows_, d_cnt_, d_tmp_, s);
-  ck(cudaMemcpyAsync(h_pin_, d_cnt_, 3 * sizeof(int), cudaMemcpyDeviceToHost, s), "counts");
-  sync();
-  const int na = (int)h_pin_[0];
+  const size_t na = finish_phase("update", (size_t)n);
   const int edges = (int)h_pin_[2 + kUpdEdges];
-  if (na > 0) {
-    ck(cudaMemcpyAsync(h_pin_, d_rows_, (size_t)na * sizeof(int), cudaMemcpyDeviceToHost, s),
-       "affected");
-    sync();
-    affected.assign(h_pin_, h_pin_ + na);
-  }
+  affected.assign(h_pin_ + kCounters, h_pin_ + kCounters + na);
   return (size_t)edges;
 }
 

@@ -99,6 +99,8 @@ class Session {
   uint32_t embed(uint32_t n_ops);
   void check_launch_error(const char *phase);
   void check_device_error(const char *phase);
+  void report_device_error(const char *phase, unsigned bits);
+  size_t finish_phase(const char *phase, size_t bound);
   void ensure_cand(size_t rows);
   void free_cand();
   void ensure_join(size_t words);
@@ -162,7 +164,11 @@ class Session {
 
   // device row lists / counters
   int *d_rows_ = nullptr, *d_rows2_ = nullptr, *d_batch_ = nullptr;
-  int *d_cnt_ = nullptr;  // [0] list count, [1] edges, [2] report count, [3] join count
+  // device words fetched together: [0] list count, [2..10) an update round's
+  // counters, kFlagsAt: an insertion's change flags, kErrAt: the error word
+  static constexpr int kCounters = 64, kFlagsAt = 16, kErrAt = 48;
+  static constexpr size_t kRowsAhead = 8192;  // rows fetched with the counters
+  int *d_cnt_ = nullptr;
   int *d_tmp_ = nullptr;
   size_t pin_bytes_ = 0;           // of each pinned staging buffer
   uint32_t *h_pin_ = nullptr;      // pinned staging (n_cap + 16 words)
