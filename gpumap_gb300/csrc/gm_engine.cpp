@@ -206,7 +206,8 @@ Session::Session(const gm_params &p) : p_(p) {
       xs_.pre = (unsigned long long *)dalloc((size_t)ex_block_ * xs_.pre_gx * xs_.pre_cap *
                                              sizeof(unsigned long long));
       xs_.pre_ub = (float *)dalloc((size_t)ex_block_ * xs_.pre_gx * xs_.pre_cap * sizeof(float));
-      xs_.mins_ld = exact_seed_tiles((int)((Nm + 255) / 256)) * 8;
+      // (no block of fewer tiles samples more of them than 32)
+      xs_.mins_ld = std::max(exact_seed_tiles((int)((Nm + 255) / 256)), 32) * 8;
       xs_.mins = (float *)dalloc((size_t)ex_block_ * xs_.mins_ld * sizeof(float));
       xs_.pre_cnt = (int *)dalloc((size_t)ex_block_ * xs_.pre_gx * sizeof(int));
       xs_.pre_over = (int *)dalloc(sizeof(int));

@@ -274,7 +274,7 @@ struct TileScreen {
 // leave the tensor memory (the tile itself is not stored).  grid.y: 128-row
 // tiles of the batch; grid.x: CTAs sharing the column tiles.  For every pair
 // (batch row m, column j) the epilogue forms D and the bound B (pair_bound);
-// its upper bound is D + B and its lower bound D - B.  Past 32 column tiles:
+// its upper bound is D + B and its lower bound D - B.  From five column tiles on:
 //  Pass 0 (kPass == 0), on an evenly spaced sample of column tiles: per row
 //    and 32-column chunk, the smallest upper bound (sc.mins).  The 32nd
 //    smallest of a row's chunk minima (k_seed_select) is the largest upper
@@ -287,7 +287,7 @@ struct TileScreen {
 //    upper bounds, then keeps the stored columns with lower bound <= T.
 //    Column side, for an existing row j: (j, m) goes to the pair pool when
 //    D - B is at most the 32nd distance of j's list.
-// Up to 32 column tiles, and for a block whose stored columns overflowed:
+// Up to four column tiles, and for a block whose stored columns overflowed:
 //  Pass 1 (kPass == 1), all column tiles: every CTA keeps, per row, a
 //    max-heap of the 32 smallest upper bounds it sees (at or below the seed
 //    when there is one) and stores it to sc.heaps; the 32nd smallest of
@@ -1154,11 +1154,19 @@ static void launch_tile(const DevState &st, const ExactMaps &maps, int dh, int r
 
 // Column tiles of the seed pass (evenly spaced over the columns): at least
 // 16, and one in 16 of the block's tiles, so that the seed stays a low
-// quantile of the row's upper bounds at any column count.
+// quantile of the row's upper bounds at any column count; all of them up to 32.
+// It needs 32 chunks of 32 columns, and some more to be low (from kSeedMin
+// tiles, 40 chunks: it then admits about 65 of 1,280 columns).  Below that the
+// heap and candidate passes run instead: a thread's heap of a row and one
+// group of epilogue warps made them 170 us a block where the seed and store
+// passes and their selections take 43 us (333 rows x 131 against 4,000).
 constexpr int kSeedTiles = 16;
 constexpr int kSeedEvery = 16;
+constexpr int kSeedMin = 5;
 
-int exact_seed_tiles(int n_tiles) { return std::max(kSeedTiles, n_tiles / kSeedEvery); }
+int exact_seed_tiles(int n_tiles) {
+  return n_tiles <= 2 * kSeedTiles ? std::max(n_tiles, 1) : std::max(kSeedTiles, n_tiles / kSeedEvery);
+}
 
 void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int row0, int blk0,
                        int nrows, int n, const ExactScreen &x, long ldD, bool keep_d, int sms,
@@ -1172,7 +1180,7 @@ void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int ro
   // entries per stored segment: the row's whole allocation shared by its
   // tile's CTAs (fewer CTAs per row tile, longer segments)
   const int cap = x.pre_fixed || gx > x.pre_gx ? x.pre_cap : (int)((long)x.pre_gx * x.pre_cap / gx);
-  if (n_tiles > 2 * kSeedTiles && x.pre && cap > 0 && gx <= x.pre_gx &&
+  if (n_tiles >= kSeedMin && x.pre && cap > 0 && gx <= x.pre_gx &&
       tiles * (kTN / 32) <= x.mins_ld) {
     // seed pass over a spread sample of tiles, then the store pass
     const int stride = n_tiles / tiles;

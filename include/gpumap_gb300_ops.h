@@ -49,7 +49,7 @@ int gm_debug_keep_tiles(struct gm_session *s, int on);
  * over the tiles may keep, fixed whatever the grid width (clamped to 64;
  * by default each of a row tile's CTAs gets an equal share of the row's
  * 64 x min(SMs, column tiles) entries; 0 runs the heap and candidate passes
- * instead, as for blocks of up to 32 column tiles).  A segment that would
+ * instead, as for blocks of up to four column tiles).  A segment that would
  * exceed it makes the heap and candidate passes run for its block
  * (gm_stats.exact_overflow_blocks). */
 int gm_debug_pre_capacity(struct gm_session *s, int cap);
