@@ -183,6 +183,7 @@ GM_D void tmem_ld_wait(uint32_t (&r)[16]) {
 // hi[0..dh) | lo[0..dh), zero padded past d.
 __global__ void k_to_bf16(const float *X, int ld, int d, int dh, int row0, int nrows,
                           __nv_bfloat16 *Xh) {
+  pdl_enter();
   const long total = (long)nrows * dh;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long)gridDim.x * blockDim.x) {
@@ -303,6 +304,7 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
     k_exact_dist(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                  int arow0, int nb, int n, int kchunks, int dh, const float *norms,
                  const float *snorms, TileScreen sc, float *D, long ldD, unsigned *err) {
+  pdl_enter();
   // a gated launch (the fallback after a pass 3 whose stored columns did
   // not overflow) does nothing: the flag is read before any barrier or
   // tensor memory is set up, by every thread alike
@@ -764,6 +766,7 @@ GM_D float warp_32nd(const float *v, int cnt, int lane) {
 __global__ void __launch_bounds__(kFinalWarps * 32)
     k_row_threshold(const float *heaps, int ncta, int nrows, int n, const float *seed, float *row_t,
                     const int *run_if, unsigned long long *stat) {
+  pdl_enter();
   if (run_if && *run_if == 0) return;
   const int lane = threadIdx.x & 31;
   const int ml = blockIdx.x * kFinalWarps + (threadIdx.x >> 5);
@@ -784,6 +787,7 @@ __global__ void __launch_bounds__(kFinalWarps * 32)
 __global__ void __launch_bounds__(kFinalWarps * 32)
     k_seed_select(const float *mins, int mins_ld, int nrows, float *seed, int *row_cnt, int *pcnt,
                   int *counter, int *pre_over) {
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   const int ml = blockIdx.x * kFinalWarps + (threadIdx.x >> 5);
   if (blockIdx.x == 0 && threadIdx.x == 0) *counter = *pre_over = 0;
@@ -811,6 +815,7 @@ __global__ void __launch_bounds__(kPreThreads)
     k_pre_select(const unsigned long long *pre, const float *pre_ub, const int *pre_cnt, int gx,
                  int cap, const int *pre_over, int n, float *row_t, int *cand, long cand_ld,
                  int *row_cnt, unsigned long long *stat) {
+  pdl_enter();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, m = blockIdx.x;
   if (*pre_over) {
     if (stat && m == 0 && threadIdx.x == 0) atomicAdd(&stat[9], 1ull);
@@ -912,6 +917,7 @@ constexpr int kMaxBlockRows = 1024;
 __global__ void __launch_bounds__(256)
     k_pool_count(const int *pool_m, const int *counter, long pool_cap, int nrows, int *cnt,
                  unsigned long long *stat) {
+  pdl_enter();
   __shared__ int s_cnt[kMaxBlockRows];
   const long total = min((long)*counter, pool_cap);
   for (int i = threadIdx.x; i < nrows; i += blockDim.x) s_cnt[i] = 0;
@@ -925,6 +931,7 @@ __global__ void __launch_bounds__(256)
 }
 __global__ void __launch_bounds__(kMaxBlockRows)
     k_pool_offsets(int nrows, const int *cnt, int *off, int *fill) {
+  pdl_enter();
   __shared__ int s_tot[32];
   const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
   const int c = i < nrows ? cnt[i] : 0;
@@ -945,6 +952,7 @@ __global__ void __launch_bounds__(kMaxBlockRows)
 }
 __global__ void k_pool_place(const int *pool_j, const int *pool_m, const int *counter, long pool_cap,
                              int *fill, int *pair_j, int *pair_m) {
+  pdl_enter();
   const long total = min((long)*counter, pool_cap);
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
     const int m = pool_m[e], q = atomicAdd(&fill[m], 1);
@@ -967,6 +975,7 @@ __global__ void __launch_bounds__(kRescoreWarps * 32)
     k_rescore(const float *X, int ld, const float *norms, int brow0, int nrows, const int *cand,
               long cand_ld, const int *row_cnt, float *cand_d, const int *pair_j, const int *pair_off,
               float *pair_d, const Key *g_key, OfferChains chains) {
+  pdl_enter();
   __shared__ __align__(16) RowDotTiles tiles[kRescoreWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int task = blockIdx.x * kRescoreWarps + warp;
@@ -1013,6 +1022,7 @@ constexpr int kRowWarps = 4;
 __global__ void k_row_select(const float *cand_d, int brow0, int nrows, const int *cand,
                              long cand_ld, const int *row_cnt, Key *g_key,
                              unsigned long long *stat) {
+  pdl_enter();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ml = blockIdx.x * kRowWarps + warp;
   if (ml >= nrows) return;
@@ -1100,8 +1110,8 @@ bool make_row_maps(void *xh, int n_cap, int dh, ExactMaps *out) {
 void launch_to_bf16(const DevState &st, void *xh, int dh, int row0, int nrows, cudaStream_t s) {
   if (nrows <= 0) return;
   const long total = (long)nrows * dh;
-  k_to_bf16<<<std::min(cdiv(total, 256), 4096), 256, 0, s>>>(st.X, st.ld, st.d, dh, row0, nrows,
-                                                           (__nv_bfloat16 *)xh);
+  launch(k_to_bf16, std::min(cdiv(total, 256), 4096), 256, 0, s, st.X, st.ld, st.d, dh, row0, nrows,
+         (__nv_bfloat16 *)xh);
   note_launch();
 }
 
@@ -1147,8 +1157,8 @@ static void launch_tile(const DevState &st, const ExactMaps &maps, int dh, int r
   sc.g_key = st.g_key;
   sc.n_exist = row0;
   sc.coef = exact_bound_coef(st.d, dh);
-  k_exact_dist<kPass, kKeepD><<<dim3(gx, m_tiles), exact_threads(kPass), kExactSmem, s>>>(
-      ta, tb, row0 + blk0, nrows, n, dh / kTK, dh, st.norms, st.snorms, sc, x.D, ldD, st.err);
+  launch(k_exact_dist<kPass, kKeepD>, dim3(gx, m_tiles), exact_threads(kPass), kExactSmem, s, ta, tb,
+         row0 + blk0, nrows, n, dh / kTK, dh, st.norms, st.snorms, sc, x.D, ldD, st.err);
   note_launch();
 }
 
@@ -1188,24 +1198,23 @@ void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int ro
     const int mins_ld = tiles * (kTN / 32);
     launch_tile<0, false>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx0, m_tiles, tiles, stride,
                           nullptr, 0, mins_ld, 0, nullptr, s);
-    k_seed_select<<<cdiv(nrows, kFinalWarps), kFinalWarps * 32, 0, s>>>(
-        x.mins, mins_ld, nrows, x.seed, x.row_cnt, x.pcnt, x.counter, x.pre_over);
+    launch(k_seed_select, cdiv(nrows, kFinalWarps), kFinalWarps * 32, 0, s, x.mins, mins_ld, nrows, x.seed,
+           x.row_cnt, x.pcnt, x.counter, x.pre_over);
     if (kd)
       launch_tile<3, true>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx, m_tiles, n_tiles, 1, x.seed,
                            cap, 0, 0, nullptr, s);
     else
       launch_tile<3, false>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx, m_tiles, n_tiles, 1, x.seed,
                             cap, 0, 0, nullptr, s);
-    k_pre_select<<<nrows, kPreThreads, 0, s>>>(
-        x.pre, x.pre_ub, x.pre_cnt, gx, cap, x.pre_over, n, x.row_t, x.cand, ldD, x.row_cnt,
-        st.stat);
+    launch(k_pre_select, nrows, kPreThreads, 0, s, x.pre, x.pre_ub, x.pre_cnt, gx, cap, x.pre_over, n,
+           x.row_t, x.cand, ldD, x.row_cnt, st.stat);
     note_launch(2);
     // after an overflow only: the heap pass (seed-capped; its pairs were
     // already pooled), the threshold and the candidate pass
     launch_tile<1, false>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx, m_tiles, n_tiles, 1, x.seed, 0,
                           0, 0, x.pre_over, s);
-    k_row_threshold<<<cdiv(nrows, kFinalWarps), kFinalWarps * 32, 0, s>>>(x.heaps, gx, nrows, n, x.seed,
-                                                                          x.row_t, x.pre_over, st.stat);
+    launch(k_row_threshold, cdiv(nrows, kFinalWarps), kFinalWarps * 32, 0, s, x.heaps, gx, nrows, n, x.seed,
+           x.row_t, x.pre_over, st.stat);
     note_launch();
     launch_tile<2, false>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx, m_tiles, n_tiles, 1, nullptr, 0,
                           0, 0, x.pre_over, s);
@@ -1220,8 +1229,8 @@ void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int ro
   else
     launch_tile<1, false>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx, m_tiles, n_tiles, 1, nullptr, 0,
                           0, 1, nullptr, s);
-  k_row_threshold<<<cdiv(nrows, kFinalWarps), kFinalWarps * 32, 0, s>>>(x.heaps, gx, nrows, n, nullptr,
-                                                                        x.row_t, nullptr, st.stat);
+  launch(k_row_threshold, cdiv(nrows, kFinalWarps), kFinalWarps * 32, 0, s, x.heaps, gx, nrows, n, nullptr,
+         x.row_t, nullptr, st.stat);
   note_launch();
   launch_tile<2, false>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx, m_tiles, n_tiles, 1, nullptr, 0,
                         0, 0, nullptr, s);
@@ -1235,16 +1244,17 @@ void launch_exact_screen(const DevState &st, int row0, int blk0, int nrows, int 
   // the pairs as found are done with once placed: pool_m holds the chains
   const OfferChains chains{x.heads, x.pool_m};
   if (row0 > 0) {
-    k_pool_count<<<grid, 256, 0, s>>>(x.pool_m, x.counter, x.pool_cap, nrows, x.pcnt, st.stat);
-    k_pool_offsets<<<1, kMaxBlockRows, 0, s>>>(nrows, x.pcnt, x.poff, x.pfill);
-    k_pool_place<<<grid, 256, 0, s>>>(x.pool_j, x.pool_m, x.counter, x.pool_cap, x.pfill, x.pair_j, x.pair_m);
+    launch(k_pool_count, grid, 256, 0, s, x.pool_m, x.counter, x.pool_cap, nrows, x.pcnt, st.stat);
+    launch(k_pool_offsets, 1, kMaxBlockRows, 0, s, nrows, x.pcnt, x.poff, x.pfill);
+    launch(k_pool_place, grid, 256, 0, s, x.pool_j, x.pool_m, x.counter, x.pool_cap, x.pfill, x.pair_j,
+           x.pair_m);
     note_launch(3);
   }
-  k_rescore<<<cdiv((long)nrows * 2 * kRescoreSplit, kRescoreWarps), kRescoreWarps * 32, 0, s>>>(
-      st.X, st.ld, st.norms, brow0, nrows, x.cand, ldD, x.row_cnt, x.cand_d, x.pair_j,
-      row0 > 0 ? x.poff : nullptr, x.pool_d, st.g_key, chains);
-  k_row_select<<<cdiv(nrows, kRowWarps), kRowWarps * 32, 0, s>>>(x.cand_d, brow0, nrows, x.cand,
-                                                                 ldD, x.row_cnt, st.g_key, st.stat);
+  launch(k_rescore, cdiv((long)nrows * 2 * kRescoreSplit, kRescoreWarps), kRescoreWarps * 32, 0, s, st.X,
+         st.ld, st.norms, brow0, nrows, x.cand, ldD, x.row_cnt, x.cand_d, x.pair_j,
+         row0 > 0 ? x.poff : nullptr, x.pool_d, st.g_key, chains);
+  launch(k_row_select, cdiv(nrows, kRowWarps), kRowWarps * 32, 0, s, x.cand_d, brow0, nrows, x.cand, ldD,
+         x.row_cnt, st.g_key, st.stat);
   note_launch(2);
   if (row0 > 0) launch_merge_offers(st, row0, brow0, chains, x.pool_d, x.pair_m, nullptr, nullptr, s);
 }

@@ -47,6 +47,7 @@ GM_D float membership(float dist, float rho, float sigma) {
 // Block sums of the embed-time distances (256 per block, FP32 tree).
 __global__ void k_mean_partial(const float *pub_dist, int n, int k, int euclid,
                                float *part, int *ipart) {
+  pdl_enter();
   __shared__ float ss[256];
   __shared__ float sc[256];
   const int t = threadIdx.x;
@@ -139,6 +140,7 @@ __global__ void __launch_bounds__(kSmoothThreads)
     k_smooth_knn(const float *pub_dist, int n, int k, int euclid, double target, float t_hi,
                  float t_lo, float *sigma, float *rho, const float *part, const int *ipart, int nb,
                  float *fscal, int *marked) {
+  pdl_enter();
   __shared__ __align__(16) float stage[kMeanStage];
   if (blockIdx.x == 0) {
     mean_final(part, ipart, nb, fscal, stage);
@@ -242,6 +244,7 @@ __global__ void __launch_bounds__(kSmoothThreads)
 
 // Rows without a positive distance: a share of the global mean.
 __global__ void k_fix_sigma(int n, const float *fscal, float *sigma, const int *marked) {
+  pdl_enter();
   if (!*marked) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && sigma[i] < 0.0f) sigma[i] = __fmul_rn(kMinKDistScale, fscal[FS_MEAN]);
@@ -254,6 +257,7 @@ __global__ void k_memb_sym(const uint32_t *pub_idx, const float *pub_dist, int n
                            int euclid, const float *sigma, const float *rho,
                            const int *batch, int nb, int *coo_row, int *coo_col,
                            float *coo_val, int *flag) {
+  pdl_enter();
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= nb * k) return;
   const int bi = tid / k, ki = tid - bi * k;
@@ -283,6 +287,7 @@ __global__ void k_memb_sym(const uint32_t *pub_idx, const float *pub_dist, int n
 
 __global__ void k_write_extras(const int *idx, const int *cnt, int ndir, int *coo_row,
                                int *coo_col, float *coo_val, int *iscal) {
+  pdl_enter();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   const int c = *cnt;
   if (q == 0) {
@@ -298,6 +303,7 @@ __global__ void k_write_extras(const int *idx, const int *cnt, int ndir, int *co
 
 // max_w over non-negative weights via the int ordering of their bits.
 __global__ void k_max_w(const float *vals, const int *iscal, float *fscal) {
+  pdl_enter();
   const int nnz = iscal[IS_NNZ];
   float m = 0.0f;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nnz; q += gridDim.x * blockDim.x)
@@ -310,6 +316,7 @@ __global__ void k_max_w(const float *vals, const int *iscal, float *fscal) {
 // Trim flag: keep w >= max_w / n_epochs (reference trim_graph, :348-400).
 __global__ void k_trim_flags(const float *vals, const int *iscal, const float *fscal,
                              int n_epochs, int *flag, int nmax) {
+  pdl_enter();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nmax) return;
   const int nnz = iscal[IS_NNZ];
@@ -325,6 +332,7 @@ __global__ void k_gather_sched(const int *idx, const int *iscal, const int *crow
                                const int *ccol, const float *cval, const float *fscal,
                                int n_epochs, float nsr_inv, int *trow, int *tcol,
                                float *eps, float *next_s, float *next_n, int *deg) {
+  pdl_enter();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= iscal[IS_NNZ2]) return;
   const int src = idx[q];
@@ -341,6 +349,7 @@ __global__ void k_gather_sched(const int *idx, const int *iscal, const int *crow
 }
 
 __global__ void k_max_deg(const int *deg, int n, int *iscal) {
+  pdl_enter();
   int m = 0;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
     m = max(m, deg[q]);
@@ -350,6 +359,7 @@ __global__ void k_max_deg(const int *deg, int n, int *iscal) {
 
 // Gradient rounding factor 2^ceil-ish via frexp (reference :433-460).
 __global__ void k_rounding(int *iscal, float *fscal, float alpha) {
+  pdl_enter();
   const int nnz = iscal[IS_NNZ2];
   const int md = iscal[IS_MAXDEG];
   float r = 1.0f;
@@ -676,7 +686,10 @@ __global__ void __launch_bounds__(kSgdThreads)
   sgd_stats(my_edges, my_negs, stat);
 }
 
-__global__ void k_set_int(int *p, int v) { *p = v; }
+__global__ void k_set_int(int *p, int v) {
+  pdl_enter();
+  *p = v;
+}
 
 __global__ void k_epoch_init(const float *eps, int nnz, float nsr_inv, float *next_s,
                              float *next_n) {
@@ -688,6 +701,7 @@ __global__ void k_epoch_init(const float *eps, int nnz, float nsr_inv, float *ne
 
 // x-range of the embedding (first component) for the noise scale.
 __global__ void k_xrange_partial(const float *emb, int n, float *part) {
+  pdl_enter();
   __shared__ float smin[256], smax[256];
   const int t = threadIdx.x;
   float mn = FLT_MAX, mx = -FLT_MAX;
@@ -717,6 +731,7 @@ __global__ void k_xrange_partial(const float *emb, int n, float *part) {
 __global__ void __launch_bounds__(256)
     k_add_noise(float *emb, const int *batch, int nb, const float *part, int nparts,
                 float noise_scale, uint64_t seed) {
+  pdl_enter();
   __shared__ float s_mn[8], s_mx[8];
   const int t = threadIdx.x, tid = blockIdx.x * blockDim.x + t;
   float mn = FLT_MAX, mx = -FLT_MAX;
@@ -761,6 +776,7 @@ constexpr int kHeurAhead = 8;
 __global__ void k_heuristic(const uint32_t *pub_idx, const float *pub_dist, int n, int k,
                             int euclid, const float *sigma, const float *rho,
                             const int *unsel, int nu, const float *snap, float *emb) {
+  pdl_enter();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nu) return;
   const int row = unsel[q];
@@ -799,6 +815,7 @@ __global__ void k_heuristic(const uint32_t *pub_idx, const float *pub_dist, int 
 }
 
 __global__ void k_mark_rows(const int *rows, int nr, int *flag) {
+  pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < nr) flag[rows[i]] = 1;
 }
@@ -809,7 +826,7 @@ inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
 void launch_mark_rows(const int *rows, int nr, int *flag, cudaStream_t s) {
   if (nr <= 0) return;
-  k_mark_rows<<<cdiv(nr, 256), 256, 0, s>>>(rows, nr, flag);
+  launch(k_mark_rows, cdiv(nr, 256), 256, 0, s, rows, nr, flag);
   note_launch();
 }
 
@@ -818,28 +835,27 @@ void launch_fuzzy_graph(const uint32_t *pub_idx, const float *pub_dist, int n, i
                         EmbedScratch &e, cudaStream_t s) {
   const long total = (long)n * k;
   const int nbl = cdiv(total, 256);
-  k_mean_partial<<<nbl, 256, 0, s>>>(pub_dist, n, k, euclidean, e.partial, e.ipartial);
+  launch(k_mean_partial, nbl, 256, 0, s, pub_dist, n, k, euclidean, e.partial, e.ipartial);
   note_launch();
   cudaMemsetAsync(e.iscal + IS_MARKED, 0, sizeof(int), s);
   const float t_hi = (float)log2_target, t_lo = (float)(log2_target - (double)t_hi);
   auto smooth = [&](auto kernel, int lanes) {
-    kernel<<<1 + cdiv((long)n * lanes, kSmoothThreads), kSmoothThreads, 0, s>>>(
-        pub_dist, n, k, euclidean, log2_target, t_hi, isfinite(log2_target) ? t_lo : 0.0f, e.sigma, e.rho,
-        e.partial, e.ipartial, nbl, e.fscal, e.iscal + IS_MARKED);
+    launch(kernel, 1 + cdiv((long)n * lanes, kSmoothThreads), kSmoothThreads, 0, s, pub_dist, n, k,
+           euclidean, log2_target, t_hi, isfinite(log2_target) ? t_lo : 0.0f, e.sigma, e.rho, e.partial,
+           e.ipartial, nbl, e.fscal, e.iscal + IS_MARKED);
   };
   if (k <= 16) smooth(k_smooth_knn<4>, 4);
   else smooth(k_smooth_knn<8>, 8);
-  k_fix_sigma<<<cdiv(n, 256), 256, 0, s>>>(n, e.fscal, e.sigma, e.iscal + IS_MARKED);
+  launch(k_fix_sigma, cdiv(n, 256), 256, 0, s, n, e.fscal, e.sigma, e.iscal + IS_MARKED);
   note_launch(2);
   const int ndir = nb * k;
   if (ndir > 0)
-    k_memb_sym<<<cdiv(ndir, 256), 256, 0, s>>>(pub_idx, pub_dist, n, k, euclidean, e.sigma,
-                                               e.rho, batch, nb, e.coo_row, e.coo_col,
-                                               e.coo_val, e.t_row);
+    launch(k_memb_sym, cdiv(ndir, 256), 256, 0, s, pub_idx, pub_dist, n, k, euclidean, e.sigma, e.rho,
+           batch, nb, e.coo_row, e.coo_col, e.coo_val, e.t_row);
     note_launch();
   compact_flags(e.t_row, ndir, -1, e.t_col, e.iscal + IS_EXTRA, e.tmp2, s);
-  k_write_extras<<<cdiv(ndir > 0 ? ndir : 1, 256), 256, 0, s>>>(
-      e.t_col, e.iscal + IS_EXTRA, ndir, e.coo_row, e.coo_col, e.coo_val, e.iscal);
+  launch(k_write_extras, cdiv(ndir > 0 ? ndir : 1, 256), 256, 0, s, e.t_col, e.iscal + IS_EXTRA, ndir,
+         e.coo_row, e.coo_col, e.coo_val, e.iscal);
   note_launch();
 }
 
@@ -853,22 +869,19 @@ void launch_schedule(int n, int nb, int k, float alpha0, int n_epochs, int neg_r
   cudaMemsetAsync(e.fscal + FS_MAXW, 0, sizeof(float), s);
   cudaMemsetAsync(e.iscal + IS_MAXDEG, 0, sizeof(int), s);
   cudaMemsetAsync(e.deg, 0, sizeof(int) * (size_t)n, s);
-  k_max_w<<<min(cdiv(nmax, 256), 1024), 256, 0, s>>>(e.coo_val, e.iscal, e.fscal);
+  launch(k_max_w, min(cdiv(nmax, 256), 1024), 256, 0, s, e.coo_val, e.iscal, e.fscal);
   note_launch();
-  k_trim_flags<<<cdiv(nmax, 256), 256, 0, s>>>(e.coo_val, e.iscal, e.fscal, n_epochs,
-                                               e.t_row, nmax);
+  launch(k_trim_flags, cdiv(nmax, 256), 256, 0, s, e.coo_val, e.iscal, e.fscal, n_epochs, e.t_row, nmax);
   note_launch();
   compact_flags_dev(e.t_row, e.iscal + IS_NNZ, nmax, e.t_col, e.iscal + IS_NNZ2, e.tmp2, s);
   // t_col holds survivor indices; gather into (t_row, flag_tail, t_val)
   const float nsr_inv = 1.0f / (float)neg_rate;  // inf when 0: no negatives
-  k_gather_sched<<<cdiv(nmax, 256), 256, 0, s>>>(e.t_col, e.iscal, e.coo_row, e.coo_col,
-                                                 e.coo_val, e.fscal, n_epochs, nsr_inv,
-                                                 e.t_row, e.flag_tail, e.t_val, e.next_s,
-                                                 e.next_n, e.deg);
+  launch(k_gather_sched, cdiv(nmax, 256), 256, 0, s, e.t_col, e.iscal, e.coo_row, e.coo_col, e.coo_val,
+         e.fscal, n_epochs, nsr_inv, e.t_row, e.flag_tail, e.t_val, e.next_s, e.next_n, e.deg);
   note_launch();
-  k_max_deg<<<min(cdiv(n, 256), 1024), 256, 0, s>>>(e.deg, n, e.iscal);
+  launch(k_max_deg, min(cdiv(n, 256), 1024), 256, 0, s, e.deg, n, e.iscal);
   note_launch();
-  k_rounding<<<1, 1, 0, s>>>(e.iscal, e.fscal, alpha0);
+  launch(k_rounding, 1, 1, 0, s, e.iscal, e.fscal, alpha0);
   note_launch();
 }
 
@@ -883,7 +896,7 @@ void launch_optimize_layout(float *emb, int n, int nb, int k, float alpha0, floa
 }
 
 void launch_set_int(int *p, int v, cudaStream_t s) {
-  k_set_int<<<1, 1, 0, s>>>(p, v);
+  launch(k_set_int, 1, 1, 0, s, p, v);
   note_launch();
 }
 
@@ -967,10 +980,9 @@ void launch_add_noise(float *emb, int n, const int *batch, int nb, float noise_s
                       uint64_t seed, EmbedScratch &e, cudaStream_t s) {
   if (nb <= 0 || noise_scale == 0.0f || n <= 0) return;
   const int nparts = min(cdiv(n, 256), 256);
-  k_xrange_partial<<<nparts, 256, 0, s>>>(emb, n, e.partial);
+  launch(k_xrange_partial, nparts, 256, 0, s, emb, n, e.partial);
   note_launch();
-  k_add_noise<<<cdiv(nb * 2, 256), 256, 0, s>>>(emb, batch, nb, e.partial, nparts,
-                                                noise_scale, seed);
+  launch(k_add_noise, cdiv(nb * 2, 256), 256, 0, s, emb, batch, nb, e.partial, nparts, noise_scale, seed);
   note_launch();
 }
 
@@ -979,8 +991,8 @@ void launch_heuristic(const uint32_t *pub_idx, const float *pub_dist, int n, int
                       EmbedScratch &e, cudaStream_t s) {
   if (nu <= 0 || n <= 0 || k <= 0) return;
   cudaMemcpyAsync(e.snap, emb, sizeof(float) * 2 * (size_t)n, cudaMemcpyDeviceToDevice, s);
-  k_heuristic<<<cdiv(nu, 128), 128, 0, s>>>(pub_idx, pub_dist, n, k, euclidean, e.sigma,
-                                            e.rho, unsel, nu, e.snap, emb);
+  launch(k_heuristic, cdiv(nu, 128), 128, 0, s, pub_idx, pub_dist, n, k, euclidean, e.sigma, e.rho, unsel,
+         nu, e.snap, emb);
   note_launch();
 }
 

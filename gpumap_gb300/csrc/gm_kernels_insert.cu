@@ -24,6 +24,7 @@ constexpr int kNormRows = 8, kNormChunk = 1024;
 __global__ void __launch_bounds__(256)
     k_row_norms(float *X, float *norms, float *snorms, int ld, int d, int row0, int nrows,
                 int cosine) {
+  pdl_enter();
   __shared__ __align__(16) float tile[kNormRows][kNormChunk + 4];
   __shared__ float s_scale[kNormRows];
   const int r0 = blockIdx.x * kNormRows;
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(256)
 constexpr int kInitWarps = 4;
 __global__ void __launch_bounds__(kInitWarps * 32)
     k_random_init(Key *g_key, int row0, int nrows, int n, int window_start, uint64_t seed) {
+  pdl_enter();
   __shared__ int s_list[kInitWarps][kListW];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rl = blockIdx.x * kInitWarps + warp;
@@ -170,6 +172,7 @@ struct HopOut {
 __global__ void __launch_bounds__(kSampWarps * 32)
     k_sample_candidates(const Key *g_key, int row0, int nrows, int n, int k, int slots,
                         int exist_only, HopOut o, int iter, const int *changed) {
+  pdl_enter();
   if (changed && *changed == 0) return;
   extern __shared__ __align__(16) int smem_sc[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -302,6 +305,7 @@ __global__ void __launch_bounds__(kCandWarps * 32)
                        const int *cand, const uint8_t *todo, const int *todo_cnt,
                        float *cand_dist, const Key *g_key, OfferChains chains, const int *changed,
                        unsigned long long *stat) {
+  pdl_enter();
   if (changed && *changed == 0) return;
   __shared__ __align__(16) RowDotTiles tiles[kCandWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -331,6 +335,7 @@ constexpr int kOfferWarps = 8;
 __global__ void __launch_bounds__(kOfferWarps * 32)
     k_merge_offers(Key *g_key, int row0, int first, OfferChains chains, const float *dist,
                    const int *e_row, int *dirty, int *changed_out, const int *changed) {
+  pdl_enter();
   if (changed && *changed == 0) return;
   const int lane = threadIdx.x & 31;
   const int j = blockIdx.x * kOfferWarps + (threadIdx.x >> 5);
@@ -376,6 +381,7 @@ constexpr int kFwdWarps = 4;
 __global__ void __launch_bounds__(kFwdWarps * 32)
     k_forward_merge(Key *g_key, int row0, int nrows, const int *cand, const int *cand_cnt,
                     const float *cand_dist, int *changed_out, const int *changed) {
+  pdl_enter();
   if (changed && *changed == 0) return;
   const int lane = threadIdx.x & 31;
   const int rl = blockIdx.x * kFwdWarps + (threadIdx.x >> 5);
@@ -443,6 +449,7 @@ __global__ void __launch_bounds__(kAdoptWarps * 32)
     k_adopt_publish(const Key *g_key, int *knn_ids, float *knn_dists, uint32_t *pub_idx,
                     float *pub_dist, int k, int row0, int nrows, const int *rows,
                     const int *n_rows_dev, int n) {
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   const int total = nrows + (n_rows_dev ? *n_rows_dev : 0);
   for (int i = blockIdx.x * kAdoptWarps + (threadIdx.x >> 5); i < total; i += gridDim.x * kAdoptWarps) {
@@ -472,6 +479,7 @@ __global__ void __launch_bounds__(kAdoptWarps * 32)
 constexpr int kInitEmbWarps = 4;
 __global__ void __launch_bounds__(kInitEmbWarps * 32)
     k_embed_init(const Key *g_key, float *emb, int k, int row0, int nrows, int n) {
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   const int rl = blockIdx.x * kInitEmbWarps + (threadIdx.x >> 5);
   if (rl >= nrows) return;
@@ -514,16 +522,16 @@ inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
 void launch_row_norms(const DevState &st, int row0, int nrows, cudaStream_t s) {
   if (nrows <= 0) return;
-  k_row_norms<<<cdiv(nrows, kNormRows), 256, 0, s>>>(st.X, st.norms, st.snorms, st.ld, st.d,
-                                                      row0, nrows, st.cosine);
+  launch(k_row_norms, cdiv(nrows, kNormRows), 256, 0, s, st.X, st.norms, st.snorms, st.ld, st.d, row0,
+         nrows, st.cosine);
   note_launch();
 }
 
 void launch_merge_offers(const DevState &st, int row0, int first, const OfferChains &chains,
                          const float *dist, const int *e_row, int *changed_out, const int *changed,
                          cudaStream_t s) {
-  k_merge_offers<<<cdiv(row0, kOfferWarps), kOfferWarps * 32, 0, s>>>(
-      st.g_key, row0, first, chains, dist, e_row, st.dirty, changed_out, changed);
+  launch(k_merge_offers, cdiv(row0, kOfferWarps), kOfferWarps * 32, 0, s, st.g_key, row0, first, chains,
+         dist, e_row, st.dirty, changed_out, changed);
   note_launch();
 }
 
@@ -531,8 +539,8 @@ void launch_nnd_insert(const DevState &st, const UpdScratch &u, int row0, int nr
                        uint64_t seed, const CandScratch &c, int *changed, int sms,
                        const std::function<void(bool)> &timed, cudaStream_t s) {
   if (nrows <= 0) return;
-  k_random_init<<<cdiv(nrows, kInitWarps), kInitWarps * 32, 0, s>>>(st.g_key, row0, nrows, n,
-                                                                    window_start, seed);
+  launch(k_random_init, cdiv(nrows, kInitWarps), kInitWarps * 32, 0, s, st.g_key, row0, nrows, n,
+         window_start, seed);
   note_launch();
   const int k = st.k, P = k * k;
   // Below 256 positions (k <= 15) the forward merge, which wants 256
@@ -561,25 +569,25 @@ void launch_nnd_insert(const DevState &st, const UpdScratch &u, int row0, int nr
     // launches return at once
     const int *go = it > 0 ? changed + it - 1 : nullptr;
     int *mark = merges ? changed + it : nullptr;
-    k_sample_candidates<<<cdiv(nrows, kSampWarps), kSampWarps * 32, smem, s>>>(
-        st.g_key, row0, nrows, n, k, slots, merges ? 0 : 1,
-        HopOut{c.cand, c.cnt, c.dist, merges ? c.todo : nullptr, c.todo_cnt}, it, go);
+    launch(k_sample_candidates, cdiv(nrows, kSampWarps), kSampWarps * 32, smem, s, st.g_key, row0, nrows, n,
+           k, slots, merges ? 0 : 1, HopOut{c.cand, c.cnt, c.dist, merges ? c.todo : nullptr, c.todo_cnt},
+           it, go);
     note_launch();
     for (int r = 0; r < nrows; r += kOfferRows) {
       const int m = std::min(kOfferRows, nrows - r);
       const size_t at = (size_t)r * kMaxCand;
       const int grid = (int)std::min<long>(cdiv((long)m * chunks, kCandWarps), 24L * std::max(sms, 1));
       timed(true);
-      k_candidate_offers<<<grid, kCandWarps * 32, 0, s>>>(
-          st.X, st.norms, st.ld, row0, row0 + r, m, chunks, c.cand + at, merges ? c.todo + at : nullptr,
-          (merges ? c.todo_cnt : c.cnt) + r, c.dist + at, st.g_key, chains, go, st.stat);
+      launch(k_candidate_offers, grid, kCandWarps * 32, 0, s, st.X, st.norms, st.ld, row0, row0 + r, m,
+             chunks, c.cand + at, merges ? c.todo + at : nullptr, (merges ? c.todo_cnt : c.cnt) + r,
+             c.dist + at, st.g_key, chains, go, st.stat);
       note_launch();
       timed(false);
       if (row0 > 0) launch_merge_offers(st, row0, row0 + r, chains, c.dist + at, nullptr, mark, go, s);
     }
     if (merges) {
-      k_forward_merge<<<cdiv(nrows, kFwdWarps), kFwdWarps * 32, 0, s>>>(
-          st.g_key, row0, nrows, c.cand, c.cnt, c.dist, mark, go);
+      launch(k_forward_merge, cdiv(nrows, kFwdWarps), kFwdWarps * 32, 0, s, st.g_key, row0, nrows, c.cand,
+             c.cnt, c.dist, mark, go);
       note_launch();
     }
   }
@@ -590,16 +598,16 @@ void launch_adopt_and_publish(const DevState &st, int row0, int nrows,
                               int n, cudaStream_t s) {
   const int total = nrows + n_rows_max;
   if (total <= 0) return;
-  k_adopt_publish<<<std::min(cdiv(total, kAdoptWarps), 2048), kAdoptWarps * 32, 0, s>>>(
-      st.g_key, st.knn_ids, st.knn_dists, st.pub_idx, st.pub_dist, st.k, row0, nrows,
-      rows, n_rows_dev, n);
+  launch(k_adopt_publish, std::min(cdiv(total, kAdoptWarps), 2048), kAdoptWarps * 32, 0, s, st.g_key,
+         st.knn_ids, st.knn_dists, st.pub_idx, st.pub_dist, st.k, row0, nrows, rows, n_rows_dev, n);
   note_launch();
 }
 
 void launch_embed_init(const DevState &st, int row0, int nrows, int n,
                        cudaStream_t s) {
   if (nrows <= 0) return;
-  k_embed_init<<<cdiv(nrows, kInitEmbWarps), kInitEmbWarps * 32, 0, s>>>(st.g_key, st.emb, st.k, row0, nrows, n);
+  launch(k_embed_init, cdiv(nrows, kInitEmbWarps), kInitEmbWarps * 32, 0, s, st.g_key, st.emb, st.k, row0,
+         nrows, n);
   note_launch();
 }
 

@@ -39,6 +39,7 @@ GM_D int bloom_bit(uint32_t key, int i) {
 // Zeroes the per-row state of an update round and its counters.
 __global__ void k_update_reset(int n, int4 *sizes, int *dirty, int *cnt_new, int *cnt_old,
                                int *counters, int n_counters) {
+  pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n_counters) counters[i] = 0;
   if (i >= n) return;
@@ -63,6 +64,7 @@ __global__ void __launch_bounds__(kSgWarps * 32)
     k_sample_graph(int *knn_ids, uint32_t *bloom, const int *batch, int nb, int n, int k,
                    int *fwd_new, int *fwd_old, int *pos_new, int *pos_old, int *cnt_new,
                    int *cnt_old, int4 *sizes) {
+  pdl_enter();
   __shared__ uint32_t s_bits[kSgWarps][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * kSgWarps + warp;
@@ -127,6 +129,7 @@ __global__ void __launch_bounds__(kSgWarps * 32)
 // of the batch, so n_cap x 32 entries are enough).
 __global__ void k_rev_segments(int n, const int *cnt_new, const int *cnt_old, int *off_new,
                                int *off_old, int *total) {
+  pdl_enter();
   const int j = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
   const int a = j < n ? cnt_new[j] : 0, c = j < n ? cnt_old[j] : 0;
   int v = a + c;
@@ -147,6 +150,7 @@ __global__ void k_rev_segments(int n, const int *cnt_new, const int *cnt_old, in
 __global__ void k_rev_place(const int *batch, int nb, const int *fwd_new, const int *fwd_old,
                             const int *pos_new, const int *pos_old, const int4 *sizes,
                             const int *off_new, const int *off_old, int *src) {
+  pdl_enter();
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= nb * kSamples) return;
   const int row = batch[tid / kSamples], s = tid % kSamples;
@@ -197,6 +201,7 @@ __global__ void __launch_bounds__(kListWarps * 32)
                  const int *cnt_new, const int *cnt_old, int *off_new, int *off_old,
                  const int *src, int4 *sizes, int *small_nodes, int *large_nodes, int *counts,
                  unsigned long long *pool_words) {
+  pdl_enter();
   __shared__ int s_cls[kListWarps], s_words[kListWarps];
   __shared__ int s_base[2];
   __shared__ unsigned long long s_pool;
@@ -472,6 +477,7 @@ static_assert(kJoinRing * kJoinCols * kJoinLd >= kJoinMax * (kJoinCols + 1) && k
               "a node's tile does not fit its ring");
 __global__ void __launch_bounds__(kJoinWarps * 32, 4)
     k_join_tiles(const int *small_nodes, const int *large_nodes, int *counts, JoinArgs g) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char join_raw[];
   JoinSmem &S = *reinterpret_cast<JoinSmem *>(join_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -499,6 +505,7 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 4)
 constexpr int kJmWarps = 8;
 __global__ void __launch_bounds__(kJmWarps * 32)
     k_join_merge(int n, JoinArgs g, Key *g_key, int *dirty, int k) {
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * kJmWarps + (threadIdx.x >> 5);
   if (t >= n) return;
@@ -579,6 +586,7 @@ __global__ void __launch_bounds__(kMpWarps * 32)
     k_merge_publish(const Key *g_key, int *knn_ids, float *knn_dists, const int *dirty,
                     uint32_t *pub_idx, float *pub_dist, int k, int n, int *edge_counter,
                     int *report_flag) {
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * kMpWarps + (threadIdx.x >> 5);
   if (row >= n) return;
@@ -671,17 +679,17 @@ void launch_join_nodes(const DevState &st, const UpdScratch &u, const int *batch
   // new sources are counted in u.cnt, old ones in u.fill; the positions of the
   // samples wait in the batch rows' reverse lists until k_join_lists writes them
   int *off_new = u.off, *off_old = u.hflag;
-  k_update_reset<<<cdiv(std::max(n, kUpdCounters), 256), 256, 0, s>>>(n, u.sizes, st.dirty, u.cnt, u.fill,
-                                                                      counters, kUpdCounters);
-  k_sample_graph<<<cdiv(nb, kSgWarps), kSgWarps * 32, 0, s>>>(
-      st.knn_ids, st.bloom, batch, nb, n, st.k, u.fwd_new, u.fwd_old, u.rev_new, u.rev_old, u.cnt, u.fill,
-      u.sizes);
-  k_rev_segments<<<cdiv(n, 256), 256, 0, s>>>(n, u.cnt, u.fill, off_new, off_old, counters + kUpdSources);
-  k_rev_place<<<cdiv((long)nb * kSamples, 256), 256, 0, s>>>(batch, nb, u.fwd_new, u.fwd_old, u.rev_new,
-                                                            u.rev_old, u.sizes, off_new, off_old, u.csr);
-  k_join_lists<<<cdiv(n, kListWarps), kListWarps * 32, 0, s>>>(
-      n, u.fwd_new, u.fwd_old, u.rev_new, u.rev_old, u.cnt, u.fill, off_new, off_old, u.csr, u.sizes,
-      small_nodes, large_nodes, counters + kUpdNodes, (unsigned long long *)(counters + kUpdPool));
+  launch(k_update_reset, cdiv(std::max(n, kUpdCounters), 256), 256, 0, s, n, u.sizes, st.dirty, u.cnt,
+         u.fill, counters, kUpdCounters);
+  launch(k_sample_graph, cdiv(nb, kSgWarps), kSgWarps * 32, 0, s, st.knn_ids, st.bloom, batch, nb, n, st.k,
+         u.fwd_new, u.fwd_old, u.rev_new, u.rev_old, u.cnt, u.fill, u.sizes);
+  launch(k_rev_segments, cdiv(n, 256), 256, 0, s, n, u.cnt, u.fill, off_new, off_old,
+         counters + kUpdSources);
+  launch(k_rev_place, cdiv((long)nb * kSamples, 256), 256, 0, s, batch, nb, u.fwd_new, u.fwd_old, u.rev_new,
+         u.rev_old, u.sizes, off_new, off_old, u.csr);
+  launch(k_join_lists, cdiv(n, kListWarps), kListWarps * 32, 0, s, n, u.fwd_new, u.fwd_old, u.rev_new,
+         u.rev_old, u.cnt, u.fill, off_new, off_old, u.csr, u.sizes, small_nodes, large_nodes,
+         counters + kUpdNodes, (unsigned long long *)(counters + kUpdPool));
   note_launch(5);
 }
 
@@ -721,16 +729,15 @@ void launch_local_join(const DevState &st, const UpdScratch &u, const int *small
                    st.stat};
   if (pass == 0) cudaMemsetAsync(u.csr, 0xff, (size_t)n * 32 * sizeof(int), s);
   else cudaMemsetAsync(counters + kUpdNodes + 2, 0, 2 * sizeof(int), s);  // the tickets
-  k_join_tiles<<<grid, kJoinWarps * 32, smem, s>>>(small_nodes, large_nodes, counters + kUpdNodes, g);
-  k_join_merge<<<cdiv(n, kJmWarps), kJmWarps * 32, 0, s>>>(n, g, st.g_key, st.dirty, st.k);
+  launch(k_join_tiles, grid, kJoinWarps * 32, smem, s, small_nodes, large_nodes, counters + kUpdNodes, g);
+  launch(k_join_merge, cdiv(n, kJmWarps), kJmWarps * 32, 0, s, n, g, st.g_key, st.dirty, st.k);
   note_launch(2);
 }
 
 void launch_merge_publish(const DevState &st, int n, int *edge_counter, int *report_flag, cudaStream_t s) {
   if (n <= 0) return;
-  k_merge_publish<<<cdiv(n, kMpWarps), kMpWarps * 32, 0, s>>>(st.g_key, st.knn_ids, st.knn_dists, st.dirty,
-                                                             st.pub_idx, st.pub_dist, st.k, n, edge_counter,
-                                                             report_flag);
+  launch(k_merge_publish, cdiv(n, kMpWarps), kMpWarps * 32, 0, s, st.g_key, st.knn_ids, st.knn_dists,
+         st.dirty, st.pub_idx, st.pub_dist, st.k, n, edge_counter, report_flag);
   note_launch();
 }
 

@@ -67,6 +67,7 @@ struct Pred {
 };
 
 __global__ void __launch_bounds__(kScanThreads) k_block_totals(Pred p, int *tot) {
+  pdl_enter();
   __shared__ int wt[kScanThreads / 32];
   const int n = p.len();
   const int base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(kScanThreads) k_block_totals(Pred p, int *tot)
 // Exclusive scan of tot[0..nb) in place; tot[nb] = grand total.  One block.
 __global__ void __launch_bounds__(kScanThreads) k_scan_totals(int *tot, int nb,
                                                               int *total_out) {
+  pdl_enter();
   __shared__ int wt[kScanThreads / 32];
   __shared__ int carry;
   if (threadIdx.x == 0) carry = 0;
@@ -115,6 +117,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_totals(int *tot, int nb,
 __global__ void __launch_bounds__(kScanThreads) k_block_write(Pred p, const int *tot,
                                                               int *out, int mode,
                                                               int n_cap_out) {
+  pdl_enter();
   __shared__ int wt[kScanThreads / 32];
   const int n = p.len();
   const int base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
@@ -146,11 +149,11 @@ inline int nblocks(int n) { return n <= 0 ? 1 : (n + kScanBlock - 1) / kScanBloc
 void run_scan(const Pred &p, int n_max, int *out, int mode, int *count, int *tmp,
               cudaStream_t s) {
   const int nb = nblocks(n_max);
-  k_block_totals<<<nb, kScanThreads, 0, s>>>(p, tmp);
+  launch(k_block_totals, nb, kScanThreads, 0, s, p, tmp);
   note_launch();
-  k_scan_totals<<<1, kScanThreads, 0, s>>>(tmp, nb, count);
+  launch(k_scan_totals, 1, kScanThreads, 0, s, tmp, nb, count);
   note_launch();
-  k_block_write<<<nb, kScanThreads, 0, s>>>(p, tmp, out, mode, n_max);
+  launch(k_block_write, nb, kScanThreads, 0, s, p, tmp, out, mode, n_max);
   note_launch();
 }
 

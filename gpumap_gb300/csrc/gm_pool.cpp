@@ -20,7 +20,7 @@ namespace gm {
 
 namespace {
 
-constexpr unsigned long long kDeviceKeep = 8ull << 30;
+constexpr unsigned long long kDeviceKeep = 16ull << 30;
 constexpr size_t kHostKeep = (size_t)64 << 20;
 constexpr int kMaxDevices = 64;
 
