@@ -215,6 +215,7 @@ Session::Session(const gm_params &p) : p_(p) {
       xs_.pcnt = (int *)dalloc((size_t)ex_block_ * sizeof(int));
       xs_.poff = (int *)dalloc(((size_t)ex_block_ + 1) * sizeof(int));
       xs_.pfill = (int *)dalloc((size_t)ex_block_ * sizeof(int));
+      xs_.ptask = (int *)dalloc(((size_t)ex_block_ + 1) * sizeof(int));
       xs_.heads = us_.fwd_new;  // not in use during an insertion
       xs_.counter = (int *)dalloc(16 * sizeof(int));
     }

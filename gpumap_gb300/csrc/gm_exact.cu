@@ -929,25 +929,40 @@ __global__ void __launch_bounds__(256)
     if (s_cnt[i]) atomicAdd(&cnt[i], s_cnt[i]);
   if (stat && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&stat[6], (unsigned long long)total);
 }
+// off: the groups' offsets, fill: the same, as cursors; task: prefix of the
+// groups of 32 chains (candidates, then pairs) that each row takes.
 __global__ void __launch_bounds__(kMaxBlockRows)
-    k_pool_offsets(int nrows, const int *cnt, int *off, int *fill) {
+    k_pool_offsets(int nrows, const int *cnt, const int *row_cnt, int *off, int *fill, int *task) {
   pdl_enter();
-  __shared__ int s_tot[32];
+  __shared__ int s_tot[2][32];
   const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
   const int c = i < nrows ? cnt[i] : 0;
-  int v = c;
+  const int g = i < nrows ? (row_cnt[i] + 31) / 32 + (c + 31) / 32 : 0;
+  int v = c, w = g;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += y;
+    const int y = __shfl_up_sync(0xffffffffu, v, o), z = __shfl_up_sync(0xffffffffu, w, o);
+    if (lane >= o) {
+      v += y;
+      w += z;
+    }
   }
-  if (lane == 31) s_tot[warp] = v;
+  if (lane == 31) {
+    s_tot[0][warp] = v;
+    s_tot[1][warp] = w;
+  }
   __syncthreads();
-  int base = 0;
-  for (int w = 0; w < warp; ++w) base += s_tot[w];
+  for (int q = 0; q < warp; ++q) {
+    v += s_tot[0][q];
+    w += s_tot[1][q];
+  }
   if (i < nrows) {
-    off[i] = fill[i] = base + v - c;
-    if (i == nrows - 1) off[nrows] = base + v;
+    off[i] = fill[i] = v - c;
+    task[i] = w - g;
+    if (i == nrows - 1) {
+      off[nrows] = v;
+      task[nrows] = w;
+    }
   }
 }
 __global__ void k_pool_place(const int *pool_j, const int *pool_m, const int *counter, long pool_cap,
@@ -962,37 +977,42 @@ __global__ void k_pool_place(const int *pool_j, const int *pool_m, const int *co
 }
 
 // Canonical distances, 32 chains per warp against one batch row
-// (gm_rowdot.cuh): kRescoreSplit warps walk each row's candidates, as many its
-// column pairs.  A pair's offer goes on one of its existing row's chains, as
-// in the NN-Descent insertion (its entry is its place in pair_j).
-// Bound by memory (a feature row per chain).  500 rows x 784 features
-// against 70,000: candidates by a CTA of four warps per row (4-byte copies, 1.1
-// waves) 73 us and pairs with both rows gathered 57 us; together 79 us now, of which
-// reading most of the 220 MB of rows once is half.
-constexpr int kRescoreWarps = 2;
-constexpr int kRescoreSplit = 4;
-__global__ void __launch_bounds__(kRescoreWarps * 32)
+// (gm_rowdot.cuh): a warp takes groups of 32 of a row's candidates or column
+// pairs in a grid stride, found in the groups' prefix by two 32-way steps.  A
+// pair's offer goes on one of its existing row's chains, as in the NN-Descent
+// insertion (its entry is its place in pair_j).
+// Pairs are spread very unevenly: a row near the middle of its cluster enters
+// thousands of lists, so a fixed number of warps per row waits for such rows.
+// 500 rows x 784 features against 70,000 (60 candidates and 60 pairs a row on
+// average): candidates by a CTA of four warps per row and pairs with both rows
+// gathered 130 us, four warps per row and kind 79 us, groups 33 us.
+__global__ void __launch_bounds__(32)
     k_rescore(const float *X, int ld, const float *norms, int brow0, int nrows, const int *cand,
               long cand_ld, const int *row_cnt, float *cand_d, const int *pair_j, const int *pair_off,
-              float *pair_d, const Key *g_key, OfferChains chains) {
+              float *pair_d, const int *task, const Key *g_key, OfferChains chains) {
   pdl_enter();
-  __shared__ __align__(16) RowDotTiles tiles[kRescoreWarps];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int task = blockIdx.x * kRescoreWarps + warp;
-  const int ml = task / (2 * kRescoreSplit), part = task % (2 * kRescoreSplit);
-  if (ml >= nrows) return;
-  const int row = brow0 + ml;
-  const float *xa = X + (size_t)row * ld;
-  const bool pairs = part >= kRescoreSplit;
-  if (pairs && !pair_off) return;
-  const int begin = pairs ? pair_off[ml] : 0;
-  const int cnt = pairs ? pair_off[ml + 1] - begin : row_cnt[ml];
-  const int *ids = pairs ? pair_j + begin : cand + (long)ml * cand_ld;
-  float *out = pairs ? pair_d + begin : cand_d + (long)ml * cand_ld;
-  for (int i0 = (part % kRescoreSplit) * 32; i0 < cnt; i0 += kRescoreSplit * 32) {
-    const int i = i0 + lane;
+  __shared__ __align__(16) RowDotTiles tiles;
+  const int lane = threadIdx.x;
+  const unsigned full = 0xffffffffu;
+  const int total = task[nrows];
+  const int step = (nrows + 31) / 32;  // (at most 32: kMaxBlockRows)
+  for (int t = blockIdx.x; t < total; t += gridDim.x) {
+    // the last row whose groups begin at or before t
+    int at = lane * step;
+    unsigned le = __ballot_sync(full, at < nrows && task[at] <= t);
+    const int base = (31 - __clz(le)) * step;
+    at = base + lane;
+    le = __ballot_sync(full, lane < step && at < nrows && task[at] <= t);
+    const int ml = base + 31 - __clz(le), row = brow0 + ml;
+    const int n_cand = row_cnt[ml], g = t - task[ml], gc = (n_cand + 31) / 32;
+    const bool pairs = g >= gc;
+    const int begin = pairs ? pair_off[ml] : 0;
+    const int cnt = pairs ? pair_off[ml + 1] - begin : n_cand;
+    const int *ids = pairs ? pair_j + begin : cand + (long)ml * cand_ld;
+    float *out = pairs ? pair_d + begin : cand_d + (long)ml * cand_ld;
+    const int i = (pairs ? g - gc : g) * 32 + lane;
     const int j = i < cnt ? ids[i] : row;
-    const float dv = canon_dist(norms[row], norms[j], warp_row_dot(X, ld, xa, j, tiles[warp]));
+    const float dv = canon_dist(norms[row], norms[j], warp_row_dot(X, ld, X + (size_t)row * ld, j, tiles));
     if (i < cnt) {
       out[i] = dv;
       if (pairs && make_key(dv, row) < g_key[(size_t)j * kListW + kListW - 1])
@@ -1245,14 +1265,17 @@ void launch_exact_screen(const DevState &st, int row0, int blk0, int nrows, int 
   const OfferChains chains{x.heads, x.pool_m};
   if (row0 > 0) {
     launch(k_pool_count, grid, 256, 0, s, x.pool_m, x.counter, x.pool_cap, nrows, x.pcnt, st.stat);
-    launch(k_pool_offsets, 1, kMaxBlockRows, 0, s, nrows, x.pcnt, x.poff, x.pfill);
+    note_launch();
+  }
+  launch(k_pool_offsets, 1, kMaxBlockRows, 0, s, nrows, x.pcnt, x.row_cnt, x.poff, x.pfill, x.ptask);
+  if (row0 > 0) {
     launch(k_pool_place, grid, 256, 0, s, x.pool_j, x.pool_m, x.counter, x.pool_cap, x.pfill, x.pair_j,
            x.pair_m);
-    note_launch(3);
+    note_launch();
   }
-  launch(k_rescore, cdiv((long)nrows * 2 * kRescoreSplit, kRescoreWarps), kRescoreWarps * 32, 0, s, st.X,
-         st.ld, st.norms, brow0, nrows, x.cand, ldD, x.row_cnt, x.cand_d, x.pair_j,
-         row0 > 0 ? x.poff : nullptr, x.pool_d, st.g_key, chains);
+  // (twelve CTAs fit an SM)
+  launch(k_rescore, 12 * std::max(sms, 1), 32, 0, s, st.X, st.ld, st.norms, brow0, nrows, x.cand, ldD,
+         x.row_cnt, x.cand_d, x.pair_j, x.poff, x.pool_d, x.ptask, st.g_key, chains);
   launch(k_row_select, cdiv(nrows, kRowWarps), kRowWarps * 32, 0, s, x.cand_d, brow0, nrows, x.cand, ldD,
          x.row_cnt, st.g_key, st.stat);
   note_launch(2);

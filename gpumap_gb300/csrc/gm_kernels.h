@@ -153,6 +153,7 @@ struct ExactScreen {
   int *pcnt = nullptr;        // pairs per batch row
   int *poff = nullptr;        // the groups' offsets (rows + 1) and fill cursors
   int *pfill = nullptr;
+  int *ptask = nullptr;       // prefix of the rows' groups of 32 chains (rows + 1)
   int *heads = nullptr;       // chain heads of the existing rows (n_cap x 32, all -1)
   int *counter = nullptr;     // pairs in the pool
   long pool_cap = 0;

@@ -23,12 +23,6 @@ struct RowDotTiles {
   float b[kDotRing][32][kDotLd];
   float a[kDotRing][kDotChunk];
 };
-// Slots of one warp whose lanes have a pair of rows each.
-struct PairDotTiles {
-  float a[kDotRing][32][kDotLd];
-  float b[kDotRing][32][kDotLd];
-};
-
 GM_D void dot_cp16(float *dst, const float *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
                    (uint32_t)__cvta_generic_to_shared(dst)),
@@ -74,47 +68,6 @@ GM_D float warp_row_dot(const float *X, int ld, const float *xa, int rb, RowDotT
     __syncwarp();
     const int slot = c % kDotRing, nq = min(kDotChunk, ld - c * kDotChunk) >> 2;
     const float4 *av = reinterpret_cast<const float4 *>(t.a[slot]);
-    const float4 *bv = reinterpret_cast<const float4 *>(t.b[slot][lane]);
-    if (nq == 8) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) dot = dot_fma4(av[i], bv[i], dot);
-    } else {
-      for (int i = 0; i < nq; ++i) dot = dot_fma4(av[i], bv[i], dot);
-    }
-    __syncwarp();
-  }
-  return dot;
-}
-
-// Lane l: dot of its rows ra and rb.
-GM_D float warp_pair_dot(const float *X, int ld, int ra, int rb, PairDotTiles &t) {
-  const int lane = threadIdx.x & 31, q = lane & 7, r0 = lane >> 3;
-  const float *sa[8], *sb[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    sa[i] = X + (size_t)__shfl_sync(0xffffffffu, ra, r0 + 4 * i) * ld + 4 * q;
-    sb[i] = X + (size_t)__shfl_sync(0xffffffffu, rb, r0 + 4 * i) * ld + 4 * q;
-  }
-  const int nch = (ld + kDotChunk - 1) / kDotChunk;
-  auto issue = [&](int c) {
-    if (c * kDotChunk + 4 * q < ld) {
-      const int slot = c % kDotRing;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        dot_cp16(&t.a[slot][r0 + 4 * i][4 * q], sa[i] + c * kDotChunk);
-        dot_cp16(&t.b[slot][r0 + 4 * i][4 * q], sb[i] + c * kDotChunk);
-      }
-    }
-    dot_commit();
-  };
-  for (int c = 0; c < kDotRing - 1; ++c) issue(c);
-  float dot = 0.0f;
-  for (int c = 0; c < nch; ++c) {
-    issue(c + kDotRing - 1);
-    dot_wait();
-    __syncwarp();
-    const int slot = c % kDotRing, nq = min(kDotChunk, ld - c * kDotChunk) >> 2;
-    const float4 *av = reinterpret_cast<const float4 *>(t.a[slot][lane]);
     const float4 *bv = reinterpret_cast<const float4 *>(t.b[slot][lane]);
     if (nq == 8) {
 #pragma unroll
