@@ -209,6 +209,12 @@ GM_D float pair_bound(float coef, float sa, float sb, float na, float nb) {
 }
 
 
+// A tile's distance |a|^2 + |b|^2 - 2 a.b from the sum of the norms, rounded,
+// and the accumulator (doubling it is exact, so one rounding remains).
+GM_D float tile_dist(float na, float nb, float acc) {
+  return __fmaf_rn(-2.0f, acc, __fadd_rn(na, nb));
+}
+
 // Max-heap of the 32 smallest upper bounds of one row, in shared memory with
 // stride kTM (element i of row r at h[i * kTM]).  Pushes x (the caller has
 // checked x < the current threshold) and returns the new threshold: the
@@ -435,14 +441,17 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
     const bool live = m < nb;
     const int row = arow0 + m;
     const int gt = threadIdx.x - 64 - 128 * group;  // 0..127 within the group
-    const float nm = live ? norms[row] : 0.0f;
-    const float sm = live ? snorms[row] : 0.0f;
     const float inf = __int_as_float(0x7f800000);
+    // rows past the block's last have an infinite norm and no limit: no
+    // column passes their tests (with a limit of +inf every column did, and
+    // a warp with such a row took all of them through the exact tests)
+    const float nm = live ? norms[row] : inf;
+    const float sm = live ? snorms[row] : 0.0f;
     float *heap = heaps + r;
     int hcnt = 0;
     float t_loc = inf;  // passes 0 and 1: the heap's largest once it holds 32
-    const float t_row = (kPass == 2 && live) ? sc.row_t[m] : inf;
-    const float seed = ((kPass == 1 || kPass == 3) && live && sc.seed) ? sc.seed[m] : inf;
+    const float t_row = (kPass == 2 && live) ? sc.row_t[m] : -inf;
+    const float seed = (kPass == 1 || kPass == 3) ? (!live ? -inf : sc.seed ? sc.seed[m] : inf) : -inf;
     int *cand_m = sc.cand + (long)m * sc.cand_ld;
     // pass 3: the segment of stored columns of (row m, this CTA), filled by
     // the row's threads of every group through a shared-memory counter
@@ -508,7 +517,7 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
       }
       // the largest pair bound of the row over this group's columns
       // (pair_bound is nondecreasing in the column's norm and factor)
-      float bmax;
+      float bmax, nmax;
       {
         unsigned mn = 0, ms = 0;
 #pragma unroll
@@ -516,7 +525,8 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
           mn = max(mn, mx[4 * group + q]);
           ms = max(ms, mx[16 + 4 * group + q]);
         }
-        bmax = pair_bound(sc.coef, sm, __uint_as_float(ms), nm, __uint_as_float(mn));
+        nmax = __uint_as_float(mn);
+        bmax = pair_bound(sc.coef, sm, __uint_as_float(ms), nm, nmax);
       }
       if (t + (int)gridDim.x < sc.tile_count) load_cols(t + gridDim.x);
       if (eok && !mbar_wait(&tmem_full[b], (tc >> 1) & 1)) {
@@ -526,10 +536,16 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
       if (!eok) continue;
       tc_fence_after();
       const int ctile = t * sc.tile_stride * kTN;
-      // passes 2 and 3: D - B of every column of the group is at least
-      // RD(D - bmax); when that exceeds the row's limit and the column's list
-      // bar in every lane, no test can pass for the column
+      // passes 2 and 3: a column needs no exact test unless some lane's
+      // nj - 2 a is at most L + slack, L the larger of the row's limit and the
+      // column's list bar, both 0 or more, or -inf.  With M = nm + nmax and
+      // u = 2^-24, |2 a| below 1.1 M: for L > 4 M it always is.  For L below
+      // that, a test that passes has RD(D - B) <= L, hence D <= L + bmax +
+      // 8 u M, and D = fl(fl(nm + nj) - 2 a) is at least nm + nj - 2 a -
+      // 3.1 u M; the slack adds 1e-6 M = 16.8 u M to bmax - nm, and the two
+      // per-column roundings are directed to the safe side.
       const float lim = kPass == 3 ? seed : t_row;
+      const float slack = __fadd_ru(__fsub_ru(bmax, nm), __fmul_ru(1e-6f, __fadd_ru(nm, nmax)));
       float cmin = inf;    // pass 0: the 32-column chunk's smallest D over other columns
       unsigned hmask = 0;  // column test: the chunk's hit columns (bit i)
       // the exact tests of column c + i of the tile (chunk bit (c & 16) + i),
@@ -565,19 +581,23 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
       // in v and at tensor-memory address tah
       auto half = [&](uint32_t(&v)[16], int c, uint32_t tah) {
         const int col0 = ctile + c;
-        // fast phase: D of the 16 columns and, for passes 2 and 3, a
+        // fast phase: D of the 16 columns or, for passes 2 and 3, a
         // warp-uniform mask of the columns where some lane may pass a test;
         // 16 independent chains without branches
         unsigned need = 0u;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const float dv = __fsub_rn(__fadd_rn(nm, cn[c + i]), __fmul_rn(2.0f, __uint_as_float(v[i])));
-          if (kPass == 1) v[i] = __float_as_uint(dv);
-          if (kKeepD && live && col0 + i < n) D[(long)m * ldD + col0 + i] = dv;
-          if (kPass == 0 && live && col0 + i < n && col0 + i != row) cmin = fminf(cmin, dv);
+          const float acc = __uint_as_float(v[i]);
           if (kPass == 2 || kPass == 3) {
             const float wj = kPass == 3 ? cn[2 * kTN + c + i] : -inf;
-            if (__any_sync(0xffffffffu, __fsub_rd(dv, bmax) <= fmaxf(lim, wj))) need |= 1u << i;
+            const float part = __fmaf_rd(-2.0f, acc, cn[c + i]);
+            if (__any_sync(0xffffffffu, part <= __fadd_ru(fmaxf(lim, wj), slack))) need |= 1u << i;
+          }
+          if (kPass < 2 || kKeepD) {
+            const float dv = tile_dist(nm, cn[c + i], acc);
+            if (kPass == 1) v[i] = __float_as_uint(dv);
+            if (kKeepD && live && col0 + i < n) D[(long)m * ldD + col0 + i] = dv;
+            if (kPass == 0 && live && col0 + i < n && col0 + i != row) cmin = fminf(cmin, dv);
           }
         }
         // slow phase, in column order: every column for the heap pass; for
@@ -592,7 +612,7 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
             const int i = __ffs(need) - 1;
             need &= need - 1;
             const float acc = __uint_as_float(tmem_ld1(tah + (uint32_t)i));
-            slow(i, __fsub_rn(__fadd_rn(nm, cn[c + i]), __fmul_rn(2.0f, acc)), c);
+            slow(i, tile_dist(nm, cn[c + i], acc), c);
           }
         }
       };
