@@ -780,6 +780,76 @@ GM_D float warp_32nd(const float *v, int cnt, int lane) {
   return __shfl_sync(0xffffffffu, top, 31);
 }
 
+// The 32nd smallest of cnt values >= 0 (inf included), value i at get(i), by a
+// whole CTA: inf when there are fewer.  The values' bits are counted in up to
+// 256 equal bins of their range, then of the bin that holds the 32nd, and so
+// on: at most four rounds of two barriers, where a search by bits takes 31
+// rounds and compares every value in each.  Every thread returns it.
+struct Select32 {
+  int bins[2][256];
+  unsigned lo, hi;
+};
+template <int kThreads, typename F>
+GM_D float cta_32nd(int cnt, F &&get, Select32 &sh) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  if (cnt < kListTop) return __int_as_float(0x7f800000);  // (the same for every thread)
+  unsigned lo = full, hi = 0u;
+  for (int i = threadIdx.x; i < cnt; i += kThreads) {
+    const unsigned v = __float_as_uint(get(i));
+    lo = min(lo, v);
+    hi = max(hi, v);
+  }
+  if (threadIdx.x == 0) {
+    sh.lo = full;
+    sh.hi = 0u;
+  }
+  for (int i = threadIdx.x; i < 256; i += kThreads) sh.bins[0][i] = 0;
+  __syncthreads();
+  lo = __reduce_min_sync(full, lo);
+  hi = __reduce_max_sync(full, hi);
+  if (lane == 0) {
+    atomicMin(&sh.lo, lo);
+    atomicMax(&sh.hi, hi);
+  }
+  __syncthreads();
+  lo = sh.lo;
+  hi = sh.hi;
+  int want = kListTop;  // the rank of the value among those in [lo, hi]
+  for (int buf = 0; lo < hi; buf ^= 1) {
+    const int shift = max(0, 24 - __clz((int)(hi - lo)));  // (hi - lo) >> shift < 256
+    for (int i = threadIdx.x; i < cnt; i += kThreads) {
+      const unsigned v = __float_as_uint(get(i));
+      if (v >= lo && v <= hi) atomicAdd(&sh.bins[buf][(v - lo) >> shift], 1);
+    }
+    for (int i = threadIdx.x; i < 256; i += kThreads) sh.bins[buf ^ 1][i] = 0;
+    __syncthreads();
+    // each warp finds the bin: eight of them a lane
+    int c[8], sum = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) sum += c[q] = sh.bins[buf][lane * 8 + q];
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(full, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const int src = __ffs(__ballot_sync(full, incl >= want)) - 1;
+    int rank = want - (incl - sum), bin = 0;
+#pragma unroll
+    for (int q = 0; q < 7; ++q)
+      if (bin == q && rank > c[q]) {
+        rank -= c[q];
+        ++bin;
+      }
+    want = __shfl_sync(full, rank, src);
+    lo += (unsigned)__shfl_sync(full, lane * 8 + bin, src) << shift;
+    hi = min(hi, lo + ((1u << shift) - 1u));
+    __syncthreads();
+  }
+  return __uint_as_float(lo);
+}
+
 // Warp per batch row: T = the 32nd smallest of the union of the CTAs' heaps
 // (pass 1), capped by the seed; both bound the row's 32nd smallest upper
 // bound from above.  With run_if, only when *run_if != 0.
@@ -801,21 +871,27 @@ __global__ void __launch_bounds__(kFinalWarps * 32)
   }
 }
 
-// Warp per batch row: the seed, the 32nd smallest of the row's chunk minima
+// CTA per batch row: the seed, the 32nd smallest of the row's chunk minima
 // from pass 0 (the largest upper bound of 32 distinct columns).  Clears the
-// counters of the passes after it.
-__global__ void __launch_bounds__(kFinalWarps * 32)
-    k_seed_select(const float *mins, int mins_ld, int nrows, float *seed, int *row_cnt, int *pcnt,
-                  int *counter, int *pre_over) {
+// counters of the passes after it.  1,000 rows of 600 minima: 25 us by a warp
+// per row (insertion above 512 values), 10.4 us.
+constexpr int kSeedThreads = 128, kSeedStage = 4096;
+__global__ void __launch_bounds__(kSeedThreads)
+    k_seed_select(const float *mins, int mins_ld, float *seed, int *row_cnt, int *pcnt, int *counter,
+                  int *pre_over) {
   pdl_enter();
-  const int lane = threadIdx.x & 31;
-  const int ml = blockIdx.x * kFinalWarps + (threadIdx.x >> 5);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *counter = *pre_over = 0;
-  if (ml >= nrows) return;
-  const float T = warp_32nd(mins + (size_t)ml * mins_ld, mins_ld, lane);
-  if (lane == 0) {
-    seed[ml] = T;
-    row_cnt[ml] = pcnt[ml] = 0;
+  extern __shared__ float s_min[];
+  __shared__ Select32 sh;
+  const int m = blockIdx.x;
+  const float *v = mins + (size_t)m * mins_ld;
+  const int staged = min(mins_ld, kSeedStage);
+  for (int i = threadIdx.x; i < staged; i += kSeedThreads) s_min[i] = v[i];
+  // (each thread reads back what it wrote)
+  const float T = cta_32nd<kSeedThreads>(mins_ld, [&](int i) { return i < kSeedStage ? s_min[i] : v[i]; }, sh);
+  if (threadIdx.x == 0) {
+    seed[m] = T;
+    row_cnt[m] = pcnt[m] = 0;
+    if (m == 0) *counter = *pre_over = 0;
   }
 }
 
@@ -823,12 +899,12 @@ __global__ void __launch_bounds__(kFinalWarps * 32)
 // bound (exact: every column whose upper bound is at most T was stored),
 // then the row's candidates, the stored columns with lower bound <= T.  Does
 // nothing when a segment overflowed (the heap passes then run instead).
-// The entries (about 0.8 % of the columns: the seed is a 32 / 4096 quantile)
-// are gathered from the row's segments, a warp per segment, into shared memory,
-// and the bounds, held in registers, searched by bits with one barrier a bit.
+// The entries (about 0.4 % of the columns: the seed is a 32 / 8192 quantile)
+// are gathered from the row's segments, a warp per segment, into shared memory.
 // A warp per row that inserted the bounds one at a time was bound by latency: 33
-// us for 500 rows of ~600 entries, this form 18 us.  A row with more than
-// kPreStage entries is worked through where they lie, by its first warp.
+// us for 500 rows of ~600 entries, a CTA that searched them by bits 24 us in a
+// run (31 rounds over all values, bound by issue), this form 13 us.  A row with
+// more than kPreStage entries is worked through where they lie, by its first warp.
 constexpr int kPreThreads = 128, kPreWarps = kPreThreads / 32;
 constexpr int kPreStage = 2048, kPreSegs = 512;
 __global__ void __launch_bounds__(kPreThreads)
@@ -843,13 +919,13 @@ __global__ void __launch_bounds__(kPreThreads)
   }
   __shared__ float s_ub[kPreStage];
   __shared__ unsigned long long s_ent[kPreStage];
-  __shared__ int s_off[kPreSegs + 1], s_count[32], s_kept;
+  __shared__ int s_off[kPreSegs + 1], s_kept;
+  __shared__ Select32 sel;
   const unsigned full = 0xffffffffu;
   const float inf = __int_as_float(0x7f800000);
   const int *cnts = pre_cnt + (size_t)m * gx;
   const size_t seg0 = (size_t)m * gx * (size_t)cap;
   if (warp == 0) {
-    s_count[lane] = 0;
     int run = 0;
     for (int c0 = 0; c0 < gx; c0 += 32) {
       const int v = c0 + lane < gx ? cnts[c0 + lane] : 0;
@@ -889,24 +965,7 @@ __global__ void __launch_bounds__(kPreThreads)
       }
     }
     __syncthreads();
-    float u[kPreStage / kPreThreads];
-#pragma unroll
-    for (int q = 0; q < kPreStage / kPreThreads; ++q) {
-      const int i = q * kPreThreads + threadIdx.x;
-      u[q] = i < total ? s_ub[i] : inf;
-    }
-    const int used = (total + kPreThreads - 1) / kPreThreads;
-    int bit = 30;
-    T = bits_32nd([&](float x) {
-      int c = 0;
-#pragma unroll
-      for (int q = 0; q < kPreStage / kPreThreads; ++q)
-        if (q < used) c += u[q] <= x;
-      c = (int)__reduce_add_sync(full, (unsigned)c);
-      if (lane == 0 && c) atomicAdd(&s_count[bit], c);
-      __syncthreads();
-      return s_count[bit--];
-    });
+    T = cta_32nd<kPreThreads>(total, [&](int i) { return s_ub[i]; }, sel);
     // fewer than 32 other rows: every column is a candidate
     if (n - 1 < kListTop) T = inf;
     for (int i = warp * 32; i < total; i += kPreThreads)
@@ -1203,15 +1262,18 @@ static void launch_tile(const DevState &st, const ExactMaps &maps, int dh, int r
 }
 
 // Column tiles of the seed pass (evenly spaced over the columns): at least
-// 16, and one in 16 of the block's tiles, so that the seed stays a low
+// 16, and one in 8 of the block's tiles, so that the seed stays a low
 // quantile of the row's upper bounds at any column count; all of them up to 32.
+// One in 16, 8, 4 (the seed and store passes of 1,000 rows x 128 against
+// 160,000, on average over an insertion): 120, 107, 103 us; of 500 rows x 784
+// against 70,000: 88, 87, 92 us.
 // It needs 32 chunks of 32 columns, and some more to be low (from kSeedMin
 // tiles, 40 chunks: it then admits about 65 of 1,280 columns).  Below that the
 // heap and candidate passes run instead: a thread's heap of a row and one
 // group of epilogue warps made them 170 us a block where the seed and store
 // passes and their selections take 43 us (333 rows x 131 against 4,000).
 constexpr int kSeedTiles = 16;
-constexpr int kSeedEvery = 16;
+constexpr int kSeedEvery = 8;
 constexpr int kSeedMin = 5;
 
 int exact_seed_tiles(int n_tiles) {
@@ -1238,8 +1300,8 @@ void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int ro
     const int mins_ld = tiles * (kTN / 32);
     launch_tile<0, false>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx0, m_tiles, tiles, stride,
                           nullptr, 0, mins_ld, 0, nullptr, s);
-    launch(k_seed_select, cdiv(nrows, kFinalWarps), kFinalWarps * 32, 0, s, x.mins, mins_ld, nrows, x.seed,
-           x.row_cnt, x.pcnt, x.counter, x.pre_over);
+    launch(k_seed_select, nrows, kSeedThreads, std::min(mins_ld, kSeedStage) * sizeof(float), s, x.mins, mins_ld,
+           x.seed, x.row_cnt, x.pcnt, x.counter, x.pre_over);
     if (kd)
       launch_tile<3, true>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx, m_tiles, n_tiles, 1, x.seed,
                            cap, 0, 0, nullptr, s);
