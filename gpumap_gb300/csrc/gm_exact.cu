@@ -159,17 +159,6 @@ GM_D void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
-// One column of this thread's lane, waited for.
-GM_D uint32_t tmem_ld1(uint32_t taddr) {
-  uint32_t r;
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r)
-      : "r"(taddr)
-      : "memory");
-  return r;
-}
 GM_D void tmem_ld_wait(uint32_t (&r)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
                : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
@@ -536,8 +525,8 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
       if (!eok) continue;
       tc_fence_after();
       const int ctile = t * sc.tile_stride * kTN;
-      // passes 2 and 3: a column needs no exact test unless some lane's
-      // nj - 2 a is at most L + slack, L the larger of the row's limit and the
+      // passes 2 and 3: a column needs no exact test unless its nj - 2 a is
+      // at most L + slack, L the larger of the row's limit and the
       // column's list bar, both 0 or more, or -inf.  With M = nm + nmax and
       // u = 2^-24, |2 a| below 1.1 M: for L > 4 M it always is.  For L below
       // that, a test that passes has RD(D - B) <= L, hence D <= L + bmax +
@@ -578,20 +567,20 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
         }
       };
       // 16 columns from c (a half of a 32-column chunk), their accumulators
-      // in v and at tensor-memory address tah
-      auto half = [&](uint32_t(&v)[16], int c, uint32_t tah) {
+      // in v
+      auto half = [&](uint32_t(&v)[16], int c) {
         const int col0 = ctile + c;
-        // fast phase: D of the 16 columns or, for passes 2 and 3, a
-        // warp-uniform mask of the columns where some lane may pass a test;
-        // 16 independent chains without branches
-        unsigned need = 0u;
+        // fast phase: D of the 16 columns or, for passes 2 and 3, a mask of
+        // the columns where this row may pass a test; 16 independent chains
+        // without branches
+        unsigned may = 0u;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const float acc = __uint_as_float(v[i]);
           if (kPass == 2 || kPass == 3) {
             const float wj = kPass == 3 ? cn[2 * kTN + c + i] : -inf;
             const float part = __fmaf_rd(-2.0f, acc, cn[c + i]);
-            if (__any_sync(0xffffffffu, part <= __fadd_ru(fmaxf(lim, wj), slack))) need |= 1u << i;
+            if (part <= __fadd_ru(fmaxf(lim, wj), slack)) may |= 1u << i;
           }
           if (kPass < 2 || kKeepD) {
             const float dv = tile_dist(nm, cn[c + i], acc);
@@ -600,20 +589,28 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
             if (kPass == 0 && live && col0 + i < n && col0 + i != row) cmin = fminf(cmin, dv);
           }
         }
-        // slow phase, in column order: every column for the heap pass; for
-        // passes 2 and 3 only the flagged ones, each accumulator read again
-        // from tensor memory (D recomputed by the same operations), so that
-        // nothing of the fast phase stays live across it
+        // slow phase: every column for the heap pass, in order; for passes 2
+        // and 3 each lane its own flagged columns, the lanes' side by side
+        // (about one pair in 250 is flagged, so 16 columns of 32 rows have two
+        // or three, rarely two in one row; a column of the warp at a time
+        // they were two thirds of the kernel's instructions)
         if constexpr (kPass == 1) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) slow(i, __uint_as_float(v[i]), c);
         } else if constexpr (kPass == 2 || kPass == 3) {
-          while (need) {  // warp-uniform
-            const int i = __ffs(need) - 1;
-            need &= need - 1;
-            const float acc = __uint_as_float(tmem_ld1(tah + (uint32_t)i));
-            slow(i, tile_dist(nm, cn[c + i], acc), c);
+          while (may) {
+            const int i = __ffs(may) - 1;
+            may &= may - 1;
+            // v[i]
+            unsigned w8[8], w4[4];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) w8[q] = (i & 1) ? v[2 * q + 1] : v[2 * q];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) w4[q] = (i & 2) ? w8[2 * q + 1] : w8[2 * q];
+            const unsigned w = (i & 8) ? ((i & 4) ? w4[3] : w4[2]) : ((i & 4) ? w4[1] : w4[0]);
+            slow(i, tile_dist(nm, cn[c + i], __uint_as_float(w)), c);
           }
+          __syncwarp();
         }
       };
       // after both halves of the 32-column chunk at c
@@ -665,10 +662,10 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
       for (int h = 0; h < kHalves; h += 2) {
         tmem_ld_wait(va);
         tmem_ld16(ta + (uint32_t)(h + 1) * 16, vb);
-        half(va, group * kGroupCols + h * 16, ta + (uint32_t)h * 16);
+        half(va, group * kGroupCols + h * 16);
         tmem_ld_wait(vb);
         if (h + 2 < kHalves) tmem_ld16(ta + (uint32_t)(h + 2) * 16, va);
-        half(vb, group * kGroupCols + (h + 1) * 16, ta + (uint32_t)(h + 1) * 16);
+        half(vb, group * kGroupCols + (h + 1) * 16);
         chunk_end(group * kGroupCols + h * 16);
       }
       tc_fence_before();
