@@ -984,12 +984,10 @@ uint32_t Session::embed(uint32_t n_ops) {
   const int nu = ni - nb;
   const uint32_t *heur_idx = st_.pub_idx;
   const float *heur_dist = st_.pub_dist;
-  // the rows the reposition step moves (those not in the batch) and the
-  // SGD's row count depend only on the batch: queued before the phase
-  // waits for the previous one (after the schedule, whose compaction
-  // shares the flag scratch)
+  // the rows the reposition step moves (those not in the batch) depend only
+  // on the batch: queued before the phase waits for the previous one (after
+  // the schedule, whose compaction shares the flag scratch)
   auto select_unsel = [&] {
-    launch_set_int(es_.iscal + kIscalN, ni, s);
     if (nu <= 0) return;
     ck(cudaMemsetAsync(es_.flag, 0, (size_t)ni * sizeof(int), s), "flags");
     launch_mark_rows(es_.batch, nb, es_.flag, s);

@@ -65,11 +65,12 @@ void exclusive_scan(const int *in, int *out, int n, int *tmp, cudaStream_t s);
 // Ordered compaction of the ids i in [0, n) with flag[i] != 0 (or, when
 // select >= 0, flag[i] == select) into out; *count receives the number.
 size_t compact_tmp_ints(int n);
-// As compact_flags, with the length read from device memory (bounded by n_max).
-void compact_flags_dev(const int *flag, const int *n_dev, int n_max, int *out,
-                       int *count, int *tmp, cudaStream_t s);
 void compact_flags(const int *flag, int n, int select, int *out, int *count,
                    int *tmp, cudaStream_t s);
+// Ordered compaction of the ids i in [0, min(*n_dev, n_max)) with vals[i] >=
+// *max_val / parts (none when *max_val is not positive).
+void compact_at_least(const float *vals, const float *max_val, int parts, const int *n_dev, int n_max,
+                      int *out, int *count, int *tmp, cudaStream_t s);
 // Ordered compaction of list[i] (i < *n_dev) where pred[list[i]] != 0.
 void compact_list(const int *list, const int *n_dev, int n_max, const int *pred,
                   int *out, int *count, int *tmp, cudaStream_t s);
@@ -241,8 +242,9 @@ void launch_optimize_layout(float *emb, int n, int nb, int k, float alpha0,
                             float gamma, float a, float b, int n_epochs,
                             int neg_rate, uint64_t seed, EmbedScratch &e,
                             cudaStream_t s);
-// Edge scheduling only: max weight, trim, epochs_per_sample, degrees,
-// rounding factor (results in e.t_row/e.flag_tail/e.t_val, e.iscal, e.fscal).
+// Edge scheduling only: trim, epochs_per_sample, degrees, rounding factor
+// (results in e.t_row/e.flag_tail/e.t_val, e.iscal, e.fscal).  After
+// launch_fuzzy_graph, which also leaves the largest weight and cleared degrees.
 void launch_schedule(int n, int nb, int k, float alpha0, int n_epochs, int neg_rate,
                      EmbedScratch &e, cudaStream_t s);
 void launch_mark_rows(const int *rows, int nr, int *flag, cudaStream_t s);
@@ -272,7 +274,6 @@ cudaError_t launch_sgd_call(float *emb, const int *head, const int *tail, const 
                             int max_edges, float alpha0, float gamma, float a, float b, int n_epochs,
                             int neg_rate, uint64_t seed, unsigned *bar, unsigned *err, int device,
                             cudaStream_t s, unsigned long long *stat = nullptr, int max_ctas = 0);
-void launch_set_int(int *p, int v, cudaStream_t s);
 constexpr int kIscalN = 4;
 constexpr int kIscalBarrier = 8;  // iscal[8..9]: SGD grid-barrier words
 void launch_epoch_init(const float *eps, int nnz, int neg_rate, float *next_s,

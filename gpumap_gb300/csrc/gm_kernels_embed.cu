@@ -44,36 +44,46 @@ GM_D float membership(float dist, float rho, float sigma) {
   return v < FLT_MIN ? FLT_MIN : v;
 }
 
-// Block sums of the embed-time distances (256 per block, FP32 tree).
-__global__ void k_mean_partial(const float *pub_dist, int n, int k, int euclid,
-                               float *part, int *ipart) {
+// Block sums of the embed-time distances (256 per block, FP32 tree).  Clears
+// what the kernels after it count into: the head degrees, their maximum, the
+// largest weight, the rows left for k_fix_sigma.
+__global__ void __launch_bounds__(256)
+    k_mean_partial(const float *pub_dist, int n, int k, int euclid, float *part, int *ipart, int *deg,
+                   int *iscal, float *fscal) {
   pdl_enter();
   __shared__ float ss[256];
-  __shared__ float sc[256];
   const int t = threadIdx.x;
   const long g = (long)blockIdx.x * 256 + t;
-  float v = 0.0f, c = 0.0f;
+  if (g < n) deg[g] = 0;
+  if (g == 0) {
+    iscal[IS_MAXDEG] = iscal[IS_MARKED] = 0;
+    fscal[FS_MAXW] = 0.0f;
+  }
+  float v = 0.0f;
+  bool ok = false;
   if (g < (long)n * k) {
-    const int row = (int)(g / k), ki = (int)(g % k);
-    const float raw = edist(pub_dist, k, row, ki, euclid);
+    const int row0 = (int)((long)blockIdx.x * 256 / k);
+    const int in = (int)((long)blockIdx.x * 256 - (long)row0 * k) + t;
+    const float raw = edist(pub_dist, k, row0 + in / k, in % k, euclid);
     if (raw >= 0.0f && raw < FLT_MAX / 2.0f) {
       v = raw;
-      c = 1.0f;
+      ok = true;
     }
   }
   ss[t] = v;
-  sc[t] = c;
-  __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (t < s) {
-      ss[t] = __fadd_rn(ss[t], ss[t + s]);
-      sc[t] = __fadd_rn(sc[t], sc[t + s]);
-    }
+  const int c = __syncthreads_count(ok);
+#pragma unroll
+  for (int s = 128; s >= 32; s >>= 1) {
+    if (t < s) ss[t] = __fadd_rn(ss[t], ss[t + s]);
     __syncthreads();
   }
+  if (t >= 32) return;
+  v = ss[t];
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) v = __fadd_rn(v, __shfl_down_sync(0xffffffffu, v, s));
   if (t == 0) {
-    part[blockIdx.x] = ss[0];
-    ipart[blockIdx.x] = (int)sc[0];
+    part[blockIdx.x] = v;
+    ipart[blockIdx.x] = c;
   }
 }
 
@@ -118,6 +128,66 @@ GM_D void two_sum(float a, float b, float &s, float &e) {
   e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 
+// Where the bisection's sum is known to lie outside the tolerance: at sigma <=
+// .x below the target, at sigma >= .y above it (-1 and infinity: nowhere).  The
+// sum over sigma rises, so one value decides for all beyond it.  Newton's
+// method on the logarithm of g(l) = sum exp(-d l), l = 1 / sigma, which is
+// convex in l, from l = 0 (g = the number of terms); then g at both sides of
+// where it stopped, about kAside from the target.
+// Rounding: __expf is good to 2 + 1.17 |x| units in the last place, so with up
+// to 31 terms g, near a target of at most 5, is off by less than 3e-6 for that,
+// 1.5e-6 for the additions and 1.5e-6 for the roundings of l d and 1 / l; the
+// bisection's own sum (gm_expf, a rounded quotient) by 2e-6 there and by 8e-6
+// at the largest sums.  With g kSure from the target the bisection's sum is more
+// than twice the tolerance from it, on the same side, there and beyond.
+constexpr float kSure = 4e-5f, kAside = 8e-5f;
+constexpr int kNewtonSteps = 8;
+template <int L>
+GM_D float2 sigma_bracket(const float (&dj)[4], const bool (&contrib)[4], float target) {
+  const unsigned full = 0xffffffffu;
+  auto row_sum = [&](float v) {
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(full, v, o));
+    return v;
+  };
+  float d[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) d[j] = fmaxf(dj[j], 0.0f);
+  auto terms = [&](float l, float &g, float &slope) {
+    float e[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) e[j] = contrib[j] ? __expf(__fmul_rn(-d[j], l)) : 0.0f;
+    g = row_sum(__fadd_rn(__fadd_rn(e[0], e[1]), __fadd_rn(e[2], e[3])));
+    slope = __fadd_rn(__fadd_rn(__fmul_rn(d[0], e[0]), __fmul_rn(d[1], e[1])),
+                      __fadd_rn(__fmul_rn(d[2], e[2]), __fmul_rn(d[3], e[3])));
+  };
+  float ones = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) ones = __fadd_rn(ones, contrib[j] && !(dj[j] > 0.0f) ? 1.0f : 0.0f);
+  ones = row_sum(ones);
+  float l = 0.0f, slope = 0.0f;
+  for (int i = 0; i < kNewtonSteps; ++i) {
+    float g;
+    terms(l, g, slope);
+    slope = row_sum(slope);
+    const bool near = fabsf(__fsub_rn(g, target)) < 0.1f * kAside;
+    if (!near) l = __fadd_rn(l, __fmul_rn(__fdividef(g, slope), __logf(__fdividef(g, target))));
+    if (__all_sync(full, near || !(l > 0.0f) || ones > target)) break;
+  }
+  const float aside = __fdividef(kAside, slope);
+  const float la = __fadd_rn(l, aside), lb = __fsub_rn(l, aside);
+  float ga, gb, unused;
+  terms(la, ga, unused);
+  terms(lb, gb, unused);
+  float2 r = make_float2(-1.0f, __int_as_float(0x7f800000));
+  if (lb > 0.0f && isfinite(la) && target <= 5.0f) {
+    if (ga <= target - kSure) r.x = __fdiv_rn(1.0f, la);
+    if (gb >= target + kSure) r.y = __fdiv_rn(1.0f, lb);
+  }
+  if (ones >= target + kSure) r.y = 0.0f;  // (at every sigma)
+  return r;
+}
+
 // sigma / rho by bisection (reference smooth_knn_dist_kernel,
 // embedding_kernel.cuh:135-207), L lanes per row (4 for k <= 16, 8 for k <=
 // 32), terms q, q + L, q + 2L, q + 3L on lane q.  The bisection's target sum is
@@ -128,8 +198,10 @@ GM_D void two_sum(float a, float b, float &s, float &e) {
 // where that cannot decide (within kUnsure of the tolerance's edge): FP64 has
 // 1/64 of the FP32 rate here and bound the kernel.  The other terms of the
 // FP64 tree: (t0 + t2) + (t1 + t3) on each lane, then xor L/2 .. 1.
-// 70,000 rows at k = 15: 151 -> 56 us; 100,000 at k = 30 (a warp per row): 1508
-// -> 187 us.
+// Most of the bisection's steps are decided by where its sum is known to lie
+// (sigma_bracket), and take no sum: three or four of about twenty do.
+// 70,000 rows at k = 15: 151 us in FP64, 56 with FP32 sums, 33 so; 100,000 at k = 30:
+// 1508 (a warp per row), 187, 70.
 // The first CTA takes the global mean meanwhile, which only rows without a
 // positive distance need: those are left marked (sigma < 0, *marked set) for
 // k_fix_sigma.
@@ -184,7 +256,23 @@ __global__ void __launch_bounds__(kSmoothThreads)
     dj[j] = __fsub_rn(san[j], r);
   }
   bool done = !live || !found;
-  for (int it = 0; it < 64; ++it) {
+  const float2 known = sigma_bracket<L>(dj, contrib, t_hi);
+  // one bisection step, when the sum at mid is not within the tolerance
+  auto step = [&](bool above) {
+    if (above) {
+      hi = mid;
+      mid = __fmul_rn(__fadd_rn(lo, hi), 0.5f);
+    } else {
+      lo = mid;
+      mid = (hi == FLT_MAX) ? __fmul_rn(mid, 2.0f) : __fmul_rn(__fadd_rn(lo, hi), 0.5f);
+    }
+  };
+  for (int it = 0;; ++it) {
+    while (!done && it < 64 && (mid <= known.x || mid >= known.y)) {
+      step(mid >= known.y);
+      ++it;
+    }
+    if (it >= 64) done = true;
     if (__all_sync(full, done)) break;
     float t[4];
 #pragma unroll
@@ -218,15 +306,8 @@ __global__ void __launch_bounds__(kSmoothThreads)
       }
     }
     if (done) continue;
-    if (within) {
-      done = true;
-    } else if (above) {
-      hi = mid;
-      mid = __fmul_rn(__fadd_rn(lo, hi), 0.5f);
-    } else {
-      lo = mid;
-      mid = (hi == FLT_MAX) ? __fmul_rn(mid, 2.0f) : __fmul_rn(__fadd_rn(lo, hi), 0.5f);
-    }
+    if (within) done = true;
+    else step(above);
   }
   if (!live || q != 0) return;
   if (!found) {
@@ -250,39 +331,58 @@ __global__ void k_fix_sigma(int n, const float *fscal, float *sigma, const int *
   if (i < n && sigma[i] < 0.0f) sigma[i] = __fmul_rn(kMinKDistScale, fscal[FS_MEAN]);
 }
 
+// The block's largest m into *to (both >= 0); the whole block calls it.
+GM_D void block_max(int m, int *to) {
+  __shared__ int s_max;
+  if (threadIdx.x == 0) s_max = 0;
+  __syncthreads();
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(&s_max, m);
+  __syncthreads();
+  // (most blocks find a value that is no smaller)
+  if (threadIdx.x == 0 && s_max > *(volatile int *)to) atomicMax(to, s_max);
+}
+
 // Directed membership p_ij for batch rows and the fuzzy union
 // w = p_ij + p_ji - p_ij p_ji; flag marks edges whose reverse is absent
-// (reference: embedding_kernel.cuh:214-320).
-__global__ void k_memb_sym(const uint32_t *pub_idx, const float *pub_dist, int n, int k,
-                           int euclid, const float *sigma, const float *rho,
-                           const int *batch, int nb, int *coo_row, int *coo_col,
-                           float *coo_val, int *flag) {
+// (reference: embedding_kernel.cuh:214-320).  Their largest w goes to
+// fscal[FS_MAXW] by the order of the bits (w >= 0; an extra edge has the w of
+// the edge it reverses).
+// Bound by the reads of the other rows' lists out of L2 (120 bytes an edge at k
+// = 30: 128 us for 3 million edges; 16 or 32 lanes that read a list in one
+// request take as long, and 8.5 us instead of 5.6 for 15,000 edges).
+__global__ void __launch_bounds__(256)
+    k_memb_sym(const uint32_t *pub_idx, const float *pub_dist, int n, int k, int euclid,
+               const float *sigma, const float *rho, const int *batch, int nb, int *coo_row,
+               int *coo_col, float *coo_val, int *flag, float *fscal) {
   pdl_enter();
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= nb * k) return;
-  const int bi = tid / k, ki = tid - bi * k;
-  const int row = batch[bi];
-  const uint32_t raw_col = eidx(pub_idx, k, row, ki);
-  const bool valid_col = raw_col < (uint32_t)n;
-  const int col = valid_col ? (int)raw_col : row;
-  const float dist = edist(pub_dist, k, row, ki, euclid);
-  float pij = 0.0f;
-  if (valid_col && col != row && valid_d(dist)) pij = membership(dist, rho[row], sigma[row]);
-  const int i = row, j = col;
-  float pji = 0.0f;
-  for (int kj = 0; kj < k; ++kj) {
-    if ((int)eidx(pub_idx, k, j, kj) == i) {
-      const float dji = edist(pub_dist, k, j, kj, euclid);
-      if (!valid_d(dji)) break;
-      pji = membership(dji, rho[j], sigma[j]);
-      break;
+  float w = 0.0f;
+  if (tid < nb * k) {
+    const int bi = tid / k, ki = tid - bi * k;
+    const int row = batch[bi];
+    const uint32_t raw_col = eidx(pub_idx, k, row, ki);
+    const bool valid_col = raw_col < (uint32_t)n;
+    const int col = valid_col ? (int)raw_col : row;
+    const float dist = edist(pub_dist, k, row, ki, euclid);
+    float pij = 0.0f;
+    if (valid_col && col != row && valid_d(dist)) pij = membership(dist, rho[row], sigma[row]);
+    float pji = 0.0f;
+    for (int kj = 0; kj < k; ++kj) {
+      if ((int)eidx(pub_idx, k, col, kj) == row) {
+        const float dji = edist(pub_dist, k, col, kj, euclid);
+        if (!valid_d(dji)) break;
+        pji = membership(dji, rho[col], sigma[col]);
+        break;
+      }
     }
+    w = __fmaf_rn(-pij, pji, __fadd_rn(pij, pji));
+    coo_row[tid] = row;
+    coo_col[tid] = col;
+    coo_val[tid] = w;
+    flag[tid] = (pji == 0.0f) ? 1 : 0;
   }
-  const float w = __fmaf_rn(-pij, pji, __fadd_rn(pij, pji));
-  coo_row[tid] = i;
-  coo_col[tid] = j;
-  coo_val[tid] = w;
-  flag[tid] = (pji == 0.0f) ? 1 : 0;
+  block_max(w > 0.0f ? __float_as_int(w) : 0, reinterpret_cast<int *>(&fscal[FS_MAXW]));
 }
 
 __global__ void k_write_extras(const int *idx, const int *cnt, int ndir, int *coo_row,
@@ -301,64 +401,61 @@ __global__ void k_write_extras(const int *idx, const int *cnt, int ndir, int *co
   coo_val[ndir + q] = coo_val[src];
 }
 
-// max_w over non-negative weights via the int ordering of their bits.
-__global__ void k_max_w(const float *vals, const int *iscal, float *fscal) {
+// Gather survivors; epochs_per_sample; head degrees and their maximum; epoch
+// state (reference: :469-495, :405-460).  A row's edges stand together but
+// for the extras: the first of each run in a warp adds the run's length (one
+// atomic for up to 32 edges).  Bound by the chain of loads from an edge's index
+// to its degree: kGatherAhead edges a thread, their loads together.
+// 4.3 million edges: 67 us with one a thread and an atomic each, 43 us so.
+constexpr int kGatherAhead = 4;
+__global__ void __launch_bounds__(256)
+    k_gather_sched(const int *idx, int *iscal, const int *crow, const int *ccol, const float *cval,
+                   const float *fscal, int n_epochs, float nsr_inv, int *trow, int *tcol, float *eps,
+                   float *next_s, float *next_n, int *deg) {
   pdl_enter();
-  const int nnz = iscal[IS_NNZ];
-  float m = 0.0f;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nnz; q += gridDim.x * blockDim.x)
-    m = fmaxf(m, vals[q]);
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0.0f)
-    atomicMax(reinterpret_cast<int *>(&fscal[FS_MAXW]), __float_as_int(m));
-}
-
-// Trim flag: keep w >= max_w / n_epochs (reference trim_graph, :348-400).
-__global__ void k_trim_flags(const float *vals, const int *iscal, const float *fscal,
-                             int n_epochs, int *flag, int nmax) {
-  pdl_enter();
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nmax) return;
-  const int nnz = iscal[IS_NNZ];
+  const int nnz = iscal[IS_NNZ2], q0 = blockIdx.x * 256 * kGatherAhead;
+  if (q0 >= nnz) return;
+  const int lane = threadIdx.x & 31;
   const float mw = fscal[FS_MAXW];
-  int keep = 0;
-  if (q < nnz && mw > 0.0f) keep = vals[q] >= __fdiv_rn(mw, (float)n_epochs) ? 1 : 0;
-  flag[q] = keep;
+  int src[kGatherAhead], head[kGatherAhead], tail[kGatherAhead], dmax = 0;
+  float w[kGatherAhead];
+#pragma unroll
+  for (int u = 0; u < kGatherAhead; ++u) {
+    const int q = q0 + u * 256 + threadIdx.x;
+    src[u] = q < nnz ? idx[q] : -1;
+  }
+#pragma unroll
+  for (int u = 0; u < kGatherAhead; ++u) {
+    head[u] = src[u] >= 0 ? crow[src[u]] : -1;
+    tail[u] = src[u] >= 0 ? ccol[src[u]] : 0;
+    w[u] = src[u] >= 0 ? cval[src[u]] : 0.0f;
+  }
+#pragma unroll
+  for (int u = 0; u < kGatherAhead; ++u) {
+    const int prev = __shfl_up_sync(0xffffffffu, head[u], 1);
+    const bool first = lane == 0 || head[u] != prev;
+    const unsigned starts = __ballot_sync(0xffffffffu, first);
+    if (head[u] < 0) continue;
+    const int q = q0 + u * 256 + threadIdx.x;
+    const float ns = __fmul_rn((float)n_epochs, __fdiv_rn(w[u], mw));
+    const float e = (ns > 0.0f) ? __fdiv_rn((float)n_epochs, ns) : -1.0f;
+    trow[q] = head[u];
+    tcol[q] = tail[u];
+    eps[q] = e;
+    next_s[q] = e;
+    next_n[q] = __fmul_rn(e, nsr_inv);
+    if (first) {
+      const unsigned later = lane == 31 ? 0u : starts >> (lane + 1);
+      const int run = later ? __ffs(later) : 32 - lane;
+      dmax = max(dmax, atomicAdd(&deg[head[u]], run) + run);
+    }
+  }
+  block_max(dmax, &iscal[IS_MAXDEG]);
 }
 
-// Gather survivors; epochs_per_sample; head degrees; epoch state
-// (reference: :469-495, :405-460).
-__global__ void k_gather_sched(const int *idx, const int *iscal, const int *crow,
-                               const int *ccol, const float *cval, const float *fscal,
-                               int n_epochs, float nsr_inv, int *trow, int *tcol,
-                               float *eps, float *next_s, float *next_n, int *deg) {
-  pdl_enter();
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= iscal[IS_NNZ2]) return;
-  const int src = idx[q];
-  const float mw = fscal[FS_MAXW];
-  const float w = cval[src];
-  const float ns = __fmul_rn((float)n_epochs, __fdiv_rn(w, mw));
-  const float e = (ns > 0.0f) ? __fdiv_rn((float)n_epochs, ns) : -1.0f;
-  trow[q] = crow[src];
-  tcol[q] = ccol[src];
-  eps[q] = e;
-  next_s[q] = e;
-  next_n[q] = __fmul_rn(e, nsr_inv);
-  atomicAdd(&deg[crow[src]], 1);
-}
-
-__global__ void k_max_deg(const int *deg, int n, int *iscal) {
-  pdl_enter();
-  int m = 0;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
-    m = max(m, deg[q]);
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(&iscal[IS_MAXDEG], m);
-}
-
-// Gradient rounding factor 2^ceil-ish via frexp (reference :433-460).
-__global__ void k_rounding(int *iscal, float *fscal, float alpha) {
+// Gradient rounding factor 2^ceil-ish via frexp (reference :433-460), and the
+// SGD's row count.
+__global__ void k_rounding(int *iscal, float *fscal, float alpha, int n) {
   pdl_enter();
   const int nnz = iscal[IS_NNZ2];
   const int md = iscal[IS_MAXDEG];
@@ -372,6 +469,7 @@ __global__ void k_rounding(int *iscal, float *fscal, float alpha) {
     r = ldexpf(1.0f, ex);
   }
   fscal[FS_ROUND] = r;
+  iscal[IS_N] = n;
 }
 
 GM_D float fclip(float v) {
@@ -686,11 +784,6 @@ __global__ void __launch_bounds__(kSgdThreads)
   sgd_stats(my_edges, my_negs, stat);
 }
 
-__global__ void k_set_int(int *p, int v) {
-  pdl_enter();
-  *p = v;
-}
-
 __global__ void k_epoch_init(const float *eps, int nnz, float nsr_inv, float *next_s,
                              float *next_n) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -835,9 +928,9 @@ void launch_fuzzy_graph(const uint32_t *pub_idx, const float *pub_dist, int n, i
                         EmbedScratch &e, cudaStream_t s) {
   const long total = (long)n * k;
   const int nbl = cdiv(total, 256);
-  launch(k_mean_partial, nbl, 256, 0, s, pub_dist, n, k, euclidean, e.partial, e.ipartial);
+  launch(k_mean_partial, nbl, 256, 0, s, pub_dist, n, k, euclidean, e.partial, e.ipartial, e.deg, e.iscal,
+         e.fscal);
   note_launch();
-  cudaMemsetAsync(e.iscal + IS_MARKED, 0, sizeof(int), s);
   const float t_hi = (float)log2_target, t_lo = (float)(log2_target - (double)t_hi);
   auto smooth = [&](auto kernel, int lanes) {
     launch(kernel, 1 + cdiv((long)n * lanes, kSmoothThreads), kSmoothThreads, 0, s, pub_dist, n, k,
@@ -849,10 +942,11 @@ void launch_fuzzy_graph(const uint32_t *pub_idx, const float *pub_dist, int n, i
   launch(k_fix_sigma, cdiv(n, 256), 256, 0, s, n, e.fscal, e.sigma, e.iscal + IS_MARKED);
   note_launch(2);
   const int ndir = nb * k;
-  if (ndir > 0)
-    launch(k_memb_sym, cdiv(ndir, 256), 256, 0, s, pub_idx, pub_dist, n, k, euclidean, e.sigma, e.rho,
-           batch, nb, e.coo_row, e.coo_col, e.coo_val, e.t_row);
+  if (ndir > 0) {
+    launch(k_memb_sym, cdiv(ndir, 256), 256, 0, s, pub_idx, pub_dist, n, k,
+           euclidean, e.sigma, e.rho, batch, nb, e.coo_row, e.coo_col, e.coo_val, e.t_row, e.fscal);
     note_launch();
+  }
   compact_flags(e.t_row, ndir, -1, e.t_col, e.iscal + IS_EXTRA, e.tmp2, s);
   launch(k_write_extras, cdiv(ndir > 0 ? ndir : 1, 256), 256, 0, s, e.t_col, e.iscal + IS_EXTRA, ndir,
          e.coo_row, e.coo_col, e.coo_val, e.iscal);
@@ -866,22 +960,15 @@ void launch_schedule(int n, int nb, int k, float alpha0, int n_epochs, int neg_r
     return;
   }
   const int nmax = 2 * nb * k;
-  cudaMemsetAsync(e.fscal + FS_MAXW, 0, sizeof(float), s);
-  cudaMemsetAsync(e.iscal + IS_MAXDEG, 0, sizeof(int), s);
-  cudaMemsetAsync(e.deg, 0, sizeof(int) * (size_t)n, s);
-  launch(k_max_w, min(cdiv(nmax, 256), 1024), 256, 0, s, e.coo_val, e.iscal, e.fscal);
-  note_launch();
-  launch(k_trim_flags, cdiv(nmax, 256), 256, 0, s, e.coo_val, e.iscal, e.fscal, n_epochs, e.t_row, nmax);
-  note_launch();
-  compact_flags_dev(e.t_row, e.iscal + IS_NNZ, nmax, e.t_col, e.iscal + IS_NNZ2, e.tmp2, s);
+  // keep w >= max_w / n_epochs (reference trim_graph, :348-400)
+  compact_at_least(e.coo_val, e.fscal + FS_MAXW, n_epochs, e.iscal + IS_NNZ, nmax, e.t_col, e.iscal + IS_NNZ2,
+                   e.tmp2, s);
   // t_col holds survivor indices; gather into (t_row, flag_tail, t_val)
   const float nsr_inv = 1.0f / (float)neg_rate;  // inf when 0: no negatives
-  launch(k_gather_sched, cdiv(nmax, 256), 256, 0, s, e.t_col, e.iscal, e.coo_row, e.coo_col, e.coo_val,
+  launch(k_gather_sched, cdiv(nmax, 256 * kGatherAhead), 256, 0, s, e.t_col, e.iscal, e.coo_row, e.coo_col, e.coo_val,
          e.fscal, n_epochs, nsr_inv, e.t_row, e.flag_tail, e.t_val, e.next_s, e.next_n, e.deg);
   note_launch();
-  launch(k_max_deg, min(cdiv(n, 256), 1024), 256, 0, s, e.deg, n, e.iscal);
-  note_launch();
-  launch(k_rounding, 1, 1, 0, s, e.iscal, e.fscal, alpha0);
+  launch(k_rounding, 1, 1, 0, s, e.iscal, e.fscal, alpha0, n);
   note_launch();
 }
 
@@ -890,14 +977,8 @@ void launch_optimize_layout(float *emb, int n, int nb, int k, float alpha0, floa
                             EmbedScratch &e, cudaStream_t s) {
   launch_schedule(n, nb, k, alpha0, n_epochs, neg_rate, e, s);
   if (n <= 0 || n_epochs <= 0 || nb <= 0) return;
-  launch_set_int(e.iscal + IS_N, n, s);
   launch_sgd(emb, e.t_row, e.flag_tail, e.t_val, e.next_s, e.next_n, e.iscal, e.fscal,
              cdiv(2 * nb * k, 256), alpha0, gamma, a, b, n_epochs, neg_rate, seed, s, nullptr);
-}
-
-void launch_set_int(int *p, int v, cudaStream_t s) {
-  launch(k_set_int, 1, 1, 0, s, p, v);
-  note_launch();
 }
 
 void launch_epoch_init(const float *eps, int nnz, int neg_rate, float *next_s,

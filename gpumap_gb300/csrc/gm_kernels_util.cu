@@ -66,7 +66,22 @@ struct Pred {
   __device__ __forceinline__ int id(int i) const { return list ? list[i] : i; }
 };
 
-__global__ void __launch_bounds__(kScanThreads) k_block_totals(Pred p, int *tot) {
+// Item i stays when its value is at least *max_val / parts (none does when the
+// maximum is not positive).
+struct PredAtLeast {
+  const float *vals, *max_val;
+  const int *n_dev;
+  int n_host, parts;
+  __device__ __forceinline__ int len() const { return min(*n_dev, n_host); }
+  __device__ __forceinline__ int at(int i) const {
+    const float mw = *max_val;
+    return mw > 0.0f && vals[i] >= __fdiv_rn(mw, (float)parts) ? 1 : 0;
+  }
+  __device__ __forceinline__ int id(int i) const { return i; }
+};
+
+template <typename P>
+__global__ void __launch_bounds__(kScanThreads) k_block_totals(P p, int *tot) {
   pdl_enter();
   __shared__ int wt[kScanThreads / 32];
   const int n = p.len();
@@ -114,8 +129,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_totals(int *tot, int nb,
 }
 
 // mode 0: exclusive scan output out[i]; mode 1: compaction out[pos] = id(i).
-__global__ void __launch_bounds__(kScanThreads) k_block_write(Pred p, const int *tot,
-                                                              int *out, int mode,
+template <typename P>
+__global__ void __launch_bounds__(kScanThreads) k_block_write(P p, const int *tot, int *out, int mode,
                                                               int n_cap_out) {
   pdl_enter();
   __shared__ int wt[kScanThreads / 32];
@@ -146,14 +161,15 @@ __global__ void __launch_bounds__(kScanThreads) k_block_write(Pred p, const int 
 
 inline int nblocks(int n) { return n <= 0 ? 1 : (n + kScanBlock - 1) / kScanBlock; }
 
-void run_scan(const Pred &p, int n_max, int *out, int mode, int *count, int *tmp,
+template <typename P>
+void run_scan(const P &p, int n_max, int *out, int mode, int *count, int *tmp,
               cudaStream_t s) {
   const int nb = nblocks(n_max);
-  launch(k_block_totals, nb, kScanThreads, 0, s, p, tmp);
+  launch(k_block_totals<P>, nb, kScanThreads, 0, s, p, tmp);
   note_launch();
   launch(k_scan_totals, 1, kScanThreads, 0, s, tmp, nb, count);
   note_launch();
-  launch(k_block_write, nb, kScanThreads, 0, s, p, tmp, out, mode, n_max);
+  launch(k_block_write<P>, nb, kScanThreads, 0, s, p, tmp, out, mode, n_max);
   note_launch();
 }
 
@@ -234,9 +250,9 @@ void compact_flags(const int *flag, int n, int select, int *out, int *count,
   run_scan(p, n, out, 1, count, tmp, s);
 }
 
-void compact_flags_dev(const int *flag, const int *n_dev, int n_max, int *out,
-                       int *count, int *tmp, cudaStream_t s) {
-  Pred p{flag, nullptr, n_dev, n_max, -1};
+void compact_at_least(const float *vals, const float *max_val, int parts, const int *n_dev, int n_max,
+                      int *out, int *count, int *tmp, cudaStream_t s) {
+  PredAtLeast p{vals, max_val, n_dev, n_max, parts};
   run_scan(p, n_max, out, 1, count, tmp, s);
 }
 
