@@ -201,8 +201,9 @@ Session::Session(const gm_params &p) : p_(p) {
       xs_.seed = (float *)dalloc((size_t)ex_block_ * sizeof(float));
       // pre-candidate segments: one per (block row, CTA of a row tile), for
       // every grid width a block can take (at most one CTA per column tile)
-      xs_.pre_cap = pre_cap_alloc_ = 64;
+      // and room for every column up to four column tiles
       xs_.pre_gx = (int)std::min<size_t>(std::max(sms_, 1), (Nm + 255) / 256);
+      xs_.pre_cap = pre_cap_alloc_ = std::max(64, (1024 + xs_.pre_gx - 1) / xs_.pre_gx);
       xs_.pre = (unsigned long long *)dalloc((size_t)ex_block_ * xs_.pre_gx * xs_.pre_cap *
                                              sizeof(unsigned long long));
       xs_.pre_ub = (float *)dalloc((size_t)ex_block_ * xs_.pre_gx * xs_.pre_cap * sizeof(float));

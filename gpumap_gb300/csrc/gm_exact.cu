@@ -270,7 +270,7 @@ struct TileScreen {
 // leave the tensor memory (the tile itself is not stored).  grid.y: 128-row
 // tiles of the batch; grid.x: CTAs sharing the column tiles.  For every pair
 // (batch row m, column j) the epilogue forms D and the bound B (pair_bound);
-// its upper bound is D + B and its lower bound D - B.  From five column tiles on:
+// its upper bound is D + B and its lower bound D - B.
 //  Pass 0 (kPass == 0), on an evenly spaced sample of column tiles: per row
 //    and 32-column chunk, the smallest upper bound (sc.mins).  The 32nd
 //    smallest of a row's chunk minima (k_seed_select) is the largest upper
@@ -283,7 +283,8 @@ struct TileScreen {
 //    upper bounds, then keeps the stored columns with lower bound <= T.
 //    Column side, for an existing row j: (j, m) goes to the pair pool when
 //    D - B is at most the 32nd distance of j's list.
-// Up to four column tiles, and for a block whose stored columns overflowed:
+// Up to four column tiles there is no pass 0 and the seed is infinite.  For a
+// block whose stored columns overflowed, or have no room:
 //  Pass 1 (kPass == 1), all column tiles: every CTA keeps, per row, a
 //    max-heap of the 32 smallest upper bounds it sees (at or below the seed
 //    when there is one) and stores it to sc.heaps; the 32nd smallest of
@@ -1265,10 +1266,13 @@ static void launch_tile(const DevState &st, const ExactMaps &maps, int dh, int r
 // 160,000, on average over an insertion): 120, 107, 103 us; of 500 rows x 784
 // against 70,000: 88, 87, 92 us.
 // It needs 32 chunks of 32 columns, and some more to be low (from kSeedMin
-// tiles, 40 chunks: it then admits about 65 of 1,280 columns).  Below that the
-// heap and candidate passes run instead: a thread's heap of a row and one
-// group of epilogue warps made them 170 us a block where the seed and store
-// passes and their selections take 43 us (333 rows x 131 against 4,000).
+// tiles, 40 chunks: it then admits about 65 of 1,280 columns).  Below that
+// there is no seed and every column is stored, where the segments have room for
+// them all.  The heap and candidate passes, which need no room: a thread's heap
+// of a row and one group of epilogue warps make them 170 us a block where the
+// seed and store passes and their selections take 43 us (333 rows x 131 against
+// 4,000), and 147 us where the store of every column takes 34 (333 rows against
+// 333 to 999).
 constexpr int kSeedTiles = 16;
 constexpr int kSeedEvery = 8;
 constexpr int kSeedMin = 5;
@@ -1289,14 +1293,18 @@ void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int ro
   // entries per stored segment: the row's whole allocation shared by its
   // tile's CTAs (fewer CTAs per row tile, longer segments)
   const int cap = x.pre_fixed || gx > x.pre_gx ? x.pre_cap : (int)((long)x.pre_gx * x.pre_cap / gx);
-  if (n_tiles >= kSeedMin && x.pre && cap > 0 && gx <= x.pre_gx &&
-      tiles * (kTN / 32) <= x.mins_ld) {
-    // seed pass over a spread sample of tiles, then the store pass
-    const int stride = n_tiles / tiles;
-    const int gx0 = std::max(1, std::min(tiles, std::max(1, sms / m_tiles)));
-    const int mins_ld = tiles * (kTN / 32);
-    launch_tile<0, false>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx0, m_tiles, tiles, stride,
-                          nullptr, 0, mins_ld, 0, nullptr, s);
+  // columns of a CTA: with room for all of them no segment overflows
+  const int cta_cols = cdiv(n_tiles, gx) * kTN;
+  const bool seeded = n_tiles >= kSeedMin;
+  if (x.pre && cap > 0 && gx <= x.pre_gx &&
+      (seeded ? tiles * (kTN / 32) <= x.mins_ld : cap >= cta_cols)) {
+    // seed pass over a spread sample of tiles (or no seed: every column is
+    // stored), then the store pass
+    const int mins_ld = seeded ? tiles * (kTN / 32) : 0;
+    if (seeded)
+      launch_tile<0, false>(st, maps, dh, row0, blk0, nrows, n, x, ldD,
+                            std::max(1, std::min(tiles, std::max(1, sms / m_tiles))), m_tiles, tiles,
+                            n_tiles / tiles, nullptr, 0, mins_ld, 0, nullptr, s);
     launch(k_seed_select, nrows, kSeedThreads, std::min(mins_ld, kSeedStage) * sizeof(float), s, x.mins, mins_ld,
            x.seed, x.row_cnt, x.pcnt, x.counter, x.pre_over);
     if (kd)
@@ -1308,6 +1316,7 @@ void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int ro
     launch(k_pre_select, nrows, kPreThreads, 0, s, x.pre, x.pre_ub, x.pre_cnt, gx, cap, x.pre_over, n,
            x.row_t, x.cand, ldD, x.row_cnt, st.stat);
     note_launch(2);
+    if (cap >= cta_cols) return;
     // after an overflow only: the heap pass (seed-capped; its pairs were
     // already pooled), the threshold and the candidate pass
     launch_tile<1, false>(st, maps, dh, row0, blk0, nrows, n, x, ldD, gx, m_tiles, n_tiles, 1, x.seed, 0,
