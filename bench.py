@@ -411,8 +411,8 @@ def roofline(stats, d, peaks):
     add("k_exact_dist", st["exact_ms"], st["exact_flops"], st["exact_launches"], "tensor")
     add("exact_screen", st["screen_ms"], st["exact_rescored"] * 2 * d * 4 + st["exact_pairs"] * 8,
         st["exact_launches"], "hbm")
-    add("k_local_join", st["join_ms"], st["join_rows"] * d * 4 + st["join_pairs"] * 8, st["join_launches"], "hbm")
-    add("k_candidate_dists", st["cand_ms"], st["cand_rows"] * d * 4, st["cand_launches"], "hbm")
+    add("local_join", st["join_ms"], st["join_rows"] * d * 4 + st["join_pairs"] * 8, st["join_launches"], "hbm")
+    add("candidate_offers", st["cand_ms"], st["cand_rows"] * d * 4, st["cand_launches"], "hbm")
     add("k_sgd_persistent", st["sgd_ms"], st["sgd_edges"] * 28 + (st["sgd_edges"] + st["sgd_negatives"]) * 8,
         st["sgd_launches"], "hbm")
     for name, t in NCU_TRAFFIC.items():

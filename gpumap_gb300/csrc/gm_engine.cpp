@@ -138,8 +138,7 @@ Session::Session(const gm_params &p) : p_(p) {
     d_batch_ = (int *)dalloc(Nm * sizeof(int));
     d_cnt_ = (int *)dalloc(kCounters * sizeof(int));
     st_.err = (unsigned *)(d_cnt_ + kErrAt);
-    d_tmp_ = (int *)dalloc(std::max(scan_tmp_ints((int)Nm), compact_tmp_ints((int)Nm)) *
-                           sizeof(int) + 64);
+    d_tmp_ = (int *)dalloc(compact_tmp_ints((int)Nm) * sizeof(int) + 64);
 
     // the embedding phase has its own batch, scan scratch, counters and
     // pinned staging, so that it can run beside the other phases (two sets
@@ -157,8 +156,7 @@ Session::Session(const gm_params &p) : p_(p) {
       e.partial = (float *)dalloc(e.cap_partial * 2 * sizeof(float));
       e.ipartial = (int *)dalloc(e.cap_partial * sizeof(int));
       e.batch = (int *)dalloc(Nm * sizeof(int));
-      e.tmp = (int *)dalloc(std::max(scan_tmp_ints((int)Nm), compact_tmp_ints((int)Nm)) *
-                            sizeof(int) + 64);
+      e.tmp = (int *)dalloc(compact_tmp_ints((int)Nm) * sizeof(int) + 64);
       if (p.overlap) {
         e.pub_idx_snap = (uint32_t *)dalloc(Nm * (k + 1) * sizeof(uint32_t));
         e.pub_dist_snap = (float *)dalloc(Nm * (k + 1) * sizeof(float));

@@ -58,12 +58,9 @@ void launch_counter_reset();
 // Rows x d floats at src, memory the device can read (host memory included),
 // into dst with row stride ld.
 void launch_copy_rows(const float *src, float *dst, size_t rows, int d, int ld, int sms, cudaStream_t s);
-// Exclusive scan of in[0..n) into out[0..n]; out[n] = total.  tmp needs
-// scan_tmp_ints(n) ints.
-size_t scan_tmp_ints(int n);
-void exclusive_scan(const int *in, int *out, int n, int *tmp, cudaStream_t s);
 // Ordered compaction of the ids i in [0, n) with flag[i] != 0 (or, when
-// select >= 0, flag[i] == select) into out; *count receives the number.
+// select >= 0, flag[i] == select) into out; *count receives the number.  tmp
+// needs compact_tmp_ints(n) ints.
 size_t compact_tmp_ints(int n);
 void compact_flags(const int *flag, int n, int select, int *out, int *count,
                    int *tmp, cudaStream_t s);
@@ -71,9 +68,6 @@ void compact_flags(const int *flag, int n, int select, int *out, int *count,
 // *max_val / parts (none when *max_val is not positive).
 void compact_at_least(const float *vals, const float *max_val, int parts, const int *n_dev, int n_max,
                       int *out, int *count, int *tmp, cudaStream_t s);
-// Ordered compaction of list[i] (i < *n_dev) where pred[list[i]] != 0.
-void compact_list(const int *list, const int *n_dev, int n_max, const int *pred,
-                  int *out, int *count, int *tmp, cudaStream_t s);
 
 // ---- insertion (gm_kernels_insert.cu) ----
 void launch_row_norms(const DevState &st, int row0, int nrows, cudaStream_t s);

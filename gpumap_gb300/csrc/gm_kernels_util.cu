@@ -1,6 +1,6 @@
-// Device-wide exclusive scan and order-preserving compaction.  Three passes
-// (per-block totals, a single-block scan of the totals, per-block write);
-// results are deterministic and keep ascending index order.
+// Order-preserving compaction.  Three passes (per-block totals, a single-block
+// scan of the totals, per-block write); results are deterministic and keep
+// ascending index order.
 #include "gm_common.cuh"
 #include "gm_kernels.h"
 
@@ -48,22 +48,12 @@ __device__ __forceinline__ int block_inclusive_scan(int v, int *warp_tot) {
   return v;
 }
 
-// Predicate value of item i for the three input kinds.
+// Item i stays when its flag is not 0, or is `select` when that is >= 0.
 struct Pred {
-  const int *vals;     // plain values (scan) or flags
-  const int *list;     // optional indirection list
-  const int *n_dev;    // optional device length of list
-  int n_host;          // host length bound
-  int select;          // -1: value != 0 ; >= 0: value == select ; -2: raw value
-  __device__ __forceinline__ int len() const { return n_dev ? min(*n_dev, n_host) : n_host; }
-  __device__ __forceinline__ int at(int i) const {
-    const int src = list ? list[i] : i;
-    const int v = vals[src];
-    if (select == -2) return v;
-    if (select == -1) return v != 0 ? 1 : 0;
-    return v == select ? 1 : 0;
-  }
-  __device__ __forceinline__ int id(int i) const { return list ? list[i] : i; }
+  const int *vals;
+  int n, select;
+  __device__ __forceinline__ int len() const { return n; }
+  __device__ __forceinline__ int at(int i) const { return (select < 0 ? vals[i] != 0 : vals[i] == select) ? 1 : 0; }
 };
 
 // Item i stays when its value is at least *max_val / parts (none does when the
@@ -77,7 +67,6 @@ struct PredAtLeast {
     const float mw = *max_val;
     return mw > 0.0f && vals[i] >= __fdiv_rn(mw, (float)parts) ? 1 : 0;
   }
-  __device__ __forceinline__ int id(int i) const { return i; }
 };
 
 template <typename P>
@@ -128,9 +117,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_totals(int *tot, int nb,
   }
 }
 
-// mode 0: exclusive scan output out[i]; mode 1: compaction out[pos] = id(i).
 template <typename P>
-__global__ void __launch_bounds__(kScanThreads) k_block_write(P p, const int *tot, int *out, int mode,
+__global__ void __launch_bounds__(kScanThreads) k_block_write(P p, const int *tot, int *out,
                                                               int n_cap_out) {
   pdl_enter();
   __shared__ int wt[kScanThreads / 32];
@@ -147,29 +135,21 @@ __global__ void __launch_bounds__(kScanThreads) k_block_write(P p, const int *to
   int run = tot[blockIdx.x] + incl - s;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
-    if (base + i < n) {
-      if (mode == 0) {
-        out[base + i] = run;
-      } else if (v[i] && run < n_cap_out) {
-        out[run] = p.id(base + i);
-      }
-    }
+    if (v[i] && run < n_cap_out) out[run] = base + i;
     run += v[i];
   }
-  if (mode == 0 && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = tot[gridDim.x];
 }
 
 inline int nblocks(int n) { return n <= 0 ? 1 : (n + kScanBlock - 1) / kScanBlock; }
 
 template <typename P>
-void run_scan(const P &p, int n_max, int *out, int mode, int *count, int *tmp,
-              cudaStream_t s) {
+void compact(const P &p, int n_max, int *out, int *count, int *tmp, cudaStream_t s) {
   const int nb = nblocks(n_max);
   launch(k_block_totals<P>, nb, kScanThreads, 0, s, p, tmp);
   note_launch();
   launch(k_scan_totals, 1, kScanThreads, 0, s, tmp, nb, count);
   note_launch();
-  launch(k_block_write<P>, nb, kScanThreads, 0, s, p, tmp, out, mode, n_max);
+  launch(k_block_write<P>, nb, kScanThreads, 0, s, p, tmp, out, n_max);
   note_launch();
 }
 
@@ -236,30 +216,16 @@ void fill_u32(void *p, uint32_t v, size_t n, cudaStream_t s) {
   note_launch();
 }
 
-size_t scan_tmp_ints(int n) { return (size_t)nblocks(n) + 2; }
 size_t compact_tmp_ints(int n) { return (size_t)nblocks(n) + 2; }
-
-void exclusive_scan(const int *in, int *out, int n, int *tmp, cudaStream_t s) {
-  Pred p{in, nullptr, nullptr, n, -2};
-  run_scan(p, n, out, 0, nullptr, tmp, s);
-}
 
 void compact_flags(const int *flag, int n, int select, int *out, int *count,
                    int *tmp, cudaStream_t s) {
-  Pred p{flag, nullptr, nullptr, n, select >= 0 ? select : -1};
-  run_scan(p, n, out, 1, count, tmp, s);
+  compact(Pred{flag, n, select}, n, out, count, tmp, s);
 }
 
 void compact_at_least(const float *vals, const float *max_val, int parts, const int *n_dev, int n_max,
                       int *out, int *count, int *tmp, cudaStream_t s) {
-  PredAtLeast p{vals, max_val, n_dev, n_max, parts};
-  run_scan(p, n_max, out, 1, count, tmp, s);
-}
-
-void compact_list(const int *list, const int *n_dev, int n_max, const int *pred,
-                  int *out, int *count, int *tmp, cudaStream_t s) {
-  Pred p{pred, list, n_dev, n_max, -1};
-  run_scan(p, n_max, out, 1, count, tmp, s);
+  compact(PredAtLeast{vals, max_val, n_dev, n_max, parts}, n_max, out, count, tmp, s);
 }
 
 }  // namespace gm
