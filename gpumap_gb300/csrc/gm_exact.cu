@@ -781,10 +781,11 @@ GM_D float warp_32nd(const float *v, int cnt, int lane) {
 // The 32nd smallest of cnt values >= 0 (inf included), value i at get(i), by a
 // whole CTA: inf when there are fewer.  The values' bits are counted in up to
 // 256 equal bins of their range, then of the bin that holds the 32nd, and so
-// on: at most four rounds of two barriers, where a search by bits takes 31
-// rounds and compares every value in each.  Every thread returns it.
+// on until it is alone in its bin: at most four rounds of two barriers, where
+// a search by bits takes 31 rounds and compares every value in each.  Every
+// thread returns it.
 struct Select32 {
-  int bins[2][256];
+  int4 bins[2][64];
   unsigned lo, hi;
 };
 template <int kThreads, typename F>
@@ -802,7 +803,7 @@ GM_D float cta_32nd(int cnt, F &&get, Select32 &sh) {
     sh.lo = full;
     sh.hi = 0u;
   }
-  for (int i = threadIdx.x; i < 256; i += kThreads) sh.bins[0][i] = 0;
+  if (threadIdx.x < 64) sh.bins[0][threadIdx.x] = make_int4(0, 0, 0, 0);
   __syncthreads();
   lo = __reduce_min_sync(full, lo);
   hi = __reduce_max_sync(full, hi);
@@ -818,14 +819,14 @@ GM_D float cta_32nd(int cnt, F &&get, Select32 &sh) {
     const int shift = max(0, 24 - __clz((int)(hi - lo)));  // (hi - lo) >> shift < 256
     for (int i = threadIdx.x; i < cnt; i += kThreads) {
       const unsigned v = __float_as_uint(get(i));
-      if (v >= lo && v <= hi) atomicAdd(&sh.bins[buf][(v - lo) >> shift], 1);
+      if (v >= lo && v <= hi) atomicAdd(reinterpret_cast<int *>(sh.bins[buf]) + ((v - lo) >> shift), 1);
     }
-    for (int i = threadIdx.x; i < 256; i += kThreads) sh.bins[buf ^ 1][i] = 0;
+    if (threadIdx.x < 64) sh.bins[buf ^ 1][threadIdx.x] = make_int4(0, 0, 0, 0);
     __syncthreads();
     // each warp finds the bin: eight of them a lane
-    int c[8], sum = 0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) sum += c[q] = sh.bins[buf][lane * 8 + q];
+    const int4 b0 = sh.bins[buf][lane * 2], b1 = sh.bins[buf][lane * 2 + 1];
+    const int c[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+    const int sum = ((b0.x + b0.y) + (b0.z + b0.w)) + ((b1.x + b1.y) + (b1.z + b1.w));
     int incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -833,16 +834,26 @@ GM_D float cta_32nd(int cnt, F &&get, Select32 &sh) {
       if (lane >= o) incl += y;
     }
     const int src = __ffs(__ballot_sync(full, incl >= want)) - 1;
-    int rank = want - (incl - sum), bin = 0;
+    int rank = want - (incl - sum), bin = 0, in_bin = c[0];
 #pragma unroll
     for (int q = 0; q < 7; ++q)
       if (bin == q && rank > c[q]) {
         rank -= c[q];
         ++bin;
+        in_bin = c[q + 1];
       }
     want = __shfl_sync(full, rank, src);
+    in_bin = __shfl_sync(full, in_bin, src);
     lo += (unsigned)__shfl_sync(full, lane * 8 + bin, src) << shift;
     hi = min(hi, lo + ((1u << shift) - 1u));
+    if (in_bin == 1) {  // (the same for every thread)
+      for (int i = threadIdx.x; i < cnt; i += kThreads) {
+        const unsigned v = __float_as_uint(get(i));
+        if (v >= lo && v <= hi) sh.lo = v;
+      }
+      __syncthreads();
+      return __uint_as_float(sh.lo);
+    }
     __syncthreads();
   }
   return __uint_as_float(lo);
@@ -872,7 +883,7 @@ __global__ void __launch_bounds__(kFinalWarps * 32)
 // CTA per batch row: the seed, the 32nd smallest of the row's chunk minima
 // from pass 0 (the largest upper bound of 32 distinct columns).  Clears the
 // counters of the passes after it.  1,000 rows of 600 minima: 25 us by a warp
-// per row (insertion above 512 values), 10.4 us.
+// per row (insertion above 512 values), 8.0 us.
 constexpr int kSeedThreads = 128, kSeedStage = 4096;
 __global__ void __launch_bounds__(kSeedThreads)
     k_seed_select(const float *mins, int mins_ld, float *seed, int *row_cnt, int *pcnt, int *counter,
@@ -898,12 +909,13 @@ __global__ void __launch_bounds__(kSeedThreads)
 // then the row's candidates, the stored columns with lower bound <= T.  Does
 // nothing when a segment overflowed (the heap passes then run instead).
 // The entries (about 0.4 % of the columns: the seed is a 32 / 8192 quantile)
-// are gathered from the row's segments, a warp per segment, into shared memory.
+// are gathered from the row's segments into shared memory, each by its own
+// thread (a warp per segment waited for one segment after another).
 // A warp per row that inserted the bounds one at a time was bound by latency: 33
 // us for 500 rows of ~600 entries, a CTA that searched them by bits 24 us in a
-// run (31 rounds over all values, bound by issue), this form 13 us.  A row with
+// run (31 rounds over all values, bound by issue), this form 11 us.  A row with
 // more than kPreStage entries is worked through where they lie, by its first warp.
-constexpr int kPreThreads = 128, kPreWarps = kPreThreads / 32;
+constexpr int kPreThreads = 128;
 constexpr int kPreStage = 2048, kPreSegs = 512;
 __global__ void __launch_bounds__(kPreThreads)
     k_pre_select(const unsigned long long *pre, const float *pre_ub, const int *pre_cnt, int gx,
@@ -954,13 +966,15 @@ __global__ void __launch_bounds__(kPreThreads)
   };
   float T = inf;
   if (total <= kPreStage && gx <= kPreSegs) {
-    for (int c = warp; c < gx; c += kPreWarps) {
-      const int off = s_off[c], len = (c + 1 < gx ? s_off[c + 1] : total) - off;
-      const size_t from = seg0 + (size_t)c * cap;
-      for (int i = lane; i < len; i += 32) {
-        s_ub[off + i] = pre_ub[from + i];
-        s_ent[off + i] = pre[from + i];
-      }
+    // entry i is in the last segment that begins at or before it
+#pragma unroll 4
+    for (int i = threadIdx.x; i < total; i += kPreThreads) {
+      int c = 0;
+      for (int step = kPreSegs / 2; step > 0; step >>= 1)
+        if (c + step < gx && s_off[c + step] <= i) c += step;
+      const size_t from = seg0 + (size_t)c * cap + (i - s_off[c]);
+      s_ub[i] = pre_ub[from];
+      s_ent[i] = pre[from];
     }
     __syncthreads();
     T = cta_32nd<kPreThreads>(total, [&](int i) { return s_ub[i]; }, sel);
