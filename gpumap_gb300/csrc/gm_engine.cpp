@@ -201,7 +201,7 @@ Session::Session(const gm_params &p) : p_(p) {
       // every grid width a block can take (at most one CTA per column tile)
       // and room for every column up to four column tiles
       xs_.pre_gx = (int)std::min<size_t>(std::max(sms_, 1), (Nm + 255) / 256);
-      xs_.pre_cap = pre_cap_alloc_ = std::max(64, (1024 + xs_.pre_gx - 1) / xs_.pre_gx);
+      xs_.pre_cap = std::max(kPreCap, (1024 + xs_.pre_gx - 1) / xs_.pre_gx);
       xs_.pre = (unsigned long long *)dalloc((size_t)ex_block_ * xs_.pre_gx * xs_.pre_cap *
                                              sizeof(unsigned long long));
       xs_.pre_ub = (float *)dalloc((size_t)ex_block_ * xs_.pre_gx * xs_.pre_cap * sizeof(float));
@@ -448,7 +448,7 @@ void Session::set_join_part(size_t words) {
 
 void Session::set_pre_cap(int cap) {
   drain();
-  xs_.pre_cap = std::max(0, std::min(cap, pre_cap_alloc_));
+  xs_.pre_cap = std::max(0, std::min(cap, kPreCap));
   xs_.pre_fixed = true;
 }
 

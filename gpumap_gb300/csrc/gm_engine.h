@@ -192,7 +192,7 @@ class Session {
   // statistics
   bool stats_on_ = false;
   bool keep_tile_ = false;
-  int pre_cap_alloc_ = 0;  // pre-candidate segment length allocated (precision 1)
+  static constexpr int kPreCap = 64;  // pre-candidate segment length, at least (precision 1)
   gm_stats stats_{};
   struct EvPair { cudaEvent_t a, b; int slot; };
   std::vector<EvPair> ev_pending_;

@@ -17,7 +17,9 @@
 //                stored): per batch row, the columns that may be among its
 //                32 nearest; per existing row, the batch rows that may enter
 //                its list
-//  k_row_threshold  per batch row: its exact threshold from the CTAs' heaps
+//  k_seed_select, k_pre_select  per batch row: its seed, then its exact
+//                threshold and candidates from the stored columns
+//  k_row_threshold  the same from the CTAs' heaps (after an overflow)
 //  k_rescore     canonical FP32 re-score of the survivors
 //  k_row_select / k_merge_offers   exact top-32 merges
 #include <cuda.h>

@@ -48,10 +48,10 @@ int gm_debug_keep_tiles(struct gm_session *s, int on);
 /* Precision 1: entries per segment of stored columns that the store pass
  * over the tiles may keep, fixed whatever the grid width (clamped to 64;
  * by default each of a row tile's CTAs gets an equal share of the row's
- * 64 x min(SMs, column tiles) entries; 0 runs the heap and candidate passes
- * instead, as for blocks of up to four column tiles).  A segment that would
- * exceed it makes the heap and candidate passes run for its block
- * (gm_stats.exact_overflow_blocks). */
+ * 64 x min(SMs, column tiles) entries, or of 1,024 when that is more; 0 runs
+ * the heap and candidate passes instead, and so does any value for blocks of
+ * up to four column tiles).  A segment that would exceed it makes the heap and
+ * candidate passes run for its block (gm_stats.exact_overflow_blocks). */
 int gm_debug_pre_capacity(struct gm_session *s, int cap);
 /* Words of the join pool that one pass of an update round covers, at most
  * (clamped to [2, 2^25], the default; frees the pool).  A round whose node
