@@ -609,6 +609,15 @@ void Session::get_stats(gm_stats *out) {
   *out = stats_;
 }
 
+// The kernel loads whole floats, so rows at an address that is not a multiple
+// of four go through the staging copy, for which alignment does not matter (a
+// misaligned load would end the context).
+Ingest ingest_route(const void *rows, bool page_locked, bool reads_host) {
+  if (page_locked) return Ingest::kCopy;
+  const bool aligned = (reinterpret_cast<uintptr_t>(rows) & (alignof(float) - 1)) == 0;
+  return reads_host && aligned ? Ingest::kInPlace : Ingest::kStaged;
+}
+
 // ---------------------------------------------------------------------------
 // append (reference impl.cuh:77-101)
 // ---------------------------------------------------------------------------
@@ -618,8 +627,8 @@ void Session::get_stats(gm_stats *out) {
 // transfer runs beside work still going (an overlapped embedding); the main
 // stream waits for it on the device.  Rows in page-locked memory are copied
 // from where they are.  Pageable rows are read in place by a kernel where the
-// GPU shares the CPU's page tables (launch_copy_rows); elsewhere they go
-// through two pinned staging slots (waiting only for the slot's previous
+// GPU shares the CPU's page tables (launch_copy_rows) and the rows are aligned
+// to floats; else they go through two pinned staging slots (waiting only for the slot's previous
 // transfer).  Where the caller's buffer is read, the call returns after the
 // copy, so that the buffer can be reused.
 void Session::append(const float *rows, size_t n_rows, size_t n_cols, bool on_device) {
@@ -647,8 +656,8 @@ void Session::append(const float *rows, size_t n_rows, size_t n_cols, bool on_de
     RingSlot &slot = ring_[ring_next_];
     ring_next_ = (ring_next_ + 1) % kRingSlots;
     const float *src = rows;
-    const bool direct = !pinned && reads_host_;
-    if (!pinned && !direct) {
+    const Ingest route = ingest_route(rows, pinned, reads_host_);
+    if (route == Ingest::kStaged) {
       const size_t bytes = n_rows * width;
       ck(cudaEventSynchronize(slot.done), "ingest slot");  // its previous transfer
       if (slot.cap < bytes) {
@@ -661,7 +670,7 @@ void Session::append(const float *rows, size_t n_rows, size_t n_cols, bool on_de
       std::memcpy(slot.buf, rows, bytes);
       src = (const float *)slot.buf;
     }
-    if (direct) {
+    if (route == Ingest::kInPlace) {
       // one read per page on the CPU: a page whose entry the kernel has
       // withdrawn for a moment (NUMA balancing does, also of a VM on its host) costs the
       // GPU a fault of 0.7 ms, the CPU one of a microsecond
@@ -677,7 +686,7 @@ void Session::append(const float *rows, size_t n_rows, size_t n_cols, bool on_de
     }
     ck(cudaEventRecord(slot.done, cstream_), "ingest event");
     ck(cudaStreamWaitEvent(stream_, slot.done, 0), "ingest wait");
-    if (pinned || direct) {
+    if (route != Ingest::kStaged) {
       // the caller's buffer is in use until the transfer ends: block here
       // rather than let the caller overwrite it (the slot event covers it)
       ck(cudaEventSynchronize(slot.done), "append copy");

@@ -53,6 +53,12 @@ class DedupQueue {
   std::vector<char> in_;
 };
 
+// How host rows reach the device: by the copy engine from where they are
+// (page-locked memory), read in place by a kernel, or copied into a pinned slot
+// first.
+enum class Ingest { kCopy = 0, kInPlace = 1, kStaged = 2 };
+Ingest ingest_route(const void *rows, bool page_locked, bool reads_host);
+
 class Session {
  public:
   explicit Session(const gm_params &p);

@@ -57,6 +57,11 @@ int gm_debug_pre_capacity(struct gm_session *s, int cap);
  * (clamped to [2, 2^25], the default; frees the pool).  A round whose node
  * blocks take more words runs in several passes; its lists are the same. */
 int gm_debug_join_words(struct gm_session *s, uint64_t words);
+/* How gm_append takes host rows at `address`: 0 copied by the copy engine from
+ * where they are (page-locked memory), 1 read in place by a kernel (the device
+ * reads host memory, and the address is a multiple of 4), 2 copied into a pinned
+ * staging slot first. */
+int gm_debug_ingest_route(uint64_t address, int page_locked, int reads_host);
 /* Host and device scalars, out[0..n):
  *  0 n_inserted, 1 insertion-queue head, 2 new-row embedding-queue head,
  *  3 embedding cursor (-1 = none), 4 embedding sweeps, 5 last nnz,
