@@ -16,6 +16,7 @@ _EXPORTS = {
     "GPUMAP": ".gpumap",
     "GPUMAPParams": "._core",
     "Metric": ".metric",
+    "release_memory": "._native",
     "BaseStrategy": ".schedule",
     "WeightedStrategy": ".schedule",
     "SequentialPriorityStrategy": ".schedule",

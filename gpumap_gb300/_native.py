@@ -84,6 +84,8 @@ _SIGS = [
     ("gm_get_device", C.c_int, [_P, C.POINTER(C.c_int32)]),
     ("gm_close", C.c_int, [_P]),
     ("gm_destroy", None, [_P]),
+    ("gm_release_memory", C.c_int, []),
+    ("gm_memory_held", C.c_int, [C.c_int32, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]),
     ("gm_last_error", C.c_char_p, []),
     ("gm_set_stats", C.c_int, [_P, C.c_int]),
     ("gm_get_stats", C.c_int, [_P, C.POINTER(gm_stats)]),
@@ -143,6 +145,18 @@ def check(rc: int) -> None:
         if rc == GM_ERR_OOM:
             raise MemoryError(msg)
         raise GMError(rc, msg or f"gpumap_gb300 error {rc}")
+
+
+def release_memory() -> None:
+    """Gives the memory kept for coming sessions back to the device and the host."""
+    check(load().gm_release_memory())
+
+
+def memory_held(device: int = 0) -> tuple[int, int]:
+    """Device bytes the library holds for sessions and operators, and those in use."""
+    reserved, used = C.c_uint64(), C.c_uint64()
+    check(load().gm_memory_held(device, C.byref(reserved), C.byref(used)))
+    return reserved.value, used.value
 
 
 def default_params(**kw) -> gm_params:

@@ -182,6 +182,25 @@ void gm_destroy(gm_session *s) {
   delete s;
 }
 
+int gm_release_memory(void) {
+  return guarded([&] {
+    const cudaError_t e = gm::memory_release();
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      throw gm::Error(GM_ERR_CUDA, std::string("release memory: ") + cudaGetErrorString(e));
+    }
+  });
+}
+
+int gm_memory_held(int32_t device, uint64_t *reserved, uint64_t *used) {
+  if (!reserved || !used) return fail(GM_ERR_INVALID, "null argument");
+  size_t r = 0, u = 0;
+  if (gm::device_held(device, &r, &u) != cudaSuccess) return fail(GM_ERR_INVALID, "device ordinal out of range");
+  *reserved = r;
+  *used = u;
+  return GM_OK;
+}
+
 const char *gm_last_error(void) { return g_last_error.c_str(); }
 
 int gm_set_stats(gm_session *s, int enable) {
@@ -365,6 +384,7 @@ int gm_op_fuzzy_schedule(const uint32_t *pub_idx, const float *pub_dist, int64_t
     cudaMemcpyAsync(fscal, e.fscal, sizeof(fscal), cudaMemcpyDeviceToHost, s);
     const cudaError_t err = cudaStreamSynchronize(s);
     for (void *q : al) gm::device_free(q, s);
+    gm::device_bound(dev);
     if (err != cudaSuccess) throw gm::Error(GM_ERR_CUDA, cudaGetErrorString(err));
     if (counts_out) {
       counts_out[0] = iscal[0];
@@ -421,6 +441,7 @@ int gm_op_sgd(float *emb, int64_t n, const int32_t *head, const int32_t *tail,
     const cudaError_t err = le != cudaSuccess ? le : cudaStreamSynchronize(s);
     if (le != cudaSuccess) cudaGetLastError();
     release();
+    gm::device_bound(dev);
     if (err != cudaSuccess) throw gm::Error(GM_ERR_CUDA, cudaGetErrorString(err));
     if (dev_err) throw gm::Error(GM_ERR_DEVICE, "SGD grid barrier wait ran out");
   });

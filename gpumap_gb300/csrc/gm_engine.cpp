@@ -268,6 +268,8 @@ void Session::release_memory() {
   if (stream_) cudaStreamSynchronize(stream_);
   for (void *q : allocs_) device_free(q, stream_);
   allocs_.clear();
+  // (the pool can give a block back only after its free has been waited for)
+  if (stream_) cudaStreamSynchronize(stream_);
   for (uint32_t **h : {&h_pin_, &h_emb_pin_, &h_emb_pin_alt_}) {
     host_free(*h, pin_bytes_);
     *h = nullptr;
@@ -309,6 +311,7 @@ Session::~Session() {
   if (current != device_) cudaSetDevice(device_);
   cudaDeviceSynchronize();
   if (current != device_) cudaSetDevice(current);
+  const size_t held = device_bytes();
   for (auto &e : ev_pool_) cudaEventDestroy(e);
   for (auto &pr : ev_pending_) {
     cudaEventDestroy(pr.a);
@@ -326,6 +329,7 @@ Session::~Session() {
   }
   if (cstream_) cudaStreamDestroy(cstream_);
   release_streams();
+  device_closed(device_, held);
 }
 
 void Session::sync() { ck(cudaStreamSynchronize(stream_), "cudaStreamSynchronize"); }

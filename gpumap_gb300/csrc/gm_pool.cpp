@@ -5,12 +5,18 @@
 // cost 0.6 ms (600 x 24) to 6 ms (160,000 x 128, precision 1) of every session
 // where the same memory had just been freed.
 //
-// Bounds: at most kDeviceKeep bytes of freed device memory stay with the pool
-// (what is above goes back at the next synchronisation), and kHostKeep bytes
-// of page-locked memory.  An allocation that fails gives everything unused
-// back and tries once more.  Both lists are safe with several threads; a block
-// is only freed after its streams have been waited for, so the next owner may
-// use it on any stream once its allocation's stream has been waited for.
+// Unused device memory that stays with a pool: what the session closed last
+// held, or half of what was kept before when that is more (so that small
+// sessions among large ones do not give it all up, and small ones alone do so
+// soon), and never more than a 32nd of the device's memory: a session beyond
+// that takes seconds to fill, and its memory is not worth keeping from others.
+// Each close gives back what is above.  kHostKeep bounds the page-locked blocks.
+// An allocation that fails, and memory_release(), give everything unused back.
+//
+// Both lists are safe with several threads; a block is only freed after its
+// streams have been waited for, so the next owner may use it on any stream once
+// its allocation's stream has been waited for.
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -20,17 +26,23 @@ namespace gm {
 
 namespace {
 
-constexpr unsigned long long kDeviceKeep = 16ull << 30;
 constexpr size_t kHostKeep = (size_t)64 << 20;
+constexpr size_t kDeviceShare = 32;
 constexpr int kMaxDevices = 64;
 
+struct DevicePool {
+  cudaMemPool_t pool = nullptr;
+  size_t keep = 0;   // unused bytes to hold on to
+  size_t most = 0;   // a 32nd of the device's memory
+};
 std::mutex g_mu;
-cudaMemPool_t g_pools[kMaxDevices] = {};
+DevicePool g_pools[kMaxDevices];
 
-cudaError_t pool_of(int device, cudaMemPool_t *out) {
+// The device's pool, made on first use (g_mu held).
+cudaError_t pool_of(int device, DevicePool **out) {
   if (device < 0 || device >= kMaxDevices) return cudaErrorInvalidDevice;
-  std::lock_guard<std::mutex> g(g_mu);
-  if (!g_pools[device]) {
+  DevicePool &d = g_pools[device];
+  if (!d.pool) {
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -38,16 +50,36 @@ cudaError_t pool_of(int device, cudaMemPool_t *out) {
     cudaMemPool_t p = nullptr;
     cudaError_t e = cudaMemPoolCreate(&p, &props);
     if (e != cudaSuccess) return e;
-    unsigned long long keep = kDeviceKeep;
-    e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    // (the runtime gives nothing back by itself: its threshold counts the memory
+    // in use as well)
+    unsigned long long never = ~0ull;
+    e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &never);
+    size_t free_b = 0, total = 0;
+    if (e == cudaSuccess) e = cudaMemGetInfo(&free_b, &total);
     if (e != cudaSuccess) {
       cudaMemPoolDestroy(p);
       return e;
     }
-    g_pools[device] = p;
+    d.pool = p;
+    d.most = total / kDeviceShare;
   }
-  *out = g_pools[device];
+  *out = &d;
   return cudaSuccess;
+}
+
+void held(cudaMemPool_t p, size_t *reserved, size_t *used) {
+  unsigned long long r = 0, u = 0;
+  cudaMemPoolGetAttribute(p, cudaMemPoolAttrReservedMemCurrent, &r);
+  cudaMemPoolGetAttribute(p, cudaMemPoolAttrUsedMemCurrent, &u);
+  *reserved = (size_t)r;
+  *used = (size_t)u;
+}
+
+// At most `keep` unused bytes stay.
+void trim(cudaMemPool_t p, size_t keep) {
+  size_t reserved = 0, used = 0;
+  held(p, &reserved, &used);
+  if (reserved > used + keep) cudaMemPoolTrimTo(p, used + keep);
 }
 
 struct HostBlock {
@@ -55,8 +87,11 @@ struct HostBlock {
   size_t bytes;
 };
 std::mutex g_host_mu;
-std::vector<HostBlock> g_host;
 size_t g_host_bytes = 0;
+std::vector<HostBlock> &host_blocks() {  // (never destroyed: a session may go after the statics)
+  static std::vector<HostBlock> *v = new std::vector<HostBlock>;
+  return *v;
+}
 
 size_t host_size(size_t bytes) {  // whole 64 KB pages
   return (bytes + 65535) / 65536 * 65536;
@@ -67,11 +102,18 @@ size_t host_size(size_t bytes) {  // whole 64 KB pages
 cudaError_t device_alloc(void **out, size_t bytes, int device, cudaStream_t s) {
   *out = nullptr;
   cudaMemPool_t p = nullptr;
-  cudaError_t e = pool_of(device, &p);
-  if (e != cudaSuccess) return e;
-  e = cudaMallocFromPoolAsync(out, bytes, p, s);
+  {
+    std::lock_guard<std::mutex> g(g_mu);
+    DevicePool *d = nullptr;
+    const cudaError_t e = pool_of(device, &d);
+    if (e != cudaSuccess) return e;
+    p = d->pool;
+  }
+  cudaError_t e = cudaMallocFromPoolAsync(out, bytes, p, s);
   if (e == cudaErrorMemoryAllocation) {
+    // a freed block goes back to the device once its free has been waited for
     cudaGetLastError();
+    cudaDeviceSynchronize();
     cudaMemPoolTrimTo(p, 0);
     e = cudaMallocFromPoolAsync(out, bytes, p, s);
   }
@@ -86,15 +128,60 @@ void device_free(void *p, cudaStream_t s) {
   if (p) cudaFreeAsync(p, s);
 }
 
+void device_closed(int device, size_t bytes) {
+  std::lock_guard<std::mutex> g(g_mu);
+  if (device < 0 || device >= kMaxDevices || !g_pools[device].pool) return;
+  DevicePool &d = g_pools[device];
+  d.keep = std::min(d.most, std::max(bytes, d.keep / 2));
+  trim(d.pool, d.keep);
+}
+
+void device_bound(int device) {
+  std::lock_guard<std::mutex> g(g_mu);
+  if (device < 0 || device >= kMaxDevices || !g_pools[device].pool) return;
+  trim(g_pools[device].pool, g_pools[device].most);
+}
+
+cudaError_t device_held(int device, size_t *reserved, size_t *used) {
+  std::lock_guard<std::mutex> g(g_mu);
+  *reserved = *used = 0;
+  if (device < 0 || device >= kMaxDevices) return cudaErrorInvalidDevice;
+  if (g_pools[device].pool) held(g_pools[device].pool, reserved, used);
+  return cudaSuccess;
+}
+
+cudaError_t memory_release() {
+  cudaError_t first = cudaSuccess;
+  {
+    std::lock_guard<std::mutex> g(g_mu);
+    int current = 0;
+    const bool back = cudaGetDevice(&current) == cudaSuccess;
+    for (int dev = 0; dev < kMaxDevices; ++dev) {
+      if (!g_pools[dev].pool) continue;
+      cudaError_t e = cudaSetDevice(dev);
+      if (e == cudaSuccess) e = cudaDeviceSynchronize();
+      if (e == cudaSuccess) e = cudaMemPoolTrimTo(g_pools[dev].pool, 0);
+      if (first == cudaSuccess) first = e;
+    }
+    if (back) cudaSetDevice(current);
+  }
+  std::lock_guard<std::mutex> g(g_host_mu);
+  for (const HostBlock &b : host_blocks()) cudaFreeHost(b.p);
+  host_blocks().clear();
+  g_host_bytes = 0;
+  return first;
+}
+
 cudaError_t host_alloc(void **out, size_t bytes) {
   const size_t want = host_size(bytes);
   {
     std::lock_guard<std::mutex> g(g_host_mu);
-    for (size_t i = 0; i < g_host.size(); ++i)
-      if (g_host[i].bytes == want) {
-        *out = g_host[i].p;
+    std::vector<HostBlock> &v = host_blocks();
+    for (size_t i = 0; i < v.size(); ++i)
+      if (v[i].bytes == want) {
+        *out = v[i].p;
         g_host_bytes -= want;
-        g_host.erase(g_host.begin() + (long)i);
+        v.erase(v.begin() + (long)i);
         return cudaSuccess;
       }
   }
@@ -112,7 +199,7 @@ void host_free(void *p, size_t bytes) {
   {
     std::lock_guard<std::mutex> g(g_host_mu);
     if (g_host_bytes + size <= kHostKeep) {
-      g_host.push_back({p, size});
+      host_blocks().push_back({p, size});
       g_host_bytes += size;
       return;
     }

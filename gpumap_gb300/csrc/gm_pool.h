@@ -10,7 +10,16 @@ namespace gm {
 cudaError_t device_alloc(void **out, size_t bytes, int device, cudaStream_t s);
 // After every stream that used the block has been waited for.
 void device_free(void *p, cudaStream_t s);
+// After a session's `bytes` were freed and its stream waited for: gives back
+// what the pool holds beyond what it keeps for the next session.
+void device_closed(int device, size_t bytes);
+// Gives back what is above the most that a pool may keep (operators).
+void device_bound(int device);
+// Bytes the device's pool holds, and those of them in use.
+cudaError_t device_held(int device, size_t *reserved, size_t *used);
 cudaError_t host_alloc(void **out, size_t bytes);
 void host_free(void *p, size_t bytes);
+// Waits for the devices and gives back everything unused, on the host too.
+cudaError_t memory_release();
 
 }  // namespace gm

@@ -161,6 +161,15 @@ int gm_close(struct gm_session *s);
 /* Frees the session (reference destructor). NULL is ignored. */
 void gm_destroy(struct gm_session *s);
 
+/* Gives the memory that the library keeps for coming sessions back to the
+ * device and the host (waits for the devices).  Closed sessions' memory is kept
+ * to be used again: as much as the last one held, at most a 32nd of the
+ * device's memory, and up to 64 MB page-locked.  Live sessions keep theirs. */
+int gm_release_memory(void);
+/* Device memory the library holds on `device` for sessions and operators, and
+ * how much of it is in use. */
+int gm_memory_held(int32_t device, uint64_t *reserved, uint64_t *used);
+
 /* Thread-local message of the last failing call on this thread. */
 const char *gm_last_error(void);
 
