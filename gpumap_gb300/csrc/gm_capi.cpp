@@ -313,6 +313,11 @@ int gm_debug_ingest_route(uint64_t address, int page_locked, int reads_host) {
   return (int)gm::ingest_route(reinterpret_cast<const void *>((uintptr_t)address), page_locked != 0, reads_host != 0);
 }
 
+int gm_debug_fail_alloc(int nth) {
+  gm::device_fail_in(std::max(0, nth));
+  return GM_OK;
+}
+
 int gm_debug_scalars(const gm_session *s, int64_t *out, int n) {
   if (!s || !out) return fail(GM_ERR_INVALID, "null argument");
   s->impl->debug_scalars(out, n);

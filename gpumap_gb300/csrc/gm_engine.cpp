@@ -35,6 +35,18 @@ void ck(cudaError_t e, const char *what) {
 
 size_t round_up(size_t v, size_t m) { return (v + m - 1) / m * m; }
 
+// Takes a half-made set of buffers back when one of them cannot be had.
+template <typename F>
+struct Undo {
+  F f;
+  bool done = false;
+  ~Undo() {
+    if (!done) f();
+  }
+};
+template <typename F>
+Undo(F) -> Undo<F>;
+
 // From 256 two-hop positions on, insertion iterates and keeps distances.
 bool reuses_dists(int k) { return k * k >= kMaxCand; }
 // Insertion scratch for r batch rows (CandScratch).
@@ -72,6 +84,18 @@ Session::Session(const gm_params &p) : p_(p) {
   if (p.device >= 0) ck(cudaSetDevice(p.device), "cudaSetDevice");
   ck(cudaGetDevice(&device_), "cudaGetDevice");
   ck(cudaFree(nullptr), "CUDA context");
+  try {
+    build();
+  } catch (...) {
+    release_all();
+    device_bound(device_);
+    throw;
+  }
+}
+
+// Streams, buffers and their first contents.
+void Session::build() {
+  const gm_params &p = p_;
   ck(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
   ck(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_), "attr");
   int host_tables = 0;
@@ -107,121 +131,115 @@ Session::Session(const gm_params &p) : p_(p) {
     fixed_bytes_ += std::max<size_t>(bytes, 16);
     return ptr;
   };
-  try {
-    st_.X = (float *)dalloc(Nm * st_.ld * sizeof(float));
-    st_.norms = (float *)dalloc(Nm * sizeof(float));
-    st_.snorms = (float *)dalloc(Nm * sizeof(float));
-    st_.g_key = (unsigned long long *)dalloc(Nm * kListW * sizeof(unsigned long long));
-    st_.dirty = (int *)dalloc(Nm * sizeof(int));
-    st_.knn_ids = (int *)dalloc(Nm * k * sizeof(int));
-    st_.knn_dists = (float *)dalloc(Nm * k * sizeof(float));
-    st_.pub_idx = (uint32_t *)dalloc(Nm * (k + 1) * sizeof(uint32_t));
-    st_.pub_dist = (float *)dalloc(Nm * (k + 1) * sizeof(float));
-    st_.emb = (float *)dalloc(Nm * 2 * sizeof(float));
-    st_.bloom = (uint32_t *)dalloc(Nm * 64 * sizeof(uint32_t));
-    d_stat_ = (unsigned long long *)dalloc(16 * sizeof(unsigned long long));
-    st_.stat = d_stat_;
+  st_.X = (float *)dalloc(Nm * st_.ld * sizeof(float));
+  st_.norms = (float *)dalloc(Nm * sizeof(float));
+  st_.snorms = (float *)dalloc(Nm * sizeof(float));
+  st_.g_key = (unsigned long long *)dalloc(Nm * kListW * sizeof(unsigned long long));
+  st_.dirty = (int *)dalloc(Nm * sizeof(int));
+  st_.knn_ids = (int *)dalloc(Nm * k * sizeof(int));
+  st_.knn_dists = (float *)dalloc(Nm * k * sizeof(float));
+  st_.pub_idx = (uint32_t *)dalloc(Nm * (k + 1) * sizeof(uint32_t));
+  st_.pub_dist = (float *)dalloc(Nm * (k + 1) * sizeof(float));
+  st_.emb = (float *)dalloc(Nm * 2 * sizeof(float));
+  st_.bloom = (uint32_t *)dalloc(Nm * 64 * sizeof(uint32_t));
+  d_stat_ = (unsigned long long *)dalloc(16 * sizeof(unsigned long long));
+  st_.stat = d_stat_;
 
-    us_.fwd_new = (int *)dalloc(Nm * kSamples * sizeof(int));
-    us_.fwd_old = (int *)dalloc(Nm * kSamples * sizeof(int));
-    us_.rev_new = (int *)dalloc(Nm * kSamples * sizeof(int));
-    us_.rev_old = (int *)dalloc(Nm * kSamples * sizeof(int));
-    us_.sizes = (int4 *)dalloc(Nm * sizeof(int4));
-    us_.cnt = (int *)dalloc(Nm * sizeof(int));
-    us_.off = (int *)dalloc((Nm + 1) * sizeof(int));
-    us_.fill = (int *)dalloc(Nm * sizeof(int));
-    us_.csr = (int *)dalloc(Nm * kSamples * sizeof(int));
-    us_.hflag = (int *)dalloc(Nm * sizeof(int));
+  us_.fwd_new = (int *)dalloc(Nm * kSamples * sizeof(int));
+  us_.fwd_old = (int *)dalloc(Nm * kSamples * sizeof(int));
+  us_.rev_new = (int *)dalloc(Nm * kSamples * sizeof(int));
+  us_.rev_old = (int *)dalloc(Nm * kSamples * sizeof(int));
+  us_.sizes = (int4 *)dalloc(Nm * sizeof(int4));
+  us_.cnt = (int *)dalloc(Nm * sizeof(int));
+  us_.off = (int *)dalloc((Nm + 1) * sizeof(int));
+  us_.fill = (int *)dalloc(Nm * sizeof(int));
+  us_.csr = (int *)dalloc(Nm * kSamples * sizeof(int));
+  us_.hflag = (int *)dalloc(Nm * sizeof(int));
 
-    d_rows_ = (int *)dalloc(Nm * sizeof(int));
-    d_rows2_ = (int *)dalloc(Nm * sizeof(int));
-    d_batch_ = (int *)dalloc(Nm * sizeof(int));
-    d_cnt_ = (int *)dalloc(kCounters * sizeof(int));
-    st_.err = (unsigned *)(d_cnt_ + kErrAt);
-    d_tmp_ = (int *)dalloc(compact_tmp_ints((int)Nm) * sizeof(int) + 64);
+  d_rows_ = (int *)dalloc(Nm * sizeof(int));
+  d_rows2_ = (int *)dalloc(Nm * sizeof(int));
+  d_batch_ = (int *)dalloc(Nm * sizeof(int));
+  d_cnt_ = (int *)dalloc(kCounters * sizeof(int));
+  st_.err = (unsigned *)(d_cnt_ + kErrAt);
+  d_tmp_ = (int *)dalloc(compact_tmp_ints((int)Nm) * sizeof(int) + 64);
 
-    // the embedding phase has its own batch, scan scratch, counters and
-    // pinned staging, so that it can run beside the other phases (two sets
-    // in overlap mode, one per side)
-    auto alloc_side = [&](EmbedScratch &e, int *&cnt) {
-      e.flag = (int *)dalloc(Nm * sizeof(int));
-      e.unsel = (int *)dalloc(Nm * sizeof(int));
-      e.sigma = (float *)dalloc(Nm * sizeof(float));
-      e.rho = (float *)dalloc(Nm * sizeof(float));
-      e.deg = (int *)dalloc(Nm * sizeof(int));
-      e.snap = (float *)dalloc(Nm * 2 * sizeof(float));
-      e.fscal = (float *)dalloc(16 * sizeof(float));
-      e.iscal = (int *)dalloc(16 * sizeof(int));
-      e.cap_partial = (Nm * k + 255) / 256 + 512;
-      e.partial = (float *)dalloc(e.cap_partial * 2 * sizeof(float));
-      e.ipartial = (int *)dalloc(e.cap_partial * sizeof(int));
-      e.batch = (int *)dalloc(Nm * sizeof(int));
-      e.tmp = (int *)dalloc(compact_tmp_ints((int)Nm) * sizeof(int) + 64);
-      if (p.overlap) {
-        e.pub_idx_snap = (uint32_t *)dalloc(Nm * (k + 1) * sizeof(uint32_t));
-        e.pub_dist_snap = (float *)dalloc(Nm * (k + 1) * sizeof(float));
-      }
-      cnt = (int *)dalloc(16 * sizeof(int));
-    };
-    alloc_side(es_, es_cnt_);
-    if (p.overlap) alloc_side(es_alt_, es_cnt_alt_);
-
-    pin_bytes_ = (Nm + kCounters) * sizeof(uint32_t);
-    ck(host_alloc((void **)&h_pin_, pin_bytes_), "cudaMallocHost");
-    ck(host_alloc((void **)&h_emb_pin_, pin_bytes_), "cudaMallocHost");
-    if (p.overlap) ck(host_alloc((void **)&h_emb_pin_alt_, pin_bytes_), "cudaMallocHost");
-    if (p.precision == 1) {
-      // split-BF16 shadow rows (hi | lo, 2 x dh bf16 each) plus a block of
-      // candidate / pair scratch for the worst case (every column a
-      // candidate of every block row): 28 bytes per (block row, row).  The
-      // block takes up to 1,024 rows (fewer, longer launches) within an
-      // eighth of the device's memory and at most 32 GB, and at least 128
-      dh_ = exact_dh((int)d);
-      xh_ = dalloc(Nm * (size_t)dh_ * 4);
-      size_t free_b = 0, total_b = 0;
-      ck(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-      const size_t budget = std::min<size_t>(total_b / 8, (size_t)32 << 30);
-      ex_block_ = (int)std::max<size_t>(128, std::min<size_t>(1024, budget / (Nm * 28)));
-      ex_block_ = ex_block_ / 128 * 128;
-      // the approximate tile itself is only stored on request (tests), in
-      // a buffer allocated then
-      ex_cand_ = (int *)dalloc((size_t)ex_block_ * Nm * sizeof(int));
-      xs_.cand = ex_cand_;
-      xs_.cand_d = (float *)dalloc((size_t)ex_block_ * Nm * sizeof(float));
-      xs_.row_cnt = (int *)dalloc((size_t)ex_block_ * sizeof(int));
-      xs_.pool_cap = (long)ex_block_ * (long)Nm;
-      xs_.pool_j = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
-      xs_.pool_m = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
-      xs_.pool_d = (float *)dalloc((size_t)xs_.pool_cap * sizeof(float));
-      xs_.pair_j = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
-      xs_.pair_m = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
-      xs_.row_t = (float *)dalloc((size_t)ex_block_ * sizeof(float));
-      xs_.seed = (float *)dalloc((size_t)ex_block_ * sizeof(float));
-      // pre-candidate segments: one per (block row, CTA of a row tile), for
-      // every grid width a block can take (at most one CTA per column tile)
-      // and room for every column up to four column tiles
-      xs_.pre_gx = (int)std::min<size_t>(std::max(sms_, 1), (Nm + 255) / 256);
-      xs_.pre_cap = std::max(kPreCap, (1024 + xs_.pre_gx - 1) / xs_.pre_gx);
-      xs_.pre = (unsigned long long *)dalloc((size_t)ex_block_ * xs_.pre_gx * xs_.pre_cap *
-                                             sizeof(unsigned long long));
-      xs_.pre_ub = (float *)dalloc((size_t)ex_block_ * xs_.pre_gx * xs_.pre_cap * sizeof(float));
-      // (no block of fewer tiles samples more of them than 32)
-      xs_.mins_ld = std::max(exact_seed_tiles((int)((Nm + 255) / 256)), 32) * 8;
-      xs_.mins = (float *)dalloc((size_t)ex_block_ * xs_.mins_ld * sizeof(float));
-      xs_.pre_cnt = (int *)dalloc((size_t)ex_block_ * xs_.pre_gx * sizeof(int));
-      xs_.pre_over = (int *)dalloc(sizeof(int));
-      xs_.heaps = (float *)dalloc((size_t)ex_block_ * std::max(sms_, 1) * 32 * sizeof(float));
-      xs_.pcnt = (int *)dalloc((size_t)ex_block_ * sizeof(int));
-      xs_.poff = (int *)dalloc(((size_t)ex_block_ + 1) * sizeof(int));
-      xs_.pfill = (int *)dalloc((size_t)ex_block_ * sizeof(int));
-      xs_.ptask = (int *)dalloc(((size_t)ex_block_ + 1) * sizeof(int));
-      xs_.heads = us_.fwd_new;  // not in use during an insertion
-      xs_.counter = (int *)dalloc(16 * sizeof(int));
+  // the embedding phase has its own batch, scan scratch, counters and
+  // pinned staging, so that it can run beside the other phases (two sets
+  // in overlap mode, one per side)
+  auto alloc_side = [&](EmbedScratch &e, int *&cnt) {
+    e.flag = (int *)dalloc(Nm * sizeof(int));
+    e.unsel = (int *)dalloc(Nm * sizeof(int));
+    e.sigma = (float *)dalloc(Nm * sizeof(float));
+    e.rho = (float *)dalloc(Nm * sizeof(float));
+    e.deg = (int *)dalloc(Nm * sizeof(int));
+    e.snap = (float *)dalloc(Nm * 2 * sizeof(float));
+    e.fscal = (float *)dalloc(16 * sizeof(float));
+    e.iscal = (int *)dalloc(16 * sizeof(int));
+    e.cap_partial = (Nm * k + 255) / 256 + 512;
+    e.partial = (float *)dalloc(e.cap_partial * 2 * sizeof(float));
+    e.ipartial = (int *)dalloc(e.cap_partial * sizeof(int));
+    e.batch = (int *)dalloc(Nm * sizeof(int));
+    e.tmp = (int *)dalloc(compact_tmp_ints((int)Nm) * sizeof(int) + 64);
+    if (p.overlap) {
+      e.pub_idx_snap = (uint32_t *)dalloc(Nm * (k + 1) * sizeof(uint32_t));
+      e.pub_dist_snap = (float *)dalloc(Nm * (k + 1) * sizeof(float));
     }
-  } catch (...) {
-    release_memory();
-    release_streams();
-    throw;
+    cnt = (int *)dalloc(16 * sizeof(int));
+  };
+  alloc_side(es_, es_cnt_);
+  if (p.overlap) alloc_side(es_alt_, es_cnt_alt_);
+
+  pin_bytes_ = (Nm + kCounters) * sizeof(uint32_t);
+  ck(host_alloc((void **)&h_pin_, pin_bytes_), "cudaMallocHost");
+  ck(host_alloc((void **)&h_emb_pin_, pin_bytes_), "cudaMallocHost");
+  if (p.overlap) ck(host_alloc((void **)&h_emb_pin_alt_, pin_bytes_), "cudaMallocHost");
+  if (p.precision == 1) {
+    // split-BF16 shadow rows (hi | lo, 2 x dh bf16 each) plus a block of
+    // candidate / pair scratch for the worst case (every column a
+    // candidate of every block row): 28 bytes per (block row, row).  The
+    // block takes up to 1,024 rows (fewer, longer launches) within an
+    // eighth of the device's memory and at most 32 GB, and at least 128
+    dh_ = exact_dh((int)d);
+    xh_ = dalloc(Nm * (size_t)dh_ * 4);
+    size_t free_b = 0, total_b = 0;
+    ck(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+    const size_t budget = std::min<size_t>(total_b / 8, (size_t)32 << 30);
+    ex_block_ = (int)std::max<size_t>(128, std::min<size_t>(1024, budget / (Nm * 28)));
+    ex_block_ = ex_block_ / 128 * 128;
+    // the approximate tile itself is only stored on request (tests), in
+    // a buffer allocated then
+    ex_cand_ = (int *)dalloc((size_t)ex_block_ * Nm * sizeof(int));
+    xs_.cand = ex_cand_;
+    xs_.cand_d = (float *)dalloc((size_t)ex_block_ * Nm * sizeof(float));
+    xs_.row_cnt = (int *)dalloc((size_t)ex_block_ * sizeof(int));
+    xs_.pool_cap = (long)ex_block_ * (long)Nm;
+    xs_.pool_j = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
+    xs_.pool_m = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
+    xs_.pool_d = (float *)dalloc((size_t)xs_.pool_cap * sizeof(float));
+    xs_.pair_j = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
+    xs_.pair_m = (int *)dalloc((size_t)xs_.pool_cap * sizeof(int));
+    xs_.row_t = (float *)dalloc((size_t)ex_block_ * sizeof(float));
+    xs_.seed = (float *)dalloc((size_t)ex_block_ * sizeof(float));
+    // pre-candidate segments: one per (block row, CTA of a row tile), for
+    // every grid width a block can take (at most one CTA per column tile)
+    // and room for every column up to four column tiles
+    xs_.pre_gx = (int)std::min<size_t>(std::max(sms_, 1), (Nm + 255) / 256);
+    xs_.pre_cap = std::max(kPreCap, (1024 + xs_.pre_gx - 1) / xs_.pre_gx);
+    xs_.pre = (unsigned long long *)dalloc((size_t)ex_block_ * xs_.pre_gx * xs_.pre_cap *
+                                           sizeof(unsigned long long));
+    xs_.pre_ub = (float *)dalloc((size_t)ex_block_ * xs_.pre_gx * xs_.pre_cap * sizeof(float));
+    // (no block of fewer tiles samples more of them than 32)
+    xs_.mins_ld = std::max(exact_seed_tiles((int)((Nm + 255) / 256)), 32) * 8;
+    xs_.mins = (float *)dalloc((size_t)ex_block_ * xs_.mins_ld * sizeof(float));
+    xs_.pre_cnt = (int *)dalloc((size_t)ex_block_ * xs_.pre_gx * sizeof(int));
+    xs_.pre_over = (int *)dalloc(sizeof(int));
+    xs_.heaps = (float *)dalloc((size_t)ex_block_ * std::max(sms_, 1) * 32 * sizeof(float));
+    xs_.pcnt = (int *)dalloc((size_t)ex_block_ * sizeof(int));
+    xs_.poff = (int *)dalloc(((size_t)ex_block_ + 1) * sizeof(int));
+    xs_.pfill = (int *)dalloc((size_t)ex_block_ * sizeof(int));
+    xs_.ptask = (int *)dalloc(((size_t)ex_block_ + 1) * sizeof(int));
+    xs_.heads = us_.fwd_new;  // not in use during an insertion
+    xs_.counter = (int *)dalloc(16 * sizeof(int));
   }
 
   // Initial contents: zero features (padding must stay zero), empty lists,
@@ -252,11 +270,8 @@ Session::Session(const gm_params &p) : p_(p) {
   ck(cudaGetLastError(), "init fill");
   ck(cudaStreamSynchronize(s), "init sync");
   if (xh_) {
-    if (!make_row_maps(xh_, (int)Nm, dh_, &maps_)) {
-      release_memory();
-      release_streams();
+    if (!make_row_maps(xh_, (int)Nm, dh_, &maps_))
       throw Error(GM_ERR_CUDA, "cuTensorMapEncodeTiled unavailable or failed");
-    }
   }
   upd_q_.reset(N);
   ensure_embed(es_, 1);
@@ -294,13 +309,29 @@ void Session::sync_embed_streams() {
 }
 
 void Session::free_embed(EmbedScratch &e) {
-  if (!e.coo_row) return;
-  for (void *q : {(void *)e.coo_row, (void *)e.coo_col, (void *)e.coo_val, (void *)e.t_row,
-                  (void *)e.t_col, (void *)e.flag_tail, (void *)e.t_val, (void *)e.next_s,
-                  (void *)e.next_n, (void *)e.tmp2})
-    device_free(q, stream_);
-  e.coo_row = nullptr;
+  auto drop = [&](auto *&...p) { ((device_free(p, stream_), p = nullptr), ...); };
+  drop(e.coo_row, e.coo_col, e.coo_val, e.t_row, e.t_col, e.flag_tail, e.t_val, e.next_s, e.next_n, e.tmp2);
   e.cap_coo = 0;
+}
+
+// Everything the session holds, however far it was built; its work has been
+// waited for.
+void Session::release_all() {
+  if (cstream_) cudaStreamSynchronize(cstream_);
+  for (cudaStream_t q : {estream_, estream_alt_})
+    if (q) cudaStreamSynchronize(q);
+  free_cand();
+  device_free(join_pool_, stream_);
+  join_pool_ = nullptr;
+  free_embed(es_);
+  free_embed(es_alt_);
+  release_memory();
+  for (auto &slot : ring_) {
+    if (slot.done) cudaEventDestroy(slot.done);
+    host_free(slot.buf, slot.cap);
+  }
+  if (cstream_) cudaStreamDestroy(cstream_);
+  release_streams();
 }
 
 Session::~Session() {
@@ -317,18 +348,7 @@ Session::~Session() {
     cudaEventDestroy(pr.a);
     cudaEventDestroy(pr.b);
   }
-  if (cstream_) cudaStreamSynchronize(cstream_);
-  free_cand();
-  device_free(join_pool_, stream_);
-  free_embed(es_);
-  free_embed(es_alt_);
-  release_memory();
-  for (auto &slot : ring_) {
-    if (slot.done) cudaEventDestroy(slot.done);
-    host_free(slot.buf, slot.cap);
-  }
-  if (cstream_) cudaStreamDestroy(cstream_);
-  release_streams();
+  release_all();
   device_closed(device_, held);
 }
 
@@ -415,6 +435,7 @@ void Session::ensure_cand(size_t rows) {
   sync();
   free_cand();
   const size_t r = std::max<size_t>(rows, 1024), slots = r * kMaxCand;
+  Undo whole{[&] { free_cand(); }};
   auto get = [&](auto *&p, size_t n) {
     ck(device_alloc((void **)&p, n * sizeof(*p), device_, stream_), "cudaMalloc cand");
   };
@@ -426,6 +447,7 @@ void Session::ensure_cand(size_t rows) {
     get(cs_.todo_cnt, r);
   }
   get(cs_.next, std::min<size_t>(r, kOfferRows) * kMaxCand);
+  whole.done = true;
   cand_rows_ = r;
 }
 
@@ -475,7 +497,7 @@ size_t Session::device_bytes() const {
   b += cand_bytes(cand_rows_, st_.k);
   if (join_pool_) b += (join_words_ + kJoinSlackWords) * sizeof(int);
   for (const EmbedScratch *e : {&es_, &es_alt_})
-    if (e->coo_row) b += e->cap_coo * 9 * 4 + (compact_tmp_ints((int)e->cap_coo) + 64) * sizeof(int);
+    if (e->cap_coo) b += e->cap_coo * 9 * 4 + (compact_tmp_ints((int)e->cap_coo) + 64) * sizeof(int);
   return b;
 }
 
@@ -506,6 +528,7 @@ void Session::ensure_embed(EmbedScratch &e, size_t nb) {
   sync_embed_streams();
   free_embed(e);
   const size_t c = std::max(need, (size_t)4096);
+  Undo whole{[&] { free_embed(e); }};
   auto get = [&](auto *&p, size_t n) {
     ck(device_alloc((void **)&p, n * sizeof(*p), device_, stream_), "cudaMalloc coo");
   };
@@ -520,6 +543,7 @@ void Session::ensure_embed(EmbedScratch &e, size_t nb) {
   get(e.next_n, c);
   get(e.tmp2, compact_tmp_ints((int)c) + 64);
   sync();  // (the embedding may run on another stream)
+  whole.done = true;
   e.cap_coo = c;
 }
 

@@ -119,6 +119,8 @@ class Session {
   void flush_init();
   template <typename... A> void log(const char *fmt, A... a) const;
   void sync();
+  void build();
+  void release_all();
   void release_streams();
   void release_memory();
   void timed_begin(int slot, cudaStream_t s = nullptr);

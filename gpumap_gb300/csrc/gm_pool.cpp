@@ -99,8 +99,14 @@ size_t host_size(size_t bytes) {  // whole 64 KB pages
 
 }  // namespace
 
+namespace {
+thread_local int g_fail_in = 0;
+}
+void device_fail_in(int n) { g_fail_in = n; }
+
 cudaError_t device_alloc(void **out, size_t bytes, int device, cudaStream_t s) {
   *out = nullptr;
+  if (g_fail_in > 0 && --g_fail_in == 0) return cudaErrorMemoryAllocation;
   cudaMemPool_t p = nullptr;
   {
     std::lock_guard<std::mutex> g(g_mu);

@@ -62,6 +62,9 @@ int gm_debug_join_words(struct gm_session *s, uint64_t words);
  * reads host memory, and the address is a multiple of 4), 2 copied into a pinned
  * staging slot first. */
 int gm_debug_ingest_route(uint64_t address, int page_locked, int reads_host);
+/* The nth device allocation of this library from here on in the calling thread
+ * (1: the next) reports out of memory; 0 takes that back. */
+int gm_debug_fail_alloc(int nth);
 /* Host and device scalars, out[0..n):
  *  0 n_inserted, 1 insertion-queue head, 2 new-row embedding-queue head,
  *  3 embedding cursor (-1 = none), 4 embedding sweeps, 5 last nnz,
