@@ -95,6 +95,7 @@ _SIGS = [
     ("gm_debug_pre_capacity", C.c_int, [_P, C.c_int]),
     ("gm_debug_join_words", C.c_int, [_P, C.c_uint64]),
     ("gm_debug_ingest_route", C.c_int, [C.c_uint64, C.c_int, C.c_int]),
+    ("gm_debug_raise", C.c_int, [_P, C.c_uint32]),
     ("gm_debug_fail_alloc", C.c_int, [C.c_int]),
     ("gm_debug_scalars", C.c_int, [_P, C.POINTER(C.c_int64), C.c_int]),
     ("gm_debug_update_queue", C.c_int, [_P, _P, C.c_uint64, C.POINTER(C.c_uint64)]),

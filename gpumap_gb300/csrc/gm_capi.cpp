@@ -313,6 +313,11 @@ int gm_debug_ingest_route(uint64_t address, int page_locked, int reads_host) {
   return (int)gm::ingest_route(reinterpret_cast<const void *>((uintptr_t)address), page_locked != 0, reads_host != 0);
 }
 
+int gm_debug_raise(gm_session *s, uint32_t bits) {
+  if (!s) return fail(GM_ERR_INVALID, "null session");
+  return guarded([&] { s->impl->raise_device_error(bits); });
+}
+
 int gm_debug_fail_alloc(int nth) {
   gm::device_fail_in(std::max(0, nth));
   return GM_OK;

@@ -378,6 +378,11 @@ void Session::drain() {
   check_device_error("embedding");
 }
 
+void Session::raise_device_error(unsigned bits) {
+  ck(cudaMemcpyAsync(st_.err, &bits, sizeof(bits), cudaMemcpyHostToDevice, stream_), "error bits");
+  sync();
+}
+
 void Session::check_launch_error(const char *phase) {
   // a launch the runtime refused (resources, configuration) is reported
   // once, by the next query of the last error
@@ -403,7 +408,8 @@ void Session::report_device_error(const char *phase, unsigned e) {
 // most `bound` rows): its counters, error word and first rows come in one wait
 // (three waits, for the count, the rows and the error word, were 30 us a
 // phase).  Counters are then at h_pin_, the rows after them; returns their
-// number.
+// number.  Error bits are kept for end_phase, so that the caller's queues are
+// brought up to date first.
 size_t Session::finish_phase(const char *phase, size_t bound) {
   check_launch_error(phase);
   const size_t ahead = std::min(bound, kRowsAhead);
@@ -412,7 +418,8 @@ size_t Session::finish_phase(const char *phase, size_t bound) {
   if (ahead)
     ck(cudaMemcpyAsync(rows, d_rows_, ahead * sizeof(int), cudaMemcpyDeviceToHost, stream_), "rows");
   sync();
-  report_device_error(phase, h_pin_[kErrAt]);
+  err_bits_ |= h_pin_[kErrAt];
+  err_read_ = true;
   const size_t n = h_pin_[0];
   if (n > ahead) {
     ck(cudaMemcpyAsync(rows + ahead, d_rows_ + ahead, (n - ahead) * sizeof(int), cudaMemcpyDeviceToHost,
@@ -420,6 +427,19 @@ size_t Session::finish_phase(const char *phase, size_t bound) {
     sync();
   }
   return n;
+}
+
+// After a phase: reports the error bits it read.  A phase that had nothing to do
+// read none; then, in overlap mode, the word is read here, because the embedding
+// still in flight at the last report may have set it since.
+void Session::end_phase(const char *phase) {
+  const bool read = err_read_;
+  const unsigned bits = err_bits_;
+  err_read_ = false;
+  err_bits_ = 0;
+  if (read) report_device_error(phase, bits);
+  else if (p_.overlap) check_device_error(phase);
+  else check_launch_error(phase);
 }
 
 void Session::free_cand() {
@@ -738,6 +758,7 @@ gm_result Session::run(uint32_t n_ins, uint32_t n_upd, uint32_t n_emb) {
   if (!ins_done_) {
     const auto t0 = Clock::now();
     r.n_insertion_ops = insert(n_ins);
+    end_phase("insertion");
     const auto t1 = Clock::now();
     r.insertion_time = std::chrono::duration<float>(t1 - t0).count();
     ins_done_ = (ins_head_ == n_inserted_) && n_inserted_ == p_.n_instances;
@@ -747,6 +768,7 @@ gm_result Session::run(uint32_t n_ins, uint32_t n_upd, uint32_t n_emb) {
     size_t changed = 0;
     const auto t0 = Clock::now();
     r.n_update_ops = update(n_upd, changed);
+    end_phase("update");
     const auto t1 = Clock::now();
     r.n_update_changed_edges = changed;
     r.update_time = std::chrono::duration<float>(t1 - t0).count();

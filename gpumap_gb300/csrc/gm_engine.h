@@ -87,6 +87,8 @@ class Session {
   // words of the join pool a pass covers, at most (tests)
   void set_join_part(size_t words);
   void drain();
+  // sets device error bits, as a wait that ran out would (tests)
+  void raise_device_error(unsigned bits);
   // consumer waits (on the device) for everything queued on this session
   void order_after(cudaStream_t consumer) const;
   void get_stats(gm_stats *out);
@@ -107,6 +109,7 @@ class Session {
   void check_device_error(const char *phase);
   void report_device_error(const char *phase, unsigned bits);
   size_t finish_phase(const char *phase, size_t bound);
+  void end_phase(const char *phase);
   void ensure_cand(size_t rows);
   void free_cand();
   void ensure_join(size_t words);
@@ -177,6 +180,8 @@ class Session {
   static constexpr int kCounters = 64, kFlagsAt = 16, kErrAt = 48;
   static constexpr size_t kRowsAhead = 8192;  // rows fetched with the counters
   int *d_cnt_ = nullptr;
+  unsigned err_bits_ = 0;  // read by finish_phase, not reported yet
+  bool err_read_ = false;
   int *d_tmp_ = nullptr;
   size_t pin_bytes_ = 0;           // of each pinned staging buffer
   uint32_t *h_pin_ = nullptr;      // pinned staging (n_cap + 16 words)

@@ -62,6 +62,9 @@ int gm_debug_join_words(struct gm_session *s, uint64_t words);
  * reads host memory, and the address is a multiple of 4), 2 copied into a pinned
  * staging slot first. */
 int gm_debug_ingest_route(uint64_t address, int page_locked, int reads_host);
+/* Sets the session's device error word, as a bounded wait that ran out would;
+ * the next check reports it. */
+int gm_debug_raise(struct gm_session *s, uint32_t bits);
 /* The nth device allocation of this library from here on in the calling thread
  * (1: the next) reports out of memory; 0 takes that back. */
 int gm_debug_fail_alloc(int nth);
