@@ -63,6 +63,7 @@ constexpr uint32_t kWaitLimit = 1u << 24;      // bounded mbarrier waits
 // list bars of a tile, double buffered (two tiles), then per buffer sixteen
 // per-warp maxima of the norms and bound factors (float bits: both >= 0)
 constexpr size_t kEpiBytes = (size_t)2 * 3 * kTN * sizeof(float) + (size_t)2 * 2 * 16 * sizeof(float);
+constexpr uint32_t kInfBits = 0x7f800000u;     // floats >= 0 below it are finite
 constexpr int kListTop = 32;                   // list width the screen keeps exact
 constexpr size_t kHeapBytes = (size_t)kListTop * kTM * sizeof(float);
 constexpr size_t kExactSmem = (size_t)kStages * kStageBytes + 1024 + 256 + kEpiBytes + kHeapBytes;
@@ -490,8 +491,13 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
             cn[jj] = cv[3 * h];
             cn[kTN + jj] = cv[3 * h + 1];
             cn[2 * kTN + jj] = cv[3 * h + 2];
-            mn = max(mn, __float_as_uint(cv[3 * h]));
-            ms = max(ms, __float_as_uint(cv[3 * h + 1]));
+            // a column whose norm is infinite or NaN (its row has such a
+            // feature, or overflows) passes no test: D - B is NaN for every
+            // row.  Its norm would make the filter's slack NaN for the whole
+            // group
+            const unsigned un = __float_as_uint(cv[3 * h]), us = __float_as_uint(cv[3 * h + 1]);
+            mn = max(mn, un < kInfBits ? un : 0u);
+            ms = max(ms, us < kInfBits ? us : 0u);
           }
         }
         mn = __reduce_max_sync(0xffffffffu, mn);
@@ -507,7 +513,7 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
         case 2: asm volatile("bar.sync 3, 128;" ::: "memory"); break;
         default: asm volatile("bar.sync 4, 128;" ::: "memory"); break;
       }
-      // the largest pair bound of the row over this group's columns
+      // the largest pair bound of the row over this group's finite columns
       // (pair_bound is nondecreasing in the column's norm and factor)
       float bmax, nmax;
       {
@@ -550,7 +556,8 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
         const float sj = cn[kTN + c + i];
         const float bnd = pair_bound(sc.coef, sm, sj, nm, nj);
         if (kPass == 1 && other) {
-          const float ub = fmaxf(__fadd_ru(dv, bnd), 0.0f);
+          // (the clamp keeps a NaN, which fails the test; fmaxf would make it 0)
+          const float sum = __fadd_ru(dv, bnd), ub = sum <= 0.0f ? 0.0f : sum;
           if (ub < t_loc && ub <= seed) t_loc = heap_push(heap, hcnt, ub);
         }
         if (kPass == 3 && other) {
