@@ -418,7 +418,10 @@ __global__ void __launch_bounds__(kFwdWarps * 32)
   for (int c0 = 0; c0 < kMaxCand; c0 += 32) {
     const int id = cand[(size_t)rl * kMaxCand + c0 + lane];
     const float dv = cand_dist[(size_t)rl * kMaxCand + c0 + lane];
+    // (a NaN passes and can take the tail's place, and anything passes a NaN
+    // there: with one among the 32 each is tested in its turn)
     unsigned todo = c0 ? __ballot_sync(full, !(dv >= __shfl_sync(full, sd, 31))) : full;
+    if (__any_sync(full, dv != dv)) todo = full;
     while (todo) {
       const int src = __ffs(todo) - 1;
       todo &= todo - 1u;

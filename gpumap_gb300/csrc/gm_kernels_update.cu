@@ -635,17 +635,38 @@ __global__ void __launch_bounds__(kMpWarps * 32)
   int report = 0;
   if (h >= 1) {
     // sort_lists: ascending (dist, id_with_flag)
-    int rank = 0;
-    for (int q = 0; q < k; ++q) {
-      const float v = __shfl_sync(full, lv, q);
-      const int e = __shfl_sync(full, le, q);
-      rank += v < lv || (v == lv && (e < le || (e == le && q < lane)));
+    if (__any_sync(full, lane < k && lv != lv)) {
+      // (a NaN has no rank: the insertion sort itself, an entry at a time; an
+      // entry goes behind the last one before it that is not above it)
+      for (int a = 1; a < k; ++a) {
+        const int e = __shfl_sync(full, le, a);
+        const float v = __shfl_sync(full, lv, a);
+        const bool above = lv > v || (lv == v && le > e);
+        const unsigned stay = __ballot_sync(full, !above) & ((1u << a) - 1u);
+        const int pos = stay ? 32 - __clz(stay) : 0;
+        const int pe = __shfl_up_sync(full, le, 1);
+        const float pv = __shfl_up_sync(full, lv, 1);
+        if (lane > pos && lane <= a) {
+          le = pe;
+          lv = pv;
+        } else if (lane == pos) {
+          le = e;
+          lv = v;
+        }
+      }
+    } else {
+      int rank = 0;
+      for (int q = 0; q < k; ++q) {
+        const float v = __shfl_sync(full, lv, q);
+        const int e = __shfl_sync(full, le, q);
+        rank += v < lv || (v == lv && (e < le || (e == le && q < lane)));
+      }
+      int from = 0;
+      for (int q = 0; q < k; ++q)
+        if (__shfl_sync(full, rank, q) == lane) from = q;
+      le = __shfl_sync(full, le, from);
+      lv = __shfl_sync(full, lv, from);
     }
-    int from = 0;
-    for (int q = 0; q < k; ++q)
-      if (__shfl_sync(full, rank, q) == lane) from = q;
-    le = __shfl_sync(full, le, from);
-    lv = __shfl_sync(full, lv, from);
     if (lane < k) {
       kl[lane] = le;
       kd[lane] = lv;
