@@ -1139,7 +1139,9 @@ void Session::debug_scalars(int64_t *out, int cnt) const {
     if (q) cudaStreamSynchronize(q);
   cudaMemcpy(iscal, es_.iscal, sizeof(iscal), cudaMemcpyDeviceToHost);
   cudaMemcpy(&err, st_.err, sizeof(err), cudaMemcpyDeviceToHost);
-  int64_t v[11] = {(int64_t)n_inserted_,
+  unsigned long long wide = 0;
+  cudaMemcpy(&wide, d_stat_ + 10, sizeof(wide), cudaMemcpyDeviceToHost);
+  int64_t v[12] = {(int64_t)n_inserted_,
                    (int64_t)ins_head_,
                    (int64_t)emb_new_head_,
                    emb_cursor_ == SIZE_MAX ? -1 : (int64_t)emb_cursor_,
@@ -1149,8 +1151,9 @@ void Session::debug_scalars(int64_t *out, int cnt) const {
                    iscal[2],
                    iscal[3],
                    (int64_t)upd_q_.size(),
-                   (int64_t)err};
-  for (int i = 0; i < cnt && i < 11; ++i) out[i] = v[i];
+                   (int64_t)err,
+                   (int64_t)wide};
+  for (int i = 0; i < cnt && i < 12; ++i) out[i] = v[i];
 }
 
 }  // namespace gm

@@ -923,7 +923,10 @@ __global__ void __launch_bounds__(kSeedThreads)
 // A warp per row that inserted the bounds one at a time was bound by latency: 33
 // us for 500 rows of ~600 entries, a CTA that searched them by bits 24 us in a
 // run (31 rounds over all values, bound by issue), this form 11 us.  A row with
-// more than kPreStage entries is worked through where they lie, by its first warp.
+// more than kPreStage entries (data far from the origin, whose bounds are wide) is
+// worked through where they lie, by the same search: by one warp a bit at a time
+// 9,600 such rows x 8 in cycles of 300 took 38.2 ms (31.8 with the insertion before
+// that), 24.7 so.
 constexpr int kPreThreads = 128;
 constexpr int kPreStage = 2048, kPreSegs = 512;
 __global__ void __launch_bounds__(kPreThreads)
@@ -941,7 +944,6 @@ __global__ void __launch_bounds__(kPreThreads)
   __shared__ int s_off[kPreSegs + 1], s_kept;
   __shared__ Select32 sel;
   const unsigned full = 0xffffffffu;
-  const float inf = __int_as_float(0x7f800000);
   const int *cnts = pre_cnt + (size_t)m * gx;
   const size_t seg0 = (size_t)m * gx * (size_t)cap;
   if (warp == 0) {
@@ -954,7 +956,7 @@ __global__ void __launch_bounds__(kPreThreads)
         const int y = __shfl_up_sync(full, incl, o);
         if (lane >= o) incl += y;
       }
-      if (c0 + lane < min(gx, kPreSegs)) s_off[c0 + lane] = run + incl - v;
+      if (c0 + lane < gx) s_off[c0 + lane] = run + incl - v;
       run += __shfl_sync(full, incl, 31);
     }
     if (lane == 0) {
@@ -973,35 +975,34 @@ __global__ void __launch_bounds__(kPreThreads)
     base = __shfl_sync(full, base, 0);
     if (ok) out[base + __popc(bal & ((1u << lane) - 1u))] = (int)(unsigned)e;
   };
-  float T = inf;
-  if (total <= kPreStage && gx <= kPreSegs) {
-    // entry i is in the last segment that begins at or before it
+  // entry i is in the last segment that begins at or before it
+  auto place = [&](int i) {
+    int c = 0;
+    for (int step = kPreSegs / 2; step > 0; step >>= 1)
+      if (c + step < gx && s_off[c + step] <= i) c += step;
+    return seg0 + (size_t)c * cap + (i - s_off[c]);
+  };
+  auto select = [&](auto &&ub, auto &&entry) {
+    // fewer than 32 other rows: every column is a candidate
+    float T = cta_32nd<kPreThreads>(total, ub, sel);
+    if (n - 1 < kListTop) T = __int_as_float(0x7f800000);
+    for (int i = warp * 32; i < total; i += kPreThreads)
+      keep(i + lane < total, i + lane < total ? entry(i + lane) : 0ull, T);
+    return T;
+  };
+  float T;
+  if (total <= kPreStage) {
 #pragma unroll 4
     for (int i = threadIdx.x; i < total; i += kPreThreads) {
-      int c = 0;
-      for (int step = kPreSegs / 2; step > 0; step >>= 1)
-        if (c + step < gx && s_off[c + step] <= i) c += step;
-      const size_t from = seg0 + (size_t)c * cap + (i - s_off[c]);
+      const size_t from = place(i);
       s_ub[i] = pre_ub[from];
       s_ent[i] = pre[from];
     }
     __syncthreads();
-    T = cta_32nd<kPreThreads>(total, [&](int i) { return s_ub[i]; }, sel);
-    // fewer than 32 other rows: every column is a candidate
-    if (n - 1 < kListTop) T = inf;
-    for (int i = warp * 32; i < total; i += kPreThreads)
-      keep(i + lane < total, i + lane < total ? s_ent[i + lane] : 0ull, T);
-  } else if (warp == 0) {
-    T = bits_32nd([&](float x) {
-      int c = 0;
-      for (int g = 0; g < gx; ++g)
-        for (int i = lane; i < cnts[g]; i += 32) c += pre_ub[seg0 + (size_t)g * cap + i] <= x;
-      return (int)__reduce_add_sync(full, (unsigned)c);
-    });
-    if (n - 1 < kListTop) T = inf;
-    for (int g = 0; g < gx; ++g)
-      for (int i = 0; i < cnts[g]; i += 32)
-        keep(i + lane < cnts[g], i + lane < cnts[g] ? pre[seg0 + (size_t)g * cap + i + lane] : 0ull, T);
+    T = select([&](int i) { return s_ub[i]; }, [&](int i) { return s_ent[i]; });
+  } else {
+    T = select([&](int i) { return pre_ub[place(i)]; }, [&](int i) { return pre[place(i)]; });
+    if (stat && threadIdx.x == 0) atomicAdd(&stat[10], 1ull);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -1319,7 +1320,7 @@ void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int ro
   // columns of a CTA: with room for all of them no segment overflows
   const int cta_cols = cdiv(n_tiles, gx) * kTN;
   const bool seeded = n_tiles >= kSeedMin;
-  if (x.pre && cap > 0 && gx <= x.pre_gx &&
+  if (x.pre && cap > 0 && gx <= x.pre_gx && gx <= kPreSegs &&
       (seeded ? tiles * (kTN / 32) <= x.mins_ld : cap >= cta_cols)) {
     // seed pass over a spread sample of tiles (or no seed: every column is
     // stored), then the store pass

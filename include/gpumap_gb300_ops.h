@@ -72,7 +72,8 @@ int gm_debug_fail_alloc(int nth);
  *  0 n_inserted, 1 insertion-queue head, 2 new-row embedding-queue head,
  *  3 embedding cursor (-1 = none), 4 embedding sweeps, 5 last nnz,
  *  6 last extras, 7 last trimmed nnz, 8 last max degree, 9 update queue size,
- * 10 device error bits. */
+ * 10 device error bits, 11 rows of the exact screen with more stored columns than
+ * its selection stages (since the statistics were last reset). */
 int gm_debug_scalars(const struct gm_session *s, int64_t *out, int n);
 /* Update-queue contents in FIFO order. */
 int gm_debug_update_queue(const struct gm_session *s, uint32_t *out, uint64_t cap,
