@@ -221,10 +221,13 @@ void Session::build() {
     xs_.row_t = (float *)dalloc((size_t)ex_block_ * sizeof(float));
     xs_.seed = (float *)dalloc((size_t)ex_block_ * sizeof(float));
     // pre-candidate segments: one per (block row, CTA of a row tile), for
-    // every grid width a block can take (at most one CTA per column tile)
-    // and room for every column up to four column tiles
-    xs_.pre_gx = (int)std::min<size_t>(std::max(sms_, 1), (Nm + 255) / 256);
-    xs_.pre_cap = std::max(kPreCap, (1024 + xs_.pre_gx - 1) / xs_.pre_gx);
+    // every grid width a block can take (at most one CTA per column tile),
+    // and room for every column up to kExactRoomTiles column tiles (one more,
+    // as CTAs with two tiles each may make one up)
+    const int tiles = (int)((Nm + 255) / 256);
+    const int room = (std::min(tiles, kExactRoomTiles) + 1) * 256;
+    xs_.pre_gx = std::min(std::max(sms_, 1), tiles);
+    xs_.pre_cap = std::max(kPreCap, (room + xs_.pre_gx - 1) / xs_.pre_gx);
     xs_.pre = (unsigned long long *)dalloc((size_t)ex_block_ * xs_.pre_gx * xs_.pre_cap *
                                            sizeof(unsigned long long));
     xs_.pre_ub = (float *)dalloc((size_t)ex_block_ * xs_.pre_gx * xs_.pre_cap * sizeof(float));

@@ -1283,6 +1283,14 @@ static void launch_tile(const DevState &st, const ExactMaps &maps, int dh, int r
   note_launch();
 }
 
+// Up to kExactRoomTiles column tiles the segments hold every column.  Rows that
+// come ordered, by cluster say, need it: a row's neighbours then lie in few
+// chunks, its seed in another cluster, and the store pass admits whole tiles.
+// With segments of 64 entries 13 of the 16 blocks of 4,999 rows x 131 in ten
+// ordered clusters overflowed and ran the heap passes as well: a build of cycles
+// of 333 took 4.4 ms, 2.7 with the room (shuffled rows 2.3 and 2.1).  Twelve bytes
+// for each of 8,448 columns and 1,024 block rows are 104 MB; from 132 tiles on the
+// segments of 64 entries take as much.
 // Column tiles of the seed pass (evenly spaced over the columns): at least
 // 16, and one in 8 of the block's tiles, so that the seed stays a low
 // quantile of the row's upper bounds at any column count; all of them up to 32.
@@ -1310,8 +1318,11 @@ void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int ro
                        cudaStream_t s) {
   const int n_tiles = cdiv(n, kTN);
   const int m_tiles = cdiv(nrows, kTM);
-  // CTAs per row tile so that the grid covers the SMs once
-  const int gx = std::max(1, std::min(n_tiles, std::max(1, sms / m_tiles)));
+  // CTAs per row tile so that the grid covers the SMs once; where the segments
+  // are to hold every column, no more than the column tiles per CTA call for
+  // (the longest CTA stays, and the segments are as long as those tiles)
+  int gx = std::max(1, std::min(n_tiles, std::max(1, sms / m_tiles)));
+  if (n_tiles <= kExactRoomTiles) gx = cdiv(n_tiles, cdiv(n_tiles, gx));
   const bool kd = keep_d && x.D;
   const int tiles = exact_seed_tiles(n_tiles);
   // entries per stored segment: the row's whole allocation shared by its

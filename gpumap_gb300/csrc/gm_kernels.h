@@ -158,6 +158,8 @@ struct ExactScreen {
 // per-row exact threshold, then the candidates): candidate columns per batch
 // row and (existing row, batch row) pairs land in x.  With keep_d the
 // approximate tile is also written to x.D (nrows x ldD), for tests.
+// Up to so many column tiles a block's stored columns have room for every column.
+constexpr int kExactRoomTiles = 32;
 // Column tiles the seed pass samples out of n_tiles.
 int exact_seed_tiles(int n_tiles);
 void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int row0, int blk0,

@@ -48,7 +48,8 @@ int gm_debug_keep_tiles(struct gm_session *s, int on);
 /* Precision 1: entries per segment of stored columns that the store pass
  * over the tiles may keep, fixed whatever the grid width (clamped to 64;
  * by default each of a row tile's CTAs gets an equal share of the row's
- * 64 x min(SMs, column tiles) entries, or of 1,024 when that is more; 0 runs
+ * 64 x min(SMs, column tiles) entries, or of 256 x (min(column tiles, 32) + 1)
+ * when that is more, so that no segment overflows up to 32 tiles; 0 runs
  * the heap and candidate passes instead, and so does any value for blocks of
  * up to four column tiles).  A segment that would exceed it makes the heap and
  * candidate passes run for its block (gm_stats.exact_overflow_blocks). */
