@@ -319,7 +319,7 @@ int gm_debug_raise(gm_session *s, uint32_t bits) {
 }
 
 int gm_debug_fail_alloc(int nth) {
-  gm::device_fail_in(std::max(0, nth));
+  gm::device_fail_in(nth);
   return GM_OK;
 }
 

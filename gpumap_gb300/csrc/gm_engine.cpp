@@ -474,16 +474,22 @@ void Session::ensure_cand(size_t rows) {
   cand_rows_ = r;
 }
 
-// The join pool: words for every block of a round, up to kJoinPartWords.
+// The join pool: words for every block of a round, up to kJoinPartWords.  Where
+// the device has no room for them a smaller pool does, with more passes: the
+// round's batch has left the queue, and the update needed no memory of its own
+// before it had a pool.
 void Session::ensure_join(size_t words) {
-  const size_t w = join_part(words);
+  size_t w = join_part(words);
   if (w <= join_words_) return;
   sync();
   device_free(join_pool_, stream_);
   join_pool_ = nullptr;
   join_words_ = 0;
-  ck(device_alloc((void **)&join_pool_, (w + kJoinSlackWords) * sizeof(int), device_, stream_),
-     "cudaMalloc join");
+  for (;; w = (w / 2 + 1) & ~(size_t)1) {
+    const cudaError_t e = device_alloc((void **)&join_pool_, (w + kJoinSlackWords) * sizeof(int), device_, stream_);
+    if (e == cudaSuccess) break;
+    if (e != cudaErrorMemoryAllocation || w <= kJoinLeastWords) ck(e, "cudaMalloc join");
+  }
   join_words_ = w;
 }
 

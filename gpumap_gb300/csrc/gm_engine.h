@@ -112,9 +112,10 @@ class Session {
   void end_phase(const char *phase);
   void ensure_cand(size_t rows);
   void free_cand();
+  static constexpr size_t kJoinLeastWords = 4096;
   void ensure_join(size_t words);
   size_t join_part(size_t words) const {
-    return std::min(std::max<size_t>((words + 1) & ~(size_t)1, 4096), join_part_max_);
+    return std::min(std::max<size_t>((words + 1) & ~(size_t)1, kJoinLeastWords), join_part_max_);
   }
   void ensure_embed(EmbedScratch &e, size_t nb);
   void free_embed(EmbedScratch &e);

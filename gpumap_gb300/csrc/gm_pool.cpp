@@ -107,6 +107,10 @@ void device_fail_in(int n) { g_fail_in = n; }
 cudaError_t device_alloc(void **out, size_t bytes, int device, cudaStream_t s) {
   *out = nullptr;
   if (g_fail_in > 0 && --g_fail_in == 0) return cudaErrorMemoryAllocation;
+  if (g_fail_in < 0) {
+    ++g_fail_in;
+    return cudaErrorMemoryAllocation;
+  }
   cudaMemPool_t p = nullptr;
   {
     std::lock_guard<std::mutex> g(g_mu);

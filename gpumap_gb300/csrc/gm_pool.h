@@ -9,7 +9,7 @@ namespace gm {
 // Ready on stream s; on another stream after s has been waited for.
 cudaError_t device_alloc(void **out, size_t bytes, int device, cudaStream_t s);
 // The n-th device_alloc from here on in the calling thread fails with
-// cudaErrorMemoryAllocation (0: none; tests).
+// cudaErrorMemoryAllocation (n < 0: the next -n do, 0: none; tests).
 void device_fail_in(int n);
 // After every stream that used the block has been waited for.
 void device_free(void *p, cudaStream_t s);

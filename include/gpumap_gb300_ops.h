@@ -67,7 +67,8 @@ int gm_debug_ingest_route(uint64_t address, int page_locked, int reads_host);
  * the next check reports it. */
 int gm_debug_raise(struct gm_session *s, uint32_t bits);
 /* The nth device allocation of this library from here on in the calling thread
- * (1: the next) reports out of memory; 0 takes that back. */
+ * (1: the next) reports out of memory, for a negative value the next -nth do;
+ * 0 takes that back. */
 int gm_debug_fail_alloc(int nth);
 /* Host and device scalars, out[0..n):
  *  0 n_inserted, 1 insertion-queue head, 2 new-row embedding-queue head,

@@ -91,3 +91,21 @@ def test_failed_insertion_growth(native, k):
         assert native.memory_held(0)[1] <= used
         r = s.run(1500, 0, 0)
         assert r.n_insertion_ops == 1500
+
+
+@pytest.mark.parametrize("failures", [1, 3])
+def test_update_with_a_smaller_pool(native, oracle_mod, failures):
+    # the join pool of the whole round cannot be had: more passes, the same lists
+    from test_gpu_parity import pair, same_result, same_state
+
+    X, _ = gaussian_mixture(2000, 20, seed=6)
+    s, o = pair(native, oracle_mod, 2000, 20, k=15, max_epoch=5)
+    s.append_host(X)
+    o.append(X)
+    same_result(s.run(2000, 0, 0), o.run(2000, 0, 0))
+    native.load().gm_debug_fail_alloc(-failures)
+    same_result(s.run(0, 2000, 0), o.run(0, 2000, 0))
+    native.load().gm_debug_fail_alloc(0)
+    same_state(s, o, tag="smaller pool")
+    same_result(s.run(0, 900, 0), o.run(0, 900, 0))
+    same_state(s, o, tag="after it")
