@@ -524,7 +524,7 @@ void Session::set_keep_tile(bool on) {
 size_t Session::device_bytes() const {
   size_t b = fixed_bytes_;
   b += cand_bytes(cand_rows_, st_.k);
-  if (join_pool_) b += (join_words_ + kJoinSlackWords) * sizeof(int);
+  b += join_bytes();
   for (const EmbedScratch *e : {&es_, &es_alt_})
     if (e->cap_coo) b += e->cap_coo * 9 * 4 + (compact_tmp_ints((int)e->cap_coo) + 64) * sizeof(int);
   return b;
@@ -535,7 +535,8 @@ size_t Session::growth_bytes(uint32_t n_ins, uint32_t n_upd, uint32_t n_emb) con
   if (n_upd > 0 && !upd_done_) {
     const size_t rows = std::min<size_t>(n_upd, n_inserted_ + n_ins);
     const size_t w = join_part(join_pool_words((int)rows, st_.k));
-    if (w > join_words_) g += (w + kJoinSlackWords) * sizeof(int);
+    // (the pool it has goes first)
+    if (w > join_words_) g += (w + kJoinSlackWords) * sizeof(int) - join_bytes();
   }
   if (p_.precision == 0 && n_ins > cand_rows_) {
     const size_t r = std::max<size_t>(n_ins, 1024);

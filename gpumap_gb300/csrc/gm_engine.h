@@ -86,6 +86,15 @@ class Session {
   void set_pre_cap(int cap);
   // words of the join pool a pass covers, at most (tests)
   void set_join_part(size_t words);
+  // bytes that the join pool may grow to in the next runs (at least
+  // kJoinLeastBytes); a smaller pool takes more passes
+  void limit_join(size_t bytes) {
+    const size_t words = bytes / sizeof(int);
+    join_limit_ = std::max(kJoinLeastWords, words > kJoinSlackWords ? (words - kJoinSlackWords) & ~(size_t)1 : 0);
+  }
+  size_t join_bytes() const { return join_pool_ ? (join_words_ + kJoinSlackWords) * sizeof(int) : 0; }
+  static constexpr size_t kJoinLeastWords = 4096;
+  static constexpr size_t kJoinLeastBytes = (kJoinLeastWords + kJoinSlackWords) * sizeof(int);
   void drain();
   // sets device error bits, as a wait that ran out would (tests)
   void raise_device_error(unsigned bits);
@@ -112,10 +121,9 @@ class Session {
   void end_phase(const char *phase);
   void ensure_cand(size_t rows);
   void free_cand();
-  static constexpr size_t kJoinLeastWords = 4096;
   void ensure_join(size_t words);
   size_t join_part(size_t words) const {
-    return std::min(std::max<size_t>((words + 1) & ~(size_t)1, kJoinLeastWords), join_part_max_);
+    return std::min({std::max<size_t>((words + 1) & ~(size_t)1, kJoinLeastWords), join_part_max_, join_limit_});
   }
   void ensure_embed(EmbedScratch &e, size_t nb);
   void free_embed(EmbedScratch &e);
@@ -171,7 +179,7 @@ class Session {
   // insertion candidates (grow on demand)
   CandScratch cs_;
   int *join_pool_ = nullptr;  // join blocks of an update round (grows on demand)
-  size_t join_words_ = 0, join_part_max_ = kJoinPartWords;
+  size_t join_words_ = 0, join_part_max_ = kJoinPartWords, join_limit_ = SIZE_MAX;
   size_t cand_rows_ = 0;
 
   // device row lists / counters

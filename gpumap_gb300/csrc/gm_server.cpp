@@ -89,14 +89,26 @@ struct gm_server {
 };
 
 // Next request a slot may run: the oldest whose session is idle and whose
-// possible scratch growth fits the budget.  A request that cannot fit while
-// nothing else runs (so nothing can free memory) fails with GM_ERR_CAPACITY.
+// possible scratch growth fits the budget; where only the update's join pool
+// does not, the pool is kept to the rest of the budget.  A request that cannot
+// fit while nothing else runs (so nothing can free memory) fails with
+// GM_ERR_CAPACITY.
 Request *gm_server::take(std::unique_lock<std::mutex> &) {
   for (auto it = pending.begin(); it != pending.end(); ++it) {
     Request *r = *it;
     Slot &sl = sessions.at(r->session);
     if (sl.busy) continue;
-    const size_t grow = sl.h->impl->growth_bytes((uint32_t)r->n_rows, r->n_upd, r->n_emb);
+    gm::Session &se = *sl.h->impl;
+    se.limit_join(SIZE_MAX);
+    size_t grow = se.growth_bytes((uint32_t)r->n_rows, r->n_upd, r->n_emb);
+    if (bytes_in_use + grow > p.hbm_budget) {
+      const size_t others = bytes_in_use + se.growth_bytes((uint32_t)r->n_rows, 0, r->n_emb);
+      const size_t pool = se.join_bytes();
+      if (others + (pool ? 0 : gm::Session::kJoinLeastBytes) <= p.hbm_budget) {
+        se.limit_join(pool + (p.hbm_budget - others));
+        grow = p.hbm_budget - bytes_in_use;
+      }
+    }
     if (bytes_in_use + grow > p.hbm_budget) {
       if (running > 0) continue;
       pending.erase(it);
