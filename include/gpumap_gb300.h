@@ -163,8 +163,9 @@ void gm_destroy(struct gm_session *s);
 
 /* Gives the memory that the library keeps for coming sessions back to the
  * device and the host (waits for the devices).  Closed sessions' memory is kept
- * to be used again: as much as the last one held, at most a 32nd of the
- * device's memory, and up to 64 MB page-locked.  Live sessions keep theirs. */
+ * to be used again: as much as brings the library back to the most that was in
+ * use at one of the last 16 closes, at most a 16th of the device's memory, and
+ * up to 64 MB page-locked.  Live sessions keep theirs. */
 int gm_release_memory(void);
 /* Device memory the library holds on `device` for sessions and operators, and
  * how much of it is in use. */
