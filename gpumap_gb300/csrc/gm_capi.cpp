@@ -442,7 +442,7 @@ int gm_op_sgd(float *emb, int64_t n, const int32_t *head, const int32_t *tail,
     // scalars: iscal[0..16) at sc, fscal at sc + 64; grid-barrier words in
     // iscal[8..9], device error word in iscal[10]
     int *isc = (int *)sc;
-    const cudaError_t le = gm::launch_sgd_call(
+    const cudaError_t le = gm::launch_sgd_persistent(
         emb, head, tail, eps, (float *)ns, (float *)nn, isc, (const float *)((char *)sc + 64),
         (int)nnz, alpha0, gamma, a, b, n_epochs, neg_rate, seed, (unsigned *)(isc + gm::kIscalBarrier),
         (unsigned *)(isc + 10), dev, s);

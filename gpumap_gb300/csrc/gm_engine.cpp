@@ -1125,7 +1125,7 @@ void Session::run_sgd(int max_edges, cudaStream_t s) {
   // overlapped: half the SMs, the other half stays free for the next cycle's
   // distance work (the per-epoch time does not depend on it)
   const int max_ctas = p_.overlap ? std::max(1, sms_ / 2) : 0;
-  ck(launch_sgd_call(st_.emb, es_.t_row, es_.flag_tail, es_.t_val, es_.next_s, es_.next_n,
+  ck(launch_sgd_persistent(st_.emb, es_.t_row, es_.flag_tail, es_.t_val, es_.next_s, es_.next_n,
                      es_.iscal, es_.fscal, max_edges, p_.alpha, 1.0f, p_.a, p_.b, (int)p_.max_epoch,
                      (int)p_.negative_sample_rate, 42ull, (unsigned *)(es_.iscal + kIscalBarrier),
                      st_.err, device_, s, st_.stat, max_ctas),

@@ -193,7 +193,7 @@ class Session {
   bool err_read_ = false;
   int *d_tmp_ = nullptr;
   size_t pin_bytes_ = 0;           // of each pinned staging buffer
-  uint32_t *h_pin_ = nullptr;      // pinned staging (n_cap + 16 words)
+  uint32_t *h_pin_ = nullptr;      // pinned staging (n_cap + kCounters words)
   uint32_t *h_emb_pin_ = nullptr;  // the embedding phase's pinned staging
   int *es_cnt_ = nullptr;          // the embedding phase's compaction counter
   uint32_t *h_emb_pin_alt_ = nullptr;  // the other side's (overlap mode)

@@ -111,7 +111,9 @@ GM_D void tma_load_2d(const CUtensorMap *map, uint64_t *bar, void *dst, int x, i
       "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
 }
-// The same with an L2 cache policy (createpolicy) for the lines it reads.
+// The same with an L2 cache policy (createpolicy) for the lines it reads: the
+// column tiles stream through L2 once per row tile while other kernels of the
+// session (the embedding's SGD) work out of L2, so their lines go first.
 GM_D void tma_load_2d_hint(const CUtensorMap *map, uint64_t *bar, void *dst, int x, int y,
                            uint64_t policy) {
   asm volatile(
@@ -120,10 +122,6 @@ GM_D void tma_load_2d_hint(const CUtensorMap *map, uint64_t *bar, void *dst, int
       "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(policy)
       : "memory");
 }
-// Column tiles stream through L2 once per row tile while other kernels of
-// the session (the embedding's SGD) work out of L2: their lines go first.
-constexpr bool kStreamEvictFirst = true;
-
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle,
 // 8-row groups 1024 bytes apart (stride byte offset), descriptor version 1.
 GM_D uint64_t sw128_desc(uint32_t addr) {
@@ -351,8 +349,8 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
   if (warp == 0) {
     if (lane == 0) {
       uint32_t it = 0;
-      uint64_t pol = 0;
-      if (kStreamEvictFirst) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+      uint64_t pol;
+      asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
       for (int t = blockIdx.x; t < sc.tile_count && ok; t += gridDim.x) {
         const int ct = t * sc.tile_stride;
         // kchunks K chunks, each with the hi and lo halves of both operands
@@ -368,13 +366,8 @@ __global__ void __launch_bounds__(exact_threads(kPass), 1)
           mbar_expect_tx(&full[s], kStageBytes);
           tma_load_2d(&tm_a, &full[s], a, kx, arow0 + m0);
           tma_load_2d(&tm_a, &full[s], a + kABytes, dh + kx, arow0 + m0);
-          if (kStreamEvictFirst) {
-            tma_load_2d_hint(&tm_b, &full[s], a + 2 * kABytes, kx, ct * kTN, pol);
-            tma_load_2d_hint(&tm_b, &full[s], a + 2 * kABytes + kBBytes, dh + kx, ct * kTN, pol);
-          } else {
-            tma_load_2d(&tm_b, &full[s], a + 2 * kABytes, kx, ct * kTN);
-            tma_load_2d(&tm_b, &full[s], a + 2 * kABytes + kBBytes, dh + kx, ct * kTN);
-          }
+          tma_load_2d_hint(&tm_b, &full[s], a + 2 * kABytes, kx, ct * kTN, pol);
+          tma_load_2d_hint(&tm_b, &full[s], a + 2 * kABytes + kBBytes, dh + kx, ct * kTN, pol);
         }
       }
       if (!ok) atomicOr(err, kDevErrSpin);

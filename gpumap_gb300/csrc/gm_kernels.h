@@ -153,15 +153,17 @@ struct ExactScreen {
   int *counter = nullptr;     // pairs in the pool
   long pool_cap = 0;
 };
-// Distances of batch rows [row0+blk0, +nrows) against rows [0, n) on the
-// tensor cores, screened as the accumulators drain, in two passes (the
-// per-row exact threshold, then the candidates): candidate columns per batch
-// row and (existing row, batch row) pairs land in x.  With keep_d the
-// approximate tile is also written to x.D (nrows x ldD), for tests.
 // Up to so many column tiles a block's stored columns have room for every column.
 constexpr int kExactRoomTiles = 32;
 // Column tiles the seed pass samples out of n_tiles.
 int exact_seed_tiles(int n_tiles);
+// Distances of batch rows [row0+blk0, +nrows) against rows [0, n) on the
+// tensor cores, screened as the accumulators drain: a seed pass over a sample of
+// the columns, the store pass over all of them and the selection of each row's
+// threshold and candidates (after an overflow, or without room, the heap and
+// candidate passes).  Candidate columns per batch row and (existing row, batch
+// row) pairs land in x.  With keep_d the approximate tile is also written to
+// x.D (nrows x ldD), for tests.
 void launch_exact_dist(const DevState &st, const ExactMaps &maps, int dh, int row0, int blk0,
                        int nrows, int n, const ExactScreen &x, long ldD, bool keep_d, int sms,
                        cudaStream_t s);
@@ -233,12 +235,7 @@ struct EmbedScratch {
 void launch_fuzzy_graph(const uint32_t *pub_idx, const float *pub_dist, int n,
                         int k, int euclidean, const int *batch, int nb,
                         double log2_target, EmbedScratch &e, cudaStream_t s);
-// Edge scheduling + SGD epochs on the COO in e (nnz in e.iscal[0]).
-void launch_optimize_layout(float *emb, int n, int nb, int k, float alpha0,
-                            float gamma, float a, float b, int n_epochs,
-                            int neg_rate, uint64_t seed, EmbedScratch &e,
-                            cudaStream_t s);
-// Edge scheduling only: trim, epochs_per_sample, degrees, rounding factor
+// Edge scheduling: trim, epochs_per_sample, degrees, rounding factor
 // (results in e.t_row/e.flag_tail/e.t_val, e.iscal, e.fscal).  After
 // launch_fuzzy_graph, which also leaves the largest weight and cleared degrees.
 void launch_schedule(int n, int nb, int k, float alpha0, int n_epochs, int neg_rate,
@@ -264,12 +261,6 @@ cudaError_t launch_sgd_persistent(float *emb, const int *head, const int *tail,
                                   int neg_rate, uint64_t seed, unsigned *bar, unsigned *err,
                                   int device, cudaStream_t s,
                                   unsigned long long *stat = nullptr, int max_ctas = 0);
-// One embedding call's SGD (all epochs): launch_sgd_persistent.
-cudaError_t launch_sgd_call(float *emb, const int *head, const int *tail, const float *eps,
-                            float *next_s, float *next_n, const int *iscal, const float *fscal,
-                            int max_edges, float alpha0, float gamma, float a, float b, int n_epochs,
-                            int neg_rate, uint64_t seed, unsigned *bar, unsigned *err, int device,
-                            cudaStream_t s, unsigned long long *stat = nullptr, int max_ctas = 0);
 constexpr int kIscalN = 4;
 constexpr int kIscalBarrier = 8;  // iscal[8..9]: SGD grid-barrier words
 void launch_epoch_init(const float *eps, int nnz, int neg_rate, float *next_s,

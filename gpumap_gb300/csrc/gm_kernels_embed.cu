@@ -972,15 +972,6 @@ void launch_schedule(int n, int nb, int k, float alpha0, int n_epochs, int neg_r
   note_launch();
 }
 
-void launch_optimize_layout(float *emb, int n, int nb, int k, float alpha0, float gamma,
-                            float a, float b, int n_epochs, int neg_rate, uint64_t seed,
-                            EmbedScratch &e, cudaStream_t s) {
-  launch_schedule(n, nb, k, alpha0, n_epochs, neg_rate, e, s);
-  if (n <= 0 || n_epochs <= 0 || nb <= 0) return;
-  launch_sgd(emb, e.t_row, e.flag_tail, e.t_val, e.next_s, e.next_n, e.iscal, e.fscal,
-             cdiv(2 * nb * k, 256), alpha0, gamma, a, b, n_epochs, neg_rate, seed, s, nullptr);
-}
-
 void launch_epoch_init(const float *eps, int nnz, int neg_rate, float *next_s,
                        float *next_n, cudaStream_t s) {
   if (nnz <= 0) return;
@@ -1046,15 +1037,6 @@ cudaError_t launch_sgd_persistent(float *emb, const int *head, const int *tail,
                                   args, (size_t)held * kSgdTurnBytes, s);
   note_launch();
   return e;
-}
-
-cudaError_t launch_sgd_call(float *emb, const int *head, const int *tail, const float *eps,
-                            float *next_s, float *next_n, const int *iscal, const float *fscal,
-                            int max_edges, float alpha0, float gamma, float a, float b, int n_epochs,
-                            int neg_rate, uint64_t seed, unsigned *bar, unsigned *err, int device,
-                            cudaStream_t s, unsigned long long *stat, int max_ctas) {
-  return launch_sgd_persistent(emb, head, tail, eps, next_s, next_n, iscal, fscal, max_edges, alpha0, gamma,
-                               a, b, n_epochs, neg_rate, seed, bar, err, device, s, stat, max_ctas);
 }
 
 void launch_add_noise(float *emb, int n, const int *batch, int nb, float noise_scale,

@@ -12,15 +12,14 @@ namespace gm {
 
 namespace {
 
-// ||x||^2 for each batch row by a sequential fma chain over the features.
-// Cosine: normalises the row in place first and stores 1.0
-// (reference: preprocess_l2_norms_kernel, insertion_kernel.cuh:31-81).
-// Squared norms of kNormRows rows per CTA: the rows are staged in shared
-// memory a chunk of up to kNormChunk features at a time (16-byte cp.async by
-// all threads: rows are 16-byte aligned, ld a multiple of 4), then lanes
-// 0..kNormRows-1 of warp 0 run the sequential fma chains, four features a read
-// (the padding is zero, which adds nothing).  Cosine rows are normalised in
-// place, and snorms gets sqrt(norm) rounded up.  Bound by the chain, 1.6 us for
+// ||x||^2 for each batch row by a sequential fma chain over the features, and
+// its square root rounded up (snorms).  Cosine: the row is normalised in place
+// afterwards and its norm is 1.0 (reference: preprocess_l2_norms_kernel,
+// insertion_kernel.cuh:31-81).  kNormRows rows per CTA, staged in shared memory
+// a chunk of up to kNormChunk features at a time (16-byte cp.async by all
+// threads: rows are 16-byte aligned, ld a multiple of 4); lanes 0..kNormRows-1
+// of warp 0 run the chains, four features a read (the padding is zero, which
+// adds nothing).  Bound by the chain, 1.6 us for
 // 784 features: 500 rows x 784 took 9.2 us with a read per feature and a row's
 // loads waiting for the row's before, 6.2 us so.
 constexpr int kNormRows = 4, kNormChunk = 1024;

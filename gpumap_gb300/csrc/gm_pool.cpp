@@ -98,6 +98,13 @@ std::vector<HostBlock> &host_blocks() {  // (never destroyed: a session may go a
   return *v;
 }
 
+void host_release() {
+  std::lock_guard<std::mutex> g(g_host_mu);
+  for (const HostBlock &b : host_blocks()) cudaFreeHost(b.p);
+  host_blocks().clear();
+  g_host_bytes = 0;
+}
+
 size_t host_size(size_t bytes) {  // whole 64 KB pages
   return (bytes + 65535) / 65536 * 65536;
 }
@@ -186,10 +193,7 @@ cudaError_t memory_release() {
     }
     if (back) cudaSetDevice(current);
   }
-  std::lock_guard<std::mutex> g(g_host_mu);
-  for (const HostBlock &b : host_blocks()) cudaFreeHost(b.p);
-  host_blocks().clear();
-  g_host_bytes = 0;
+  host_release();
   return first;
 }
 
@@ -206,7 +210,12 @@ cudaError_t host_alloc(void **out, size_t bytes) {
         return cudaSuccess;
       }
   }
-  const cudaError_t e = cudaHostAlloc(out, want, cudaHostAllocPortable);
+  cudaError_t e = cudaHostAlloc(out, want, cudaHostAllocPortable);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    host_release();
+    e = cudaHostAlloc(out, want, cudaHostAllocPortable);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     *out = nullptr;
