@@ -380,10 +380,10 @@ def run_target_latency(X_host, n, d, q_idx, exact, precision, overlap, target_s=
 NCU_TRAFFIC = {
     # one insertion block of 500 rows against 15,500 columns (dh 832): the
     # seed pass plus the store pass, DRAM read + write; scaled by FLOPs
-    "k_exact_dist": {"bytes": (15401728 + 512) + (54068736 + 2715904), "per": "flop",
+    "k_exact_dist": {"bytes": 15402752 + (54209280 + 1729280), "per": "flop",
                      "units": 6 * 500 * 15500 * 832},
     # one embedding call (1,000 rows, ~26.7k edges, 200 epochs)
-    "k_sgd_persistent": {"bytes": 870400 + 75008, "per": "launch", "units": 1},
+    "k_sgd_persistent": {"bytes": 789248 + 78080, "per": "launch", "units": 1},
 }
 
 

@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kOfferWarps * 32)
 // ties with the tail; then those into the list) run one element at a time,
 // each scan from the tail as one ballot: lane q holds entry q, and the place
 // is after the last entry the element does not precede.  One thread per row
-// took 468 us for 10,000 rows at k = 30, this form 20 us.
+// took 468 us for 10,000 rows at k = 30, this form 52 us.
 constexpr int kFwdWarps = 4;
 __global__ void __launch_bounds__(kFwdWarps * 32)
     k_forward_merge(Key *g_key, int row0, int nrows, const int *cand, const int *cand_cnt,
