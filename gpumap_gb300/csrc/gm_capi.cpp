@@ -350,10 +350,12 @@ int gm_op_fuzzy_schedule(const uint32_t *pub_idx, const float *pub_dist, int64_t
   return guarded([&] {
     gm::EmbedScratch e;
     std::vector<void *> al;
+    size_t scratch = 0;
     int dev = 0;
     cudaGetDevice(&dev);
     auto dalloc = [&](size_t bytes) {
       void *p = nullptr;
+      scratch += bytes;
       if (gm::device_alloc(&p, std::max<size_t>(bytes, 16), dev, s) != cudaSuccess) {
         for (void *q : al) gm::device_free(q, s);
         throw gm::Error(GM_ERR_OOM, "cudaMalloc");
@@ -394,7 +396,7 @@ int gm_op_fuzzy_schedule(const uint32_t *pub_idx, const float *pub_dist, int64_t
     cudaMemcpyAsync(fscal, e.fscal, sizeof(fscal), cudaMemcpyDeviceToHost, s);
     const cudaError_t err = cudaStreamSynchronize(s);
     for (void *q : al) gm::device_free(q, s);
-    gm::device_bound(dev);
+    gm::device_bound(dev, scratch);
     if (err != cudaSuccess) throw gm::Error(GM_ERR_CUDA, cudaGetErrorString(err));
     if (counts_out) {
       counts_out[0] = iscal[0];
@@ -451,7 +453,7 @@ int gm_op_sgd(float *emb, int64_t n, const int32_t *head, const int32_t *tail,
     const cudaError_t err = le != cudaSuccess ? le : cudaStreamSynchronize(s);
     if (le != cudaSuccess) cudaGetLastError();
     release();
-    gm::device_bound(dev);
+    gm::device_bound(dev, (size_t)nnz * 8);
     if (err != cudaSuccess) throw gm::Error(GM_ERR_CUDA, cudaGetErrorString(err));
     if (dev_err) throw gm::Error(GM_ERR_DEVICE, "SGD grid barrier wait ran out");
   });

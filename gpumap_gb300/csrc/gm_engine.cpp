@@ -88,7 +88,7 @@ Session::Session(const gm_params &p) : p_(p) {
     build();
   } catch (...) {
     release_all();
-    device_bound(device_);
+    device_bound(device_, fixed_bytes_);
     throw;
   }
 }

@@ -164,7 +164,8 @@ void device_closed(int device, size_t bytes) {
   trim(d.pool, std::min(d.most, peak > used ? peak - used : 0));
 }
 
-void device_bound(int device) {
+void device_bound(int device, size_t bytes) {
+  if (bytes < kPoolSlack) return;
   std::lock_guard<std::mutex> g(g_mu);
   if (device < 0 || device >= kMaxDevices || !g_pools[device].pool) return;
   trim(g_pools[device].pool, g_pools[device].most);

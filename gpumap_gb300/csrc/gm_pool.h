@@ -16,8 +16,10 @@ void device_free(void *p, cudaStream_t s);
 // After a session's `bytes` were freed and its stream waited for: gives back
 // what the pool holds beyond what it keeps for the next session.
 void device_closed(int device, size_t bytes);
-// Gives back what is above the most that a pool may keep (operators).
-void device_bound(int device);
+// After an operator freed `bytes` of scratch: gives back what is above the most
+// that a pool may keep (small operators take what is there and are not worth
+// the question).
+void device_bound(int device, size_t bytes);
 // Bytes the device's pool holds, and those of them in use.
 cudaError_t device_held(int device, size_t *reserved, size_t *used);
 cudaError_t host_alloc(void **out, size_t bytes);
