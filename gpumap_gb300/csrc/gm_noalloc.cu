@@ -1,5 +1,5 @@
 // gm_op_sgd_noalloc: the SGD operator of gm_op_sgd with its scratch in a
-// fixed device array instead of cudaMalloc'd buffers.
+// fixed device array instead of allocated buffers.
 //
 // Who needs it: callers that must not allocate device memory while they run
 // -- a host framework whose own memory pool owns the GPU's memory (a
